@@ -1,6 +1,6 @@
-// tcgen05 GEMM kernels: the plain GEMM, the fused all-gather -> GEMM and the producer GEMM of the
-// copy-engine reduce-scatter, plus the host-side pieces every GEMM translation unit shares (tensor-map
-// cache, operand set-up, tile-order defaults). The reduce-scatter GEMMs live in gemm_rs.cu, the
+// tcgen05 GEMM kernels: the fused all-gather -> GEMM and the producer GEMM of the copy-engine
+// reduce-scatter, plus the host-side pieces every GEMM translation unit shares (tensor-map
+// cache, operand set-up, tile-order defaults). The plain GEMM lives in gemm_plain.cu, the reduce-scatter GEMMs live in gemm_rs.cu, the
 // decode GEMM -> all-reduce in gemm_ar.cu, the tf32 kernels in gemm_tf32.cu.
 //
 //  * all-gather -> GEMM (reference: kraken/fused/all_gather_matmul.py:222-325): comm CTAs of the
@@ -22,6 +22,7 @@ namespace kraken {
 // hooks
 // ---------------------------------------------------------------------------------------------
 struct AgHooks : HookDefaults {
+  static constexpr bool kAct = true;
   int bn;
   __device__ __forceinline__ bool begin_tile(const GemmParams&, int, int, int, int) { return true; }
   __device__ __forceinline__ void add_to_chunk(const GemmParams&, int, int, int, int, uint32_t (&)[32], int) {}
@@ -351,11 +352,7 @@ template <int BN>
 __device__ __forceinline__ void gemm_body(const GemmParams& p, unsigned bid, unsigned nb) {
   extern __shared__ unsigned char smem_raw[];
   const unsigned n_mma = (unsigned)p.num_mma_ctas;
-  if (p.mode == GEMM_PLAIN) {
-    PlainHooks h;
-    h.bn = BN;
-    gemm_mainloop<BN>(p, bid, nb, h, smem_raw);
-  } else if (p.mode == GEMM_AG) {
+  if (p.mode == GEMM_AG) {
     if (bid >= n_mma) {
       if (p.ag_push && p.ag_mc_out != nullptr) ag_mc_cta(p, bid - n_mma, nb - n_mma, smem_raw);
       else if (p.ag_push) ag_push_cta(p, bid - n_mma, nb - n_mma, smem_raw);
@@ -377,11 +374,7 @@ __device__ __forceinline__ void gemm_body(const GemmParams& p, unsigned bid, uns
 __device__ __forceinline__ void gemm_pair_body(const GemmParams& p, unsigned bid, unsigned nb) {
   extern __shared__ unsigned char smem_raw[];
   const unsigned n_mma = (unsigned)p.num_mma_ctas;   // even
-  if (p.mode == GEMM_PLAIN) {
-    PlainHooks h;
-    h.bn = 256;
-    gemm_mainloop_pair(p, bid / 2, nb / 2, h, smem_raw);
-  } else if (p.mode == GEMM_AG) {
+  if (p.mode == GEMM_AG) {
     if (bid >= n_mma) {
       if (p.ag_push && p.ag_mc_out != nullptr) ag_mc_cta(p, bid - n_mma, nb - n_mma, smem_raw);
       else if (p.ag_push) ag_push_cta(p, bid - n_mma, nb - n_mma, smem_raw);
@@ -571,7 +564,7 @@ static int launch_pair(GemmParams p, unsigned cap, unsigned n_comm, cudaStream_t
 }
 
 int launch_gemm(int bn, const GemmParams& p, unsigned nb, cudaStream_t stream) {
-  if (p.in_fp32) return launch_gemm_tf32(bn, p, nb, stream);
+  if (p.in_fp32) return launch_gemm_tf32(bn, p, nb, stream);   // GEMM_AR
   if (p.mode == GEMM_AR) return launch_gemm_ar(bn, p, nb, stream);
   const size_t floor_smem = p.mode == GEMM_AG ? kAgSmem : 0;   // comm CTAs reuse the block's shared memory
   auto sm = [&](size_t s) { return s > floor_smem ? s : floor_smem; };
@@ -596,7 +589,7 @@ unsigned grid_cap(const DeviceState* d) {
 // Fills the operand/tiling part of the parameter block for C[M,N] = A[M,K] * Bt[N,K]^T.
 // swap: the weights (Bt) become the 128-row operand and the tile is stored transposed.
 int setup_problem(GemmParams& p, const void* a, long long lda, const void* bt, long long ldb, int M, int N,
-                         int K, bool swap, int bn_override, int* bn_out, int elt) {
+                         int K, bool swap, int bn_override, int* bn_out, int elt, int c_box_rows) {
   KR_REQUIRE(M >= 1 && N >= 1 && K >= 8 && (K * elt) % 16 == 0, "GEMM needs K rows of whole 16-byte units and positive sizes");
   p.in_fp32 = elt == 4 ? 1 : 0;
   const void* r = swap ? bt : a;
@@ -614,7 +607,7 @@ int setup_problem(GemmParams& p, const void* a, long long lda, const void* bt, l
   p.transposed = swap ? 1 : 0;
   int rc = get_tmap(r, p.rows_r, K, ldr, kBM, &p.tmap_r, elt);
   if (rc) return rc;
-  rc = get_tmap(c, p.rows_c, K, ldc, bn, &p.tmap_c, elt);
+  rc = get_tmap(c, p.rows_c, K, ldc, c_box_rows > 0 ? c_box_rows : bn, &p.tmap_c, elt);
   if (rc) return rc;
   p.host_c_ptr = c;
   p.host_ldc = ldc;
@@ -633,41 +626,6 @@ KR_API int kr_tmap_cache_stats(unsigned long long* hits, unsigned long long* mis
   return KR_SUCCESS;
 }
 
-// out[M,N] (bf16 or fp32, row stride ldo) = a[M,K] (row stride lda) * bt[N,K]^T (row stride ldb).
-// swap_ab: -1 auto (weights on the 128-row side when M <= 64), 0/1 forced.
-// use_pair: 0 forces the single-CTA kernel, anything else lets eligible shapes use CTA pairs.
-// in_fp32: a and bt hold fp32 and are multiplied as tf32 (single-CTA kernels; strides in elements).
-KR_API int kr_gemm_bf16(const void* a, long long lda, const void* bt, long long ldb, void* out, long long ldo, int M,
-                        int N, int K, int out_fp32, int swap_ab, int bn_override, int max_ctas, int use_pair,
-                        int in_fp32, cudaStream_t stream) {
-  DeviceState* d = device_state();
-  if (!d) return KR_FAIL_CUDA;
-  GemmParams p;
-  memset(&p, 0, sizeof(p));
-  const bool swap = swap_ab < 0 ? (M <= 64 && N >= 128) : swap_ab != 0;
-  int bn = 0;
-  if (in_fp32 && bn_override <= 0) bn_override = tf32_bn(swap ? M : N);
-  int rc = setup_problem(p, a, lda, bt, ldb, M, N, K, swap, bn_override, &bn, in_fp32 ? 4 : 2);
-  if (rc) return rc;
-  if (in_fp32) KR_REQUIRE(bn == 16 || bn == 64 || bn == 256, "tf32 GEMM supports column tiles of 16, 64 and 256");
-  p.mode = GEMM_PLAIN;
-  p.out = out;
-  p.ldo = ldo;
-  p.out_rows = M;
-  p.out_cols = N;
-  p.out_fp32 = out_fp32;
-  p.ws = 1;
-  p.sync = sync_ctx(d);
-  if (!swap && !out_fp32 && bn >= 64) p.use_tma_store = store_tmap(out, M, N, ldo, &p.tmap_out[0]) ? 1 : 0;
-  unsigned nb = (unsigned)(p.tiles_r * p.tiles_c);
-  unsigned cap = grid_cap(d);
-  if (max_ctas > 0 && (unsigned)max_ctas < cap) cap = (unsigned)max_ctas;
-  if (pair_eligible(bn, p) && cap >= 2 && use_pair != 0) return launch_pair(p, cap, 0, stream);
-  if (nb > cap) nb = cap;
-  p.num_mma_ctas = (int)nb;
-  return launch_gemm(bn, p, nb, stream);
-}
-
 // Fused all-gather -> GEMM. a_out [ws*shard_rows, K] receives the gathered A; c[ws*shard_rows, N] =
 // a_out * bt^T. progress [ws*splits] must be zero on entry; counters [ws*splits + 1] zero
 // (self-resetting). Engines that fill a_out:
@@ -682,11 +640,12 @@ KR_API int kr_gemm_bf16(const void* a, long long lda, const void* bt, long long 
 //              flag word flag_base — then the shard is written once, through the NVSwitch, and the
 //              tile order after the own shard goes chunk by chunk over all peers; nullptr: one
 //              unicast copy per peer, the peer that needs the shard first served first.
+// act: activation of the result, 0 none, 1 GELU (tanh form).
 KR_API int kr_ag_gemm_bf16(void* const* bufs, uint32_t* const* pads, const void* own_shard, int rank, int ws,
                            void* a_out, const void* bt, long long ldb, void* c, long long ldc, int shard_rows, int N,
                            int K, int splits, uint32_t* progress, uint32_t* counters, int num_comm_ctas,
                            uint32_t pad_base, int push, unsigned long long a_out_off, uint32_t flag_base,
-                           unsigned long long pad_words, int entry_barrier, void* mc_out, uint32_t* mc_flags,
+                           unsigned long long pad_words, int entry_barrier, void* mc_out, uint32_t* mc_flags, int act,
                            cudaStream_t stream) {
   DeviceState* d = device_state();
   if (!d) return KR_FAIL_CUDA;
@@ -704,6 +663,7 @@ KR_API int kr_ag_gemm_bf16(void* const* bufs, uint32_t* const* pads, const void*
   rc = get_tmap(own_shard, shard_rows, K, K, kBM, &p.tmap_r_local);
   if (rc) return rc;
   p.mode = GEMM_AG;
+  p.act = act;
   p.out = c;
   p.ldo = ldc;
   p.out_rows = M;

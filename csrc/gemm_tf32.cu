@@ -1,5 +1,6 @@
 // Single-CTA tcgen05 GEMM kernels for fp32 operands, multiplied as tf32 (kind::tf32, K = 8 per
-// instruction, fp32 accumulation in TMEM): the plain GEMM and the decode GEMM -> all-reduce. The
+// instruction, fp32 accumulation in TMEM) of the decode GEMM -> all-reduce (the plain tf32 GEMM is in
+// gemm_plain.cu). The
 // reference's GEMM + all-reduce and GEMM + reduce-scatter tests feed fp32 operands to tl.dot, which
 // multiplies them as tf32 as well (test/test_gemm_allreduce.py:57-58).
 #include "kraken/gemm_host.h"
@@ -10,15 +11,9 @@ namespace kraken {
 template <int BN>
 __device__ __forceinline__ void gemm_tf32_body(const GemmParams& p, unsigned bid, unsigned nb) {
   extern __shared__ unsigned char smem_raw[];
-  if (p.mode == GEMM_AR) {
-    ArHooksT<(BN <= 64)> h;   // the tagged push only exists for decode rows (column tiles up to 64)
-    h.bn = BN;
-    gemm_mainloop<BN, ArHooksT<(BN <= 64)>, 4>(p, bid, nb, h, smem_raw);
-  } else {
-    PlainHooks h;
-    h.bn = BN;
-    gemm_mainloop<BN, PlainHooks, 4>(p, bid, nb, h, smem_raw);
-  }
+  ArHooksT<(BN <= 64)> h;   // the tagged push only exists for decode rows (column tiles up to 64)
+  h.bn = BN;
+  gemm_mainloop<BN, ArHooksT<(BN <= 64)>, 4>(p, bid, nb, h, smem_raw);
 }
 
 #define KR_DEFINE_GEMM_TF32(BN)                                                                                \
@@ -33,8 +28,7 @@ KR_DEFINE_GEMM_TF32(64)
 KR_DEFINE_GEMM_TF32(16)
 
 int launch_gemm_tf32(int bn, const GemmParams& p, unsigned nb, cudaStream_t stream) {
-  if (p.mode != GEMM_PLAIN && p.mode != GEMM_AR)
-    return fail(KR_FAIL_UNSUPPORTED, "fp32 operands are supported by the plain GEMM and the GEMM all-reduce");
+  if (p.mode != GEMM_AR) return fail(KR_FAIL_UNSUPPORTED, "fp32 operands are supported by the plain GEMM and the GEMM all-reduce");
   switch (bn) {
     case 256: return launch_ranked(gemm_tf32_256_kernel, gemm_tf32_256_emu_kernel, p, nb, kGemmThreads, GemmCfg<256>::SMEM, stream);
     case 64: return launch_ranked(gemm_tf32_64_kernel, gemm_tf32_64_emu_kernel, p, nb, kGemmThreads, GemmCfg<64>::SMEM, stream);

@@ -1,0 +1,428 @@
+// One-wave GEMM: every CTA (or CTA pair) computes ONE output tile, or one of `splits` equal K ranges of
+// it, and the splits of a tile form a thread-block cluster that sums them through distributed shared
+// memory. For the problems whose tiles do not fill the chip once — decode batches above all, where the
+// time is the weights' way out of HBM and a tile per CTA leaves most SMs idle.
+//
+//   C[M,N] = act(A[M,K] * Bt[N,K]^T), bf16 operands or fp32 multiplied as tf32, fp32 sums in K order
+//   (split by split), bf16 or fp32 result.
+//
+// Why clusters and not partial sums in global memory: a 256 x 256 tile split in two costs 15-18 us there
+// (slots out to L2, an atomic, slots back in: measured with %globaltimer stamps) and about 4 us here.
+// The accumulators go TMEM -> own shared memory (the operand stages are free by then); after one
+// cluster barrier every CTA of the cluster sums and stores an equal share of the tile, reading the
+// others' shared memory, with all ten warps, so that the store is shared out as well. A warp reads 512
+// consecutive bytes of a peer at a time (scattered 16-byte units measured a third of the rate), hence two
+// staging layouts: [unit of four columns][row] for a transposed store, [row][unit] with the units of a row
+// permuted by the row number (no bank conflicts for the row-per-lane writes) for a row-major one.
+#include <algorithm>
+#include <map>
+#include <mutex>
+#include "kraken/gemm_host.h"
+
+namespace kraken {
+
+constexpr int kTileThreads = 320;      // TMA warp, MMA warp, eight warps that empty the accumulator
+
+struct alignas(64) TileParams {
+  CUtensorMap tmap_r, tmap_c;
+  int tiles_r, tiles_c, num_kb;
+  int transposed, out_fp32, act;
+  int out_rows, out_cols;
+  void* out;
+  long long ldo;
+  const void* cp_src;                  // optional copy of the row operand, as in gemm_plain.cu
+  void* cp_dst;
+  unsigned long long cp_bytes;
+  SyncCtx sync;
+};
+
+template <int BN, bool PAIR>
+struct TileCfg {
+  static constexpr int A_BYTES = kBM * 128;
+  static constexpr int B_BYTES = (PAIR ? BN / 2 : BN) * 128;
+  static constexpr int B_BYTES_AL = (B_BYTES + 1023) / 1024 * 1024;
+  static constexpr int STAGE = A_BYTES + B_BYTES_AL;
+  static constexpr int RAW_STAGES = (kSmemLimit - 1024 - 512) / STAGE;
+  static constexpr int STAGES = RAW_STAGES > 12 ? 12 : RAW_STAGES;
+  static constexpr int TMEM_COLS = BN < 32 ? 32 : BN;
+  static constexpr int SMEM = 1024 + STAGES * STAGE + 512;
+  static_assert(BN * kBM * 4 <= STAGES * STAGE, "the accumulator has to fit the stages");
+};
+
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_shared_u4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_size() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+
+// acc[k] = sum over the splits, in order, of the four columns at staging offset off[k]. Loops, not
+// straight-line code: the epilogue runs once per launch out of a cold instruction cache, and code that
+// was unrolled over splits and units spent more time on fetching itself than on the sums.
+template <int UN>
+__device__ __forceinline__ void sum_splits(uint32_t slot0, uint32_t ctas, uint32_t half, int splits, const uint32_t (&off)[UN], float4 (&acc)[UN]) {
+#pragma unroll
+  for (int k = 0; k < UN; ++k) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+  for (int i = 0; i < splits; i += 2) {
+    const uint32_t a = mapa_shared(slot0, (uint32_t)i * ctas + half), b = mapa_shared(slot0, (uint32_t)min(i + 1, splits - 1) * ctas + half);
+    float4 x[UN], y[UN];
+#pragma unroll
+    for (int k = 0; k < UN; ++k) x[k] = ld_cluster_f4(a + off[k]);
+#pragma unroll
+    for (int k = 0; k < UN; ++k) y[k] = ld_cluster_f4(b + off[k]);
+    const float s = i + 1 < splits ? 1.f : 0.f;
+#pragma unroll
+    for (int k = 0; k < UN; ++k) {
+      acc[k].x = (acc[k].x + x[k].x) + s * y[k].x;
+      acc[k].y = (acc[k].y + x[k].y) + s * y[k].y;
+      acc[k].z = (acc[k].z + x[k].z) + s * y[k].z;
+      acc[k].w = (acc[k].w + x[k].w) + s * y[k].w;
+    }
+  }
+}
+
+template <int BN, int ELT, bool PAIR>
+__global__ void __launch_bounds__(kTileThreads, 1) gemm_tile_kernel(const __grid_constant__ TileParams p) {
+  using Cfg = TileCfg<BN, PAIR>;
+  constexpr int kStageK = 128 / ELT;
+  constexpr uint32_t CTAS = PAIR ? 2 : 1;
+  extern __shared__ unsigned char smem_raw[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_ctarank(), csize = cluster_size();
+  const uint32_t half = PAIR ? (rank & 1u) : 0u;           // which CTA of the pair
+  const bool leader = half == 0;
+  const int split = (int)(rank / CTAS), splits = (int)(csize / CTAS);
+  const int tile = (int)(blockIdx.x / csize);
+  // consecutive tiles share the column operand of a column sweep
+  const int tr2 = tile % p.tiles_r, tc = tile / p.tiles_r;
+  const int tr = PAIR ? 2 * tr2 + (int)half : tr2;
+  const int kb_lo = (int)((long long)p.num_kb * split / splits), kb_hi = (int)((long long)p.num_kb * (split + 1) / splits);
+
+  const uint32_t stage0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const uint32_t bars = stage0 + Cfg::STAGES * Cfg::STAGE;
+  auto full_bar = [&](int s) { return bars + 8u * s; };
+  auto empty_bar = [&](int s) { return bars + 8u * (Cfg::STAGES + s); };
+  auto row_unit_off = [](int row, int unit) {
+    constexpr int PERM = BN / 4 < 8 ? BN / 4 - 1 : 7;
+    return (uint32_t)(row * (BN / 4) + (unit ^ (row & PERM))) * 16u;
+  };
+  const uint32_t done_bar = bars + 8u * (2 * Cfg::STAGES);
+  const uint32_t tmem_slot = done_bar + 8;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < Cfg::STAGES; ++s) {
+      mbar_init(full_bar(s), 1);
+      mbar_init(empty_bar(s), 1);
+    }
+    mbar_init(done_bar, 1);
+    mbar_fence_init();
+    tma_prefetch_desc(&p.tmap_r);
+    tma_prefetch_desc(&p.tmap_c);
+  }
+  if (warp == 1) {
+    if (PAIR) { tmem_alloc_pair(tmem_slot, Cfg::TMEM_COLS); tmem_relinquish_pair(); }
+    else { tmem_alloc(tmem_slot, Cfg::TMEM_COLS); tmem_relinquish(); }
+  }
+  tc_fence_before();
+  if (PAIR) cluster_sync_all();      // both CTAs' barriers exist before anyone signals across the pair
+  else __syncthreads();
+  tc_fence_after();
+  uint32_t tmem_base;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
+  pdl_launch();
+  pdl_wait();
+
+  if (warp == 0) {
+    if (elect_one()) {
+      int s = 0;
+      uint32_t ph = 0;
+      for (int kb = kb_lo; kb < kb_hi; ++kb) {
+        if (!mbar_wait(empty_bar(s), ph ^ 1u, p.sync, 80)) break;
+        const uint32_t sa = stage0 + s * Cfg::STAGE;
+        if (PAIR) {
+          const uint32_t lead_full = mapa_shared(full_bar(s), rank & ~1u);
+          if (leader) mbar_expect_tx(full_bar(s), 2 * (Cfg::A_BYTES + Cfg::B_BYTES));
+          tma_load_2d_pair(sa, &p.tmap_r, lead_full, kb * kStageK, tr * kBM);
+          tma_load_2d_pair(sa + Cfg::A_BYTES, &p.tmap_c, lead_full, kb * kStageK, tc * BN + (int)half * (BN / 2));
+        } else {
+          mbar_expect_tx(full_bar(s), Cfg::A_BYTES + Cfg::B_BYTES);
+          tma_load_2d(sa, &p.tmap_r, full_bar(s), kb * kStageK, tr * kBM);
+          tma_load_2d(sa + Cfg::A_BYTES, &p.tmap_c, full_bar(s), kb * kStageK, tc * BN);
+        }
+        if (++s == Cfg::STAGES) { s = 0; ph ^= 1u; }
+      }
+    }
+  } else if (warp == 1) {
+    if (leader && elect_one()) {
+      constexpr int UM = PAIR ? 256 : 128;
+      constexpr uint32_t idesc = ELT == 2 ? make_idesc_bf16(UM, BN) : make_idesc_tf32(UM, BN);
+      int s = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      for (int kb = kb_lo; kb < kb_hi; ++kb) {
+        ok = mbar_wait(full_bar(s), ph, p.sync, 81);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t sa = stage0 + s * Cfg::STAGE;
+        const uint64_t adesc = make_smem_desc_sw128(sa), bdesc = make_smem_desc_sw128(sa + Cfg::A_BYTES);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const uint32_t accumulate = (kb > kb_lo || k != 0) ? 1u : 0u;
+          const uint64_t a = adesc + (uint64_t)(2 * k), b = bdesc + (uint64_t)(2 * k);
+          if (PAIR) {
+            if (ELT == 2) umma_bf16_pair(tmem_base, a, b, idesc, accumulate);
+            else umma_tf32_pair(tmem_base, a, b, idesc, accumulate);
+          } else {
+            if (ELT == 2) umma_bf16(tmem_base, a, b, idesc, accumulate);
+            else umma_tf32(tmem_base, a, b, idesc, accumulate);
+          }
+        }
+        if (PAIR) {
+          umma_commit_pair(empty_bar(s));
+          umma_commit_pair(mapa_shared(empty_bar(s), rank | 1u));
+        } else {
+          umma_commit(empty_bar(s));
+        }
+        if (++s == Cfg::STAGES) { s = 0; ph ^= 1u; }
+      }
+      if (ok) {
+        if (PAIR) {
+          umma_commit_pair(done_bar);
+          umma_commit_pair(mapa_shared(done_bar, rank | 1u));
+        } else {
+          umma_commit(done_bar);
+        }
+      }
+    }
+  } else {
+    if (p.cp_bytes != 0) {
+      // the copy of the row operand: this CTA's share, by the eight warps that have nothing to do yet
+      const size_t nvec = p.cp_bytes / 16, lo = nvec * blockIdx.x / gridDim.x, hi = nvec * (blockIdx.x + 1) / gridDim.x;
+      constexpr int T = kTileThreads - 64;
+      size_t v = lo + threadIdx.x - 64;
+      for (; v + 7 * T < hi; v += 8 * T) {
+        U4 x[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] = ld16((const char*)p.cp_src + (v + (size_t)i * T) * 16);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) st16((char*)p.cp_dst + (v + (size_t)i * T) * 16, x[i]);
+      }
+      for (; v < hi; v += T) st16((char*)p.cp_dst + v * 16, ld16((const char*)p.cp_src + v * 16));
+    }
+    // ---- accumulator -> own shared memory, as 16-byte units of four columns
+    bool ok = mbar_wait(done_bar, 0, p.sync, 82);
+    ok = __all_sync(0xffffffffu, ok);
+    tc_fence_after();
+    constexpr int HALVES = BN >= 32 ? 2 : 1;               // two warps per TMEM lane quarter
+    constexpr int COLS = BN / HALVES, CH = COLS < 32 ? COLS : 32;
+    const int q = warp & 3, h = (warp - 2) >> 2;
+    if (ok && h < HALVES) {
+      const int row = q * 32 + lane;
+#pragma unroll 1
+      for (int c0 = h * COLS; c0 < (h + 1) * COLS; c0 += CH) {
+        uint32_t r[32];
+        const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c0;
+        if (CH == 32) tmem_ld32(t_addr, r);
+        else tmem_ld16(t_addr, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int u = 0; u < CH / 4; ++u)
+          st_shared_u4(stage0 + (p.transposed ? (uint32_t)((c0 / 4 + u) * kBM + row) * 16u : row_unit_off(row, c0 / 4 + u)), r[4 * u], r[4 * u + 1], r[4 * u + 2], r[4 * u + 3]);
+      }
+    }
+  }
+  __syncwarp();
+  tc_fence_before();
+  if (csize > 1) cluster_sync_all();
+  else __syncthreads();
+  tc_fence_after();
+
+  // ---- sum over the splits and store: share `split` of this CTA's 128 x BN part of the tile
+  constexpr int UN = 2;                                    // 16-byte units per thread and split in flight
+  constexpr int UNITS = BN / 4 * kBM;
+  const int lo = UNITS / 64 * split / splits * 64, hi = UNITS / 64 * (split + 1) / splits * 64;
+  const uint32_t slot0 = stage0;
+  const bool fp32 = p.out_fp32 != 0, act = p.act != 0;
+  if (p.transposed) {
+    // D(i, j) -> out[tc*BN + j][tr*128 + i]; lanes = consecutive i
+    const int cols_left = p.out_rows - tc * BN, rows_left = p.out_cols - tr * kBM;
+    char* const out = (char*)p.out + ((long long)tc * BN * p.ldo + tr * kBM) * (fp32 ? 4 : 2);
+#pragma unroll 1
+    for (int e0 = lo + (int)threadIdx.x; e0 < hi; e0 += UN * kTileThreads) {
+      float4 acc[UN];
+      uint32_t off[UN];
+#pragma unroll
+      for (int k = 0; k < UN; ++k) off[k] = (uint32_t)min(e0 + k * kTileThreads, hi - 1) * 16u;
+      sum_splits<UN>(slot0, CTAS, half, splits, off, acc);
+#pragma unroll
+      for (int k = 0; k < UN; ++k) {
+        const int e = e0 + k * kTileThreads, i = e % kBM;
+        if (e < hi && i < rows_left) {
+          const float v[4] = {acc[k].x, acc[k].y, acc[k].z, acc[k].w};
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const int j = e / kBM * 4 + c;
+            if (j < cols_left) {
+              const float y = act ? gelu_tanh(v[c]) : v[c];
+              if (fp32) ((float*)out)[(long long)j * p.ldo + i] = y;
+              else ((__nv_bfloat16*)out)[(long long)j * p.ldo + i] = __float2bfloat16(y);
+            }
+          }
+        }
+      }
+    }
+  } else {
+    // D(i, j) -> out[tr*128 + i][tc*BN + j]; lanes = consecutive groups of eight columns
+    constexpr int GROUPS = BN / 8;                         // per row
+    const bool vec_ok = (p.ldo * (fp32 ? 4 : 2)) % 16 == 0 && ((uintptr_t)p.out & 15) == 0;
+#pragma unroll 1
+    for (int e = lo / 2 + (int)threadIdx.x; e < hi / 2; e += kTileThreads) {
+      const int i = e / GROUPS, u = e % GROUPS * 2;
+      const int row = tr * kBM + i, col = tc * BN + u * 4;
+      float4 acc[2];
+      const uint32_t off[2] = {row_unit_off(i, u), row_unit_off(i, u + 1)};
+      sum_splits<2>(slot0, CTAS, half, splits, off, acc);
+      if (row < p.out_rows && col < p.out_cols) {
+        float v[8] = {acc[0].x, acc[0].y, acc[0].z, acc[0].w, acc[1].x, acc[1].y, acc[1].z, acc[1].w};
+        if (act) {
+#pragma unroll
+          for (int c = 0; c < 8; ++c) v[c] = gelu_tanh(v[c]);
+        }
+        char* o = (char*)p.out + ((long long)row * p.ldo + col) * (fp32 ? 4 : 2);
+        if (vec_ok && col + 8 <= p.out_cols) {
+          if (fp32) {
+            st16(o, U4{__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3])});
+            st16(o + 16, U4{__float_as_uint(v[4]), __float_as_uint(v[5]), __float_as_uint(v[6]), __float_as_uint(v[7])});
+          } else {
+            st16(o, pack8(v));
+          }
+        } else {
+#pragma unroll
+          for (int c = 0; c < 8; ++c)
+            if (col + c < p.out_cols) {
+              if (fp32) ((float*)o)[c] = v[c];
+              else ((__nv_bfloat16*)o)[c] = __float2bfloat16(v[c]);
+            }
+        }
+      }
+    }
+  }
+  // nobody leaves while the cluster may still read its shared memory (or the pair its barriers)
+  tc_fence_before();
+  if (csize > 1) cluster_sync_all();
+  else __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    if (PAIR) tmem_dealloc_pair(tmem_base, Cfg::TMEM_COLS);
+    else tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
+  }
+}
+
+// ---- host ---------------------------------------------------------------------------------------
+struct TileVariant {
+  const void* fn;
+  size_t smem;
+};
+template <int ELT>
+static TileVariant tile_variant(int bn, bool pair) {
+  if (pair) {
+    if (bn == 128) return {(const void*)gemm_tile_kernel<128, ELT, true>, TileCfg<128, true>::SMEM};
+    return {(const void*)gemm_tile_kernel<256, ELT, true>, TileCfg<256, true>::SMEM};
+  }
+  switch (bn) {
+    case 16: return {(const void*)gemm_tile_kernel<16, ELT, false>, TileCfg<16, false>::SMEM};
+    case 32: return {(const void*)gemm_tile_kernel<32, ELT, false>, TileCfg<32, false>::SMEM};
+    case 64: return {(const void*)gemm_tile_kernel<64, ELT, false>, TileCfg<64, false>::SMEM};
+    default: return {nullptr, 0};
+  }
+}
+
+// How many clusters of `cluster` CTAs of this kernel the device holds at once (asked once; 0: none).
+static int max_clusters(int device, const TileVariant& v, unsigned cluster) {
+  static std::mutex mu;
+  static std::map<std::tuple<int, const void*, unsigned>, int> known;
+  std::lock_guard<std::mutex> lk(mu);
+  auto key = std::make_tuple(device, v.fn, cluster);
+  auto it = known.find(key);
+  if (it != known.end()) return it->second;
+  int n = 0;
+  if (ensure_dynamic_smem(v.fn, v.smem) == KR_SUCCESS) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cluster;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(cluster);
+    cfg.blockDim = dim3(kTileThreads);
+    cfg.dynamicSmemBytes = v.smem;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, v.fn, &cfg) != cudaSuccess) {
+      (void)cudaGetLastError();
+      n = 0;
+    }
+  }
+  known[key] = n;
+  return n;
+}
+
+// The split count of a one-wave problem, 0 when its tiles do not fit the chip at once. Times in us as
+// measured: K blocks at the rate the MMAs (256-column pairs 0.30 per block) or the operand loads (0.18,
+// single CTAs 0.25) allow, but never below the operands' time out of HBM, plus what summing S splits
+// adds: little for the narrow tiles of single CTAs, a lot once a cluster of pairs spans more than four
+// CTAs (M = 256, N = 4096, K = 2048: 1 / 2 / 3 splits 17.5 / 14.2 / 20.5 us).
+int tile_gemm_splits(const DeviceState* d, int tiles, int num_kb, int bn, bool pair, int elt) {
+  const TileVariant v = elt == 4 ? tile_variant<4>(bn, pair) : tile_variant<2>(bn, pair);
+  if (v.fn == nullptr) return 0;
+  const int ctas = pair ? 2 : 1, most = 8 / ctas;
+  const double kb_us = !pair ? 0.25 : (bn == 256 ? 0.30 : 0.18);
+  const double hbm_us = (double)tiles * ctas * num_kb * kBM * 128 / 6.5e6;
+  auto sum_us = [&](int s) { return !pair ? 0.25 * s : (s <= 2 ? 1.5 * s : 4.0 * s - 2.0) * bn / 256; };
+  int best = 0;
+  double best_us = 1e30;
+  for (int s = 1; s <= most && (s == 1 || num_kb >= 4 * s); ++s) {
+    if (tiles * s * ctas > d->num_sms || tiles > max_clusters(d->device, v, (unsigned)(s * ctas))) continue;
+    const double us = std::max((num_kb + s - 1) / s * kb_us, hbm_us) + sum_us(s);
+    if (us < best_us) {
+      best_us = us;
+      best = s;
+    }
+  }
+  return best;
+}
+
+int launch_tile_gemm(const GemmParams& g, int bn, bool pair, int splits, cudaStream_t stream) {
+  const TileVariant v = g.in_fp32 ? tile_variant<4>(bn, pair) : tile_variant<2>(bn, pair);
+  if (v.fn == nullptr) return fail(KR_FAIL_ARG, "no one-wave kernel of this tile width");
+  TileParams p;
+  p.tmap_r = g.tmap_r;
+  p.tmap_c = g.tmap_c;
+  p.tiles_r = g.tiles_r;
+  p.tiles_c = g.tiles_c;
+  p.num_kb = (g.K + (g.in_fp32 ? 32 : 64) - 1) / (g.in_fp32 ? 32 : 64);
+  p.transposed = g.transposed;
+  p.out_fp32 = g.out_fp32;
+  p.act = g.act;
+  p.out_rows = g.out_rows;
+  p.out_cols = g.out_cols;
+  p.out = g.out;
+  p.ldo = g.ldo;
+  p.cp_src = g.cp_src;
+  p.cp_dst = g.cp_dst;
+  p.cp_bytes = g.cp_bytes;
+  p.sync = g.sync;
+  const unsigned cluster = (unsigned)splits * (pair ? 2 : 1);
+  void* args[] = {(void*)&p};
+  return launch_overlapped(v.fn, (unsigned)(g.tiles_r * g.tiles_c) * cluster, kTileThreads, args, v.smem, stream, cluster);
+}
+
+}  // namespace kraken

@@ -6,7 +6,26 @@
 namespace kraken {
 
 struct PlainHooks : HookDefaults {
+  static constexpr bool kStreamK = true;
+  static constexpr bool kOverlap = true;
+  static constexpr bool kAct = true;
   int bn;
+  // The copy warps: this CTA's contiguous share of the row operand, eight 16-byte loads in flight per thread.
+  __device__ __forceinline__ void side_role(const GemmParams& p, unsigned worker, unsigned workers, int half, int tid) {
+    const size_t ctas = half < 0 ? workers : 2 * workers, id = half < 0 ? worker : 2 * worker + half;
+    const size_t nvec = p.cp_bytes / 16, lo = nvec * id / ctas, hi = nvec * (id + 1) / ctas;
+    const char* src = (const char*)p.cp_src;
+    char* dst = (char*)p.cp_dst;
+    size_t v = lo + tid;
+    for (; v + 7 * kCopyThreads < hi; v += 8 * kCopyThreads) {
+      U4 x[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[i] = ld16(src + (v + (size_t)i * kCopyThreads) * 16);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) st16(dst + (v + (size_t)i * kCopyThreads) * 16, x[i]);
+    }
+    for (; v < hi; v += kCopyThreads) st16(dst + v * 16, ld16(src + v * 16));
+  }
   __device__ __forceinline__ bool begin_tile(const GemmParams&, int, int, int, int) { return true; }
   __device__ __forceinline__ void add_to_chunk(const GemmParams&, int, int, int, int, uint32_t (&)[32], int) {}
   __device__ __forceinline__ bool before_load(const GemmParams&, int, const CUtensorMap*&, int&) { return true; }

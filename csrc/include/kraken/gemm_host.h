@@ -18,14 +18,17 @@ int default_group_r();
 bool pair_enabled();
 unsigned grid_cap(const DeviceState* d);
 int setup_problem(GemmParams& p, const void* a, long long lda, const void* bt, long long ldb, int M, int N, int K,
-                  bool swap, int bn_override, int* bn_out, int elt = 2);
-// Single-CTA kernels for fp32 operands multiplied as tf32 (plain GEMM and GEMM -> all-reduce;
-// column tiles of 16, 64 or 256). Defined in gemm_tf32.cu.
+                  bool swap, int bn_override, int* bn_out, int elt = 2, int c_box_rows = 0);
+// Single-CTA kernels for fp32 operands multiplied as tf32 (GEMM -> all-reduce; column tiles of 16, 64 or 256). Defined in gemm_tf32.cu.
 int launch_gemm_tf32(int bn, const GemmParams& p, unsigned nb, cudaStream_t stream);
 // Single-CTA kernels of the decode GEMM -> all-reduce. Defined in gemm_ar.cu.
 int launch_gemm_ar(int bn, const GemmParams& p, unsigned nb, cudaStream_t stream);
 // Routes a parameter block to the kernel family of its mode and operand type (gemm.cu).
 int launch_gemm(int bn, const GemmParams& p, unsigned nb, cudaStream_t stream);
+// One-wave GEMM (gemm_tile.cu): the most K splits with which `tiles` tiles of this kernel run at once,
+// 0 when it does not apply; and its launch.
+int tile_gemm_splits(const DeviceState* d, int tiles, int num_kb, int bn, bool pair, int elt);
+int launch_tile_gemm(const GemmParams& g, int bn, bool pair, int splits, cudaStream_t stream);
 int pick_bn(int rows_c);      // column-tile width for `rows_c` rows of the column operand
 int tf32_bn(int rows_c);      // the same among the widths the tf32 kernels exist for
 

@@ -65,6 +65,12 @@ int emu_record(const void* emu_kernel, const void* p, size_t psize, unsigned nbl
 // Raises the kernel's dynamic shared-memory limit once per (device, kernel).
 int ensure_dynamic_smem(const void* func, size_t smem);
 
+// Launches `fn` so that its set-up overlaps the end of the kernel before it on the stream (the
+// launch gap of 2-3 us is much of a small call): the kernel has to call pdl_wait(). cluster > 0: as
+// clusters of that many blocks.
+int launch_overlapped(const void* fn, unsigned nblocks, unsigned nthreads, void** args, size_t smem, cudaStream_t stream,
+                      unsigned cluster = 0);
+
 // Launches `real` with the parameter block by value, or — while an emulation is being recorded —
 // stores the block so that kr_emu_end() can launch `emu` once for all ranks.
 template <class P>

@@ -164,6 +164,15 @@ __device__ __forceinline__ void fence_acq_rel_gpu() { asm volatile("fence.acq_re
 // Orders generic-proxy accesses with async-proxy (TMA) accesses of the executing thread.
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
 
+// ---- programmatic dependent launch --------------------------------------------------------------
+// A kernel launched with launch_overlapped() (host.h) may start while its predecessor on the stream
+// still runs: it does its set-up, then pdl_wait() returns once the predecessor has completed and its
+// writes are visible. Call it before the first access to global memory that anyone else touches.
+// pdl_launch() lets such a successor start as soon as this grid's blocks have all called it (or left).
+// Both do nothing in a launch without the attribute.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- bounded spinning ------------------------------------------------------------------------
 
 // Polls `pred()` until it holds, the deadline passes, or another waiter already failed.

@@ -82,6 +82,30 @@ int ensure_dynamic_smem(const void* func, size_t smem) {
   return KR_SUCCESS;
 }
 
+int launch_overlapped(const void* fn, unsigned nblocks, unsigned nthreads, void** args, size_t smem, cudaStream_t stream,
+                      unsigned cluster) {
+  if (smem > 48 * 1024) {
+    int rc = ensure_dynamic_smem(fn, smem);
+    if (rc) return rc;
+  }
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(nblocks);
+  cfg.blockDim = dim3(nthreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 0 ? 2 : 1;
+  KR_CUDA(cudaLaunchKernelExC(&cfg, fn, args));
+  return KR_SUCCESS;
+}
+
 EmuRecorder& emu_recorder() {
   static thread_local EmuRecorder r;
   return r;

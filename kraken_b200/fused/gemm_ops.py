@@ -199,7 +199,7 @@ def all_gather_matmul(a_shared: torch.Tensor, b: torch.Tensor, a_out: torch.Tens
         _lib.check(L.kr_ag_gemm_bf16(oh.buffer_ptrs_dev, oh.signal_pad_ptrs_dev, a_shared.data_ptr(), rank, ws,
                                      gathered.data_ptr(), bt.data_ptr(), ldb, c.data_ptr(), N, shard_rows, N, K, splits,
                                      progress.data_ptr() if progress is not None else None, counters.data_ptr(), n_comm,
-                                     0, 1, off, flag_base, oh.signal_pad_words, barrier, mc_out, mc_flags, stream))
+                                     0, 1, off, flag_base, oh.signal_pad_words, barrier, mc_out, mc_flags, 0, stream))
         if user_out is not None:
             user_out.copy_(gathered)
             gathered = user_out
@@ -209,7 +209,7 @@ def all_gather_matmul(a_shared: torch.Tensor, b: torch.Tensor, a_out: torch.Tens
         a_out = torch.empty((M, K), dtype=a_shared.dtype, device=dev)
     if progress is None:
         progress = torch.zeros(ws * splits, dtype=torch.uint32, device=dev)
-    args_tail = (0, 0, 0, 0, 0, None, None, stream)     # the push arguments (unused)
+    args_tail = (0, 0, 0, 0, 0, None, None, 0, stream)     # the push arguments (unused)
     if ws == 1 and emu is None:
         # nothing to gather: a device copy fills a_out while the GEMM reads the shard in place
         a_out.copy_(a_shared)

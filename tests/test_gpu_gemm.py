@@ -407,3 +407,19 @@ def test_tensor_map_cache_is_hit_on_repeated_calls():
     klib.check(klib.lib().kr_tmap_cache_stats(ctypes.byref(h1), ctypes.byref(m1)))
     assert h1.value - h0.value >= 10           # both operand maps, five calls
     assert m1.value - m0.value <= 5            # at most the output map of a fresh output tensor
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 1024, 4096), (3, 8200, 264), (17, 520, 1032), (64, 1000, 8192), (65, 520, 2048),
+                                   (128, 4096, 520), (129, 4096, 4104), (300, 1032, 136), (777, 5120, 1032), (2049, 1160, 264)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_gemm_split_tiles_match_fp32_reference(M, N, K, dtype):
+    # the launcher's own choice: clusters that split a tile along K, tiles dealt in parts, swapped operands
+    g = torch.Generator().manual_seed(31)
+    a = torch.randn(M, K, generator=g).to(dtype).cuda()
+    bt = (0.05 * torch.randn(N, K, generator=g)).to(dtype).cuda()
+    ref = (a.double() @ bt.double().t()).float()
+    for out_dtype in (torch.float32, torch.bfloat16):
+        c = fused.matmul(a, bt.t(), out_dtype=out_dtype)
+        rel = ((c.float() - ref).norm() / ref.norm()).item()
+        assert rel < (3e-3 if out_dtype == torch.bfloat16 else (1e-5 if dtype == torch.bfloat16 else 1e-3)), rel
+        assert torch.equal(c, fused.matmul(a, bt.t(), out_dtype=out_dtype))      # the parts are summed in K order
