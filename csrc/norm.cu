@@ -1,4 +1,5 @@
-// RMSNorm and the tensor-parallel decode epilogue: all-reduce + bias + RMSNorm in one kernel.
+// The tensor-parallel decode epilogue: all-reduce + bias + RMSNorm in one kernel (the standalone RMSNorm
+// and the form of one rank are in local.cu).
 // A block owns whole rows (row r belongs to block r % gridDim.x on every rank), keeps the summed
 // row in registers between the reduction and the normalisation, and loops over its rows, so the
 // grid never exceeds the SM count whatever the batch size.
@@ -30,70 +31,6 @@ struct NormParams {
 };
 
 __device__ __forceinline__ char* symm_buf(const NormParams& p, int r) { return (char*)p.bufs[r] + p.buf_off; }
-
-// ---- standalone RMSNorm ----------------------------------------------------------------------
-// A block walks rows r, r + gridDim.x, ...; the NEXT row's vectors are requested before the current
-// row is reduced and stored, so every block always has a row of loads in flight (the reduction's
-// two block barriers would otherwise leave the memory pipe idle once per row).
-__global__ void __launch_bounds__(kNormMaxThreads) rms_norm_kernel(const __grid_constant__ NormParams p) {
-  __shared__ float smem[32];
-  const int nvec = p.D / 8;
-  U4 nx[kNormVpt];
-  int r = blockIdx.x;
-  if (r < p.rows) {
-    const char* xrow = (const char*)p.x + (size_t)r * p.D * 2;
-#pragma unroll
-    for (int i = 0; i < kNormVpt; ++i) {
-      const int v = threadIdx.x + i * blockDim.x;
-      if (v < nvec) nx[i] = ld16(xrow + (size_t)v * 16);
-    }
-  }
-  for (; r < p.rows; r += gridDim.x) {
-    float f[kNormVpt][8];
-#pragma unroll
-    for (int i = 0; i < kNormVpt; ++i) {
-      const int v = threadIdx.x + i * blockDim.x;
-      if (v < nvec) unpack8(nx[i], f[i]);
-    }
-    const int rn = r + gridDim.x;
-    if (rn < p.rows) {
-      const char* xrow = (const char*)p.x + (size_t)rn * p.D * 2;
-#pragma unroll
-      for (int i = 0; i < kNormVpt; ++i) {
-        const int v = threadIdx.x + i * blockDim.x;
-        if (v < nvec) nx[i] = ld16(xrow + (size_t)v * 16);
-      }
-    }
-    rms_finish<kNormVpt>(f, nvec, p.D, p.eps, (const char*)p.w, (char*)p.y + (size_t)r * p.D * 2, smem);
-  }
-}
-
-// Rows longer than the register budget: two passes over global memory.
-__global__ void __launch_bounds__(kNormMaxThreads) rms_norm_long_kernel(const __grid_constant__ NormParams p) {
-  __shared__ float smem[32];
-  const int nvec = p.D / 8;
-  for (int r = blockIdx.x; r < p.rows; r += gridDim.x) {
-    const char* xrow = (const char*)p.x + (size_t)r * p.D * 2;
-    char* yrow = (char*)p.y + (size_t)r * p.D * 2;
-    float ss = 0.f;
-    for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
-      float f[8];
-      unpack8(ld16(xrow + (size_t)v * 16), f);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
-    }
-    ss = block_sum(ss, smem);
-    const float inv = rsqrtf(ss / (float)p.D + p.eps);
-    for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
-      float f[8], g[8];
-      unpack8(ld16(xrow + (size_t)v * 16), f);
-      unpack8(ld16_nc((const char*)p.w + (size_t)v * 16), g);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) g[j] = f[j] * inv * g[j];
-      st16(yrow + (size_t)v * 16, pack8(g));
-    }
-  }
-}
 
 __device__ __forceinline__ void norm_add_bias8(const NormParams& p, size_t elem, float (&f)[8]) {
   acc8(ld16_nc((const char*)p.bias + (elem % p.bias_period) * 2), f);
@@ -231,40 +168,13 @@ KR_DEFINE_RANKED_KERNEL(ar_norm_two_shot_mc_long, NormParams, kNormMaxThreads)
 
 using namespace kraken;
 
-// Threads per row. vpt = 16-byte vectors each thread keeps: 1 when the loads cross NVLink (every
-// load of a row in flight at once matters more than occupancy), up to kNormVpt for the local
-// kernel (smaller blocks, several rows resident per SM, four independent loads per thread).
-static unsigned norm_threads(int D, int vpt) {
-  unsigned nvec = (unsigned)D / 8;
-  unsigned t = (nvec + vpt - 1) / vpt;
-  t = (t + 31) / 32 * 32;
+// Threads per row: one 16-byte vector each while the row allows (the loads cross NVLink: every load of a
+// row in flight at once matters more than occupancy).
+static unsigned norm_threads(int D) {
+  unsigned t = ((unsigned)D / 8 + 31) / 32 * 32;
   if (t < 64) t = 64;
   if (t > kNormMaxThreads) t = kNormMaxThreads;
   return t;
-}
-
-KR_API int kr_rms_norm(const void* x, const void* w, void* y, int rows, int D, float eps, cudaStream_t stream) {
-  DeviceState* d = device_state();
-  if (!d) return KR_FAIL_CUDA;
-  KR_REQUIRE(rows >= 0 && D > 0 && D % 8 == 0, "rms_norm needs D % 8 == 0");
-  KR_REQUIRE((((uintptr_t)x | (uintptr_t)y | (uintptr_t)w) & 15) == 0, "tensors must be 16-byte aligned");
-  if (rows == 0) return KR_SUCCESS;
-  NormParams p;
-  memset(&p, 0, sizeof(p));
-  p.x = x; p.y = y; p.w = w; p.rows = rows; p.D = D; p.eps = eps;
-  const unsigned nt = norm_threads(D, rows >= 2 * d->num_sms ? kNormVpt : 1);
-  // one wave of co-resident blocks (the register file, not the thread count, is what limits it)
-  int per_sm = 0;
-  KR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rms_norm_kernel, (int)nt, 0));
-  const unsigned resident = per_sm > 0 ? (unsigned)per_sm : 1u;
-  const unsigned cap = (unsigned)d->num_sms * resident;
-  unsigned nb = (unsigned)rows < cap ? (unsigned)rows : cap;
-  if (D / 8 <= kNormVpt * kNormMaxThreads)
-    rms_norm_kernel<<<nb, nt, 0, stream>>>(p);
-  else
-    rms_norm_long_kernel<<<nb, kNormMaxThreads, 0, stream>>>(p);
-  KR_CUDA(cudaGetLastError());
-  return KR_SUCCESS;
 }
 
 // y = rms_norm(bias + sum_r x_r) ; algo 0: one-shot pull, 1: two-shot, 2: two-shot NVLS (mc_ptr)
@@ -293,7 +203,7 @@ KR_API int kr_all_reduce_bias_rms_norm(void* const* bufs, unsigned long long buf
   unsigned cap = (unsigned)d->num_sms;
   if (emu_recorder().active) cap = cap / (unsigned)emu_recorder().ws ? cap / (unsigned)emu_recorder().ws : 1;
   unsigned nb = (unsigned)rows < cap ? (unsigned)rows : cap;
-  unsigned nt = norm_threads(D, 1);
+  unsigned nt = norm_threads(D);
   const bool longrow = (unsigned)D / 8 > nt;       // more than one vector per thread
   if (algo == 0)
     return longrow ? launch_ranked(ar_norm_one_shot_long_kernel, ar_norm_one_shot_long_emu_kernel, p, nb, nt, 0, stream)

@@ -14,6 +14,7 @@ import torch
 from .. import _reference as ref
 from .. import config
 from .._logging import utils as _log
+from ..ops import host as _host
 from ..ops import lib as _lib
 from ..parallel import symm_mem
 
@@ -93,12 +94,21 @@ def _max_blocks(kwargs) -> int:
     return int(kwargs.get("max_num_blocks", 0) or 0)
 
 
+def _alone(tensor: torch.Tensor, group, symmetric: bool) -> bool:
+    """World size 1: a reduction over ranks is a copy (local.cu), without staging and barriers."""
+    return tensor.is_cuda and symm_mem.solo(group) and (not symmetric or symm_mem.native_allocation(tensor) is not None)
+
+
 def one_shot_all_reduce(tensor: torch.Tensor, **kwargs) -> torch.Tensor:
     """output = sum over ranks of `tensor`. `tensor` must live in symmetric memory
     (``symm_mem.empty``). Small messages are pushed: every rank writes its data into a slot of each
     peer's workspace, one barrier, local sum. Larger ones are pulled: every rank reads all peers'
     copies directly. fp32 accumulation in rank order. kwargs: group, max_num_blocks,
     algo="push"|"pull" (default KRAKEN_ONE_SHOT)."""
+    if _alone(tensor, kwargs.get("group"), True):
+        out = _host.all_reduce(tensor, None, None)
+        if out is not None:
+            return out
     if tensor.device.type != "cuda":
         return ref.all_reduce(tensor, kwargs.get("group"))
     _check_bf16(tensor)
@@ -138,6 +148,10 @@ def two_shot_all_reduce(tensor: torch.Tensor, **kwargs) -> torch.Tensor:
     but slower than it on 2), else with peer loads and stores.
     kwargs: group, max_num_blocks, nvls=False forces the peer-load form (as does
     KRAKEN_FORCE_ALGO=two_shot)."""
+    if _alone(tensor, kwargs.get("group"), False):
+        out = _host.all_reduce(tensor, None, None)
+        if out is not None:
+            return out
     if tensor.device.type != "cuda":
         return ref.all_reduce(tensor, kwargs.get("group"))
     _check_bf16(tensor)
@@ -152,6 +166,8 @@ def multimem_all_reduce(tensor: torch.Tensor, **kwargs) -> torch.Tensor:
     ``multimem.ld_reduce`` (the NVSwitch adds) and broadcasts it with ``multimem.st``. Returns
     `tensor`. Falls back to the P2P two-shot form (still in place) when the buffer has no
     multicast mapping (NVLS disabled or unsupported)."""
+    if _alone(tensor, kwargs.get("group"), True) and _host.all_reduce(tensor, None, tensor) is not None:
+        return tensor
     if tensor.device.type != "cuda":
         tensor.copy_(ref.all_reduce(tensor, kwargs.get("group")))
         return tensor
@@ -172,6 +188,10 @@ def reduce_scatter(tensor: torch.Tensor, **kwargs) -> torch.Tensor:
     [r*n, (r+1)*n). A symmetric `tensor` is read in place; an ordinary one is staged through the
     group workspace. fp32 accumulation in rank order (bitwise identical run to run)."""
     group = kwargs.get("group")
+    if tensor.dim() > 0 and _alone(tensor, group, False):
+        out = _host.all_reduce(tensor, None, None)
+        if out is not None:
+            return out
     if tensor.device.type != "cuda":
         return ref.reduce_scatter(tensor, group)
     _check_bf16(tensor)
@@ -199,6 +219,10 @@ def all_reduce(tensor: torch.Tensor, **kwargs) -> torch.Tensor:
     up to about 16 MB at 2 GPUs and 1-2 MB at 8 — hence a threshold of 64 MiB / ws^2; above it the
     two-shot form runs, through NVLS when the workspace has a multicast mapping. One-shot needs the
     input itself in symmetric memory; ordinary tensors always take the staged two-shot form."""
+    if _alone(tensor, kwargs.get("group"), False):
+        out = _host.all_reduce(tensor, None, None)
+        if out is not None:
+            return out
     if tensor.device.type != "cuda":
         return ref.all_reduce(tensor, kwargs.get("group"))
     algo = config.force_algo()

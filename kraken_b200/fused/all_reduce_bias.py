@@ -16,6 +16,7 @@ import torch
 from .. import _reference as ref
 from .. import config
 from ..comm.all_reduce import _bias_args, _check_bf16, _dump, _push_all_reduce, push_eligible, push_workspace
+from ..ops import host as _host
 from ..ops import lib as _lib
 from ..parallel import symm_mem
 
@@ -27,12 +28,23 @@ def _scratch(symm_buf: torch.Tensor, x: torch.Tensor, group):
     return hdl, hdl.offset_of(symm_buf)
 
 
+def _alone(symm_buf: torch.Tensor, x: torch.Tensor, group) -> bool:
+    """World size 1 with a proper scratch tensor: the op needs neither scratch nor exchange."""
+    if not (x.is_cuda and symm_mem.solo(group)):
+        return False
+    alloc = symm_mem.native_allocation(symm_buf)
+    return alloc is not None and symm_buf.numel() * symm_buf.element_size() >= x.numel() * x.element_size()
+
+
 def one_shot_all_reduce_bias(symm_mem_buffer: torch.Tensor, input_tensor: torch.Tensor, bias: torch.Tensor | None,
                              output: torch.Tensor, max_num_blocks: int = 0, BLOCK_SIZE: int = 4096,
                              group=None, algo: str | None = None) -> None:
     """output = all_reduce(input) (+ bias). Small messages: every rank writes its data into the
     peers' workspace, one barrier, local sum (`symm_mem_buffer` is then not touched). Larger ones:
-    copy into `symm_mem_buffer`, barrier, every rank pulls all peers' copies and sums."""
+    copy into `symm_mem_buffer`, barrier, every rank pulls all peers' copies and sums. One rank: output =
+    input (+ bias), in one pass."""
+    if _alone(symm_mem_buffer, input_tensor, group) and _host.all_reduce(input_tensor, bias, output) is not None:
+        return None
     if input_tensor.device.type != "cuda":
         output.copy_(ref.all_reduce_bias(input_tensor, bias, group))
         return None
@@ -56,6 +68,8 @@ def two_shot_all_reduce_bias(symm_mem_input: torch.Tensor, input_tensor: torch.T
                              group=None) -> torch.Tensor:
     """output = all_reduce(input) (+ bias): each rank reduces 1/ws of the elements, adds the bias
     and publishes the result to every rank (through NVLS when the buffer has a multicast mapping)."""
+    if _alone(symm_mem_input, input_tensor, group) and _host.all_reduce(input_tensor, bias, output) is not None:
+        return output
     if input_tensor.device.type != "cuda":
         output.copy_(ref.all_reduce_bias(input_tensor, bias, group))
         return output
@@ -108,6 +122,8 @@ def one_shot_all_reduce_bias_rms_norm(symm_mem_input: torch.Tensor, x: torch.Ten
                                       group=None, algo: str | None = None) -> None:
     """y = rms_norm(all_reduce(x) + bias) * w; the summed row never leaves registers. Small inputs
     take the push form (one barrier), larger ones the pull form; algo="push"|"pull" overrides."""
+    if _alone(symm_mem_input, x, group) and _host.bias_rms_norm(x, bias, w, y, eps):
+        return
     _ar_bias_rms_norm(symm_mem_input, x, bias, w, y, eps, group, 0, algo)
 
 
@@ -115,6 +131,8 @@ def two_shot_all_reduce_bias_rms_norm(symm_mem_input: torch.Tensor, x: torch.Ten
                                       w: torch.Tensor, y: torch.Tensor, eps: float = 1e-5, group=None) -> None:
     """Same result with the two-shot exchange: rank k reduces columns [k*D/ws, (k+1)*D/ws) of each
     row and publishes them, then every rank normalises. Needs D % (8 * world_size) == 0."""
+    if _alone(symm_mem_input, x, group) and _host.bias_rms_norm(x, bias, w, y, eps):
+        return
     D = x.shape[-1]
     info = symm_mem.resolve_group(group)
     algo = 1 if D % (8 * info.world_size) == 0 else 0

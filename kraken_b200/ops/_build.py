@@ -2,7 +2,8 @@
 
 Every ``csrc/*.cu`` file is compiled with ``nvcc -gencode arch=compute_100a,code=sm_100a`` into an
 object file and linked into ``kraken_b200/_C/libkraken_b200.so`` in the source tree, so the
-library travels with the checkout and no JIT cache is involved. A source hash stored next to the
+library travels with the checkout and no JIT cache is involved; ``csrc/host/bindings.cpp`` becomes the
+Python extension ``kraken_b200/_C/kraken_b200_host.so`` next to it. A source hash stored next to the
 library makes rebuilds incremental. nvcc cross-compiles without a GPU.
 
 ``build(debug=True)`` compiles the same sources with ``-DKRAKEN_DEBUG=1`` into
@@ -26,6 +27,9 @@ CSRC = REPO / "csrc"
 OUT_DIR = REPO / "kraken_b200" / "_C"
 LIB_PATH = OUT_DIR / "libkraken_b200.so"
 DEBUG_LIB_PATH = OUT_DIR / "libkraken_b200_debug.so"
+HOST_NAME = "kraken_b200_host"
+HOST_SRC = CSRC / "host" / "bindings.cpp"
+HOST_PATH = OUT_DIR / (HOST_NAME + ".so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -79,6 +83,8 @@ def build(verbose: bool = False, force: bool = False, debug: bool = False) -> Pa
     with open(OUT_DIR / ".build.lock", "w") as lock:
         fcntl.flock(lock, fcntl.LOCK_EX)
         try:
+            if force or host_is_stale():
+                _build_host_locked(verbose)
             if not force and not is_stale(debug):
                 return lib_path(debug)
             return _build_locked(verbose, force, debug)
@@ -126,6 +132,54 @@ def _build_locked(verbose: bool, force: bool, debug: bool = False) -> Path:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
         os.replace(tmp, target)
     return target
+
+
+# ---- the Python extension of the host path (g++ against the installed torch) ---------------------
+def _host_digest() -> str:
+    import torch
+
+    h = hashlib.sha256(HOST_SRC.read_bytes())
+    h.update(f"{torch.__version__} {sys.version}".encode())
+    return h.hexdigest()
+
+
+def host_is_stale() -> bool:
+    stamp = OUT_DIR / (HOST_NAME + ".hash")
+    return not HOST_PATH.exists() or not stamp.exists() or stamp.read_text() != _host_digest()
+
+
+def _build_host_locked(verbose: bool) -> None:
+    import sysconfig
+
+    import torch
+
+    root = Path(torch.__file__).parent
+    cuda = Path(_nvcc()).resolve().parents[1]
+    tmp = HOST_PATH.with_suffix(f".so.tmp{os.getpid()}")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f"-I{root / 'include'}", f"-I{root / 'include' / 'torch' / 'csrc' / 'api' / 'include'}", f"-I{cuda / 'include'}",
+           f"-I{sysconfig.get_paths()['include']}", str(HOST_SRC), "-o", str(tmp), f"-L{root / 'lib'}",
+           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python"]
+    if verbose:
+        print(" ".join(cmd), file=sys.stderr)
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"building {HOST_NAME} failed:\n{r.stdout}\n{r.stderr}")
+    os.replace(tmp, HOST_PATH)
+    (OUT_DIR / (HOST_NAME + ".hash")).write_text(_host_digest())
+
+
+def build_host_if_stale() -> None:
+    """Builds the extension when it is missing or out of date; an out-of-date one is kept when it cannot
+    be rebuilt here."""
+    if os.environ.get("KRAKEN_NO_BUILD", "0") == "1" or not host_is_stale():
+        return
+    try:
+        build()
+    except Exception:
+        if not HOST_PATH.exists():
+            raise
 
 
 def is_stale(debug: bool = False) -> bool:

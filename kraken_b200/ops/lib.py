@@ -87,6 +87,9 @@ _PROTOS = {
                                    c_ulonglong, c_uint32, _P]),
     "kr_push_all_reduce_bias_rms_norm": (c_int, [_P, _P, _P, c_int, c_int, _P, _P, c_ulonglong, _P, _P, c_int, c_int,
                                                  c_float, c_uint32, c_ulonglong, c_ulonglong, c_uint32, _P]),
+    # ops of one rank
+    "kr_local_all_reduce": (c_int, [_P, _P, _P, c_ulonglong, c_ulonglong, _P]),
+    "kr_local_bias_rms_norm": (c_int, [_P, c_int, _P, c_ulonglong, _P, _P, c_int, c_int, c_float, c_int, _P]),
     # norm kernels
     "kr_rms_norm": (c_int, [_P, _P, _P, c_int, c_int, c_float, _P]),
     "kr_all_reduce_bias_rms_norm": (c_int, [_P, c_ulonglong, _P, c_int, c_int, _P, _P, c_ulonglong, _P, _P, c_int, c_int, c_float,
@@ -170,7 +173,7 @@ def decode_status(word: int) -> str:
 def current_stream_ptr() -> int:
     import torch
 
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def check_status(stream: int | None = None, clear: bool = True) -> None:
@@ -181,4 +184,7 @@ def check_status(stream: int | None = None, clear: bool = True) -> None:
     if word.value != 0:
         if clear:
             check(lib().kr_clear_status(s))
+        from . import host
+
+        host.reset_if_loaded()      # a kernel that gave up may have left its scratch counters set
         raise KrakenSyncTimeout(decode_status(word.value))

@@ -47,6 +47,7 @@ class GroupInfo:
 
 
 _tls = threading.local()
+_HAVE_DIST = dist.is_available()
 
 
 def _emu_ctx():
@@ -73,6 +74,16 @@ def resolve_group(group=None) -> GroupInfo:
             pg = dist.group.WORLD
     name = getattr(pg, "group_name", None) or "world"
     return GroupInfo(dist.get_rank(pg), dist.get_world_size(pg), str(name), pg)
+
+
+def solo(group=None) -> bool:
+    """Whether `group` is this process alone on a real device (world size 1, not emulated)."""
+    if getattr(_tls, "emu", None) is not None:
+        return False
+    if not isinstance(group, GroupInfo) and not (_HAVE_DIST and dist.is_initialized()):
+        return True
+    info = resolve_group(group)
+    return info.world_size == 1 and info.emu is None
 
 
 # ---------------------------------------------------------------------------------------------
@@ -146,6 +157,12 @@ def _find_allocation(t: torch.Tensor) -> SymmAllocation | None:
             _alloc_by_ptr[key] = a
             return a
     return None
+
+
+def native_allocation(t: torch.Tensor) -> SymmAllocation | None:
+    """The block of the native allocator that holds CUDA tensor `t` (None: no such block); the cheap form of
+    ``rendezvous`` for ops that only have to know that their operand is symmetric."""
+    return _alloc_by_ptr.get((t.get_device(), t.data_ptr())) or _find_allocation(t)
 
 
 class SymmHandle:

@@ -224,3 +224,41 @@ def test_push_tagged_and_flag_forms_share_a_workspace(monkeypatch):
         for r in range(ws):
             torch.testing.assert_close(outs[r].float(), expect, atol=5e-2, rtol=5e-2)
             assert torch.equal(outs[0], outs[r])
+
+
+@pytest.mark.parametrize("rows,D", [(1, 8), (2, 1032), (1, 8200), (3, 16392), (2, 32768), (297, 1024), (300, 1032),
+                                    (297, 8192), (300, 8200), (300, 16392)])
+@pytest.mark.parametrize("bias", ["none", "row", "full"])
+def test_one_rank_forms(rows, D, bias):
+    # world size 1 outside any emulation: no exchange, one pass (few rows: a thread per vector; many: 128-thread blocks)
+    x = symm_mem.empty(rows, D, dtype=torch.bfloat16, device="cuda")
+    x.copy_(_inputs(1, (rows, D))[0])
+    w = (1 + 0.1 * torch.randn(D)).to(torch.bfloat16).cuda()
+    b = {"none": None, "row": torch.randn(D).to(torch.bfloat16).cuda(), "full": torch.randn(rows, D).to(torch.bfloat16).cuda()}[bias]
+    s = x.float() + (b.float() if b is not None else 0)
+    for fn in (fused.one_shot_all_reduce_bias_rms_norm, fused.two_shot_all_reduce_bias_rms_norm):
+        y = torch.empty_like(x)
+        _poison(y)
+        fn(x, x, b, w, y)
+        torch.testing.assert_close(y.float(), _rms_ref(s, w, 1e-5), atol=4e-2, rtol=2e-2)
+    for fn in (fused.one_shot_all_reduce_bias, fused.two_shot_all_reduce_bias):
+        out = torch.empty_like(x)
+        _poison(out)
+        fn(x, x, b, out)
+        assert torch.equal(out, s.to(torch.bfloat16))
+    assert torch.equal(comm.all_reduce(x), x) and torch.equal(comm.reduce_scatter(x), x)
+    torch.testing.assert_close(fused.rms_norm(x, w).float(), _rms_ref(x, w, 1e-5), atol=4e-2, rtol=2e-2)
+
+
+@pytest.mark.parametrize("rows,D", [(1, 8), (5, 1000), (16, 8192), (300, 5120)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_rounded_bias_rms_norm_rounds_like_separate_ops(rows, D, dtype):
+    from kraken_b200.ops import host
+
+    p = torch.randn(rows, D, device="cuda", dtype=dtype)
+    bias = torch.randn(D, device="cuda").to(torch.bfloat16)
+    w = (1 + 0.1 * torch.randn(D, device="cuda")).to(torch.bfloat16)
+    x = (p.to(torch.bfloat16).float() + bias.float()).to(torch.bfloat16)
+    y = host.rounded_bias_rms_norm(p, bias, w, 1e-5)
+    torch.testing.assert_close(y.float(), _rms_ref(x, w, 1e-5), atol=1e-2, rtol=1e-2)
+    assert torch.equal(y, fused.rms_norm(x, w))
