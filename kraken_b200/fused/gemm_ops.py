@@ -17,6 +17,7 @@ import torch
 from .. import _reference as ref
 from .. import config
 from .._logging import utils as _log
+from ..ops import host as _host
 from ..ops import lib as _lib
 from ..parallel import symm_mem
 from .gemm_common import as_k_major_a, as_k_major_bt, use_tf32
@@ -30,20 +31,36 @@ def matmul(a: torch.Tensor, b: torch.Tensor, out_dtype: torch.dtype = torch.bflo
     pair (0 forces the single-CTA kernel; default lets large shapes use CTA pairs)."""
     if a.device.type != "cuda":
         return ref.matmul_f32(a, b).to(out_dtype)
-    tf32 = use_tf32(a, b) and kwargs.get("tf32", True)
+    if out_dtype not in (torch.bfloat16, torch.float32):
+        raise TypeError("output must be bfloat16 or float32")
+    return _gemm(a, b, out_dtype == torch.float32, bool(kwargs.get("tf32", True)), int(kwargs.get("swap_ab", -1)),
+                 int(kwargs.get("bn", 0)), int(kwargs.get("max_ctas", 0)), int(kwargs.get("pair", 1)))
+
+
+_ACT = {None: 0, "gelu_tanh": 1}
+
+
+def _gemm(a: torch.Tensor, b: torch.Tensor, out_fp32: bool, tf32: bool, swap_ab: int = -1, bn: int = 0, max_ctas: int = 0,
+          pair: int = 1, act: str | None = None, copy_dst: torch.Tensor | None = None) -> torch.Tensor:
+    """act(a @ b) on this GPU alone; `copy_dst` additionally receives a copy of `a`."""
+    out = _host.gemm(a, b, out_fp32, _ACT[act], tf32, swap_ab, bn, max_ctas, pair, copy_dst)
+    if out is not None:
+        return out
+    # operands of another type or layout: cast and laid out K-major first
+    tf32 = tf32 and use_tf32(a, b)
     a2, lda = as_k_major_a(a, tf32)
     bt, ldb = as_k_major_bt(b, tf32)
     M, K = a2.shape
     N = bt.shape[0]
     if bt.shape[1] != K:
         raise ValueError("inner dimensions differ")
-    if out_dtype not in (torch.bfloat16, torch.float32):
-        raise TypeError("output must be bfloat16 or float32")
-    out = torch.empty((M, N), dtype=out_dtype, device=a.device)
-    _lib.check(_lib.lib().kr_gemm_bf16(a2.data_ptr(), lda, bt.data_ptr(), ldb, out.data_ptr(), N, M, N, K,
-                                       1 if out_dtype == torch.float32 else 0, int(kwargs.get("swap_ab", -1)),
-                                       int(kwargs.get("bn", 0)), int(kwargs.get("max_ctas", 0)),
-                                       int(kwargs.get("pair", 1)), 1 if tf32 else 0, _lib.current_stream_ptr()))
+    out = _host.gemm(a2, bt.t(), out_fp32, _ACT[act], tf32, swap_ab, bn, max_ctas, pair, copy_dst)
+    if out is not None:
+        return out
+    out = torch.empty((M, N), dtype=torch.float32 if out_fp32 else torch.bfloat16, device=a.device)
+    _lib.check(_lib.lib().kr_gemm(a2.data_ptr(), lda, bt.data_ptr(), ldb, out.data_ptr(), N, M, N, K, 1 if out_fp32 else 0, _ACT[act],
+                                  swap_ab, bn, max_ctas, pair, 1 if tf32 else 0, -1, None, 0, None, 0,
+                                  copy_dst.data_ptr() if copy_dst is not None else None, _lib.current_stream_ptr()))
     return out
 
 
@@ -102,6 +119,21 @@ def _default_push_ctas(shard_bytes: int, ws: int, flops: float, multicast: bool)
 _AG_FLAG_BANK = 2048      # chunk flags per bank in the signal pad (two banks from TILE_FLAG_BASE on)
 
 
+def all_gather_matmul_act(a_shared: torch.Tensor, b: torch.Tensor, act: str, group=None) -> torch.Tensor:
+    """act(gathered A @ b), without the gathered A: the activation is applied to the fp32 sums in the
+    GEMM's epilogue. act="gelu_tanh"."""
+    if a_shared.is_cuda and symm_mem.solo(group):
+        alloc = symm_mem.native_allocation(a_shared)
+        if alloc is not None and alloc.local_ptr == a_shared.data_ptr():
+            c = _host.gemm(a_shared, b, False, _ACT[act], False, -1, 0, 0, 1, None)
+            if c is not None:
+                return c
+    if a_shared.device.type != "cuda":
+        c = all_gather_matmul(a_shared, b, group=group)[1]
+        return torch.nn.functional.gelu(c, approximate="tanh")
+    return all_gather_matmul(a_shared, b, group=group, _act=act)[1]
+
+
 def all_gather_matmul(a_shared: torch.Tensor, b: torch.Tensor, a_out: torch.Tensor | None = None,
                       progress: torch.Tensor | None = None, **kwargs) -> tuple[torch.Tensor, torch.Tensor]:
     """(gathered A [M, K], C [M, N] = gathered A @ b). `a_shared` is this rank's [M/ws, K] shard in
@@ -124,6 +156,16 @@ def all_gather_matmul(a_shared: torch.Tensor, b: torch.Tensor, a_out: torch.Tens
 
     kwargs: splits_per_rank=1, num_comm_sms, backend, group."""
     group = kwargs.get("group")
+    if a_shared.is_cuda and a_shared.dim() == 2 and kwargs.get("backend") in (None, "auto", "push", "ce", "sm") and symm_mem.solo(group):
+        # nothing to gather: one launch multiplies the shard in place and copies it to a_out on the side
+        alloc = symm_mem.native_allocation(a_shared)
+        if alloc is not None and alloc.local_ptr == a_shared.data_ptr() and a_shared.is_contiguous() and not _log.dump_enabled():
+            gathered = torch.empty_like(a_shared) if a_out is None else a_out
+            c = _host.gemm(a_shared, b, False, 0, False, -1, 0, 0, 1, gathered)
+            if c is not None:
+                if progress is not None:
+                    progress.fill_(1)
+                return gathered, c
     if a_shared.device.type != "cuda":
         a, c = ref.all_gather_matmul(a_shared, b, group)
         if progress is not None:
@@ -166,6 +208,7 @@ def all_gather_matmul(a_shared: torch.Tensor, b: torch.Tensor, a_out: torch.Tens
     c = torch.empty((M, N), dtype=a_shared.dtype, device=dev)
     counters = _zero_counters(dev, ws * splits + 1, emu)
     L = _lib.lib()
+    act = _ACT[kwargs.get("_act")]
     _log.log_kernel_choice("all_gather_matmul", f"M={M} N={N} K={K} ws={ws} splits={splits} engine={backend}")
     stream = _lib.current_stream_ptr()
     if progress is not None:
@@ -199,7 +242,7 @@ def all_gather_matmul(a_shared: torch.Tensor, b: torch.Tensor, a_out: torch.Tens
         _lib.check(L.kr_ag_gemm_bf16(oh.buffer_ptrs_dev, oh.signal_pad_ptrs_dev, a_shared.data_ptr(), rank, ws,
                                      gathered.data_ptr(), bt.data_ptr(), ldb, c.data_ptr(), N, shard_rows, N, K, splits,
                                      progress.data_ptr() if progress is not None else None, counters.data_ptr(), n_comm,
-                                     0, 1, off, flag_base, oh.signal_pad_words, barrier, mc_out, mc_flags, 0, stream))
+                                     0, 1, off, flag_base, oh.signal_pad_words, barrier, mc_out, mc_flags, act, stream))
         if user_out is not None:
             user_out.copy_(gathered)
             gathered = user_out
@@ -209,7 +252,7 @@ def all_gather_matmul(a_shared: torch.Tensor, b: torch.Tensor, a_out: torch.Tens
         a_out = torch.empty((M, K), dtype=a_shared.dtype, device=dev)
     if progress is None:
         progress = torch.zeros(ws * splits, dtype=torch.uint32, device=dev)
-    args_tail = (0, 0, 0, 0, 0, None, None, 0, stream)     # the push arguments (unused)
+    args_tail = (0, 0, 0, 0, 0, None, None, act, stream)     # the push arguments (unused)
     if ws == 1 and emu is None:
         # nothing to gather: a device copy fills a_out while the GEMM reads the shard in place
         a_out.copy_(a_shared)
@@ -254,6 +297,10 @@ def gemm_one_shot_all_reduce(a: torch.Tensor, b: torch.Tensor, **kwargs) -> torc
     group = kwargs.get("group")
     if a.device.type != "cuda":
         return ref.gemm_all_reduce(a, b, group)
+    if symm_mem.solo(group):
+        out = _host.gemm(a, b, True, 0, True, -1, 0, 0, 1, None)
+        if out is not None:
+            return out
     tf32 = use_tf32(a, b)
     a2, lda = as_k_major_a(a, tf32)
     bt, ldb = as_k_major_bt(b, tf32)
@@ -262,12 +309,10 @@ def gemm_one_shot_all_reduce(a: torch.Tensor, b: torch.Tensor, **kwargs) -> torc
     if bt.shape[1] != K or (K * a2.element_size()) % 16:
         raise ValueError("inner dimensions must match and K rows must be whole 16-byte units")
     info = symm_mem.resolve_group(group)
+    if info.world_size == 1:
+        return _gemm(a2, bt.t(), True, tf32)
     out = torch.empty((M, N), dtype=torch.float32, device=a.device)
     L = _lib.lib()
-    if info.world_size == 1:
-        _lib.check(L.kr_gemm_bf16(a2.data_ptr(), lda, bt.data_ptr(), ldb, out.data_ptr(), N, M, N, K, 1, -1, 0, 0, 1,
-                                  1 if tf32 else 0, _lib.current_stream_ptr()))
-        return out
     ws = info.world_size
     mn4 = M * N * 4
     # one-shot: an eighth of the buffer per staging half; two-shot: ws partial slots + the result in
@@ -319,6 +364,10 @@ def gemm_reduce_scatter(a: torch.Tensor, b: torch.Tensor, **kwargs) -> torch.Ten
     group = kwargs.get("group")
     if a.device.type != "cuda":
         return ref.gemm_reduce_scatter(a, b, group)
+    if not kwargs.keys() - {"group"} and symm_mem.solo(group) and not _log.dump_enabled():
+        out = _host.gemm(a, b, False, 0, False, -1, 0, 0, 1, None)
+        if out is not None:
+            return out
     a2, lda = as_k_major_a(a)
     bt, ldb = as_k_major_bt(b)
     M, K = a2.shape
@@ -329,7 +378,6 @@ def gemm_reduce_scatter(a: torch.Tensor, b: torch.Tensor, **kwargs) -> torch.Ten
     ws = info.world_size
     if M % ws:
         raise ValueError("M must be divisible by the world size")
-    out = torch.empty((M // ws, N), dtype=torch.bfloat16, device=a.device)
     algo = str(kwargs.get("algo", config.rs_algo()))
     if algo not in ("pull", "push", "scatter"):
         raise ValueError("algo must be 'pull', 'scatter' or 'push'")
@@ -344,8 +392,10 @@ def gemm_reduce_scatter(a: torch.Tensor, b: torch.Tensor, **kwargs) -> torch.Ten
     L = _lib.lib()
     s = _lib.current_stream_ptr()
     if ws == 1 and not (force and fused_ok):
-        _lib.check(L.kr_gemm_bf16(a2.data_ptr(), lda, bt.data_ptr(), ldb, out.data_ptr(), N, M, N, K, 0, -1, 0, 0, 1, 0, s))
-    elif fused_ok:
+        out = _gemm(a2, bt.t(), False, False)
+        return out if a.dtype != torch.float32 else out.to(a.dtype)
+    out = torch.empty((M // ws, N), dtype=torch.bfloat16, device=a.device)
+    if fused_ok:
         if algo in ("pull", "scatter"):
             hdl = symm_mem.get_symm_mem_workspace(group, 2 * M * N * 2 + 2048, a.device, kind="gemm_rs")
             calls = getattr(hdl, "_gemm_rs_calls", 0)        # per staging buffer: selects the half / counter bank
@@ -396,11 +446,9 @@ def gemm_reduce_scatter_ce_persistent(a: torch.Tensor, b: torch.Tensor, reduce_o
         raise ValueError("copy-engine GEMM reduce-scatter needs (M / world_size) % 128 == 0")
     L = _lib.lib()
     dev = a.device
-    out = torch.empty((M // ws, N), dtype=torch.bfloat16, device=dev)
     if ws == 1:
-        _lib.check(L.kr_gemm_bf16(a2.data_ptr(), lda, bt.data_ptr(), ldb, out.data_ptr(), N, M, N, K, 0, -1, 0, 0, 1, 0,
-                                  _lib.current_stream_ptr()))
-        return out
+        return _gemm(a2, bt.t(), False, False)
+    out = torch.empty((M // ws, N), dtype=torch.bfloat16, device=dev)
     gemm_out = torch.empty((M, N), dtype=torch.bfloat16, device=dev)
     _log.log_kernel_choice("gemm_reduce_scatter_ce_persistent", f"M={M} N={N} K={K} ws={ws}: producer GEMM + copy engines + slab reduction")
     hdl = symm_mem.get_symm_mem_workspace(group, M * N * 2, dev)

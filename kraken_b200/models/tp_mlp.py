@@ -4,14 +4,12 @@ the ops are kraken/fused/all_gather_matmul.py, gemm_reduce_scatter_fused.py,
 gemm_one_shot_all_reduce_fused.py and two_shot_all_reduce_bias_rms_norm.py).
 
 Prefill (sequence-parallel activations, [M/ws, H] per rank):
-    h = all_gather_matmul(x_shard, W_up[:, shard])        column-parallel up projection
-    h = gelu(h)
+    h = gelu(all_gather_matmul(x_shard, W_up[:, shard]))  column-parallel up projection, GELU in its epilogue
     y_shard = gemm_reduce_scatter(h, W_down[shard, :])    row-parallel down projection
 Decode (replicated activations, [M, H] per rank, M small):
     p = gemm_one_shot_all_reduce(h_local, W_down[shard, :])     fp32 [M, H]
     y = two_shot_all_reduce_bias_rms_norm(...)  is the next layer's input norm; here the already
-        reduced p only needs bias + RMSNorm, so decode() applies them with the fused norm kernel
-        on one rank's data (world size 1 semantics of the same kernel).
+        reduced p only needs bias + RMSNorm, which decode() applies in one kernel.
 Weights are random-initialised bf16 (no checkpoints are involved anywhere in this library).
 """
 from __future__ import annotations
@@ -19,6 +17,8 @@ from __future__ import annotations
 import torch
 
 from .. import fused
+from ..fused.gemm_ops import all_gather_matmul_act, matmul
+from ..ops import host as _host
 from ..parallel import symm_mem
 
 
@@ -54,14 +54,20 @@ class TPMLP:
 
     def prefill(self, x_symm_shard: torch.Tensor) -> torch.Tensor:
         """x_symm_shard: [M/ws, H] in symmetric memory -> [M/ws, H]."""
-        _, h = fused.all_gather_matmul(x_symm_shard, self.w_up_t.t(), group=self.group)
-        h = torch.nn.functional.gelu(h, approximate="tanh")
+        h = all_gather_matmul_act(x_symm_shard, self.w_up_t.t(), "gelu_tanh", self.group)
         return fused.gemm_reduce_scatter(h, self.w_down_t.t(), group=self.group)
 
     # -- decode ------------------------------------------------------------------------------------
     def decode(self, h_local: torch.Tensor, eps: float = 1e-5) -> torch.Tensor:
         """h_local: [M, F/ws] (this rank's slice of the MLP activations) -> normalised [M, H]."""
-        p = fused.gemm_one_shot_all_reduce(h_local, self.w_down_t.t(), group=self.group)     # fp32, replicated
+        if h_local.is_cuda and h_local.dtype == torch.bfloat16 and symm_mem.solo(self.group):
+            p = matmul(h_local, self.w_down_t.t())         # one rank: nothing left to sum, so the rounding is the epilogue's
+        else:
+            p = fused.gemm_one_shot_all_reduce(h_local, self.w_down_t.t(), group=self.group)     # fp32, replicated
+        if p.is_cuda:
+            y = _host.rounded_bias_rms_norm(p, self.bias, self.norm_w, eps)
+            if y is not None:
+                return y
         x = p.to(torch.bfloat16)
         if x.device.type != "cuda":
             from .. import _reference as ref

@@ -423,3 +423,20 @@ def test_gemm_split_tiles_match_fp32_reference(M, N, K, dtype):
         rel = ((c.float() - ref).norm() / ref.norm()).item()
         assert rel < (3e-3 if out_dtype == torch.bfloat16 else (1e-5 if dtype == torch.bfloat16 else 1e-3)), rel
         assert torch.equal(c, fused.matmul(a, bt.t(), out_dtype=out_dtype))      # the parts are summed in K order
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 264, 64), (64, 1000, 136), (130, 520, 264), (777, 5120, 520), (2100, 2600, 264)])
+def test_one_rank_all_gather_matmul_and_activation(M, N, K):
+    from kraken_b200.fused.gemm_ops import all_gather_matmul_act
+    from kraken_b200.parallel import symm_mem
+
+    a, bt = _ab(M, N, K, seed=41, scale_b=0.1)
+    x = symm_mem.empty(M, K, dtype=torch.bfloat16, device="cuda")
+    x.copy_(a)
+    ref = a.float() @ bt.float().t()
+    prog = torch.zeros(1, dtype=torch.uint32, device="cuda")
+    gathered, c = fused.all_gather_matmul(x, bt.t(), progress=prog)
+    assert torch.equal(gathered, a) and gathered.data_ptr() != x.data_ptr() and int(prog[0]) == 1
+    _close(c, ref, K)
+    h = all_gather_matmul_act(x, bt.t(), "gelu_tanh")
+    _close(h, torch.nn.functional.gelu(ref, approximate="tanh"), K)
