@@ -10,9 +10,8 @@
 //    One launch, no copy engine, no second stream. A copy-engine feed is available as well.
 //  * copy-engine reduce-scatter producer (reference: gemm_reduce_scatter_ce_persistent.py:46-134).
 #include <deque>
-#include <map>
 #include <mutex>
-#include <tuple>
+#include <unordered_map>
 #include "kraken/gemm_host.h"
 #include "kraken/gemm_hooks.cuh"
 
@@ -417,12 +416,20 @@ struct TmapKey {
   unsigned long long rows, cols, ld;
   unsigned box_rows;
   int elt;
-  bool operator<(const TmapKey& o) const {
-    return std::tie(ptr, rows, cols, ld, box_rows, elt) < std::tie(o.ptr, o.rows, o.cols, o.ld, o.box_rows, o.elt);
+  bool operator==(const TmapKey& o) const {
+    return ptr == o.ptr && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows && elt == o.elt;
+  }
+};
+struct TmapHash {
+  size_t operator()(const TmapKey& k) const {
+    unsigned long long h = (unsigned long long)(uintptr_t)k.ptr >> 4;
+    for (unsigned long long v : {k.rows, k.cols, k.ld, (unsigned long long)k.box_rows * 8 + (unsigned long long)k.elt})
+      h = (h ^ v) * 0x9e3779b97f4a7c15ull;
+    return (size_t)(h ^ (h >> 32));
   }
 };
 static std::mutex g_tmap_mu;
-static std::map<TmapKey, CUtensorMap> g_tmap_cache;
+static std::unordered_map<TmapKey, CUtensorMap, TmapHash> g_tmap_cache;
 static std::deque<TmapKey> g_tmap_order;             // insertion order, for eviction
 constexpr size_t kTmapCacheEntries = 4096;
 static unsigned long long g_tmap_hits = 0, g_tmap_misses = 0;

@@ -99,7 +99,7 @@ static void deal_tiles(PlainPlan& pl, int max_workers, int sk_mode) {
 }
 
 static PlainPlan plain_plan(const DeviceState* d, int M, int N, int K, int elt, int swap_ab, int bn_override, int use_pair,
-                            int max_ctas, int sk_mode, bool have_scratch = true) {
+                            int max_ctas, int sk_mode, bool have_scratch) {
   PlainPlan pl;
   memset(&pl, 0, sizeof(pl));
   const bool emu = emu_recorder().active;
@@ -146,6 +146,27 @@ static PlainPlan plain_plan(const DeviceState* d, int M, int N, int K, int elt, 
   return pl;
 }
 
+// The plan of a problem, remembered per thread for the shapes a program repeats (a decode step calls the
+// same few again and again; working a plan out takes about a microsecond).
+static const PlainPlan& known_plan(const DeviceState* d, int M, int N, int K, int elt, int swap_ab, int bn_override, int use_pair,
+                                   int max_ctas, int sk_mode, bool have_scratch) {
+  struct Entry {
+    int key[11];
+    PlainPlan plan;
+  };
+  static thread_local Entry table[64];
+  const int key[11] = {1, d->device, M, N, K, elt, swap_ab, bn_override, use_pair, max_ctas, sk_mode * 2 + (have_scratch ? 1 : 0)};
+  unsigned h = 2166136261u;
+  for (int k : key) h = (h ^ (unsigned)k) * 16777619u;
+  Entry& e = table[(h ^ (h >> 15)) % 64];
+  if (emu_recorder().active || memcmp(e.key, key, sizeof(key)) != 0) {
+    e.plan = plain_plan(d, M, N, K, elt, swap_ab, bn_override, use_pair, max_ctas, sk_mode, have_scratch);
+    memcpy(e.key, key, sizeof(key));
+    if (emu_recorder().active) e.key[0] = 0;       // an emulated launch is planned for fewer CTAs
+  }
+  return e.plan;
+}
+
 template <int BN, int ELT>
 static int launch_plain(const GemmParams& p, unsigned ctas, unsigned threads, cudaStream_t stream) {
   if (emu_recorder().active)
@@ -169,7 +190,7 @@ KR_API int kr_gemm_scratch(int M, int N, int K, int in_fp32, int swap_ab, int bn
   DeviceState* d = device_state();
   if (!d) return KR_FAIL_CUDA;
   KR_REQUIRE(M >= 1 && N >= 1 && K >= 1, "GEMM needs positive sizes");
-  const PlainPlan pl = plain_plan(d, M, N, K, in_fp32 ? 4 : 2, swap_ab, bn_override, use_pair, max_ctas, sk_mode);
+  const PlainPlan& pl = known_plan(d, M, N, K, in_fp32 ? 4 : 2, swap_ab, bn_override, use_pair, max_ctas, sk_mode, true);
   *slot_bytes = pl.slot_bytes;
   *counter_words = pl.counters;
   return KR_SUCCESS;
@@ -192,7 +213,10 @@ KR_API int kr_gemm(const void* a, long long lda, const void* bt, long long ldb, 
   if (!d) return KR_FAIL_CUDA;
   KR_REQUIRE(M >= 1 && N >= 1, "GEMM needs positive sizes");
   const int elt = in_fp32 ? 4 : 2;
-  const PlainPlan pl = plain_plan(d, M, N, K, elt, swap_ab, bn_override, use_pair, max_ctas, sk_mode, slots != nullptr && counters != nullptr);
+  // a problem that needs no scratch has the same plan with and without
+  PlainPlan pl = known_plan(d, M, N, K, elt, swap_ab, bn_override, use_pair, max_ctas, sk_mode, true);
+  if (pl.sk_tiles > 0 && (slots == nullptr || counters == nullptr))
+    pl = known_plan(d, M, N, K, elt, swap_ab, bn_override, use_pair, max_ctas, sk_mode, false);
   KR_REQUIRE(slot_bytes >= pl.slot_bytes && counter_words >= pl.counters, "GEMM scratch too small");
   GemmParams p;
   memset(&p, 0, sizeof(p));

@@ -88,6 +88,34 @@ PyObject* py_reset(PyObject*, PyObject*) {
   Py_RETURN_NONE;
 }
 
+// Operands as the kernels take them: a [M, K] with K contiguous, bt [N, K] with K contiguous
+// (row stride `ldb`). Whether these are such operands, both bf16 or, with tf32, both fp32.
+bool gemm_operands(const at::Tensor& a, const at::Tensor& bt, int64_t N, int64_t Kb, int64_t ldb, int64_t kb_stride, bool tf32) {
+  if (a.dim() != 2 || bt.dim() != 2 || a.scalar_type() != bt.scalar_type()) return false;
+  const bool fp32 = a.scalar_type() == at::kFloat;
+  if (fp32 ? !tf32 : a.scalar_type() != at::kBFloat16) return false;
+  const int64_t M = a.size(0), K = a.size(1), unit = fp32 ? 4 : 8, lda = a.stride(0);
+  return Kb == K && fits_int(M) && fits_int(N) && fits_int(K) && K % unit == 0 && a.stride(1) == 1 && kb_stride == 1 && lda % unit == 0 &&
+         ldb % unit == 0 && lda >= K && ldb >= K && aligned(a) && aligned(bt);
+}
+int run_gemm(const at::Tensor& a, const at::Tensor& bt, int64_t N, int64_t ldb, bool out_fp32, int act, int swap, int bn, int max_ctas, int pair,
+             void* copy_dst, c10::cuda::CUDAStream stream, at::Tensor& out) {
+  const int64_t M = a.size(0), K = a.size(1);
+  const bool fp32 = a.scalar_type() == at::kFloat;
+  out = at::detail::empty_cuda({M, N}, out_fp32 ? at::kFloat : at::kBFloat16, a.device(), std::nullopt);
+  u64 slot_bytes = 0, words = 0;
+  int rc = api.gemm_scratch((int)M, (int)N, (int)K, fp32, swap, bn, pair, max_ctas, -1, &slot_bytes, &words);
+  if (rc) return rc;
+  at::Tensor slots, counters;
+  if (slot_bytes) {
+    slots = at::detail::empty_cuda({(int64_t)slot_bytes}, at::kByte, a.device(), std::nullopt);
+    counters = counters_for(a.device().index(), stream, (int64_t)words);
+  }
+  return api.gemm(a.data_ptr(), a.stride(0), bt.data_ptr(), ldb, out.data_ptr(), N, (int)M, (int)N, (int)K, out_fp32, act, swap, bn, max_ctas,
+                  pair, fp32, -1, slot_bytes ? slots.data_ptr() : nullptr, slot_bytes,
+                  slot_bytes ? (uint32_t*)counters.data_ptr() : nullptr, words, copy_dst, (void*)stream.stream());
+}
+
 // gemm(a, b, out_fp32, act, tf32, swap_ab, bn, max_ctas, pair, copy_dst): act(a @ b). a [M, K] with K contiguous, b
 // [K, N] stored transposed (N rows of contiguous K), both bf16 or, with tf32, both fp32.
 PyObject* py_gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
@@ -97,38 +125,47 @@ PyObject* py_gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
   }
   const c10::DeviceIndex dev = c10::cuda::current_device();
   const at::Tensor *a = cuda_tensor(args[0], dev), *b = cuda_tensor(args[1], dev);
-  if (!a || !b || a->dim() != 2 || b->dim() != 2 || a->scalar_type() != b->scalar_type()) Py_RETURN_NONE;
-  const bool fp32 = a->scalar_type() == at::kFloat;
-  if (fp32 ? args[4] != Py_True : a->scalar_type() != at::kBFloat16) Py_RETURN_NONE;
-  const int64_t M = a->size(0), K = a->size(1), N = b->size(1), unit = fp32 ? 4 : 8;
-  if (b->size(0) != K || !fits_int(M) || !fits_int(N) || !fits_int(K) || K % unit) Py_RETURN_NONE;
-  const int64_t lda = a->stride(0), ldb = b->stride(1);
-  if (a->stride(1) != 1 || b->stride(0) != 1 || lda % unit || ldb % unit || lda < K || ldb < K || !aligned(*a) || !aligned(*b)) Py_RETURN_NONE;
-  const bool out_fp32 = args[2] == Py_True;
+  if (!a || !b || b->dim() != 2 || !gemm_operands(*a, *b, b->size(1), b->size(0), b->stride(1), b->stride(0), args[4] == Py_True)) Py_RETURN_NONE;
   const int act = (int)PyLong_AsLong(args[3]), swap = (int)PyLong_AsLong(args[5]), bn = (int)PyLong_AsLong(args[6]),
             max_ctas = (int)PyLong_AsLong(args[7]), pair = (int)PyLong_AsLong(args[8]);
   if (PyErr_Occurred()) return nullptr;
   void* copy_dst = nullptr;
   if (args[9] != Py_None) {
     const at::Tensor* c = cuda_tensor(args[9], dev);
-    if (!c || !plain_bf16(*c) || c->numel() != M * K || fp32 || lda != K) Py_RETURN_NONE;
+    if (!c || !plain_bf16(*c) || c->numel() != a->numel() || a->scalar_type() != at::kBFloat16 || !a->is_contiguous()) Py_RETURN_NONE;
     copy_dst = c->data_ptr();
   }
-  auto stream = c10::cuda::getCurrentCUDAStream(dev);
-  at::Tensor out = at::detail::empty_cuda({M, N}, out_fp32 ? at::kFloat : at::kBFloat16, a->device(), std::nullopt);
-  u64 slot_bytes = 0, words = 0;
-  int rc = api.gemm_scratch((int)M, (int)N, (int)K, fp32, swap, bn, pair, max_ctas, -1, &slot_bytes, &words);
-  if (rc) return failed(rc);
-  at::Tensor slots, counters;
-  if (slot_bytes) {
-    slots = at::detail::empty_cuda({(int64_t)slot_bytes}, at::kByte, a->device(), std::nullopt);
-    counters = counters_for(dev, stream, (int64_t)words);
-  }
-  rc = api.gemm(a->data_ptr(), lda, b->data_ptr(), ldb, out.data_ptr(), N, (int)M, (int)N, (int)K, out_fp32, act, swap, bn, max_ctas,
-                pair, fp32, -1, slot_bytes ? slots.data_ptr() : nullptr, slot_bytes,
-                slot_bytes ? (uint32_t*)counters.data_ptr() : nullptr, words, copy_dst, (void*)stream.stream());
+  at::Tensor out;
+  const int rc = run_gemm(*a, *b, b->size(1), b->stride(1), args[2] == Py_True, act, swap, bn, max_ctas, pair, copy_dst,
+                          c10::cuda::getCurrentCUDAStream(dev), out);
   if (rc) return failed(rc);
   return THPVariable_Wrap(std::move(out));
+}
+
+// decode(h, w_t, bias, norm_w, eps) -> bf16 rms_norm(bf16(bf16(h @ w_t^T) + bias)) * norm_w; w_t [N, K], all bf16
+PyObject* py_decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 5) {
+    PyErr_SetString(PyExc_TypeError, "decode takes 5 arguments");
+    return nullptr;
+  }
+  const c10::DeviceIndex dev = c10::cuda::current_device();
+  const at::Tensor *h = cuda_tensor(args[0], dev), *wt = cuda_tensor(args[1], dev), *bias = cuda_tensor(args[2], dev),
+                   *w = cuda_tensor(args[3], dev);
+  if (!h || !wt || !bias || !w || wt->dim() != 2 || !gemm_operands(*h, *wt, wt->size(0), wt->size(1), wt->stride(0), wt->stride(1), false) || logging())
+    Py_RETURN_NONE;
+  const int64_t N = wt->size(0);
+  if (!plain_bf16(*bias) || !plain_bf16(*w) || N % 8 || N > 32768 || bias->numel() != N || w->numel() != N) Py_RETURN_NONE;
+  const double eps = PyFloat_AsDouble(args[4]);
+  if (PyErr_Occurred()) return nullptr;
+  auto stream = c10::cuda::getCurrentCUDAStream(dev);
+  at::Tensor p;
+  int rc = run_gemm(*h, *wt, N, wt->stride(0), false, 0, -1, 0, 0, 1, nullptr, stream, p);
+  if (rc) return failed(rc);
+  at::Tensor y = at::detail::empty_cuda(p.sizes(), at::kBFloat16, p.device(), std::nullopt);
+  rc = api.local_bias_rms_norm(p.data_ptr(), 0, bias->data_ptr(), (u64)N, w->data_ptr(), y.data_ptr(), (int)p.size(0), (int)N, (float)eps, 1,
+                               (void*)stream.stream());
+  if (rc) return failed(rc);
+  return THPVariable_Wrap(std::move(y));
 }
 
 // rms_norm(x, w, eps) -> y
@@ -163,21 +200,23 @@ bool bias_of(PyObject* o, c10::DeviceIndex dev, const at::Tensor& x, const void*
   return true;
 }
 
-// bias_rms_norm(x, bias, w, y, eps): y = rms_norm(x + bias) * w, the sum in fp32; True when done
+// bias_rms_norm(scratch, x, bias, w, y, eps): y = rms_norm(x + bias) * w, the sum in fp32; True when done. The
+// scratch tensor of the multi-rank form only has to be large enough.
 PyObject* py_bias_rms_norm(PyObject*, PyObject* const* args, Py_ssize_t n) {
-  if (n != 5) {
-    PyErr_SetString(PyExc_TypeError, "bias_rms_norm takes 5 arguments");
+  if (n != 6) {
+    PyErr_SetString(PyExc_TypeError, "bias_rms_norm takes 6 arguments");
     return nullptr;
   }
   const c10::DeviceIndex dev = c10::cuda::current_device();
-  const at::Tensor *x = cuda_tensor(args[0], dev), *w = cuda_tensor(args[2], dev), *y = cuda_tensor(args[3], dev);
-  if (!x || !w || !y || !plain_bf16(*x) || !plain_bf16(*w) || !plain_bf16(*y) || x->dim() < 1 || logging()) Py_RETURN_NONE;
+  const at::Tensor *scratch = cuda_tensor(args[0], dev), *x = cuda_tensor(args[1], dev), *w = cuda_tensor(args[3], dev),
+                   *y = cuda_tensor(args[4], dev);
+  if (!scratch || !x || !w || !y || scratch->nbytes() < x->nbytes() || !plain_bf16(*x) || !plain_bf16(*w) || !plain_bf16(*y) || x->dim() < 1 || logging()) Py_RETURN_NONE;
   const int64_t D = x->size(-1);
   const void* bias;
   u64 bias_n;
   if (!fits_int(D) || D % 8 || D > 32768 || w->numel() != D || y->numel() != x->numel() || !fits_int(x->numel() / D)) Py_RETURN_NONE;
-  if (!bias_of(args[1], dev, *x, bias, bias_n)) Py_RETURN_NONE;
-  const double eps = PyFloat_AsDouble(args[4]);
+  if (!bias_of(args[2], dev, *x, bias, bias_n)) Py_RETURN_NONE;
+  const double eps = PyFloat_AsDouble(args[5]);
   if (PyErr_Occurred()) return nullptr;
   int rc = api.local_bias_rms_norm(x->data_ptr(), 0, bias, bias_n, w->data_ptr(), y->data_ptr(), (int)(x->numel() / D), (int)D, (float)eps, 0,
                                    (void*)c10::cuda::getCurrentCUDAStream(dev).stream());
@@ -271,7 +310,7 @@ PyObject* guarded(PyObject* self, PyObject* const* args, Py_ssize_t n) {
 }
 #define KR_FAST(NAME) \
   { #NAME, (PyCFunction)(void (*)(void))guarded<py_##NAME>, METH_FASTCALL, nullptr }
-PyMethodDef g_methods[] = {KR_FAST(gemm), KR_FAST(rms_norm), KR_FAST(bias_rms_norm), KR_FAST(rounded_bias_rms_norm), KR_FAST(all_reduce),
+PyMethodDef g_methods[] = {KR_FAST(gemm), KR_FAST(decode), KR_FAST(rms_norm), KR_FAST(bias_rms_norm), KR_FAST(rounded_bias_rms_norm), KR_FAST(all_reduce),
                            {"bind", py_bind, METH_VARARGS, nullptr},
                            {"reset", py_reset, METH_NOARGS, nullptr},
                            {nullptr, nullptr, 0, nullptr}};

@@ -1,4 +1,5 @@
 // Host runtime: error strings, per-device status word, wait deadline, rank emulation.
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <mutex>
@@ -21,6 +22,8 @@ int cuda_fail(cudaError_t e, const char* what) {
 
 static std::mutex g_mu;
 static std::map<int, DeviceState*> g_states;
+constexpr int kMaxDevices = 64;
+static std::atomic<DeviceState*> g_state_table[kMaxDevices];   // the same, read without the lock on every call
 static uint64_t g_default_timeout_ns = 0;
 
 static uint64_t default_timeout_ns() {
@@ -40,6 +43,8 @@ DeviceState* device_state() {
     cuda_fail(e, "cudaGetDevice");
     return nullptr;
   }
+  if (dev < kMaxDevices)
+    if (DeviceState* known = g_state_table[dev].load(std::memory_order_acquire)) return known;
   std::lock_guard<std::mutex> lk(g_mu);
   auto it = g_states.find(dev);
   if (it != g_states.end()) return it->second;
@@ -55,6 +60,7 @@ DeviceState* device_state() {
   }
   d->timeout_ns = default_timeout_ns();
   g_states[dev] = d;
+  if (dev < kMaxDevices) g_state_table[dev].store(d, std::memory_order_release);
   return d;
 }
 
@@ -73,10 +79,18 @@ int ensure_dynamic_smem(const void* func, size_t smem) {
   static std::map<std::pair<int, const void*>, size_t> done;
   int dev = 0;
   KR_CUDA(cudaGetDevice(&dev));
+  // what this thread has raised before, without the lock
+  struct Seen { int dev; const void* func; size_t smem; };
+  static thread_local Seen seen[16];
+  Seen& mine = seen[((uintptr_t)func >> 4) % 16];
+  if (mine.func == func && mine.dev == dev && mine.smem >= smem) return KR_SUCCESS;
   std::lock_guard<std::mutex> lk(g_mu);
   auto key = std::make_pair(dev, func);
   auto it = done.find(key);
-  if (it != done.end() && it->second >= smem) return KR_SUCCESS;
+  if (it != done.end() && it->second >= smem) {
+    mine = Seen{dev, func, it->second};
+    return KR_SUCCESS;
+  }
   KR_CUDA(cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   done[key] = smem;
   return KR_SUCCESS;

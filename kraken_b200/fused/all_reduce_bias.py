@@ -28,12 +28,13 @@ def _scratch(symm_buf: torch.Tensor, x: torch.Tensor, group):
     return hdl, hdl.offset_of(symm_buf)
 
 
-def _alone(symm_buf: torch.Tensor, x: torch.Tensor, group) -> bool:
-    """World size 1 with a proper scratch tensor: the op needs neither scratch nor exchange."""
-    if not (x.is_cuda and symm_mem.solo(group)):
-        return False
-    alloc = symm_mem.native_allocation(symm_buf)
-    return alloc is not None and symm_buf.numel() * symm_buf.element_size() >= x.numel() * x.element_size()
+def _alone(symm_buf: torch.Tensor, group) -> bool:
+    """World size 1 with a symmetric scratch tensor: the op needs no exchange."""
+    return symm_buf.is_cuda and symm_mem.solo(group) and symm_mem.native_allocation(symm_buf) is not None
+
+
+def _fits(symm_buf: torch.Tensor, x: torch.Tensor) -> bool:
+    return symm_buf.numel() * symm_buf.element_size() >= x.numel() * x.element_size()
 
 
 def one_shot_all_reduce_bias(symm_mem_buffer: torch.Tensor, input_tensor: torch.Tensor, bias: torch.Tensor | None,
@@ -43,7 +44,7 @@ def one_shot_all_reduce_bias(symm_mem_buffer: torch.Tensor, input_tensor: torch.
     peers' workspace, one barrier, local sum (`symm_mem_buffer` is then not touched). Larger ones:
     copy into `symm_mem_buffer`, barrier, every rank pulls all peers' copies and sums. One rank: output =
     input (+ bias), in one pass."""
-    if _alone(symm_mem_buffer, input_tensor, group) and _host.all_reduce(input_tensor, bias, output) is not None:
+    if _alone(symm_mem_buffer, group) and _fits(symm_mem_buffer, input_tensor) and _host.all_reduce(input_tensor, bias, output) is not None:
         return None
     if input_tensor.device.type != "cuda":
         output.copy_(ref.all_reduce_bias(input_tensor, bias, group))
@@ -68,7 +69,7 @@ def two_shot_all_reduce_bias(symm_mem_input: torch.Tensor, input_tensor: torch.T
                              group=None) -> torch.Tensor:
     """output = all_reduce(input) (+ bias): each rank reduces 1/ws of the elements, adds the bias
     and publishes the result to every rank (through NVLS when the buffer has a multicast mapping)."""
-    if _alone(symm_mem_input, input_tensor, group) and _host.all_reduce(input_tensor, bias, output) is not None:
+    if _alone(symm_mem_input, group) and _fits(symm_mem_input, input_tensor) and _host.all_reduce(input_tensor, bias, output) is not None:
         return output
     if input_tensor.device.type != "cuda":
         output.copy_(ref.all_reduce_bias(input_tensor, bias, group))
@@ -122,7 +123,7 @@ def one_shot_all_reduce_bias_rms_norm(symm_mem_input: torch.Tensor, x: torch.Ten
                                       group=None, algo: str | None = None) -> None:
     """y = rms_norm(all_reduce(x) + bias) * w; the summed row never leaves registers. Small inputs
     take the push form (one barrier), larger ones the pull form; algo="push"|"pull" overrides."""
-    if _alone(symm_mem_input, x, group) and _host.bias_rms_norm(x, bias, w, y, eps):
+    if _alone(symm_mem_input, group) and _host.bias_rms_norm(symm_mem_input, x, bias, w, y, eps):
         return
     _ar_bias_rms_norm(symm_mem_input, x, bias, w, y, eps, group, 0, algo)
 
@@ -131,7 +132,7 @@ def two_shot_all_reduce_bias_rms_norm(symm_mem_input: torch.Tensor, x: torch.Ten
                                       w: torch.Tensor, y: torch.Tensor, eps: float = 1e-5, group=None) -> None:
     """Same result with the two-shot exchange: rank k reduces columns [k*D/ws, (k+1)*D/ws) of each
     row and publishes them, then every rank normalises. Needs D % (8 * world_size) == 0."""
-    if _alone(symm_mem_input, x, group) and _host.bias_rms_norm(x, bias, w, y, eps):
+    if _alone(symm_mem_input, group) and _host.bias_rms_norm(symm_mem_input, x, bias, w, y, eps):
         return
     D = x.shape[-1]
     info = symm_mem.resolve_group(group)

@@ -17,7 +17,7 @@ from __future__ import annotations
 import torch
 
 from .. import fused
-from ..fused.gemm_ops import all_gather_matmul_act, matmul
+from ..fused.gemm_ops import all_gather_matmul_act
 from ..ops import host as _host
 from ..parallel import symm_mem
 
@@ -60,10 +60,12 @@ class TPMLP:
     # -- decode ------------------------------------------------------------------------------------
     def decode(self, h_local: torch.Tensor, eps: float = 1e-5) -> torch.Tensor:
         """h_local: [M, F/ws] (this rank's slice of the MLP activations) -> normalised [M, H]."""
-        if h_local.is_cuda and h_local.dtype == torch.bfloat16 and symm_mem.solo(self.group):
-            p = matmul(h_local, self.w_down_t.t())         # one rank: nothing left to sum, so the rounding is the epilogue's
-        else:
-            p = fused.gemm_one_shot_all_reduce(h_local, self.w_down_t.t(), group=self.group)     # fp32, replicated
+        if h_local.is_cuda and symm_mem.solo(self.group):
+            # one rank: nothing left to sum, so the GEMM's epilogue rounds p and one native call does both steps
+            y = _host.decode(h_local, self.w_down_t, self.bias, self.norm_w, eps)
+            if y is not None:
+                return y
+        p = fused.gemm_one_shot_all_reduce(h_local, self.w_down_t.t(), group=self.group)     # fp32, replicated
         if p.is_cuda:
             y = _host.rounded_bias_rms_norm(p, self.bias, self.norm_w, eps)
             if y is not None:

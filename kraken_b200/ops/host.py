@@ -14,7 +14,7 @@ import threading
 from . import _build
 
 _lock = threading.Lock()
-_FUNCTIONS = ("gemm", "rms_norm", "bias_rms_norm", "rounded_bias_rms_norm", "all_reduce", "reset")
+_FUNCTIONS = ("gemm", "decode", "rms_norm", "bias_rms_norm", "rounded_bias_rms_norm", "all_reduce", "reset")
 _NATIVE = ("kr_last_error", "kr_rms_norm", "kr_local_bias_rms_norm", "kr_local_all_reduce", "kr_gemm_scratch", "kr_gemm")
 
 
