@@ -5,12 +5,12 @@
 //
 // All of them are bound by HBM, or by the launch for a few rows. Blocks are small, take one row (or 16 KB)
 // each and are started in address order: on a B200 that reads and writes faster than a persistent grid
-// whose blocks stride through memory. Measured on 16384 x 8192: RMSNorm with one 128-thread block per
-// row 84 us (6.39 TB/s), persistent 256-thread blocks with a prefetched next row 92 us, rows through a
-// ring of bulk copies 99 us; 256 MB copied by 512-thread blocks of two vectors per thread 82 us,
-// by a persistent grid 93 us, with bulk copies 90 us.
+// whose blocks stride through memory. Measured: RMSNorm of 16384 x 8192 83 us (6.47 TB/s; persistent
+// 256-thread blocks with a prefetched next row 92 us, rows through a ring of bulk copies 99 us); 256 MB
+// copied by 512-thread blocks of two vectors per thread 82 us, by a persistent grid 93 us, with bulk copies 90 us.
 #include "kraken/host.h"
 #include "kraken/norm_core.cuh"
+#include "kraken/tcgen05.cuh"
 
 namespace kraken {
 
@@ -118,6 +118,55 @@ __global__ void __launch_bounds__(VPT <= 2 ? 1024 : 512) norm_row_kernel(const L
   }
 }
 
+// Thousands of rows: the row is fetched into shared memory with one bulk copy and read from there twice,
+// so a block holds no row in registers and as many rows are in flight as shared memory takes (13 of 16 KB
+// per SM). Rows kept in registers measured 2-50 % slower here, following each kernel's register count
+// (16384 rows: D 8192 87.5 to 83.0 us, D 6144 95 to 62.7, D 5120 58 to 53.4; floor 81.9 / 61.4 / 51.2).
+template <int T>
+__global__ void __launch_bounds__(T) norm_stream_kernel(const LocalNormParams p, const SyncCtx sync) {
+  extern __shared__ __align__(128) unsigned char row_smem[];
+  __shared__ __align__(8) unsigned long long bar;
+  __shared__ float partial[T / 32];
+  pdl_launch();
+  const int nvec = p.D / 8;
+  const uint32_t row_bytes = (uint32_t)p.D * 2u;
+  if (threadIdx.x == 0) {
+    mbar_init(smem_u32(&bar), 1);
+    mbar_fence_init();
+    pdl_wait();
+    mbar_expect_tx(smem_u32(&bar), row_bytes);
+    bulk_load_1d(smem_u32(row_smem), (const char*)p.x + (size_t)blockIdx.x * row_bytes, row_bytes, smem_u32(&bar));
+  }
+  __syncthreads();
+  pdl_wait();
+  if (!mbar_wait(smem_u32(&bar), 0, sync, 90)) return;
+  float ss = 0.f;
+#pragma unroll 4
+  for (int v = threadIdx.x; v < nvec; v += T) {
+    float g[8];
+    unpack8(*(const U4*)(row_smem + (size_t)v * 16), g);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) ss += g[j] * g[j];
+  }
+  ss = warp_sum(ss);
+  if ((threadIdx.x & 31) == 0) partial[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < T / 32; ++k) ss += partial[k];
+  const float inv = rsqrtf(ss / (float)p.D + p.eps);
+  char* y = (char*)p.y + (size_t)blockIdx.x * row_bytes;
+#pragma unroll 4
+  for (int v = threadIdx.x; v < nvec; v += T) {
+    float g[8], h[8];
+    unpack8(*(const U4*)(row_smem + (size_t)v * 16), g);
+    unpack8(ld16_nc((const char*)p.w + (size_t)v * 16), h);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) h[j] = g[j] * inv * h[j];
+    st16(y + (size_t)v * 16, pack8(h));
+  }
+}
+
 // Rows longer than the register budget: two passes over global memory.
 __global__ void __launch_bounds__(kNormMaxThreads) rms_norm_long_kernel(const LocalNormParams p) {
   __shared__ float smem[32];
@@ -198,12 +247,21 @@ static NormKernel norm_row(int vpt) {
 
 static int launch_norm(const DeviceState* d, int mode, LocalNormParams p, int rows, cudaStream_t stream) {
   const int nvec = p.D / 8;
-  // Two rows per SM or fewer: the row's latency counts, so as many threads as it has vectors. Beyond, small
-  // blocks that keep a whole row in flight (several rows resident per SM, cheap barrier): 128 threads, more
-  // only for rows that would not fit eight vectors per thread.
-  int threads = rows <= 2 * d->num_sms ? (nvec + 31) / 32 * 32 : 128;
-  while (threads < 512 && nvec > 8 * threads) threads *= 2;
-  if (threads > 1024) threads = nvec <= 2048 ? 1024 : 512;         // kernels of three vectors and more are built for 512 threads
+  if (mode == NORM_PLAIN && rows >= 24 * d->num_sms && p.D <= 32768) {
+    // from here on the rows stream through shared memory (4096 x 4096: 12.2 us against 14.3; 2048 x 8192, which
+    // L2 mostly holds: 15 against 12.6)
+    SyncCtx sync = sync_ctx(d);
+    void* args[] = {(void*)&p, (void*)&sync};
+    const bool small = p.D < 2560;
+    return launch_overlapped(small ? (const void*)norm_stream_kernel<64> : (const void*)norm_stream_kernel<128>, (unsigned)rows, small ? 64 : 128,
+                             args, (size_t)p.D * 2, stream);
+  }
+  // Two rows per SM or fewer: the row's latency counts, so as many threads as it has vectors. Beyond, half as
+  // many: fewer barriers' worth of warps (512 x 8192 3.9 us against 4.8, with 128 threads 5.7). Kernels of
+  // three vectors and more per thread are built for 512 threads.
+  int threads = ((rows <= 2 * d->num_sms ? nvec : (nvec + 1) / 2) + 31) / 32 * 32;
+  if (threads > 1024) threads = nvec <= 2048 ? 1024 : 512;
+  if (rows > 2 * d->num_sms && threads > 512) threads = 512;
   const int vpt = (nvec + threads - 1) / threads;
   void* args[] = {(void*)&p};
   if (vpt > 8) return launch_overlapped((const void*)rms_norm_long_kernel, (unsigned)rows, kNormMaxThreads, args, 0, stream);

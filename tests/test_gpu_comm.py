@@ -262,3 +262,10 @@ def test_rounded_bias_rms_norm_rounds_like_separate_ops(rows, D, dtype):
     y = host.rounded_bias_rms_norm(p, bias, w, 1e-5)
     torch.testing.assert_close(y.float(), _rms_ref(x, w, 1e-5), atol=1e-2, rtol=1e-2)
     assert torch.equal(y, fused.rms_norm(x, w))
+
+
+@pytest.mark.parametrize("rows,D", [(3552, 8), (3552, 2552), (3600, 2560), (4000, 1000), (3552, 32768), (3552, 32776)])
+def test_rms_norm_of_thousands_of_rows(rows, D):
+    x = torch.randn(rows, D, device="cuda").to(torch.bfloat16)
+    w = (1 + 0.1 * torch.randn(D, device="cuda")).to(torch.bfloat16)
+    torch.testing.assert_close(fused.rms_norm(x, w).float(), _rms_ref(x, w, 1e-5), atol=4e-2, rtol=2e-2)
