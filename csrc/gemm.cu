@@ -416,14 +416,15 @@ struct TmapKey {
   unsigned long long rows, cols, ld;
   unsigned box_rows;
   int elt;
+  unsigned box_bytes;
   bool operator==(const TmapKey& o) const {
-    return ptr == o.ptr && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows && elt == o.elt;
+    return ptr == o.ptr && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows && elt == o.elt && box_bytes == o.box_bytes;
   }
 };
 struct TmapHash {
   size_t operator()(const TmapKey& k) const {
     unsigned long long h = (unsigned long long)(uintptr_t)k.ptr >> 4;
-    for (unsigned long long v : {k.rows, k.cols, k.ld, (unsigned long long)k.box_rows * 8 + (unsigned long long)k.elt})
+    for (unsigned long long v : {k.rows, k.cols, k.ld, (unsigned long long)k.box_rows * 2048 + k.box_bytes * 8 + (unsigned long long)k.elt})
       h = (h ^ v) * 0x9e3779b97f4a7c15ull;
     return (size_t)(h ^ (h >> 32));
   }
@@ -435,11 +436,11 @@ constexpr size_t kTmapCacheEntries = 4096;
 static unsigned long long g_tmap_hits = 0, g_tmap_misses = 0;
 
 // Tensor map of a row-major matrix [rows, cols] of bf16 (elt 2) or fp32 (elt 4) elements (cols
-// contiguous, `ld` elements per row), box = 128 bytes of columns x box_rows rows, 128-byte swizzle,
+// contiguous, `ld` elements per row), box = box_bytes (128 or 64) of columns x box_rows rows, swizzled by as much,
 // out-of-range elements read as zero.
 int get_tmap(const void* ptr, unsigned long long rows, unsigned long long cols, unsigned long long ld,
-                    unsigned box_rows, CUtensorMap* out, int elt) {
-  TmapKey key{ptr, rows, cols, ld, box_rows, elt};
+                    unsigned box_rows, CUtensorMap* out, int elt, unsigned box_bytes) {
+  TmapKey key{ptr, rows, cols, ld, box_rows, elt, box_bytes};
   {
     std::lock_guard<std::mutex> lk(g_tmap_mu);
     auto it = g_tmap_cache.find(key);
@@ -455,12 +456,12 @@ int get_tmap(const void* ptr, unsigned long long rows, unsigned long long cols, 
   KR_REQUIRE(box_rows >= 1 && box_rows <= 256, "bad TMA box");
   cuuint64_t gdim[2] = {cols, rows};
   cuuint64_t gstride[1] = {ld * (unsigned long long)elt};
-  cuuint32_t box[2] = {(cuuint32_t)(128 / elt), box_rows};
+  cuuint32_t box[2] = {(cuuint32_t)(box_bytes / elt), box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUtensorMap m;
   KR_CU(cuTensorMapEncodeTiled, &m, elt == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
         const_cast<void*>(ptr), gdim, gstride, box,
-        estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+        estr, CU_TENSOR_MAP_INTERLEAVE_NONE, box_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   {
     std::lock_guard<std::mutex> lk(g_tmap_mu);

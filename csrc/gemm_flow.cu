@@ -1,0 +1,505 @@
+// The plain GEMM for problems of a wave of tiles and more: persistent CTA pairs that draw their tiles from a
+// counter, C[M,N] = act(A[M,K] * Bt[N,K]^T) with bf16 operands or fp32 multiplied as tf32.
+//
+// What bounds it: a B200 runs long GEMMs at its power limit (1.3-1.5 GHz), so besides feeding the tensor
+// cores what counts is the data moved per operation. Two choices follow.
+//  * Tiles are handed out in order, one atomic per tile. With a fixed share per pair the pairs drift apart (some
+//    run 5 % slower), the tiles in flight stop sharing operands and HBM reads more than double: 8192 x 8192
+//    x 14336 read 3.98 GB with fixed shares, 1.98 GB in order (ncu, dram__bytes_read.sum).
+//  * RB = 2 row blocks: a pair computes 512 x 256, each operand stage feeds twice the MMAs (48 KB instead of 64
+//    per CTA and 256 x 256 x 64 block pair). The accumulators then fill TMEM, so a tile's first MMAs wait for the
+//    epilogue of the one before, row block by row block. RB = 1 keeps two accumulators in turn.
+// Narrower column tiles (BN) fit ragged sizes and waves better; the launcher picks (flow_plan).
+//
+// Warps: 0 TMA producer (the leader's also draws the tiles), 1 MMA issuer (leader), 2-9 epilogue (two per TMEM
+// lane quarter, column panels dealt alternately), 10-11 optional copy of the row operand.
+#include <algorithm>
+#include "kraken/gemm_host.h"
+
+namespace kraken {
+
+constexpr int kFlowEpiWarps = 8;
+constexpr int kFlowThreads = 64 + 32 * kFlowEpiWarps;
+constexpr int kFlowCopyThreads = 64;                      // 12 warps leave 168 registers a thread, 14 would leave 128
+constexpr int kFlowSlots = 4;                             // tiles drawn ahead of the slowest role, at most
+
+struct alignas(64) FlowParams {
+  CUtensorMap tmap_r, tmap_c, tmap_out;
+  int tiles_r, tiles_c, num_kb, group_r;                  // tiles of RB * 256 rows
+  int items, split_from;                                  // tiles from split_from on are drawn as single row blocks
+  int transposed, out_fp32, act;
+  int out_rows, out_cols;
+  uint32_t* sched;                                        // [0] items drawn beyond the first of each pair, [1] pairs done; or nullptr
+  void* out;                                              // output without a tensor map (else nullptr) and its row stride
+  long long ldo;
+  const void* cp_src;
+  void* cp_dst;
+  unsigned long long cp_bytes;
+  SyncCtx sync;
+};
+
+template <int BN, int RB>
+struct FlowCfg {
+  static constexpr int A_BYTES = kBM * 128;               // one row block of this CTA
+  static constexpr int B_BYTES = BN / 2 * 128;
+  static constexpr int STAGE = RB * A_BYTES + B_BYTES;
+  static constexpr int EPI = kFlowEpiWarps * 4096;
+  static constexpr int RAW_STAGES = (kSmemLimit - 1024 - EPI - 512) / STAGE;
+  static constexpr int STAGES = RAW_STAGES > 8 ? 8 : RAW_STAGES;
+  static constexpr int BUFS = 2 * RB * BN <= 512 ? 2 : 1;
+  static constexpr int UNITS = BUFS * RB;                 // accumulators of BN columns
+  static constexpr int TMEM_COLS = UNITS * BN <= 256 ? 256 : 512;
+  static constexpr int SMEM = 1024 + STAGES * STAGE + EPI + 512;
+  static_assert(BN % 32 == 0 && BN >= 128 && BN <= 256 && UNITS <= 4 && STAGES >= 3, "tile shape");
+  static_assert(16 * STAGES + 16 * UNITS + 16 * kFlowSlots + 4 * kFlowSlots + 8 <= 512, "barrier area");
+};
+
+// Bounded wait with cluster-scope acquire: what the other CTA wrote before it arrived is visible.
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred P;\n\t mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 P, [%1], %2;\n\t selp.u32 %0, 1, 0, P;\n\t}\n"
+      : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, const SyncCtx& c, uint32_t site) {
+  if (mbar_try_wait_cluster(bar, parity)) return true;
+  const uint64_t t0 = globaltimer_ns();
+  uint32_t n = 0;
+  while (true) {
+    if (mbar_try_wait_cluster(bar, parity)) return true;
+    if ((++n & 255u) == 0u) {
+      if (!status_ok(c)) return false;
+      if (globaltimer_ns() - t0 > c.timeout_ns) {
+        set_status(c, make_status(KR_ERR_TIMEOUT_MBAR, site, 0, blockIdx.x));
+        return false;
+      }
+    }
+  }
+}
+__device__ __forceinline__ void st_cluster_u32(uint32_t addr, uint32_t v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ uint32_t ld_shared_u32(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+
+struct FlowItem {
+  int tr, tc, rb_lo, rb_hi;      // tile coordinates and the row blocks of it
+};
+template <int RB>
+__device__ __forceinline__ FlowItem flow_item(const FlowParams& p, int t) {
+  FlowItem it;
+  int tile = t;
+  it.rb_lo = 0;
+  it.rb_hi = RB;
+  if (RB == 2 && t >= p.split_from) {
+    tile = p.split_from + ((t - p.split_from) >> 1);
+    it.rb_lo = (t - p.split_from) & 1;
+    it.rb_hi = it.rb_lo + 1;
+  }
+  const int per_group = p.group_r * p.tiles_c, g = tile / per_group, first = g * p.group_r;
+  const int gsz = min(p.group_r, p.tiles_r - first), in = tile - g * per_group;
+  it.tr = first + in % gsz;
+  it.tc = in / gsz;
+  return it;
+}
+
+template <int BN, int RB, int ELT>
+__global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_kernel(const __grid_constant__ FlowParams p) {
+  using Cfg = FlowCfg<BN, RB>;
+  constexpr int kStageK = 128 / ELT;
+  extern __shared__ unsigned char smem_raw[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t cta = cluster_ctarank();
+  const bool leader = cta == 0;
+  const int pair = (int)(blockIdx.x >> 1), pairs = (int)(gridDim.x >> 1);
+  const uint32_t stage0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const uint32_t epi0 = stage0 + Cfg::STAGES * Cfg::STAGE;
+  const uint32_t bars = epi0 + Cfg::EPI;
+  auto full_bar = [&](int s) { return bars + 8u * s; };
+  auto empty_bar = [&](int s) { return bars + 8u * (Cfg::STAGES + s); };
+  auto tfull_bar = [&](int u) { return bars + 8u * (2 * Cfg::STAGES + u); };
+  auto tempty_bar = [&](int u) { return bars + 8u * (2 * Cfg::STAGES + Cfg::UNITS + u); };
+  const uint32_t sfull = bars + 8u * (2 * Cfg::STAGES + 2 * Cfg::UNITS), sempty = sfull + 8u * kFlowSlots;
+  const uint32_t sdata = sempty + 8u * kFlowSlots, tmem_slot = sdata + 4u * kFlowSlots;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < Cfg::STAGES; ++s) {
+      mbar_init(full_bar(s), 1);
+      mbar_init(empty_bar(s), 1);
+    }
+    for (int u = 0; u < Cfg::UNITS; ++u) {
+      mbar_init(tfull_bar(u), 1);
+      mbar_init(tempty_bar(u), 2 * kFlowEpiWarps);
+    }
+    for (int k = 0; k < kFlowSlots; ++k) {
+      mbar_init(sfull + 8u * k, 1);
+      mbar_init(sempty + 8u * k, 2 + 2 * kFlowEpiWarps);     // the MMA issuer, the peer's producer, both CTAs' epilogue warps
+    }
+    mbar_fence_init();
+    tma_prefetch_desc(&p.tmap_r);
+    tma_prefetch_desc(&p.tmap_c);
+    tma_prefetch_desc(&p.tmap_out);
+  }
+  if (warp == 1) {
+    tmem_alloc_pair(tmem_slot, Cfg::TMEM_COLS);
+    tmem_relinquish_pair();
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();            // both CTAs' barriers exist before anyone signals across the pair
+  tc_fence_after();
+  const uint32_t tmem_base = ld_shared_u32(tmem_slot);
+  pdl_launch();
+  pdl_wait();
+
+  // A staged panel of 32 rows x `cols` columns to an output that TMA cannot describe (rows not whole 16-byte
+  // units), element by element.
+  auto store_plain = [&](uint32_t panel, int gx, int gy, int cols, bool fp32, int ln) {
+    const int elt = fp32 ? 4 : 2, pitch = cols * elt, mask = pitch == 128 ? 7 : 3;
+    for (int r = 0; r < 32 && gy + r < p.out_rows; ++r) {
+      const int perm = pitch == 128 ? (r & mask) : ((r >> 1) & mask);
+      for (int c = ln; c < cols && gx + c < p.out_cols; c += 32) {
+        const uint32_t a = panel + (uint32_t)(r * pitch + ((((c * elt) >> 4) ^ perm) << 4) + ((c * elt) & 15));
+        const long long o = (long long)(gy + r) * p.ldo + gx + c;
+        if (fp32) {
+          ((uint32_t*)p.out)[o] = ld_shared_u32(a);
+        } else {
+          unsigned short v;
+          asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
+          ((unsigned short*)p.out)[o] = v;
+        }
+      }
+    }
+    __syncwarp();
+  };
+
+  // The item after publication k (item k + 1 of this pair): read by every role but the leader's producer.
+  auto next_item = [&](int k, bool warp_wide, int& t) {
+    const uint32_t slot = (uint32_t)(k % kFlowSlots), parity = (uint32_t)(k / kFlowSlots) & 1u;
+    bool ok = mbar_wait_cluster(sfull + 8u * slot, parity, p.sync, 91);
+    if (warp_wide) ok = __all_sync(0xffffffffu, ok);
+    t = ok ? (int)ld_shared_u32(sdata + 4u * slot) : p.items;
+    if (warp_wide) __syncwarp();
+    if (!warp_wide || lane == 0) mbar_arrive_cluster(mapa_shared(sempty + 8u * slot, 0));
+    return ok;
+  };
+
+  if (warp == 0) {
+    // ================= TMA producer (both CTAs) =================
+    if (elect_one()) {
+      int s = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      int t = pair;
+      for (int k = 0; ok && t < p.items; ++k) {
+        int drawn = 0;
+        // Drawn now and published a few K blocks on, when the atomic has long returned: the peer's producer goes
+        // on to the next tile without a gap. Without a counter every pair takes its fixed share.
+        if (leader) drawn = p.sched != nullptr ? (int)atomicAdd(p.sched, 1u) + pairs : t + pairs;
+        const FlowItem it = flow_item<RB>(p, t);
+        const uint32_t bytes = 2u * (uint32_t)((it.rb_hi - it.rb_lo) * Cfg::A_BYTES + Cfg::B_BYTES);
+        const int row0 = it.tr * (RB * 256) + (int)cta * kBM, col0 = it.tc * BN + (int)cta * (BN / 2);
+        for (int kb = 0; kb < p.num_kb; ++kb) {
+          ok = mbar_wait(empty_bar(s), ph ^ 1u, p.sync, 92);
+          if (!ok) break;
+          const uint32_t lead_full = mapa_shared(full_bar(s), 0);
+          if (leader) mbar_expect_tx(full_bar(s), bytes);             // both CTAs' bytes complete on the leader's barrier
+          const uint32_t sa = stage0 + s * Cfg::STAGE;
+#pragma unroll
+          for (int rb = 0; rb < RB; ++rb)
+            if (rb >= it.rb_lo && rb < it.rb_hi)
+              tma_load_2d_pair(sa + rb * Cfg::A_BYTES, &p.tmap_r, lead_full, kb * kStageK, row0 + rb * 256);
+          tma_load_2d_pair(sa + RB * Cfg::A_BYTES, &p.tmap_c, lead_full, kb * kStageK, col0);
+          if (++s == Cfg::STAGES) { s = 0; ph ^= 1u; }
+          if (leader && kb == min(3, p.num_kb - 1)) {
+            // to both CTAs, even past the end (that is how the other roles learn of it)
+            const uint32_t slot = (uint32_t)(k % kFlowSlots), parity = (uint32_t)(k / kFlowSlots) & 1u;
+            ok = mbar_wait_cluster(sempty + 8u * slot, parity ^ 1u, p.sync, 93);
+            if (!ok) break;
+#pragma unroll
+            for (uint32_t c = 0; c < 2; ++c) {
+              st_cluster_u32(mapa_shared(sdata + 4u * slot, c), (uint32_t)drawn);
+              mbar_arrive_cluster(mapa_shared(sfull + 8u * slot, c));
+            }
+          }
+        }
+        if (leader) t = drawn;
+        else ok = next_item(k, false, t) && ok;
+      }
+      if (leader && p.sched != nullptr) {
+        // the last pair puts the counter back for the next launch on this stream
+        const uint32_t done = atom_add_acqrel_gpu(p.sched + 1, 1u);
+        if (done == (uint32_t)pairs - 1u) {
+          p.sched[0] = 0;
+          p.sched[1] = 0;
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ================= MMA issuer (leader CTA only) =================
+    if (leader && elect_one()) {
+      constexpr uint32_t idesc = ELT == 2 ? make_idesc_bf16(256, BN) : make_idesc_tf32(256, BN);
+      int s = 0;
+      uint32_t ph = 0, uph = 0;                            // uph: one phase bit per accumulator
+      bool ok = true;
+      int t = pair;
+      for (int k = 0; ok && t < p.items; ++k) {
+        const FlowItem it = flow_item<RB>(p, t);
+        const int u0 = Cfg::BUFS == 2 ? (k & 1) * RB : 0;
+        for (int kb = 0; kb < p.num_kb; ++kb) {
+          ok = mbar_wait(full_bar(s), ph, p.sync, 94);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t sa = stage0 + s * Cfg::STAGE;
+          const uint64_t bdesc = make_smem_desc_sw128(sa + RB * Cfg::A_BYTES);
+#pragma unroll
+          for (int rb = 0; rb < RB; ++rb) {
+            if (rb < it.rb_lo || rb >= it.rb_hi) continue;
+            const int u = u0 + rb;
+            if (kb == 0) {
+              ok = mbar_wait(tempty_bar(u), ((uph >> u) & 1u) ^ 1u, p.sync, 95) && ok;
+              tc_fence_after();
+            }
+            const uint64_t adesc = make_smem_desc_sw128(sa + rb * Cfg::A_BYTES);
+            const uint32_t d_tmem = tmem_base + (uint32_t)(u * BN);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const uint32_t accumulate = (kb > 0 || i != 0) ? 1u : 0u;
+              if (ELT == 2) umma_bf16_pair(d_tmem, adesc + (uint64_t)(2 * i), bdesc + (uint64_t)(2 * i), idesc, accumulate);
+              else umma_tf32_pair(d_tmem, adesc + (uint64_t)(2 * i), bdesc + (uint64_t)(2 * i), idesc, accumulate);
+            }
+            if (kb == p.num_kb - 1) {
+              umma_commit_pair(tfull_bar(u));
+              umma_commit_pair(mapa_shared(tfull_bar(u), 1));
+            }
+          }
+          if (!ok) break;
+          umma_commit_pair(empty_bar(s));
+          umma_commit_pair(mapa_shared(empty_bar(s), 1));
+          if (++s == Cfg::STAGES) { s = 0; ph ^= 1u; }
+        }
+        for (int rb = it.rb_lo; rb < it.rb_hi; ++rb) uph ^= 1u << (u0 + rb);
+        ok = next_item(k, false, t) && ok;
+      }
+    }
+  } else if (warp < 2 + kFlowEpiWarps) {
+    // ================= epilogue (both CTAs, own 128 rows of each block) =================
+    const int q = warp & 3, h = (warp - 2) >> 2;           // TMEM lane quarter; even or odd column panels
+    const uint32_t slot = epi0 + (uint32_t)(warp - 2) * 4096u;
+    constexpr int PW = BN % 64 == 0 ? 64 : 32;             // columns per panel of a bf16 row-major tile
+    constexpr int CHUNKS = (BN / PW + 1) / 2 * (PW / 32);  // 32-column chunks of one warp, at most
+    auto chunk_col = [&](int i) { return PW == 64 ? (h + 2 * (i >> 1)) * 64 + (i & 1) * 32 : (h + 2 * i) * 32; };
+    const bool fp32 = p.out_fp32 != 0, transposed = p.transposed != 0;
+    uint32_t uph = 0;
+    bool ok = true;
+    int t = pair;
+    for (int k = 0; ok && t < p.items; ++k) {
+      const FlowItem it = flow_item<RB>(p, t);
+      const int u0 = Cfg::BUFS == 2 ? (k & 1) * RB : 0;
+#pragma unroll 1
+      for (int rb = it.rb_lo; rb < it.rb_hi && ok; ++rb) {
+        const int u = u0 + rb;
+        ok = mbar_wait(tfull_bar(u), (uph >> u) & 1u, p.sync, 96);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        uph ^= 1u << u;
+        tc_fence_after();
+        const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(u * BN);
+        const int drow = it.tr * (RB * 256) + rb * 256 + (int)cta * kBM + q * 32;      // first row of D of this warp
+        auto release = [&] {      // this warp has read its part of the accumulator
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(mapa_shared(tempty_bar(u), 0));
+        };
+        // A panel in the slot goes out: rows gy ..., columns gx ... of the output
+        auto send = [&](int gx, int gy, int cols) {
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            if (p.out == nullptr && gx < p.out_cols && gy < p.out_rows) tma_store_2d(&p.tmap_out, slot, gx, gy);
+            bulk_commit_group();
+          }
+          if (p.out != nullptr) store_plain(slot, gx, gy, cols, fp32, lane);
+        };
+        auto slot_free = [&] {    // the store that last read the slot is done with it
+          if (lane == 0) bulk_wait_group_read<0>();
+          __syncwarp();
+        };
+        if (fp32) {
+#pragma unroll 1
+          for (int i = 0; i < CHUNKS; ++i) {
+            const int col = chunk_col(i);
+            if (col >= BN) break;
+            uint32_t r[32];
+            tmem_ld32(t_addr + (uint32_t)col, r);
+            tmem_ld_wait();
+            if (i + 1 == CHUNKS || chunk_col(i + 1) >= BN) release();
+            if (p.act != 0) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(gelu_tanh(__uint_as_float(r[j])));
+            }
+            slot_free();
+            if (transposed) {
+              // panel row j = column col + j of D; lanes = consecutive output columns
+#pragma unroll
+              for (int j = 0; j < 32; ++j)
+                asm volatile("st.shared.u32 [%0], %1;" ::"r"(slot + j * 128u + (uint32_t)((((lane >> 2) ^ (j & 7)) << 4) + (lane & 3) * 4)), "r"(r[j]) : "memory");
+              send(drow, it.tc * BN + col, 32);
+            } else {
+#pragma unroll
+              for (int v = 0; v < 8; ++v)
+                st_shared_u4(slot + lane * 128u + (uint32_t)((v ^ (lane & 7)) << 4), r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3]);
+              send(it.tc * BN + col, drow, 32);
+            }
+          }
+        } else {
+          // bf16: the warp's whole part is read and rounded before anything is stored, so that the next
+          // tile's MMAs wait for nothing but TMEM reads; the activation follows on the rounded values, as it
+          // would on a bf16 tensor.
+          uint32_t packed[CHUNKS][16];
+#pragma unroll
+          for (int i = 0; i < CHUNKS; ++i) {
+            const int col = chunk_col(i);
+            if (col < BN) {
+              uint32_t r[32];
+              tmem_ld32(t_addr + (uint32_t)col, r);
+              tmem_ld_wait();
+#pragma unroll
+              for (int v = 0; v < 16; ++v) packed[i][v] = pack_bf16x2(__uint_as_float(r[2 * v]), __uint_as_float(r[2 * v + 1]));
+            }
+          }
+          release();
+#pragma unroll
+          for (int i = 0; i < CHUNKS; ++i) {
+            const int col = chunk_col(i);
+            if (col < BN) {
+              if (p.act != 0) {
+#pragma unroll
+                for (int v = 0; v < 16; ++v)
+                  packed[i][v] = pack_bf16x2(gelu_tanh(bf16lo(packed[i][v])), gelu_tanh(bf16hi(packed[i][v])));
+              }
+              if (transposed) {
+                slot_free();
+#pragma unroll
+                for (int j = 0; j < 32; ++j) {
+                  const uint32_t a = slot + j * 64u + (uint32_t)((((lane >> 3) ^ ((j >> 1) & 3)) << 4) + (lane & 7) * 2);
+                  asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"((unsigned short)(packed[i][j >> 1] >> ((j & 1) * 16))) : "memory");
+                }
+                send(drow, it.tc * BN + col, 32);
+              } else if (PW == 64) {
+                if ((i & 1) == 0) slot_free();
+#pragma unroll
+                for (int v = 0; v < 4; ++v)
+                  st_shared_u4(slot + lane * 128u + (uint32_t)((((i & 1) * 4 + v) ^ (lane & 7)) << 4), packed[i][4 * v], packed[i][4 * v + 1],
+                               packed[i][4 * v + 2], packed[i][4 * v + 3]);
+                if ((i & 1) == 1) send(it.tc * BN + col - 32, drow, 64);
+              } else {
+                slot_free();
+#pragma unroll
+                for (int v = 0; v < 4; ++v)
+                  st_shared_u4(slot + lane * 64u + (uint32_t)((v ^ ((lane >> 1) & 3)) << 4), packed[i][4 * v], packed[i][4 * v + 1],
+                               packed[i][4 * v + 2], packed[i][4 * v + 3]);
+                send(it.tc * BN + col, drow, 32);
+              }
+            }
+          }
+        }
+      }
+      if (ok) ok = next_item(k, true, t);
+    }
+    if (lane == 0) bulk_wait_group<0>();
+  } else if (p.cp_bytes != 0) {
+    // ================= copy of the row operand: this CTA's share =================
+    const size_t nvec = p.cp_bytes / 16, lo = nvec * blockIdx.x / gridDim.x, hi = nvec * (blockIdx.x + 1) / gridDim.x;
+    size_t v = lo + threadIdx.x - kFlowThreads;
+    for (; v + 7 * kFlowCopyThreads < hi; v += 8 * kFlowCopyThreads) {
+      U4 x[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[i] = ld16((const char*)p.cp_src + (v + (size_t)i * kFlowCopyThreads) * 16);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) st16((char*)p.cp_dst + (v + (size_t)i * kFlowCopyThreads) * 16, x[i]);
+    }
+    for (; v < hi; v += kFlowCopyThreads) st16((char*)p.cp_dst + v * 16, ld16((const char*)p.cp_src + v * 16));
+  }
+  __syncwarp();
+
+  // ---- teardown: nobody leaves while the pair may still touch its shared memory or barriers
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc_pair(tmem_base, Cfg::TMEM_COLS);
+  }
+}
+
+// ---- host ---------------------------------------------------------------------------------------
+struct FlowVariant {
+  const void* fn;
+  size_t smem;
+};
+template <int ELT>
+static FlowVariant flow_variant(int bn, int rb) {
+#define KR_FLOW(BN, RB) \
+  if (bn == BN && rb == RB) return {(const void*)gemm_flow_kernel<BN, RB, ELT>, FlowCfg<BN, RB>::SMEM};
+  KR_FLOW(256, 2)
+  KR_FLOW(224, 2)
+  KR_FLOW(192, 2)
+  KR_FLOW(160, 2)
+  KR_FLOW(128, 2)
+  KR_FLOW(256, 1)
+  KR_FLOW(224, 1)
+  KR_FLOW(192, 1)
+  KR_FLOW(160, 1)
+  KR_FLOW(128, 1)
+#undef KR_FLOW
+  return {nullptr, 0};
+}
+
+int launch_flow_gemm(const GemmParams& g, int bn, int rb, int pairs, uint32_t* sched, cudaStream_t stream) {
+  const FlowVariant v = g.in_fp32 ? flow_variant<4>(bn, rb) : flow_variant<2>(bn, rb);
+  if (v.fn == nullptr) return fail(KR_FAIL_ARG, "no persistent pair kernel of this tile shape");
+  FlowParams p;
+  memset(&p, 0, sizeof(p));
+  p.tmap_r = g.tmap_r;
+  p.tmap_c = g.tmap_c;
+  const int out_elt = g.out_fp32 ? 4 : 2;
+  const unsigned box_bytes = (out_elt == 4 || (!g.transposed && bn % 64 == 0)) ? 128u : 64u;
+  if ((g.ldo * out_elt) % 16 == 0 && ((uintptr_t)g.out & 15) == 0) {
+    int rc = get_tmap(g.out, g.out_rows, g.out_cols, g.ldo, 32, &p.tmap_out, out_elt, box_bytes);
+    if (rc) return rc;
+  } else {
+    p.tmap_out = g.tmap_r;          // prefetched, not used
+    p.out = g.out;
+    p.ldo = g.ldo;
+  }
+  p.tiles_r = (g.rows_r + 256 * rb - 1) / (256 * rb);
+  p.tiles_c = (g.rows_c + bn - 1) / bn;
+  p.num_kb = (g.K + (g.in_fp32 ? 32 : 64) - 1) / (g.in_fp32 ? 32 : 64);
+  p.group_r = std::max(1, g.group_r / (2 * rb));
+  const int tiles = p.tiles_r * p.tiles_c;
+  // A last wave that is at most half full is dealt as single row blocks
+  p.split_from = tiles;
+  if (rb == 2 && 2 * (tiles % pairs) <= pairs) p.split_from = tiles - tiles % pairs;
+  p.items = p.split_from + (tiles - p.split_from) * rb;
+  p.transposed = g.transposed;
+  p.out_fp32 = g.out_fp32;
+  p.act = g.act;
+  p.out_rows = g.out_rows;
+  p.out_cols = g.out_cols;
+  p.sched = sched;
+  p.cp_src = g.cp_src;
+  p.cp_dst = g.cp_dst;
+  p.cp_bytes = g.cp_bytes;
+  p.sync = g.sync;
+  pairs = std::min(pairs, p.items);
+  if (pairs == p.items) p.sched = nullptr;        // one item each
+  void* args[] = {(void*)&p};
+  return launch_overlapped(v.fn, 2u * (unsigned)pairs, g.cp_bytes ? kFlowThreads + kFlowCopyThreads : kFlowThreads, args, v.smem, stream, 2);
+}
+
+}  // namespace kraken

@@ -1,10 +1,14 @@
 // The plain GEMM C[M,N] = act(A[M,K] * Bt[N,K]^T) on one GPU: what every fused op runs at world size 1
 // and fused.matmul everywhere. bf16 operands, or fp32 operands multiplied as tf32; fp32 accumulation;
-// bf16 or fp32 result. Kernels: CTA pairs (256 x 256 and 256 x 128 tiles) and single CTAs (128 x 16 ...
-// 128 x 256), all persistent, with the tiles of an uneven wave cut along K (stream-K, gemm_core.cuh).
-// Optionally four more warps per CTA copy the row operand somewhere else while the tiles are computed
+// bf16 or fp32 result. This file picks among three kernel families and launches:
+//   tile    one wave, a tile or a K range of it per CTA or pair (gemm_tile.cu)
+//   flow    persistent pairs that draw tiles in order (gemm_flow.cu)
+//   single  persistent single CTAs on the shared main loop (here): narrow outputs, layouts asked for
+//           explicitly, rank emulation
+// Optionally warps without another role copy the row operand somewhere else while the tiles are computed
 // (the all-gather GEMM at world size 1 returns its gathered operand).
 #include <algorithm>
+#include <cmath>
 #include "kraken/gemm_host.h"
 #include "kraken/gemm_hooks.cuh"
 
@@ -19,7 +23,6 @@ __device__ __forceinline__ void plain_body(const GemmParams& p, unsigned bid, un
   h.bn = BN;
   gemm_mainloop<BN, PlainHooks, ELT>(p, bid, nb, h, smem_raw);
 }
-
 template <int BN, int ELT>
 __global__ void __launch_bounds__(kPlainThreads, 1) gemm_plain_kernel(const __grid_constant__ GemmParams p) {
   plain_body<BN, ELT>(p, blockIdx.x, gridDim.x);
@@ -28,141 +31,130 @@ template <int BN, int ELT>
 __global__ void __launch_bounds__(kPlainThreads, 1) gemm_plain_emu_kernel(const GemmParams* ps) {
   plain_body<BN, ELT>(ps[blockIdx.y], blockIdx.x, gridDim.x);
 }
-template <int BN, int ELT>
-__global__ void __launch_bounds__(kPlainThreads, 1)
-    gemm_plain_pair_kernel(const __grid_constant__ GemmParams p) {
-  extern __shared__ unsigned char smem_raw[];
-  PlainHooks h;
-  h.bn = BN;
-  gemm_mainloop_pair<PlainHooks, BN, ELT>(p, blockIdx.x / 2, gridDim.x / 2, h, smem_raw);
-}
 
 // ---- plan -------------------------------------------------------------------------------------
-// Which kernel a problem runs on, and how its tiles are dealt. Times in microseconds, from runs of
-// this kernel on a B200; only their ratios matter.
+enum PlainKind : int { PLAIN_SINGLE = 0, PLAIN_TILE = 1, PLAIN_FLOW = 2 };
 struct PlainPlan {
-  bool swap;        // the weights (Bt) are the 128-row operand and the tile is stored transposed
-  bool pair;
-  int bn, tiles_r, tiles_c, num_kb;
-  int workers;      // CTAs, or CTA pairs
-  int sk_tiles;
-  int splits;       // > 0: the one-wave kernel, every tile cut into this many parts along K
-  size_t slot_bytes, counters;
+  int kind;
+  bool swap;        // the weights (Bt) are the row operand and the tile is stored transposed
+  bool pair;        // TILE: CTA pairs
+  int bn, rb;       // column tile; FLOW: row blocks per tile
+  int splits;       // TILE
+  int workers;      // CTAs, or pairs, of a persistent kernel
 };
 
-static size_t sk_slot_bytes(const PlainPlan& pl) {
-  return (size_t)2 * pl.workers * (pl.pair ? 2 : 1) * 4 * 32 * pl.bn * 4;
+// Time model of the pair kernels, in microseconds per K block (64 bf16 or 32 fp32 columns of K) of a
+// 256 x 256 block, from long runs on a B200. With every SM busy the chip is at its power limit (0.47);
+// fewer pairs run faster, down to 0.30 at full clock. Narrow column tiles move more operand bytes per
+// operation, two row blocks fewer.
+static double pair_kb_us(int busy, int pairs) { return std::max(0.30, 0.47 * std::sqrt((double)busy / pairs)); }
+static double tile_cost(int bn, int rb) {
+  const double one = bn == 256 ? 1.0 : bn == 224 ? 0.88 : bn == 192 ? 0.77 : bn == 160 ? 0.66 : 0.59;
+  return rb == 1 ? one : 1.93 * one;
 }
 
-// Deals the tiles of `pl` to at most `max_workers` workers. With at least one whole wave, the tiles
-// beyond the last whole wave (and one wave more when they are few, so that nobody gets slivers of
-// many tiles) are cut along K; with less than a wave all tiles are. Cutting costs a meeting of the
-// contributors, so a nearly full last wave stays whole.
-static void deal_tiles(PlainPlan& pl, int max_workers, int sk_mode) {
-  const int T = pl.tiles_r * pl.tiles_c;
-  pl.workers = std::min(T, max_workers);
-  pl.sk_tiles = 0;
-  // one K block: the MMA (or what the shared-memory port feeds it), or the bytes of all workers from HBM
-  const double mma = 0.375 * pl.bn / 256;
-  const double load = (128.0 + (pl.pair ? pl.bn / 2 : pl.bn)) * 128 / 90e3;
-  auto kb_us = [&](int w) {
-    return std::max(std::max(mma, load), (double)w * (pl.pair ? 256 : 128) * 128 / 6.5e6);
-  };
-  // partial sums out, the count, and the last one's way through the slots
-  auto meet_us = [&](double contributors) { return 1.5 + pl.bn / 128.0 * (0.8 + 0.8 * contributors); };
-  const int waves = T / max_workers, rest = T % max_workers;
-  double best = (double)((T + max_workers - 1) / max_workers) * pl.num_kb * kb_us(pl.workers);
-  if (sk_mode == 0 || (rest == 0 && sk_mode < 0)) return;
-  auto consider = [&](int tiles, int w) {
-    const long long units = (long long)tiles * pl.num_kb;
-    if (w > units || w < 2) return;
-    const double per = (double)((units + w - 1) / w);
-    if (per < 2) return;
-    const double whole = (double)((T - tiles) / w) * pl.num_kb;
-    const double n = (double)w / tiles + (w % tiles ? 1 : 0);
-    double t = (whole + per) * kb_us(w) + meet_us(n);
-    if (sk_mode > 0) t *= 1e-3;
-    if (t < best) {
-      best = t;
-      pl.workers = w;
-      pl.sk_tiles = tiles;
-    }
-  };
-  if (waves == 0) {
-    for (int i = 2; i <= 16 && i * T <= max_workers; ++i) consider(T, i * T);   // every tile in i equal parts
-    consider(T, max_workers);
-  } else {
-    if (rest == 0) return;
-    if (2 * rest >= max_workers || sk_mode == 1) consider(rest, max_workers);
-    if (2 * rest < max_workers || sk_mode == 2) consider(rest + max_workers, max_workers);
-  }
+// Rows that do not start on 128-byte lines cost an extra sector and line per 128 bytes fetched, which weighs the
+// more the less a tile reuses its operands (4000 x 6000 x 3000: 256 x 256 tiles 155 us, 512 x 224 131).
+static double flow_us(int rows, int cols, int num_kb, int bn, int rb, int pairs, bool lines) {
+  const int T = ((rows + 256 * rb - 1) / (256 * rb)) * ((cols + bn - 1) / bn);
+  const int whole = T / pairs, rest = T % pairs;
+  const double off1 = lines ? 1.0 : 1.2, off = rb == 1 ? off1 : (lines ? 1.0 : 1.06);
+  const double full = num_kb * tile_cost(bn, rb) * off * pair_kb_us(pairs, pairs);
+  double last = rest ? num_kb * tile_cost(bn, rb) * off * pair_kb_us(rest, pairs) : 0.0;
+  if (rb == 2 && rest && 2 * rest <= pairs) last = num_kb * tile_cost(bn, 1) * off1 * pair_kb_us(2 * rest, pairs);
+  // what is not hidden: start and last epilogue, and with one accumulator set the epilogue of every tile
+  const double bubble = 2 * rb * bn <= 512 ? 0.0 : 2.5;
+  return whole * (full + bubble) + last + 8.0;
 }
 
 static PlainPlan plain_plan(const DeviceState* d, int M, int N, int K, int elt, int swap_ab, int bn_override, int use_pair,
-                            int max_ctas, int sk_mode, bool have_scratch) {
+                            int max_ctas) {
   PlainPlan pl;
   memset(&pl, 0, sizeof(pl));
+  pl.rb = 1;
   const bool emu = emu_recorder().active;
-  const bool pair_ok = use_pair != 0 && pair_enabled() && !emu;
-  const bool free_choice = swap_ab < 0 && bn_override <= 0;
-  pl.swap = swap_ab < 0 ? (M <= 64 && N >= 128) : swap_ab != 0;
-  // Between one and two row tiles of 128 the tokens fit one 128-column tile of a pair: half the padding
-  // of a 256-row tile.
-  if (free_choice && pair_ok && M > 64 && M <= 128 && N >= 256) pl.swap = true;
-  const int rows = pl.swap ? N : M, cols = pl.swap ? M : N;
-  pl.bn = bn_override > 0 ? bn_override : (elt == 4 ? tf32_bn(cols) : pick_bn(cols));
-  if (free_choice && pair_ok) {
-    pl.pair = cols > 64 && rows > 128;
-    if (pl.pair) pl.bn = cols <= 128 ? 128 : 256;
-  } else {
-    pl.pair = pair_ok && !pl.swap && pl.bn == 256 && rows >= 256;
-  }
-  const int unit = pl.pair ? 256 : kBM;
-  pl.tiles_r = (rows + unit - 1) / unit;
-  pl.tiles_c = (cols + pl.bn - 1) / pl.bn;
-  pl.num_kb = (K + 128 / elt - 1) / (128 / elt);
   int cap = (int)grid_cap(d);
   if (max_ctas > 0 && max_ctas < cap) cap = max_ctas;
-  if (pl.pair && cap < 2) {
-    pl.pair = false;
-    pl.tiles_r = (rows + kBM - 1) / kBM;
+  const bool pair_ok = use_pair != 0 && pair_enabled() && !emu && cap >= 2;
+  const int num_kb = (K + 128 / elt - 1) / (128 / elt), pairs = cap / 2;
+  const bool lines = (long long)K * elt % 128 == 0;
+  const bool whole_chip = max_ctas <= 0 && !emu;
+  pl.swap = swap_ab < 0 ? (M <= 64 && N >= 128) : swap_ab != 0;
+  if (bn_override >= 1000 && pair_ok) {
+    pl.kind = PLAIN_FLOW;
+    pl.bn = bn_override % 1000;
+    pl.rb = bn_override / 1000;
+    pl.workers = pairs;
+    return pl;
   }
-  // An explicit layout is taken as given (its tests compare kernels bit by bit); parts of tiles are
-  // summed in another order than whole ones.
-  if (emu || (sk_mode < 0 && !free_choice)) sk_mode = 0;
-  if ((sk_mode < 0 && max_ctas <= 0) || sk_mode >= 10) {
-    pl.splits = tile_gemm_splits(d, pl.tiles_r * pl.tiles_c, pl.num_kb, pl.bn, pl.pair, elt);
-    if (sk_mode > 10) pl.splits = std::min(pl.splits, sk_mode - 10);
+  if (swap_ab < 0 && bn_override <= 0 && pair_ok && std::min(M, N) > 64 && std::max(M, N) > 128) {
+    // the whole choice is open: both orientations, every tile width, one wave with K splits or many
+    double best = 1e30;
+    for (int swap = 0; swap < 2; ++swap) {
+      const int rows = swap ? N : M, cols = swap ? M : N;
+      if (rows <= 128) continue;
+      for (int bn = 128; bn <= 256; bn += 32) {
+        if (bn > 128 && bn - 32 >= cols) continue;                   // wider than needed
+        if (whole_chip && (bn == 128 || bn == 256)) {
+          const int tiles = ((rows + 255) / 256) * ((cols + bn - 1) / bn);
+          double us = 1e30;
+          const int s = tiles <= pairs ? tile_gemm_splits(d, tiles, num_kb, bn, true, elt, lines ? 1.0 : 1.2, &us) : 0;
+          if (s > 0 && us < best) {
+            best = us;
+            pl.kind = PLAIN_TILE; pl.swap = swap != 0; pl.pair = true; pl.bn = bn; pl.splits = s;
+          }
+        }
+        for (int rb = 1; rb <= 2; ++rb) {
+          if (rb == 2 && rows <= 256) continue;
+          // a transposed store writes shorter runs: row-major unless the other way saves something
+          const double us = flow_us(rows, cols, num_kb, bn, rb, pairs, lines) * (swap ? 1.02 : 1.0);
+          if (us < best) {
+            best = us;
+            pl.kind = PLAIN_FLOW; pl.swap = swap != 0; pl.bn = bn; pl.rb = rb; pl.splits = 0; pl.workers = pairs;
+          }
+        }
+      }
+    }
+    if (best < 1e30) return pl;
+  }
+  const int rows = pl.swap ? N : M, cols = pl.swap ? M : N;
+  pl.bn = bn_override > 0 ? bn_override : (elt == 4 && !(pair_ok && cols > 64) ? tf32_bn(cols) : pick_bn(cols));
+  if (pair_ok && pl.bn == 256 && rows >= 256) {
+    pl.kind = PLAIN_FLOW;
+    pl.workers = pairs;
+    return pl;
+  }
+  if (elt == 4 && pl.bn == 128) pl.bn = 256;
+  const int tiles = ((rows + kBM - 1) / kBM) * ((cols + pl.bn - 1) / pl.bn);
+  if (swap_ab < 0 && bn_override <= 0 && whole_chip && tiles <= d->num_sms) {
+    pl.splits = tile_gemm_splits(d, tiles, num_kb, pl.bn, false, elt, 1.0, nullptr);
     if (pl.splits > 0) {
-      pl.workers = pl.tiles_r * pl.tiles_c;
+      pl.kind = PLAIN_TILE;
       return pl;
     }
   }
-  deal_tiles(pl, pl.pair ? cap / 2 : cap, have_scratch ? sk_mode : 0);
-  if (pl.sk_tiles > 0) {
-    pl.slot_bytes = sk_slot_bytes(pl);
-    pl.counters = (size_t)pl.sk_tiles * (pl.pair ? 2 : 1) * 4;
-  }
+  pl.kind = PLAIN_SINGLE;
+  pl.workers = std::min(tiles, cap);
   return pl;
 }
 
 // The plan of a problem, remembered per thread for the shapes a program repeats (a decode step calls the
-// same few again and again; working a plan out takes about a microsecond).
-static const PlainPlan& known_plan(const DeviceState* d, int M, int N, int K, int elt, int swap_ab, int bn_override, int use_pair,
-                                   int max_ctas, int sk_mode, bool have_scratch) {
+// same few again and again; working a plan out takes microseconds).
+static PlainPlan known_plan(const DeviceState* d, int M, int N, int K, int elt, int swap_ab, int bn_override, int use_pair,
+                            int max_ctas) {
   struct Entry {
-    int key[11];
+    int key[10];
     PlainPlan plan;
   };
   static thread_local Entry table[64];
-  const int key[11] = {1, d->device, M, N, K, elt, swap_ab, bn_override, use_pair, max_ctas, sk_mode * 2 + (have_scratch ? 1 : 0)};
+  if (emu_recorder().active) return plain_plan(d, M, N, K, elt, swap_ab, bn_override, use_pair, max_ctas);
+  const int key[10] = {1, d->device, M, N, K, elt, swap_ab, bn_override, use_pair, max_ctas};
   unsigned h = 2166136261u;
   for (int k : key) h = (h ^ (unsigned)k) * 16777619u;
   Entry& e = table[(h ^ (h >> 15)) % 64];
-  if (emu_recorder().active || memcmp(e.key, key, sizeof(key)) != 0) {
-    e.plan = plain_plan(d, M, N, K, elt, swap_ab, bn_override, use_pair, max_ctas, sk_mode, have_scratch);
+  if (memcmp(e.key, key, sizeof(key)) != 0) {
+    e.plan = plain_plan(d, M, N, K, elt, swap_ab, bn_override, use_pair, max_ctas);
     memcpy(e.key, key, sizeof(key));
-    if (emu_recorder().active) e.key[0] = 0;       // an emulated launch is planned for fewer CTAs
   }
   return e.plan;
 }
@@ -174,56 +166,44 @@ static int launch_plain(const GemmParams& p, unsigned ctas, unsigned threads, cu
   void* args[] = {(void*)&p};
   return launch_overlapped((const void*)gemm_plain_kernel<BN, ELT>, ctas, threads, args, GemmCfg<BN>::SMEM, stream);
 }
-template <int BN, int ELT>
-static int launch_plain_pair(const GemmParams& p, unsigned ctas, unsigned threads, cudaStream_t stream) {
-  void* args[] = {(void*)&p};
-  return launch_overlapped((const void*)gemm_plain_pair_kernel<BN, ELT>, ctas, threads, args, PairCfgT<BN>::SMEM, stream, 2);
-}
 
 }  // namespace kraken
 
 using namespace kraken;
 
-// Scratch a call with these arguments needs: bytes of partial-sum slots (0: none) and counter words.
+// Counter words a call with these arguments needs (0: none).
 KR_API int kr_gemm_scratch(int M, int N, int K, int in_fp32, int swap_ab, int bn_override, int use_pair, int max_ctas,
-                           int sk_mode, unsigned long long* slot_bytes, unsigned long long* counter_words) {
+                           unsigned long long* counter_words) {
   DeviceState* d = device_state();
   if (!d) return KR_FAIL_CUDA;
   KR_REQUIRE(M >= 1 && N >= 1 && K >= 1, "GEMM needs positive sizes");
-  const PlainPlan& pl = known_plan(d, M, N, K, in_fp32 ? 4 : 2, swap_ab, bn_override, use_pair, max_ctas, sk_mode, true);
-  *slot_bytes = pl.slot_bytes;
-  *counter_words = pl.counters;
+  *counter_words = known_plan(d, M, N, K, in_fp32 ? 4 : 2, swap_ab, bn_override, use_pair, max_ctas).kind == PLAIN_FLOW ? 2 : 0;
   return KR_SUCCESS;
 }
 
 // out[M,N] (bf16 or fp32, row stride ldo) = act(a[M,K] (row stride lda) * bt[N,K]^T (row stride ldb)).
 // act: 0 none, 1 GELU (tanh form), on the fp32 sums.
-// swap_ab: -1 auto (weights on the 128-row side when M <= 64), 0/1 forced.
-// use_pair: 0 forces the single-CTA kernel, anything else lets eligible shapes use CTA pairs.
+// swap_ab: -1 auto, 0/1 forced (1: the weights are the row operand).
+// bn_override: 0 auto, 16 ... 256 a column tile, 1000 * b + n persistent pairs with b row blocks x n columns.
+// use_pair: 0 forces the single-CTA kernels, anything else lets eligible shapes use CTA pairs.
 // in_fp32: a and bt hold fp32 and are multiplied as tf32 (strides in elements).
-// sk_mode: -1 auto, 0 whole tiles only, 1 / 2 forced. slots / counters: scratch as kr_gemm_scratch
-// says for the same arguments (counters zero, zero again after the call; nothing else may use either
-// while the call runs), or nullptr: whole tiles only.
+// counters: as many zero words as kr_gemm_scratch says for the same arguments (zero again after the call;
+// nothing else may use them while it runs), or nullptr: tiles are dealt in fixed shares.
 // copy_dst: when not nullptr, receives a copy of a (which then has to be contiguous).
 KR_API int kr_gemm(const void* a, long long lda, const void* bt, long long ldb, void* out, long long ldo, int M, int N, int K,
-                   int out_fp32, int act, int swap_ab, int bn_override, int max_ctas, int use_pair, int in_fp32, int sk_mode,
-                   void* slots, unsigned long long slot_bytes, uint32_t* counters, unsigned long long counter_words,
-                   void* copy_dst, cudaStream_t stream) {
+                   int out_fp32, int act, int swap_ab, int bn_override, int max_ctas, int use_pair, int in_fp32,
+                   uint32_t* counters, void* copy_dst, cudaStream_t stream) {
   DeviceState* d = device_state();
   if (!d) return KR_FAIL_CUDA;
   KR_REQUIRE(M >= 1 && N >= 1, "GEMM needs positive sizes");
   const int elt = in_fp32 ? 4 : 2;
-  // a problem that needs no scratch has the same plan with and without
-  PlainPlan pl = known_plan(d, M, N, K, elt, swap_ab, bn_override, use_pair, max_ctas, sk_mode, true);
-  if (pl.sk_tiles > 0 && (slots == nullptr || counters == nullptr))
-    pl = known_plan(d, M, N, K, elt, swap_ab, bn_override, use_pair, max_ctas, sk_mode, false);
-  KR_REQUIRE(slot_bytes >= pl.slot_bytes && counter_words >= pl.counters, "GEMM scratch too small");
+  const PlainPlan pl = known_plan(d, M, N, K, elt, swap_ab, bn_override, use_pair, max_ctas);
+  const bool pair = pl.kind == PLAIN_FLOW || pl.pair;
   GemmParams p;
   memset(&p, 0, sizeof(p));
   int bn = 0;
-  int rc = setup_problem(p, a, lda, bt, ldb, M, N, K, pl.swap, pl.bn, &bn, elt, pl.pair ? pl.bn / 2 : pl.bn);
+  int rc = setup_problem(p, a, lda, bt, ldb, M, N, K, pl.swap, pl.bn, &bn, elt, pair ? pl.bn / 2 : pl.bn);
   if (rc) return rc;
-  if (in_fp32) KR_REQUIRE(bn == 16 || bn == 64 || bn == 256 || pl.splits > 0 || (pl.pair && bn == 128), "tf32 GEMM supports column tiles of 16, 64 and 256");
   p.mode = GEMM_PLAIN;
   p.out = out;
   p.ldo = ldo;
@@ -233,34 +213,26 @@ KR_API int kr_gemm(const void* a, long long lda, const void* bt, long long ldb, 
   p.act = act;
   p.ws = 1;
   p.sync = sync_ctx(d);
-  p.sk_tiles = pl.sk_tiles;
-  p.sk_slots = (float*)slots;
-  p.sk_counters = counters;
   if (copy_dst != nullptr) {
     KR_REQUIRE(lda == K && ((uintptr_t)copy_dst & 15) == 0 && ((unsigned long long)M * K * elt) % 16 == 0, "the copied operand must be contiguous and 16-byte aligned");
     p.cp_src = a;
     p.cp_dst = copy_dst;
     p.cp_bytes = (unsigned long long)M * K * elt;
   }
-  const unsigned threads = copy_dst != nullptr ? kPlainThreads : kGemmThreads;
-  if (!pl.swap && !out_fp32 && bn >= 64) p.use_tma_store = store_tmap(out, M, N, ldo, &p.tmap_out[0]) ? 1 : 0;
-  if (pl.splits > 0) {
-    p.tiles_r = pl.tiles_r;
+  if (pl.kind == PLAIN_FLOW) return launch_flow_gemm(p, bn, pl.rb, pl.workers, counters, stream);
+  if (pl.kind == PLAIN_TILE) {
+    if (pl.pair) p.tiles_r = (p.rows_r + 255) / 256;
     return launch_tile_gemm(p, bn, pl.pair, pl.splits, stream);
   }
-  const unsigned ctas = (unsigned)pl.workers * (pl.pair ? 2 : 1);
+  const unsigned threads = copy_dst != nullptr ? kPlainThreads : kGemmThreads, ctas = (unsigned)pl.workers;
+  if (!pl.swap && !out_fp32 && bn >= 64) p.use_tma_store = store_tmap(out, M, N, ldo, &p.tmap_out[0]) ? 1 : 0;
   p.num_mma_ctas = (int)ctas;
-  if (pl.pair) {
-    p.tiles_r = pl.tiles_r;
-    p.group_r = std::max(1, p.group_r / 2);
-    if (in_fp32) return bn == 128 ? launch_plain_pair<128, 4>(p, ctas, threads, stream) : launch_plain_pair<256, 4>(p, ctas, threads, stream);
-    return bn == 128 ? launch_plain_pair<128, 2>(p, ctas, threads, stream) : launch_plain_pair<256, 2>(p, ctas, threads, stream);
-  }
   if (in_fp32) {
     switch (bn) {
       case 256: return launch_plain<256, 4>(p, ctas, threads, stream);
       case 64: return launch_plain<64, 4>(p, ctas, threads, stream);
-      default: return launch_plain<16, 4>(p, ctas, threads, stream);
+      case 16: return launch_plain<16, 4>(p, ctas, threads, stream);
+      default: return fail(KR_FAIL_ARG, "tf32 GEMM supports column tiles of 16, 64 and 256");
     }
   }
   switch (bn) {
@@ -272,10 +244,9 @@ KR_API int kr_gemm(const void* a, long long lda, const void* bt, long long ldb, 
   }
 }
 
-// The same without scratch, activation or copy: whole tiles only.
+// The same without counters, activation or copy.
 KR_API int kr_gemm_bf16(const void* a, long long lda, const void* bt, long long ldb, void* out, long long ldo, int M,
                         int N, int K, int out_fp32, int swap_ab, int bn_override, int max_ctas, int use_pair,
                         int in_fp32, cudaStream_t stream) {
-  return kr_gemm(a, lda, bt, ldb, out, ldo, M, N, K, out_fp32, 0, swap_ab, bn_override, max_ctas, use_pair, in_fp32, -1, nullptr, 0,
-                 nullptr, 0, nullptr, stream);
+  return kr_gemm(a, lda, bt, ldb, out, ldo, M, N, K, out_fp32, 0, swap_ab, bn_override, max_ctas, use_pair, in_fp32, nullptr, nullptr, stream);
 }

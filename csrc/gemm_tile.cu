@@ -15,6 +15,7 @@
 // staging layouts: [unit of four columns][row] for a transposed store, [row][unit] with the units of a row
 // permuted by the row number (no bank conflicts for the row-per-lane writes) for a row-major one.
 #include <algorithm>
+#include <cmath>
 #include <map>
 #include <mutex>
 #include "kraken/gemm_host.h"
@@ -53,9 +54,6 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
   float4 v;
   asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
   return v;
-}
-__device__ __forceinline__ void st_shared_u4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 __device__ __forceinline__ uint32_t cluster_size() {
   uint32_t r;
@@ -375,28 +373,31 @@ static int max_clusters(int device, const TileVariant& v, unsigned cluster) {
   return n;
 }
 
-// The split count of a one-wave problem, 0 when its tiles do not fit the chip at once. Times in us as
-// measured: K blocks at the rate the MMAs (256-column pairs 0.30 per block) or the operand loads (0.18,
-// single CTAs 0.25) allow, but never below the operands' time out of HBM, plus what summing S splits
-// adds: little for the narrow tiles of single CTAs, a lot once a cluster of pairs spans more than four
-// CTAs (M = 256, N = 4096, K = 2048: 1 / 2 / 3 splits 17.5 / 14.2 / 20.5 us).
-int tile_gemm_splits(const DeviceState* d, int tiles, int num_kb, int bn, bool pair, int elt) {
+// The split count of a one-wave problem, 0 when its tiles do not fit the chip at once, and its time (us).
+// Times as measured: K blocks at the rate the MMAs (256-column pairs 0.30 per block at full clock, more
+// when the chip is full and power-limited) or the operand loads (0.18-0.28, single CTAs 0.25) allow, but
+// never below the operands' time out of HBM, plus what summing S splits adds: little for the narrow tiles
+// of single CTAs, a lot once a cluster of pairs spans more than four CTAs (M = 256, N = 4096, K = 2048:
+// 1 / 2 / 3 splits 17.5 / 14.2 / 20.5 us).
+int tile_gemm_splits(const DeviceState* d, int tiles, int num_kb, int bn, bool pair, int elt, double off_line, double* us_out) {
   const TileVariant v = elt == 4 ? tile_variant<4>(bn, pair) : tile_variant<2>(bn, pair);
   if (v.fn == nullptr) return 0;
   const int ctas = pair ? 2 : 1, most = 8 / ctas;
-  const double kb_us = !pair ? 0.25 : (bn == 256 ? 0.30 : 0.18);
   const double hbm_us = (double)tiles * ctas * num_kb * kBM * 128 / 6.5e6;
   auto sum_us = [&](int s) { return !pair ? 0.25 * s : (s <= 2 ? 1.5 * s : 4.0 * s - 2.0) * bn / 256; };
   int best = 0;
   double best_us = 1e30;
   for (int s = 1; s <= most && (s == 1 || num_kb >= 4 * s); ++s) {
     if (tiles * s * ctas > d->num_sms || tiles > max_clusters(d->device, v, (unsigned)(s * ctas))) continue;
-    const double us = std::max((num_kb + s - 1) / s * kb_us, hbm_us) + sum_us(s);
+    const double busy = (double)tiles * s * ctas / d->num_sms;
+    const double kb_us = !pair ? 0.25 : std::max(0.30, 0.47 * std::sqrt(busy)) * (bn == 256 ? 1.0 : 0.59) * off_line;
+    const double us = std::max((num_kb + s - 1) / s * kb_us, hbm_us) + sum_us(s) + 8.0;
     if (us < best_us) {
       best_us = us;
       best = s;
     }
   }
+  if (us_out) *us_out = best_us;
   return best;
 }
 

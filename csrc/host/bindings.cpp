@@ -26,9 +26,9 @@ struct Api {
   int (*rms_norm)(const void*, const void*, void*, int, int, float, void*);
   int (*local_bias_rms_norm)(const void*, int, const void*, u64, const void*, void*, int, int, float, int, void*);
   int (*local_all_reduce)(const void*, void*, const void*, u64, u64, void*);
-  int (*gemm_scratch)(int, int, int, int, int, int, int, int, int, u64*, u64*);
+  int (*gemm_scratch)(int, int, int, int, int, int, int, int, u64*);
   int (*gemm)(const void*, long long, const void*, long long, void*, long long, int, int, int, int, int, int, int, int, int, int,
-              int, void*, u64, uint32_t*, u64, void*, void*);
+              uint32_t*, void*, void*);
 };
 Api api;
 PyObject* g_error = nullptr;
@@ -57,13 +57,13 @@ bool aligned(const at::Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_p
 bool plain_bf16(const at::Tensor& t) { return t.scalar_type() == at::kBFloat16 && t.is_contiguous() && aligned(t); }
 bool fits_int(int64_t v) { return v >= 1 && v < (int64_t(1) << 31); }
 
-// ---- scratch of GEMMs whose tiles are computed in parts ------------------------------------------
-// Arrival counters are zero between launches, so one small buffer per stream serves every call on it (calls
-// on one stream never overlap). The partial sums come from torch's caching allocator call by call. At most
-// kMaxStreams buffers are kept; a dropped one goes back to the allocator, which hands it out again in
-// stream order. Under stream capture the buffer is allocated and zeroed inside the graph.
+// ---- counters of GEMMs that draw their tiles ------------------------------------------------------
+// They are zero between launches, so one small buffer per stream serves every call on it (calls on one
+// stream never overlap). At most kMaxStreams buffers are kept; a dropped one goes back to torch's caching
+// allocator, which hands it out again in stream order. Under stream capture the buffer is allocated and
+// zeroed inside the graph.
 constexpr size_t kMaxStreams = 32;
-constexpr int64_t kCounterWords = 4096;
+constexpr int64_t kCounterWords = 32;
 std::mutex g_pool_mu;
 std::map<std::pair<int, void*>, at::Tensor> g_pool;
 
@@ -103,17 +103,13 @@ int run_gemm(const at::Tensor& a, const at::Tensor& bt, int64_t N, int64_t ldb, 
   const int64_t M = a.size(0), K = a.size(1);
   const bool fp32 = a.scalar_type() == at::kFloat;
   out = at::detail::empty_cuda({M, N}, out_fp32 ? at::kFloat : at::kBFloat16, a.device(), std::nullopt);
-  u64 slot_bytes = 0, words = 0;
-  int rc = api.gemm_scratch((int)M, (int)N, (int)K, fp32, swap, bn, pair, max_ctas, -1, &slot_bytes, &words);
+  u64 words = 0;
+  int rc = api.gemm_scratch((int)M, (int)N, (int)K, fp32, swap, bn, pair, max_ctas, &words);
   if (rc) return rc;
-  at::Tensor slots, counters;
-  if (slot_bytes) {
-    slots = at::detail::empty_cuda({(int64_t)slot_bytes}, at::kByte, a.device(), std::nullopt);
-    counters = counters_for(a.device().index(), stream, (int64_t)words);
-  }
+  at::Tensor counters;
+  if (words) counters = counters_for(a.device().index(), stream, (int64_t)words);
   return api.gemm(a.data_ptr(), a.stride(0), bt.data_ptr(), ldb, out.data_ptr(), N, (int)M, (int)N, (int)K, out_fp32, act, swap, bn, max_ctas,
-                  pair, fp32, -1, slot_bytes ? slots.data_ptr() : nullptr, slot_bytes,
-                  slot_bytes ? (uint32_t*)counters.data_ptr() : nullptr, words, copy_dst, (void*)stream.stream());
+                  pair, fp32, words ? (uint32_t*)counters.data_ptr() : nullptr, copy_dst, (void*)stream.stream());
 }
 
 // gemm(a, b, out_fp32, act, tf32, swap_ab, bn, max_ctas, pair, copy_dst): act(a @ b). a [M, K] with K contiguous, b

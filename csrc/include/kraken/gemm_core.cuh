@@ -118,14 +118,9 @@ struct alignas(64) GemmParams {
   int rs_algo;               // 0: push, owner reduces in its epilogue; 1: pull; 2: scatter (push + reducer warps)
   int rs_sub_rows;           // pull / scatter: rows of one reduce work item (power of two, 16 ... 128)
   uint32_t rs_done_off;      // pull / scatter: words from a tile's arrival counter to its "items done" counter
-  // Stream-K (plain GEMM): tiles [0, sk_tiles) are cut into K-block units that are dealt evenly to all
-  // workers, the rest are computed whole (see WorkIter). Partial tiles meet in sk_slots, see sk_meet.
-  int sk_tiles;
-  float* sk_slots;           // [2 * workers][CTAs per worker][4 warps][BN * 32] fp32
-  uint32_t* sk_counters;     // [sk_tiles][CTAs per worker][4 warps] arrivals (zero, self-resetting)
   int act;                   // activation applied to the fp32 result before it is rounded: 0 none, 1 GELU (tanh form)
-  // Plain GEMM launched with kCopyThreads more threads: the extra warps copy the row operand
-  // (cp_bytes bytes, a multiple of 16) from cp_src to cp_dst while the tiles are computed.
+  // Plain GEMM: warps without another role copy the row operand (cp_bytes bytes, a multiple of 16) from
+  // cp_src to cp_dst while the tiles are computed.
   const void* cp_src;
   void* cp_dst;
   unsigned long long cp_bytes;
@@ -185,14 +180,9 @@ __device__ __forceinline__ void trace_put(const GemmParams& p, int role, int slo
     p.trace[(((size_t)blockIdx.x * kTraceRoles + role) * kTraceTiles + slot) * kTraceFields + field] = globaltimer_ns();
 }
 
-// The work of one CTA (or CTA pair) as a sequence of (tile, K-block range) items. First its share of
-// the stream-K units: units of one K block, tile-major over tiles [0, sk_tiles), cut into equal
-// contiguous ranges, so every worker gets the same number of K blocks (+-1) and touches at most two
-// tiles in part. Then whole tiles sk_tiles + worker, + workers, ... (with k_splits > 1: split items,
-// split-major, so that one wave of CTAs covers every tile once). The stream-K part comes first so that
-// its partial sums meet in the epilogue warps while the MMAs of whole tiles run.
+// The work of one CTA (or CTA pair): tiles worker, worker + workers, ... With k_splits > 1 items are
+// (split, tile), split-major, so that one wave of CTAs covers every tile once.
 struct WorkIter {
-  int u, u_end;
   int t, stride, total, tiles_rc, ksp, num_kb;
   __device__ __forceinline__ WorkIter(const GemmParams& p, int worker, int workers, int num_kb_) {
     num_kb = num_kb_;
@@ -200,23 +190,9 @@ struct WorkIter {
     ksp = p.k_splits > 1 ? p.k_splits : 1;
     total = tiles_rc * ksp;
     stride = workers;
-    u = u_end = 0;
-    if (p.sk_tiles > 0) {
-      const long long units = (long long)p.sk_tiles * num_kb;
-      u = (int)(units * worker / workers);
-      u_end = (int)(units * (worker + 1) / workers);
-    }
-    t = p.sk_tiles + worker;
+    t = worker;
   }
   __device__ __forceinline__ bool next(int& tile, int& split, int& kb_lo, int& kb_hi) {
-    split = 0;
-    if (u < u_end) {
-      tile = u / num_kb;
-      kb_lo = u - tile * num_kb;
-      kb_hi = min(num_kb, kb_lo + (u_end - u));
-      u += kb_hi - kb_lo;
-      return true;
-    }
     if (t >= total) return false;
     split = ksp > 1 ? t / tiles_rc : 0;
     tile = t - split * tiles_rc;
@@ -246,7 +222,6 @@ __device__ __forceinline__ void epi_bar_sync() { asm volatile("bar.sync 1, 128;"
 //   side_role (work of the warps beyond the six pipeline warps, if the launch has any),
 //   helper_role (what the six pipeline warps do after their last tile, before the teardown).
 struct HookDefaults {
-  static constexpr bool kStreamK = false;   // whether this kernel's tiles may be computed in parts (GemmParams::sk_tiles)
   static constexpr bool kOverlap = false;   // whether the kernel is launched with launch_overlapped()
   static constexpr bool kAct = false;       // whether its epilogue can apply an activation (GemmParams::act)
   int k_split = 0;           // which K split the tile in hand belongs to (set by the main loop)
@@ -279,101 +254,6 @@ struct TileDest {
   int ll_dst = -1;
 };
 
-// ---- stream-K: partial tiles ------------------------------------------------------------------
-// A tile whose K blocks are split over several workers is summed by whichever of them finishes last
-// (per epilogue warp, i.e. per 32 rows: no barrier wider than a warp). Every contributor stores its
-// fp32 partial sums in a slot of its own and counts itself in with one acquire-release atomic; the one
-// that completes the count adds the slots up IN K ORDER, own slot included, so the result does not
-// depend on who was last. Nobody ever waits for another CTA. The slots (and the count) stay in L2.
-struct SkTile {
-  int first = 0, n = 0;      // contributing workers [first, first + n); n == 0: sums come from TMEM
-  const char* base = nullptr;      // this warp's rows in slot 0
-  size_t slot_bytes = 0;
-};
-
-// Slot of a contributor: a worker touches at most two tiles in part, the one its range starts inside
-// (slot 2w) and the one its range ends inside (2w + 1: it is that tile's first contributor).
-__device__ __forceinline__ int sk_slot(const SkTile& t, int i) { return 2 * (t.first + i) + (i == 0 ? 1 : 0); }
-
-// Stores this warp's partial sums, hands the accumulator back and counts the warp in. True when this
-// warp completes the tile and has to sum the slots (described by `st`).
-template <int BN, bool PAIR>
-__device__ __forceinline__ bool sk_meet(const GemmParams& p, int tile, int kb_lo, int num_kb, int worker, int workers,
-                                        uint32_t t_addr, int q, int cta, int lane, uint32_t tempty_addr, SkTile& st) {
-  constexpr int CTAS = PAIR ? 2 : 1;
-  constexpr int CH = BN < 32 ? BN : 32;
-  const long long units = (long long)p.sk_tiles * num_kb;
-  // owner of unit u: the largest w with floor(w * units / workers) <= u
-  const int first = (int)((((long long)tile * num_kb + 1) * workers - 1) / units);
-  const int last = (int)(((long long)(tile + 1) * num_kb * workers - 1) / units);
-  st.first = first;
-  st.n = last - first + 1;
-  st.slot_bytes = (size_t)CTAS * 4 * 32 * BN * 4;
-  st.base = (const char*)p.sk_slots + (size_t)(cta * 4 + q) * 32 * BN * 4;
-  char* mine = const_cast<char*>(st.base) + st.slot_bytes * (2 * worker + (kb_lo == 0 ? 1 : 0));
-#pragma unroll 1
-  for (int c0 = 0; c0 < BN; c0 += CH) {
-    uint32_t r[32];
-    if (CH == 32) tmem_ld32(t_addr + c0, r);
-    else tmem_ld16(t_addr + c0, r);
-    tmem_ld_wait();
-    if (c0 + CH >= BN) {
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) { if (PAIR) mbar_arrive_cluster(tempty_addr); else mbar_arrive(tempty_addr); }
-    }
-#pragma unroll
-    for (int u = 0; u < CH / 4; ++u)
-      st16(mine + ((size_t)(c0 / 4 + u) * 32 + lane) * 16, U4{r[4 * u], r[4 * u + 1], r[4 * u + 2], r[4 * u + 3]});
-  }
-  __syncwarp();
-  uint32_t* cnt = p.sk_counters + ((size_t)tile * CTAS + cta) * 4 + q;
-  uint32_t old = 0;
-  if (lane == 0) {
-    old = atom_add_acqrel_gpu(cnt, 1u);
-    if (old == (uint32_t)(st.n - 1)) *cnt = 0;       // for the next launch on this stream
-  }
-  old = __shfl_sync(0xffffffffu, old, 0);
-  return old == (uint32_t)(st.n - 1);
-}
-
-// Columns [col, col + CH) of this lane's row, summed over the contributors; the loads of two slots
-// are in flight together.
-template <int CH>
-__device__ __forceinline__ void sk_sum(const SkTile& st, int col, int lane, uint32_t (&r)[32]) {
-  const size_t off = ((size_t)(col / 4) * 32 + lane) * 16;
-  float f[CH];
-#pragma unroll
-  for (int j = 0; j < CH; ++j) f[j] = 0.f;
-#pragma unroll 1
-  for (int i = 0; i < st.n; i += 2) {
-    U4 x[CH / 4], y[CH / 4];
-    const char* a = st.base + st.slot_bytes * sk_slot(st, i) + off;
-    const char* b = st.base + st.slot_bytes * sk_slot(st, i + 1) + off;
-    const bool two = i + 1 < st.n;
-#pragma unroll
-    for (int u = 0; u < CH / 4; ++u) x[u] = ld16(a + (size_t)u * 512);
-    if (two) {
-#pragma unroll
-      for (int u = 0; u < CH / 4; ++u) y[u] = ld16(b + (size_t)u * 512);
-    }
-#pragma unroll
-    for (int u = 0; u < CH / 4; ++u) {
-      f[4 * u] += __uint_as_float(x[u].x); f[4 * u + 1] += __uint_as_float(x[u].y);
-      f[4 * u + 2] += __uint_as_float(x[u].z); f[4 * u + 3] += __uint_as_float(x[u].w);
-    }
-    if (two) {
-#pragma unroll
-      for (int u = 0; u < CH / 4; ++u) {
-        f[4 * u] += __uint_as_float(y[u].x); f[4 * u + 1] += __uint_as_float(y[u].y);
-        f[4 * u + 2] += __uint_as_float(y[u].z); f[4 * u + 3] += __uint_as_float(y[u].w);
-      }
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < CH; ++j) r[j] = __float_as_uint(f[j]);
-}
-
 // Epilogue of one tile, run by the four epilogue warps: TMEM -> registers -> (hook: add peers'
 // partial sums) -> convert -> swizzled staging in shared memory -> coalesced global stores.
 // `tempty_addr` is the mbarrier that returns the accumulator to the MMA issuer: a local barrier,
@@ -381,25 +261,21 @@ __device__ __forceinline__ void sk_sum(const SkTile& st, int col, int lane, uint
 template <int BN, bool PAIR, class Hooks>
 __device__ __forceinline__ bool gemm_epilogue_tile(const GemmParams& p, Hooks& hooks, int tr, int tc, int acc,
                                                    uint32_t tmem_base, int q, int lane, unsigned char* stg,
-                                                   uint32_t tempty_addr, bool defer, const SkTile& sk = SkTile()) {
+                                                   uint32_t tempty_addr, bool defer) {
   if (!hooks.begin_tile(p, tr, tc, q, lane)) return false;
   TileDest dst = hooks.tile_dest(p, tr, tc);
   const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN);
   constexpr int kChunk = BN < 32 ? BN : 32;
-  // One chunk of columns of this lane's row: out of TMEM (the last chunk hands the accumulator back to
-  // the MMA issuer, before the global stores), or out of the slots of a tile computed in parts.
+  // One chunk of columns of this lane's row out of TMEM; the last chunk hands the accumulator back to
+  // the MMA issuer, before the global stores.
   auto load_chunk = [&](int col, bool last, uint32_t (&r)[32]) {
-    if (Hooks::kStreamK && sk.n > 0) {
-      sk_sum<kChunk>(sk, col, lane, r);
-    } else {
-      if (kChunk == 32) tmem_ld32(t_addr + col, r);
-      else tmem_ld16(t_addr + col, r);
-      tmem_ld_wait();
-      if (last) {
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) { if (PAIR) mbar_arrive_cluster(tempty_addr); else mbar_arrive(tempty_addr); }
-      }
+    if (kChunk == 32) tmem_ld32(t_addr + col, r);
+    else tmem_ld16(t_addr + col, r);
+    tmem_ld_wait();
+    if (last) {
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) { if (PAIR) mbar_arrive_cluster(tempty_addr); else mbar_arrive(tempty_addr); }
     }
     if (Hooks::kAct && p.act != 0) {
 #pragma unroll
@@ -705,12 +581,7 @@ __device__ __forceinline__ void gemm_mainloop(const GemmParams& p, unsigned bid,
         prev_tr = -1;
         if (!ok) break;
       }
-      SkTile sk;
-      if (Hooks::kStreamK && kb_hi - kb_lo < num_kb) {
-        const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN);
-        if (!sk_meet<BN, false>(p, tile, kb_lo, num_kb, (int)bid, (int)nb, t_addr, q, 0, lane, tempty_bar(acc), sk)) continue;
-      }
-      ok = gemm_epilogue_tile<BN, false>(p, hooks, tr, tc, acc, tmem_base, q, lane, stg, tempty_bar(acc), defer, sk);
+      ok = gemm_epilogue_tile<BN, false>(p, hooks, tr, tc, acc, tmem_base, q, lane, stg, tempty_bar(acc), defer);
       if (!ok) break;
       if (q == 0 && lane == 0) trace_put(p, 1, it, 1);
       if (defer) {
@@ -759,27 +630,22 @@ __device__ __forceinline__ void gemm_mainloop(const GemmParams& p, unsigned bid,
 //   tfull[a]   one per CTA, 1 arrival: same double commit
 //   tempty[a]  in the leader, 8 arrivals: the four epilogue warps of each CTA
 // ---------------------------------------------------------------------------------------------
-template <int BN_>
-struct PairCfgT {
-  static constexpr int BN = BN_;                      // pair tile: 256 rows x BN columns
-  static constexpr int A_BYTES = kBM * kBK * 2;       // this CTA's 128 rows of the row operand
-  static constexpr int B_BYTES = (BN / 2) * kBK * 2;  // this CTA's half of the column operand
+struct PairCfg {
+  static constexpr int BN = 256;                 // pair tile: 256 rows x 256 columns
+  static constexpr int A_BYTES = kBM * kBK * 2;  // this CTA's 128 rows of the row operand
+  static constexpr int B_BYTES = 128 * kBK * 2;  // this CTA's 128 rows of the column operand
   static constexpr int STAGE = A_BYTES + B_BYTES;
   static constexpr int EPI = 4 * kEpiWarpBytes;
-  static constexpr int STAGES = BN == 256 ? 6 : 8;
-  static constexpr int TMEM_COLS = 2 * BN;
+  static constexpr int STAGES = 6;
+  static constexpr int TMEM_COLS = 512;
   static constexpr int SMEM = 1024 + STAGES * STAGE + EPI + 512;
-  static_assert(SMEM <= kSmemLimit, "pair kernel shared memory");
-  static_assert(BN == 128 || BN == 256, "pair tiles are 128 or 256 columns wide");
 };
-using PairCfg = PairCfgT<256>;
+static_assert(PairCfg::SMEM <= kSmemLimit, "pair kernel shared memory");
 
-// ELT = bytes per operand element, as in the single-CTA main loop.
-template <class Hooks, int BN = 256, int ELT = 2>
+template <class Hooks>
 __device__ __forceinline__ void gemm_mainloop_pair(const GemmParams& p, unsigned pair_id, unsigned num_pairs,
                                                    Hooks& hooks, unsigned char* smem_raw) {
-  using Cfg = PairCfgT<BN>;
-  constexpr int kStageK = 128 / ELT;            // operand elements along K per stage
+  using Cfg = PairCfg;
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const uint32_t cta = cluster_ctarank();
@@ -821,7 +687,7 @@ __device__ __forceinline__ void gemm_mainloop_pair(const GemmParams& p, unsigned
     pdl_wait();
   }
 
-  const int num_kb = (p.K + kStageK - 1) / kStageK;
+  const int num_kb = (p.K + kBK - 1) / kBK;
   WorkIter work(p, (int)pair_id, (int)num_pairs, num_kb);   // tiles_r counts 256-row pair tiles here
   int tile, split, kb_lo, kb_hi;
 
@@ -849,8 +715,8 @@ __device__ __forceinline__ void gemm_mainloop_pair(const GemmParams& p, unsigned
           // its own empty barrier, which the leader signals after the MMAs that waited on full[s].
           if (leader) mbar_expect_tx(full_bar(s), 2 * (Cfg::A_BYTES + Cfg::B_BYTES));
           const uint32_t sa = stage0 + s * Cfg::STAGE;
-          tma_load_2d_pair(sa, rmap, lead_full, kb * kStageK, row0);
-          tma_load_2d_pair(sa + Cfg::A_BYTES, &p.tmap_c, lead_full, kb * kStageK, tc * BN + (int)cta * (BN / 2));
+          tma_load_2d_pair(sa, rmap, lead_full, kb * kBK, row0);
+          tma_load_2d_pair(sa + Cfg::A_BYTES, &p.tmap_c, lead_full, kb * kBK, tc * Cfg::BN + (int)cta * 128);
           if (++s == Cfg::STAGES) { s = 0; ph ^= 1u; }
         }
       }
@@ -858,7 +724,7 @@ __device__ __forceinline__ void gemm_mainloop_pair(const GemmParams& p, unsigned
   } else if (warp == 1) {
     // ================= MMA issuer (leader CTA only) =================
     if (leader && elect_one()) {
-      constexpr uint32_t idesc = ELT == 2 ? make_idesc_bf16(256, BN) : make_idesc_tf32(256, BN);
+      constexpr uint32_t idesc = make_idesc_bf16(256, Cfg::BN);
       uint32_t peer_empty[Cfg::STAGES], peer_tfull[2];
       for (int s = 0; s < Cfg::STAGES; ++s) peer_empty[s] = mapa_shared(empty_bar(s), 1);
       for (int a = 0; a < 2; ++a) peer_tfull[a] = mapa_shared(tfull_bar(a), 1);
@@ -873,7 +739,7 @@ __device__ __forceinline__ void gemm_mainloop_pair(const GemmParams& p, unsigned
         if (!ok) break;
         tc_fence_after();
         trace_put(p, 0, it, 0);
-        const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
+        const uint32_t d_tmem = tmem_base + (uint32_t)(acc * Cfg::BN);
         for (int kb = kb_lo; kb < kb_hi; ++kb) {
           ok = mbar_wait(full_bar(s), ph, p.sync, 46);
           if (!ok) break;
@@ -883,11 +749,8 @@ __device__ __forceinline__ void gemm_mainloop_pair(const GemmParams& p, unsigned
           const uint64_t adesc = make_smem_desc_sw128(sa);
           const uint64_t bdesc = make_smem_desc_sw128(sa + Cfg::A_BYTES);
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const uint32_t accumulate = (kb > kb_lo || k != 0) ? 1u : 0u;
-            if (ELT == 2) umma_bf16_pair(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, accumulate);
-            else umma_tf32_pair(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, accumulate);
-          }
+          for (int k = 0; k < kBK / 16; ++k)
+            umma_bf16_pair(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, (kb > kb_lo || k != 0) ? 1u : 0u);
           umma_commit_pair(empty_bar(s));      // own stage free
           umma_commit_pair(peer_empty[s]);     // peer's stage free
           if (++s == Cfg::STAGES) { s = 0; ph ^= 1u; }
@@ -931,12 +794,7 @@ __device__ __forceinline__ void gemm_mainloop_pair(const GemmParams& p, unsigned
         prev_tr = -1;
         if (!ok) break;
       }
-      SkTile sk;
-      if (Hooks::kStreamK && kb_hi - kb_lo < num_kb) {
-        const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN);
-        if (!sk_meet<BN, true>(p, tile, kb_lo, num_kb, (int)pair_id, (int)num_pairs, t_addr, q, (int)cta, lane, lead_tempty[acc], sk)) continue;
-      }
-      ok = gemm_epilogue_tile<BN, true>(p, hooks, tr, tc, acc, tmem_base, q, lane, stg, lead_tempty[acc], defer, sk);
+      ok = gemm_epilogue_tile<Cfg::BN, true>(p, hooks, tr, tc, acc, tmem_base, q, lane, stg, lead_tempty[acc], defer);
       if (!ok) break;
       if (q == 0 && lane == 0) trace_put(p, 1, it, 1);
       if (defer) {

@@ -6,7 +6,6 @@
 namespace kraken {
 
 struct PlainHooks : HookDefaults {
-  static constexpr bool kStreamK = true;
   static constexpr bool kOverlap = true;
   static constexpr bool kAct = true;
   int bn;

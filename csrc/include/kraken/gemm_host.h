@@ -10,7 +10,7 @@ namespace kraken {
 // elements per row), box = 128 bytes of columns x box_rows rows, 128-byte swizzle, out-of-range
 // elements read as zero. Cached.
 int get_tmap(const void* ptr, unsigned long long rows, unsigned long long cols, unsigned long long ld,
-             unsigned box_rows, CUtensorMap* out, int elt = 2);
+             unsigned box_rows, CUtensorMap* out, int elt = 2, unsigned box_bytes = 128);
 // Tensor map for TMA stores of bf16 tiles (box of 32 rows); false when the matrix cannot be
 // described to TMA or TMA stores are switched off.
 bool store_tmap(const void* ptr, long long rows, long long cols, long long ld, CUtensorMap* m);
@@ -26,8 +26,10 @@ int launch_gemm_ar(int bn, const GemmParams& p, unsigned nb, cudaStream_t stream
 // Routes a parameter block to the kernel family of its mode and operand type (gemm.cu).
 int launch_gemm(int bn, const GemmParams& p, unsigned nb, cudaStream_t stream);
 // One-wave GEMM (gemm_tile.cu): the most K splits with which `tiles` tiles of this kernel run at once,
-// 0 when it does not apply; and its launch.
-int tile_gemm_splits(const DeviceState* d, int tiles, int num_kb, int bn, bool pair, int elt);
+// 0 when it does not apply, and its estimated time (off_line: factor for rows off 128-byte lines); and its launch.
+int tile_gemm_splits(const DeviceState* d, int tiles, int num_kb, int bn, bool pair, int elt, double off_line, double* us);
+// Persistent pairs that draw their tiles in order (gemm_flow.cu); sched: two zero words, zero again afterwards.
+int launch_flow_gemm(const GemmParams& g, int bn, int rb, int pairs, uint32_t* sched, cudaStream_t stream);
 int launch_tile_gemm(const GemmParams& g, int bn, bool pair, int splits, cudaStream_t stream);
 int pick_bn(int rows_c);      // column-tile width for `rows_c` rows of the column operand
 int tf32_bn(int rows_c);      // the same among the widths the tf32 kernels exist for

@@ -59,7 +59,7 @@ def _gemm(a: torch.Tensor, b: torch.Tensor, out_fp32: bool, tf32: bool, swap_ab:
         return out
     out = torch.empty((M, N), dtype=torch.float32 if out_fp32 else torch.bfloat16, device=a.device)
     _lib.check(_lib.lib().kr_gemm(a2.data_ptr(), lda, bt.data_ptr(), ldb, out.data_ptr(), N, M, N, K, 1 if out_fp32 else 0, _ACT[act],
-                                  swap_ab, bn, max_ctas, pair, 1 if tf32 else 0, -1, None, 0, None, 0,
+                                  swap_ab, bn, max_ctas, pair, 1 if tf32 else 0, None,
                                   copy_dst.data_ptr() if copy_dst is not None else None, _lib.current_stream_ptr()))
     return out
 

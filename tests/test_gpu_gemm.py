@@ -440,3 +440,20 @@ def test_one_rank_all_gather_matmul_and_activation(M, N, K):
     _close(c, ref, K)
     h = all_gather_matmul_act(x, bt.t(), "gelu_tanh")
     _close(h, torch.nn.functional.gelu(ref, approximate="tanh"), K)
+
+
+@pytest.mark.parametrize("bn", [1128, 1160, 1192, 1224, 1256, 2128, 2160, 2192, 2224, 2256])
+@pytest.mark.parametrize("swap", [0, 1])
+def test_gemm_persistent_pairs_every_tile_shape(bn, swap):
+    # row blocks x columns as 1000 * b + n; the last wave of two-block tiles is dealt as single blocks
+    for M, N, K, dtype in [(300, 1032, 136, torch.bfloat16), (777, 2601, 72, torch.bfloat16), (2049, 520, 68, torch.float32)]:
+        g = torch.Generator().manual_seed(51)
+        a = torch.randn(M, K, generator=g).to(dtype).cuda()
+        bt = (0.05 * torch.randn(N, K, generator=g)).to(dtype).cuda()
+        ref = (a.double() @ bt.double().t()).float()
+        for out_dtype in (torch.bfloat16, torch.float32):
+            for _ in range(2):                  # the tile counter is back at zero for the second call
+                c = fused.matmul(a, bt.t(), out_dtype=out_dtype, bn=bn, swap_ab=swap)
+                assert ((c.float() - ref).norm() / ref.norm()).item() < 3e-3
+    c = fused.matmul(a, bt.t(), bn=bn, swap_ab=swap, max_ctas=6)        # many tiles per pair
+    assert ((c.float() - ref).norm() / ref.norm()).item() < 3e-3
