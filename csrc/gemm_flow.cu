@@ -11,17 +11,19 @@
 //    epilogue of the one before, row block by row block. RB = 1 keeps two accumulators in turn.
 // Narrower column tiles (BN) fit ragged sizes and waves better; the launcher picks (flow_plan).
 //
-// Warps: 0 TMA producer (the leader's also draws the tiles), 1 MMA issuer (leader), 2-9 epilogue (two per TMEM
-// lane quarter, column panels dealt alternately), 10-11 optional copy of the row operand.
+// Warps: 0 TMA producer (the leader's also draws the tiles), 1 MMA issuer (leader), 2-5 epilogue (one per TMEM
+// lane quarter), 6-7 optional copy of the row operand. The common epilogues (MODE) are kernels of their own: with
+// every store form in one kernel its unrolled code pushed the other roles' loops out of the instruction cache
+// (8192 x 8192 x 3584 372 us against 366).
 #include <algorithm>
 #include "kraken/gemm_host.h"
 
 namespace kraken {
 
-constexpr int kFlowEpiWarps = 8;
+constexpr int kFlowEpiWarps = 4;
 constexpr int kFlowThreads = 64 + 32 * kFlowEpiWarps;
-constexpr int kFlowCopyThreads = 64;                      // 12 warps leave 168 registers a thread, 14 would leave 128
-constexpr int kFlowSlots = 4;                             // tiles drawn ahead of the slowest role, at most
+constexpr int kFlowCopyThreads = 64;
+constexpr int kFlowSlots = 16;                            // more than the slowest role can be behind the producer, see next_item
 
 struct alignas(64) FlowParams {
   CUtensorMap tmap_r, tmap_c, tmap_out;
@@ -43,7 +45,7 @@ struct FlowCfg {
   static constexpr int A_BYTES = kBM * 128;               // one row block of this CTA
   static constexpr int B_BYTES = BN / 2 * 128;
   static constexpr int STAGE = RB * A_BYTES + B_BYTES;
-  static constexpr int EPI = kFlowEpiWarps * 4096;
+  static constexpr int EPI = kFlowEpiWarps * 8192;       // two panel slots per warp
   static constexpr int RAW_STAGES = (kSmemLimit - 1024 - EPI - 512) / STAGE;
   static constexpr int STAGES = RAW_STAGES > 8 ? 8 : RAW_STAGES;
   static constexpr int BUFS = 2 * RB * BN <= 512 ? 2 : 1;
@@ -51,34 +53,16 @@ struct FlowCfg {
   static constexpr int TMEM_COLS = UNITS * BN <= 256 ? 256 : 512;
   static constexpr int SMEM = 1024 + STAGES * STAGE + EPI + 512;
   static_assert(BN % 32 == 0 && BN >= 128 && BN <= 256 && UNITS <= 4 && STAGES >= 3, "tile shape");
-  static_assert(16 * STAGES + 16 * UNITS + 16 * kFlowSlots + 4 * kFlowSlots + 8 <= 512, "barrier area");
+  static_assert(16 * STAGES + 16 * UNITS + 12 * kFlowSlots + 8 <= 512, "barrier area");
+  static_assert(STAGES + BUFS + 2 < kFlowSlots, "a role could be lapped");
 };
 
-// Bounded wait with cluster-scope acquire: what the other CTA wrote before it arrived is visible.
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred P;\n\t mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 P, [%1], %2;\n\t selp.u32 %0, 1, 0, P;\n\t}\n"
-      : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, const SyncCtx& c, uint32_t site) {
-  if (mbar_try_wait_cluster(bar, parity)) return true;
-  const uint64_t t0 = globaltimer_ns();
-  uint32_t n = 0;
-  while (true) {
-    if (mbar_try_wait_cluster(bar, parity)) return true;
-    if ((++n & 255u) == 0u) {
-      if (!status_ok(c)) return false;
-      if (globaltimer_ns() - t0 > c.timeout_ns) {
-        set_status(c, make_status(KR_ERR_TIMEOUT_MBAR, site, 0, blockIdx.x));
-        return false;
-      }
-    }
-  }
-}
-__device__ __forceinline__ void st_cluster_u32(uint32_t addr, uint32_t v) {
-  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+// One word into the shared memory of a CTA of the cluster, counted on an mbarrier there: whoever has waited for
+// that phase sees the word. No fence at either end (a release / acquire pair at cluster scope per tile and
+// role cost 0.8 us of every tile).
+__device__ __forceinline__ void publish_cluster_u32(uint32_t addr, uint32_t bar, uint32_t v) {
+  asm volatile("mbarrier.arrive.expect_tx.relaxed.cluster.shared::cluster.b64 _, [%0], 4;" ::"r"(bar) : "memory");
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.u32 [%0], %1, [%2];" ::"r"(addr), "r"(v), "r"(bar) : "memory");
 }
 __device__ __forceinline__ uint32_t ld_shared_u32(uint32_t addr) {
   uint32_t v;
@@ -107,7 +91,9 @@ __device__ __forceinline__ FlowItem flow_item(const FlowParams& p, int t) {
   return it;
 }
 
-template <int BN, int RB, int ELT>
+enum FlowMode : int { FLOW_ROWS = 0, FLOW_ROWS_ACT = 1, FLOW_ANY = 2 };     // bf16 row-major through TMA; with GELU; anything
+
+template <int BN, int RB, int ELT, int MODE>
 __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_kernel(const __grid_constant__ FlowParams p) {
   using Cfg = FlowCfg<BN, RB>;
   constexpr int kStageK = 128 / ELT;
@@ -123,8 +109,8 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
   auto empty_bar = [&](int s) { return bars + 8u * (Cfg::STAGES + s); };
   auto tfull_bar = [&](int u) { return bars + 8u * (2 * Cfg::STAGES + u); };
   auto tempty_bar = [&](int u) { return bars + 8u * (2 * Cfg::STAGES + Cfg::UNITS + u); };
-  const uint32_t sfull = bars + 8u * (2 * Cfg::STAGES + 2 * Cfg::UNITS), sempty = sfull + 8u * kFlowSlots;
-  const uint32_t sdata = sempty + 8u * kFlowSlots, tmem_slot = sdata + 4u * kFlowSlots;
+  const uint32_t sfull = bars + 8u * (2 * Cfg::STAGES + 2 * Cfg::UNITS), sdata = sfull + 8u * kFlowSlots;
+  const uint32_t tmem_slot = sdata + 4u * kFlowSlots;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < Cfg::STAGES; ++s) {
@@ -135,10 +121,7 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
       mbar_init(tfull_bar(u), 1);
       mbar_init(tempty_bar(u), 2 * kFlowEpiWarps);
     }
-    for (int k = 0; k < kFlowSlots; ++k) {
-      mbar_init(sfull + 8u * k, 1);
-      mbar_init(sempty + 8u * k, 2 + 2 * kFlowEpiWarps);     // the MMA issuer, the peer's producer, both CTAs' epilogue warps
-    }
+    for (int k = 0; k < kFlowSlots; ++k) mbar_init(sfull + 8u * k, 1);
     mbar_fence_init();
     tma_prefetch_desc(&p.tmap_r);
     tma_prefetch_desc(&p.tmap_c);
@@ -177,14 +160,14 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
     __syncwarp();
   };
 
-  // The item after publication k (item k + 1 of this pair): read by every role but the leader's producer.
+  // The item after item k of this pair, as the leader's producer published it. The slots need no "free" signal:
+  // the producer is at most STAGES items ahead of the MMA issuer (one stage per item at least), which is at
+  // most BUFS + 1 ahead of the epilogue.
   auto next_item = [&](int k, bool warp_wide, int& t) {
-    const uint32_t slot = (uint32_t)(k % kFlowSlots), parity = (uint32_t)(k / kFlowSlots) & 1u;
-    bool ok = mbar_wait_cluster(sfull + 8u * slot, parity, p.sync, 91);
+    const uint32_t slot = (uint32_t)(k % kFlowSlots);
+    bool ok = mbar_wait(sfull + 8u * slot, (uint32_t)(k / kFlowSlots) & 1u, p.sync, 91);
     if (warp_wide) ok = __all_sync(0xffffffffu, ok);
     t = ok ? (int)ld_shared_u32(sdata + 4u * slot) : p.items;
-    if (warp_wide) __syncwarp();
-    if (!warp_wide || lane == 0) mbar_arrive_cluster(mapa_shared(sempty + 8u * slot, 0));
     return ok;
   };
 
@@ -217,14 +200,10 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
           if (++s == Cfg::STAGES) { s = 0; ph ^= 1u; }
           if (leader && kb == min(3, p.num_kb - 1)) {
             // to both CTAs, even past the end (that is how the other roles learn of it)
-            const uint32_t slot = (uint32_t)(k % kFlowSlots), parity = (uint32_t)(k / kFlowSlots) & 1u;
-            ok = mbar_wait_cluster(sempty + 8u * slot, parity ^ 1u, p.sync, 93);
-            if (!ok) break;
+            const uint32_t slot = (uint32_t)(k % kFlowSlots);
 #pragma unroll
-            for (uint32_t c = 0; c < 2; ++c) {
-              st_cluster_u32(mapa_shared(sdata + 4u * slot, c), (uint32_t)drawn);
-              mbar_arrive_cluster(mapa_shared(sfull + 8u * slot, c));
-            }
+            for (uint32_t c = 0; c < 2; ++c)
+              publish_cluster_u32(mapa_shared(sdata + 4u * slot, c), mapa_shared(sfull + 8u * slot, c), (uint32_t)drawn);
           }
         }
         if (leader) t = drawn;
@@ -288,13 +267,13 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
     }
   } else if (warp < 2 + kFlowEpiWarps) {
     // ================= epilogue (both CTAs, own 128 rows of each block) =================
-    const int q = warp & 3, h = (warp - 2) >> 2;           // TMEM lane quarter; even or odd column panels
-    const uint32_t slot = epi0 + (uint32_t)(warp - 2) * 4096u;
+    const int q = warp & 3;                                // TMEM lane quarter
+    const uint32_t slots = epi0 + (uint32_t)(warp - 2) * 8192u;
     constexpr int PW = BN % 64 == 0 ? 64 : 32;             // columns per panel of a bf16 row-major tile
-    constexpr int CHUNKS = (BN / PW + 1) / 2 * (PW / 32);  // 32-column chunks of one warp, at most
-    auto chunk_col = [&](int i) { return PW == 64 ? (h + 2 * (i >> 1)) * 64 + (i & 1) * 32 : (h + 2 * i) * 32; };
-    const bool fp32 = p.out_fp32 != 0, transposed = p.transposed != 0;
-    uint32_t uph = 0;
+    constexpr int CHUNKS = BN / 32;
+    const bool fp32 = MODE == FLOW_ANY && p.out_fp32 != 0, transposed = MODE == FLOW_ANY && p.transposed != 0;
+    const bool act = MODE == FLOW_ROWS_ACT || (MODE == FLOW_ANY && p.act != 0);
+    uint32_t uph = 0, sent = 0;
     bool ok = true;
     int t = pair;
     for (int k = 0; ok && t < p.items; ++k) {
@@ -315,97 +294,92 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
           __syncwarp();
           if (lane == 0) mbar_arrive_cluster(mapa_shared(tempty_bar(u), 0));
         };
-        // A panel in the slot goes out: rows gy ..., columns gx ... of the output
-        auto send = [&](int gx, int gy, int cols) {
+        // The slot for the next panel, once the store that last read it (two panels ago) is done with it
+        auto next_slot = [&] {
+          if (lane == 0) bulk_wait_group_read<1>();
+          __syncwarp();
+          return slots + (sent++ & 1u) * 4096u;
+        };
+        // A panel in a slot goes out: rows gy ..., columns gx ... of the output
+        auto send = [&](uint32_t slot, int gx, int gy, int cols) {
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
-            if (p.out == nullptr && gx < p.out_cols && gy < p.out_rows) tma_store_2d(&p.tmap_out, slot, gx, gy);
+            if ((MODE != FLOW_ANY || p.out == nullptr) && gx < p.out_cols && gy < p.out_rows) tma_store_2d(&p.tmap_out, slot, gx, gy);
             bulk_commit_group();
           }
-          if (p.out != nullptr) store_plain(slot, gx, gy, cols, fp32, lane);
+          if (MODE == FLOW_ANY && p.out != nullptr) store_plain(slot, gx, gy, cols, fp32, lane);
         };
-        auto slot_free = [&] {    // the store that last read the slot is done with it
-          if (lane == 0) bulk_wait_group_read<0>();
-          __syncwarp();
-        };
-        if (fp32) {
+        if (MODE == FLOW_ANY && (fp32 || transposed)) {
 #pragma unroll 1
           for (int i = 0; i < CHUNKS; ++i) {
-            const int col = chunk_col(i);
-            if (col >= BN) break;
+            const int col = i * 32;
             uint32_t r[32];
             tmem_ld32(t_addr + (uint32_t)col, r);
             tmem_ld_wait();
-            if (i + 1 == CHUNKS || chunk_col(i + 1) >= BN) release();
-            if (p.act != 0) {
+            if (i + 1 == CHUNKS) release();
+            if (act) {
 #pragma unroll
               for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(gelu_tanh(__uint_as_float(r[j])));
             }
-            slot_free();
+            const uint32_t slot = next_slot();
             if (transposed) {
               // panel row j = column col + j of D; lanes = consecutive output columns
+              if (fp32) {
 #pragma unroll
-              for (int j = 0; j < 32; ++j)
-                asm volatile("st.shared.u32 [%0], %1;" ::"r"(slot + j * 128u + (uint32_t)((((lane >> 2) ^ (j & 7)) << 4) + (lane & 3) * 4)), "r"(r[j]) : "memory");
-              send(drow, it.tc * BN + col, 32);
+                for (int j = 0; j < 32; ++j)
+                  asm volatile("st.shared.u32 [%0], %1;" ::"r"(slot + j * 128u + (uint32_t)((((lane >> 2) ^ (j & 7)) << 4) + (lane & 3) * 4)), "r"(r[j]) : "memory");
+              } else {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) {
+                  const __nv_bfloat16 v = __float2bfloat16(__uint_as_float(r[j]));
+                  asm volatile("st.shared.u16 [%0], %1;" ::"r"(slot + j * 64u + (uint32_t)((((lane >> 3) ^ ((j >> 1) & 3)) << 4) + (lane & 7) * 2)),
+                               "h"(*reinterpret_cast<const unsigned short*>(&v)) : "memory");
+                }
+              }
+              send(slot, drow, it.tc * BN + col, 32);
             } else {
 #pragma unroll
               for (int v = 0; v < 8; ++v)
                 st_shared_u4(slot + lane * 128u + (uint32_t)((v ^ (lane & 7)) << 4), r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3]);
-              send(it.tc * BN + col, drow, 32);
+              send(slot, it.tc * BN + col, drow, 32);
             }
           }
         } else {
-          // bf16: the warp's whole part is read and rounded before anything is stored, so that the next
-          // tile's MMAs wait for nothing but TMEM reads; the activation follows on the rounded values, as it
-          // would on a bf16 tensor.
+          // bf16 rows: everything is read and rounded before anything is stored, so that the next tile's MMAs
+          // wait for nothing but TMEM reads; the activation follows on the rounded values, as it would on a
+          // bf16 tensor.
           uint32_t packed[CHUNKS][16];
 #pragma unroll
-          for (int i = 0; i < CHUNKS; ++i) {
-            const int col = chunk_col(i);
-            if (col < BN) {
-              uint32_t r[32];
-              tmem_ld32(t_addr + (uint32_t)col, r);
-              tmem_ld_wait();
+          for (int i = 0; i < CHUNKS; i += 2) {
+            uint32_t r0[32], r1[32];
+            tmem_ld32(t_addr + (uint32_t)(i * 32), r0);
+            if (i + 1 < CHUNKS) tmem_ld32(t_addr + (uint32_t)(i * 32 + 32), r1);
+            tmem_ld_wait();
 #pragma unroll
-              for (int v = 0; v < 16; ++v) packed[i][v] = pack_bf16x2(__uint_as_float(r[2 * v]), __uint_as_float(r[2 * v + 1]));
+            for (int v = 0; v < 16; ++v) {
+              packed[i][v] = pack_bf16x2(__uint_as_float(r0[2 * v]), __uint_as_float(r0[2 * v + 1]));
+              if (i + 1 < CHUNKS) packed[i + 1 < CHUNKS ? i + 1 : i][v] = pack_bf16x2(__uint_as_float(r1[2 * v]), __uint_as_float(r1[2 * v + 1]));
             }
           }
           release();
+          uint32_t slot = 0;
 #pragma unroll
           for (int i = 0; i < CHUNKS; ++i) {
-            const int col = chunk_col(i);
-            if (col < BN) {
-              if (p.act != 0) {
+            if (act) {
 #pragma unroll
-                for (int v = 0; v < 16; ++v)
-                  packed[i][v] = pack_bf16x2(gelu_tanh(bf16lo(packed[i][v])), gelu_tanh(bf16hi(packed[i][v])));
-              }
-              if (transposed) {
-                slot_free();
-#pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                  const uint32_t a = slot + j * 64u + (uint32_t)((((lane >> 3) ^ ((j >> 1) & 3)) << 4) + (lane & 7) * 2);
-                  asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"((unsigned short)(packed[i][j >> 1] >> ((j & 1) * 16))) : "memory");
-                }
-                send(drow, it.tc * BN + col, 32);
-              } else if (PW == 64) {
-                if ((i & 1) == 0) slot_free();
-#pragma unroll
-                for (int v = 0; v < 4; ++v)
-                  st_shared_u4(slot + lane * 128u + (uint32_t)((((i & 1) * 4 + v) ^ (lane & 7)) << 4), packed[i][4 * v], packed[i][4 * v + 1],
-                               packed[i][4 * v + 2], packed[i][4 * v + 3]);
-                if ((i & 1) == 1) send(it.tc * BN + col - 32, drow, 64);
-              } else {
-                slot_free();
-#pragma unroll
-                for (int v = 0; v < 4; ++v)
-                  st_shared_u4(slot + lane * 64u + (uint32_t)((v ^ ((lane >> 1) & 3)) << 4), packed[i][4 * v], packed[i][4 * v + 1],
-                               packed[i][4 * v + 2], packed[i][4 * v + 3]);
-                send(it.tc * BN + col, drow, 32);
-              }
+              for (int v = 0; v < 16; ++v)
+                packed[i][v] = pack_bf16x2(gelu_tanh(bf16lo(packed[i][v])), gelu_tanh(bf16hi(packed[i][v])));
             }
+            if (PW == 32 || (i & 1) == 0) slot = next_slot();
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+              const uint32_t a = PW == 64 ? slot + lane * 128u + (uint32_t)((((i & 1) * 4 + v) ^ (lane & 7)) << 4)
+                                          : slot + lane * 64u + (uint32_t)((v ^ ((lane >> 1) & 3)) << 4);
+              st_shared_u4(a, packed[i][4 * v], packed[i][4 * v + 1], packed[i][4 * v + 2], packed[i][4 * v + 3]);
+            }
+            if (PW == 32) send(slot, it.tc * BN + i * 32, drow, 32);
+            else if ((i & 1) == 1) send(slot, it.tc * BN + i * 32 - 32, drow, 64);
           }
         }
       }
@@ -442,10 +416,10 @@ struct FlowVariant {
   const void* fn;
   size_t smem;
 };
-template <int ELT>
+template <int ELT, int MODE>
 static FlowVariant flow_variant(int bn, int rb) {
 #define KR_FLOW(BN, RB) \
-  if (bn == BN && rb == RB) return {(const void*)gemm_flow_kernel<BN, RB, ELT>, FlowCfg<BN, RB>::SMEM};
+  if (bn == BN && rb == RB) return {(const void*)gemm_flow_kernel<BN, RB, ELT, MODE>, FlowCfg<BN, RB>::SMEM};
   KR_FLOW(256, 2)
   KR_FLOW(224, 2)
   KR_FLOW(192, 2)
@@ -461,7 +435,10 @@ static FlowVariant flow_variant(int bn, int rb) {
 }
 
 int launch_flow_gemm(const GemmParams& g, int bn, int rb, int pairs, uint32_t* sched, cudaStream_t stream) {
-  const FlowVariant v = g.in_fp32 ? flow_variant<4>(bn, rb) : flow_variant<2>(bn, rb);
+  const bool tma_out = (g.ldo * (g.out_fp32 ? 4 : 2)) % 16 == 0 && ((uintptr_t)g.out & 15) == 0;
+  const bool rows = tma_out && !g.out_fp32 && !g.transposed && !g.in_fp32;
+  const FlowVariant v = g.in_fp32 ? flow_variant<4, FLOW_ANY>(bn, rb) : !rows ? flow_variant<2, FLOW_ANY>(bn, rb)
+                        : g.act ? flow_variant<2, FLOW_ROWS_ACT>(bn, rb) : flow_variant<2, FLOW_ROWS>(bn, rb);
   if (v.fn == nullptr) return fail(KR_FAIL_ARG, "no persistent pair kernel of this tile shape");
   FlowParams p;
   memset(&p, 0, sizeof(p));
@@ -469,7 +446,7 @@ int launch_flow_gemm(const GemmParams& g, int bn, int rb, int pairs, uint32_t* s
   p.tmap_c = g.tmap_c;
   const int out_elt = g.out_fp32 ? 4 : 2;
   const unsigned box_bytes = (out_elt == 4 || (!g.transposed && bn % 64 == 0)) ? 128u : 64u;
-  if ((g.ldo * out_elt) % 16 == 0 && ((uintptr_t)g.out & 15) == 0) {
+  if (tma_out) {
     int rc = get_tmap(g.out, g.out_rows, g.out_cols, g.ldo, 32, &p.tmap_out, out_elt, box_bytes);
     if (rc) return rc;
   } else {
