@@ -417,14 +417,15 @@ struct TmapKey {
   unsigned box_rows;
   int elt;
   unsigned box_bytes;
+  int promote;
   bool operator==(const TmapKey& o) const {
-    return ptr == o.ptr && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows && elt == o.elt && box_bytes == o.box_bytes;
+    return ptr == o.ptr && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows && elt == o.elt && box_bytes == o.box_bytes && promote == o.promote;
   }
 };
 struct TmapHash {
   size_t operator()(const TmapKey& k) const {
     unsigned long long h = (unsigned long long)(uintptr_t)k.ptr >> 4;
-    for (unsigned long long v : {k.rows, k.cols, k.ld, (unsigned long long)k.box_rows * 2048 + k.box_bytes * 8 + (unsigned long long)k.elt})
+    for (unsigned long long v : {k.rows, k.cols, k.ld, (unsigned long long)k.box_rows * 4096 + (unsigned long long)k.promote * 8 + k.box_bytes * 16 + (unsigned long long)k.elt})
       h = (h ^ v) * 0x9e3779b97f4a7c15ull;
     return (size_t)(h ^ (h >> 32));
   }
@@ -439,8 +440,8 @@ static unsigned long long g_tmap_hits = 0, g_tmap_misses = 0;
 // contiguous, `ld` elements per row), box = box_bytes (128 or 64) of columns x box_rows rows, swizzled by as much,
 // out-of-range elements read as zero.
 int get_tmap(const void* ptr, unsigned long long rows, unsigned long long cols, unsigned long long ld,
-                    unsigned box_rows, CUtensorMap* out, int elt, unsigned box_bytes) {
-  TmapKey key{ptr, rows, cols, ld, box_rows, elt, box_bytes};
+                    unsigned box_rows, CUtensorMap* out, int elt, unsigned box_bytes, bool promote_256) {
+  TmapKey key{ptr, rows, cols, ld, box_rows, elt, box_bytes, promote_256 ? 1 : 0};
   {
     std::lock_guard<std::mutex> lk(g_tmap_mu);
     auto it = g_tmap_cache.find(key);
@@ -461,7 +462,7 @@ int get_tmap(const void* ptr, unsigned long long rows, unsigned long long cols, 
   CUtensorMap m;
   KR_CU(cuTensorMapEncodeTiled, &m, elt == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
         const_cast<void*>(ptr), gdim, gstride, box,
-        estr, CU_TENSOR_MAP_INTERLEAVE_NONE, box_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+        estr, CU_TENSOR_MAP_INTERLEAVE_NONE, box_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, promote_256 ? CU_TENSOR_MAP_L2_PROMOTION_L2_256B : CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   {
     std::lock_guard<std::mutex> lk(g_tmap_mu);
@@ -597,7 +598,7 @@ unsigned grid_cap(const DeviceState* d) {
 // Fills the operand/tiling part of the parameter block for C[M,N] = A[M,K] * Bt[N,K]^T.
 // swap: the weights (Bt) become the 128-row operand and the tile is stored transposed.
 int setup_problem(GemmParams& p, const void* a, long long lda, const void* bt, long long ldb, int M, int N,
-                         int K, bool swap, int bn_override, int* bn_out, int elt, int c_box_rows) {
+                         int K, bool swap, int bn_override, int* bn_out, int elt, int c_box_rows, bool promote_256) {
   KR_REQUIRE(M >= 1 && N >= 1 && K >= 8 && (K * elt) % 16 == 0, "GEMM needs K rows of whole 16-byte units and positive sizes");
   p.in_fp32 = elt == 4 ? 1 : 0;
   const void* r = swap ? bt : a;
@@ -613,9 +614,9 @@ int setup_problem(GemmParams& p, const void* a, long long lda, const void* bt, l
   p.group_r = default_group_r();
   p.pivot_r = 0;
   p.transposed = swap ? 1 : 0;
-  int rc = get_tmap(r, p.rows_r, K, ldr, kBM, &p.tmap_r, elt);
+  int rc = get_tmap(r, p.rows_r, K, ldr, kBM, &p.tmap_r, elt, 128, promote_256);
   if (rc) return rc;
-  rc = get_tmap(c, p.rows_c, K, ldc, c_box_rows > 0 ? c_box_rows : bn, &p.tmap_c, elt);
+  rc = get_tmap(c, p.rows_c, K, ldc, c_box_rows > 0 ? c_box_rows : bn, &p.tmap_c, elt, 128, promote_256);
   if (rc) return rc;
   p.host_c_ptr = c;
   p.host_ldc = ldc;

@@ -93,9 +93,19 @@ static PlainPlan plain_plan(const DeviceState* d, int M, int N, int K, int elt, 
     for (int swap = 0; swap < 2; ++swap) {
       const int rows = swap ? N : M, cols = swap ? M : N;
       if (rows <= 128) continue;
+      if (whole_chip && cols <= 128) {
+        // single CTAs of 128 x 128: up to eight K splits (100 x 4000 x 9000 21 us, with pairs 27)
+        const int tiles = (rows + kBM - 1) / kBM;
+        double us = 1e30;
+        const int s = tiles <= d->num_sms ? tile_gemm_splits(d, tiles, num_kb, 128, false, elt, 1.0, &us) : 0;
+        if (s > 0 && us < best) {
+          best = us;
+          pl.kind = PLAIN_TILE; pl.swap = swap != 0; pl.pair = false; pl.bn = 128; pl.splits = s; pl.rb = 1;
+        }
+      }
       for (int bn = 128; bn <= 256; bn += 32) {
         if (bn > 128 && bn - 32 >= cols) continue;                   // wider than needed
-        if (whole_chip && (bn == 128 || bn == 256)) {
+        if (whole_chip) {
           const int tiles = ((rows + 255) / 256) * ((cols + bn - 1) / bn);
           double us = 1e30;
           const int s = tiles <= pairs ? tile_gemm_splits(d, tiles, num_kb, bn, true, elt, lines ? 1.0 : 1.2, &us) : 0;
@@ -110,7 +120,7 @@ static PlainPlan plain_plan(const DeviceState* d, int M, int N, int K, int elt, 
           const double us = flow_us(rows, cols, num_kb, bn, rb, pairs, lines) * (swap ? 1.02 : 1.0);
           if (us < best) {
             best = us;
-            pl.kind = PLAIN_FLOW; pl.swap = swap != 0; pl.bn = bn; pl.rb = rb; pl.splits = 0; pl.workers = pairs;
+            pl.kind = PLAIN_FLOW; pl.swap = swap != 0; pl.pair = true; pl.bn = bn; pl.rb = rb; pl.splits = 0; pl.workers = pairs;
           }
         }
       }
@@ -202,7 +212,10 @@ KR_API int kr_gemm(const void* a, long long lda, const void* bt, long long ldb, 
   GemmParams p;
   memset(&p, 0, sizeof(p));
   int bn = 0;
-  int rc = setup_problem(p, a, lda, bt, ldb, M, N, K, pl.swap, pl.bn, &bn, elt, pair ? pl.bn / 2 : pl.bn);
+  int rc = setup_problem(p, a, lda, bt, ldb, M, N, K, pl.swap, pl.bn, &bn, elt, pair ? pl.bn / 2 : pl.bn,
+                         // Persistent pairs on rows off the 128-byte lines: fetching past the line into L2 only gets in the
+                         // way there (777 x 5120 x 13704 153 to 140 us); elsewhere it helps (16 x 8192 x 28672 78.6 to 76.0).
+                         pl.kind != PLAIN_FLOW || (lda * elt % 128 == 0 && ldb * elt % 128 == 0));
   if (rc) return rc;
   p.mode = GEMM_PLAIN;
   p.out = out;

@@ -45,7 +45,7 @@ struct TileCfg {
   static constexpr int STAGE = A_BYTES + B_BYTES_AL;
   static constexpr int RAW_STAGES = (kSmemLimit - 1024 - 512) / STAGE;
   static constexpr int STAGES = RAW_STAGES > 12 ? 12 : RAW_STAGES;
-  static constexpr int TMEM_COLS = BN < 32 ? 32 : BN;
+  static constexpr int TMEM_COLS = BN <= 32 ? 32 : BN <= 64 ? 64 : BN <= 128 ? 128 : 256;
   static constexpr int SMEM = 1024 + STAGES * STAGE + 512;
   static_assert(BN * kBM * 4 <= STAGES * STAGE, "the accumulator has to fit the stages");
 };
@@ -219,13 +219,12 @@ __global__ void __launch_bounds__(kTileThreads, 1) gemm_tile_kernel(const __grid
     bool ok = mbar_wait(done_bar, 0, p.sync, 82);
     ok = __all_sync(0xffffffffu, ok);
     tc_fence_after();
-    constexpr int HALVES = BN >= 32 ? 2 : 1;               // two warps per TMEM lane quarter
-    constexpr int COLS = BN / HALVES, CH = COLS < 32 ? COLS : 32;
+    constexpr int CH = BN < 32 ? BN : 32;                  // two warps per TMEM lane quarter take turns
     const int q = warp & 3, h = (warp - 2) >> 2;
-    if (ok && h < HALVES) {
+    if (ok) {
       const int row = q * 32 + lane;
 #pragma unroll 1
-      for (int c0 = h * COLS; c0 < (h + 1) * COLS; c0 += CH) {
+      for (int c0 = h * CH; c0 < BN; c0 += 2 * CH) {
         uint32_t r[32];
         const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c0;
         if (CH == 32) tmem_ld32(t_addr, r);
@@ -332,10 +331,16 @@ struct TileVariant {
 template <int ELT>
 static TileVariant tile_variant(int bn, bool pair) {
   if (pair) {
-    if (bn == 128) return {(const void*)gemm_tile_kernel<128, ELT, true>, TileCfg<128, true>::SMEM};
-    return {(const void*)gemm_tile_kernel<256, ELT, true>, TileCfg<256, true>::SMEM};
+    switch (bn) {
+      case 128: return {(const void*)gemm_tile_kernel<128, ELT, true>, TileCfg<128, true>::SMEM};
+      case 160: return {(const void*)gemm_tile_kernel<160, ELT, true>, TileCfg<160, true>::SMEM};
+      case 192: return {(const void*)gemm_tile_kernel<192, ELT, true>, TileCfg<192, true>::SMEM};
+      case 224: return {(const void*)gemm_tile_kernel<224, ELT, true>, TileCfg<224, true>::SMEM};
+      default: return {(const void*)gemm_tile_kernel<256, ELT, true>, TileCfg<256, true>::SMEM};
+    }
   }
   switch (bn) {
+    case 128: return {(const void*)gemm_tile_kernel<128, ELT, false>, TileCfg<128, false>::SMEM};
     case 16: return {(const void*)gemm_tile_kernel<16, ELT, false>, TileCfg<16, false>::SMEM};
     case 32: return {(const void*)gemm_tile_kernel<32, ELT, false>, TileCfg<32, false>::SMEM};
     case 64: return {(const void*)gemm_tile_kernel<64, ELT, false>, TileCfg<64, false>::SMEM};
@@ -375,7 +380,7 @@ static int max_clusters(int device, const TileVariant& v, unsigned cluster) {
 
 // The split count of a one-wave problem, 0 when its tiles do not fit the chip at once, and its time (us).
 // Times as measured: K blocks at the rate the MMAs (256-column pairs 0.30 per block at full clock, more
-// when the chip is full and power-limited) or the operand loads (0.18-0.28, single CTAs 0.25) allow, but
+// when the chip is full and power-limited) or the operand loads (single CTAs 0.25, 128 columns wide 0.36) allow, but
 // never below the operands' time out of HBM, plus what summing S splits adds: little for the narrow tiles
 // of single CTAs, a lot once a cluster of pairs spans more than four CTAs (M = 256, N = 4096, K = 2048:
 // 1 / 2 / 3 splits 17.5 / 14.2 / 20.5 us).
@@ -384,13 +389,14 @@ int tile_gemm_splits(const DeviceState* d, int tiles, int num_kb, int bn, bool p
   if (v.fn == nullptr) return 0;
   const int ctas = pair ? 2 : 1, most = 8 / ctas;
   const double hbm_us = (double)tiles * ctas * num_kb * kBM * 128 / 6.5e6;
+  const double width = bn == 256 ? 1.0 : bn == 224 ? 0.88 : bn == 192 ? 0.77 : bn == 160 ? 0.66 : 0.59;
   auto sum_us = [&](int s) { return !pair ? 0.25 * s : (s <= 2 ? 1.5 * s : 4.0 * s - 2.0) * bn / 256; };
   int best = 0;
   double best_us = 1e30;
   for (int s = 1; s <= most && (s == 1 || num_kb >= 4 * s); ++s) {
     if (tiles * s * ctas > d->num_sms || tiles > max_clusters(d->device, v, (unsigned)(s * ctas))) continue;
     const double busy = (double)tiles * s * ctas / d->num_sms;
-    const double kb_us = !pair ? 0.25 : std::max(0.30, 0.47 * std::sqrt(busy)) * (bn == 256 ? 1.0 : 0.59) * off_line;
+    const double kb_us = !pair ? (bn == 128 ? 0.36 : 0.25) : std::max(0.30, 0.47 * std::sqrt(busy)) * width * off_line;
     const double us = std::max((num_kb + s - 1) / s * kb_us, hbm_us) + sum_us(s) + 8.0;
     if (us < best_us) {
       best_us = us;
