@@ -52,7 +52,7 @@ struct FlowCfg {
   static constexpr int UNITS = BUFS * RB;                 // accumulators of BN columns
   static constexpr int TMEM_COLS = UNITS * BN <= 256 ? 256 : 512;
   static constexpr int SMEM = 1024 + STAGES * STAGE + EPI + 512;
-  static_assert(BN % 32 == 0 && BN >= 128 && BN <= 256 && UNITS <= 4 && STAGES >= 3, "tile shape");
+  static_assert(BN % 32 == 0 && BN >= 64 && BN <= 256 && UNITS <= 4 && STAGES >= 3, "tile shape");
   static_assert(16 * STAGES + 16 * UNITS + 12 * kFlowSlots + 8 <= 512, "barrier area");
   static_assert(STAGES + BUFS + 2 < kFlowSlots, "a role could be lapped");
 };
@@ -425,11 +425,15 @@ static FlowVariant flow_variant(int bn, int rb) {
   KR_FLOW(192, 2)
   KR_FLOW(160, 2)
   KR_FLOW(128, 2)
+  KR_FLOW(96, 2)
+  KR_FLOW(64, 2)
   KR_FLOW(256, 1)
   KR_FLOW(224, 1)
   KR_FLOW(192, 1)
   KR_FLOW(160, 1)
   KR_FLOW(128, 1)
+  KR_FLOW(96, 1)
+  KR_FLOW(64, 1)
 #undef KR_FLOW
   return {nullptr, 0};
 }

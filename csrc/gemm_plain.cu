@@ -43,32 +43,34 @@ struct PlainPlan {
   int workers;      // CTAs, or pairs, of a persistent kernel
 };
 
-// Time model of the pair kernels, in microseconds per K block (64 bf16 or 32 fp32 columns of K) of a
-// 256 x 256 block, from long runs on a B200. With every SM busy the chip is at its power limit (0.47);
-// fewer pairs run faster, down to 0.30 at full clock. Narrow column tiles move more operand bytes per
-// operation, two row blocks fewer.
-static double pair_kb_us(int busy, int pairs) { return std::max(0.30, 0.47 * std::sqrt((double)busy / pairs)); }
-static double tile_cost(int bn, int rb) {
-  const double one = bn == 256 ? 1.0 : bn == 224 ? 0.88 : bn == 192 ? 0.77 : bn == 160 ? 0.66 : 0.59;
-  return rb == 1 ? one : 1.93 * one;
-}
+// Where the rows of an operand start: 0 on 128-byte lines, 1 on 32-byte sectors, 2 in the middle of sectors
+// (a row length of an odd number of 16-byte units): each 128 bytes then cost a fifth sector.
+static int row_class(long long ld, int elt) { return ld * elt % 128 == 0 ? 0 : ld * elt % 32 == 0 ? 1 : 2; }
 
-// Rows that do not start on 128-byte lines cost an extra sector and line per 128 bytes fetched, which weighs the
-// more the less a tile reuses its operands (4000 x 6000 x 3000: 256 x 256 tiles 155 us, 512 x 224 131).
-static double flow_us(int rows, int cols, int num_kb, int bn, int rb, int pairs, bool lines) {
+// Time model of the pair kernels, in microseconds, fitted to long runs on a B200 with every SM busy, i.e. at
+// the power limit: per K block (64 bf16 or 32 fp32 columns of K) 0.299 for the MMAs of 256 x 256 and 0.0054 per
+// KB of operands a CTA fetches, by the class of their rows (4096 x 4096 x 9512 against x 9472: 256 x 256 tiles
+// 308 / 256 us, 512 x 256 266 / 249, 256 x 128 388 / 292).
+static double block_us(int bn, int rb, int class_r, int class_c) {
+  static const double kByClass[3] = {1.0, 1.07, 1.5};
+  return (0.299 * rb * bn / 256 + 0.0054 * (16 * rb * kByClass[class_r] + bn / 16.0 * kByClass[class_c])) * (rb == 2 ? 1.03 : 1.0);
+}
+// With fewer SMs busy the rest run faster, up to full clock.
+static double clock_factor(double busy) { return std::max(0.64, std::sqrt(busy)); }
+
+static double flow_us(int rows, int cols, int num_kb, int bn, int rb, int pairs, int class_r, int class_c) {
   const int T = ((rows + 256 * rb - 1) / (256 * rb)) * ((cols + bn - 1) / bn);
   const int whole = T / pairs, rest = T % pairs;
-  const double off1 = lines ? 1.0 : 1.2, off = rb == 1 ? off1 : (lines ? 1.0 : 1.06);
-  const double full = num_kb * tile_cost(bn, rb) * off * pair_kb_us(pairs, pairs);
-  double last = rest ? num_kb * tile_cost(bn, rb) * off * pair_kb_us(rest, pairs) : 0.0;
-  if (rb == 2 && rest && 2 * rest <= pairs) last = num_kb * tile_cost(bn, 1) * off1 * pair_kb_us(2 * rest, pairs);
+  const double full = num_kb * block_us(bn, rb, class_r, class_c);
+  double last = rest ? full * clock_factor((double)rest / pairs) : 0.0;
+  if (rb == 2 && rest && 2 * rest <= pairs) last = num_kb * block_us(bn, 1, class_r, class_c) * clock_factor(2.0 * rest / pairs);
   // what is not hidden: start and last epilogue, and with one accumulator set the epilogue of every tile
-  const double bubble = 2 * rb * bn <= 512 ? 0.0 : 2.5;
+  const double bubble = 2 * rb * bn <= 512 ? 0.0 : 3.5;
   return whole * (full + bubble) + last + 8.0;
 }
 
 static PlainPlan plain_plan(const DeviceState* d, int M, int N, int K, int elt, int swap_ab, int bn_override, int use_pair,
-                            int max_ctas) {
+                            int max_ctas, int class_a, int class_b) {
   PlainPlan pl;
   memset(&pl, 0, sizeof(pl));
   pl.rb = 1;
@@ -77,7 +79,6 @@ static PlainPlan plain_plan(const DeviceState* d, int M, int N, int K, int elt, 
   if (max_ctas > 0 && max_ctas < cap) cap = max_ctas;
   const bool pair_ok = use_pair != 0 && pair_enabled() && !emu && cap >= 2;
   const int num_kb = (K + 128 / elt - 1) / (128 / elt), pairs = cap / 2;
-  const bool lines = (long long)K * elt % 128 == 0;
   const bool whole_chip = max_ctas <= 0 && !emu;
   pl.swap = swap_ab < 0 ? (M <= 64 && N >= 128) : swap_ab != 0;
   if (bn_override >= 1000 && pair_ok) {
@@ -91,24 +92,24 @@ static PlainPlan plain_plan(const DeviceState* d, int M, int N, int K, int elt, 
     // the whole choice is open: both orientations, every tile width, one wave with K splits or many
     double best = 1e30;
     for (int swap = 0; swap < 2; ++swap) {
-      const int rows = swap ? N : M, cols = swap ? M : N;
+      const int rows = swap ? N : M, cols = swap ? M : N, cr = swap ? class_b : class_a, cc = swap ? class_a : class_b;
       if (rows <= 128) continue;
       if (whole_chip && cols <= 128) {
         // single CTAs of 128 x 128: up to eight K splits (100 x 4000 x 9000 21 us, with pairs 27)
         const int tiles = (rows + kBM - 1) / kBM;
         double us = 1e30;
-        const int s = tiles <= d->num_sms ? tile_gemm_splits(d, tiles, num_kb, 128, false, elt, 1.0, &us) : 0;
+        const int s = tiles <= d->num_sms ? tile_gemm_splits(d, tiles, num_kb, 128, false, elt, 0.36 / 0.324 * (block_us(128, 1, cr, cc) + 0.0054 * 8), &us) : 0;
         if (s > 0 && us < best) {
           best = us;
           pl.kind = PLAIN_TILE; pl.swap = swap != 0; pl.pair = false; pl.bn = 128; pl.splits = s; pl.rb = 1;
         }
       }
-      for (int bn = 128; bn <= 256; bn += 32) {
-        if (bn > 128 && bn - 32 >= cols) continue;                   // wider than needed
-        if (whole_chip) {
+      for (int bn = 64; bn <= 256; bn += 32) {
+        if (bn > 64 && bn - 32 >= cols) continue;                    // wider than needed
+        if (whole_chip && bn >= 128) {
           const int tiles = ((rows + 255) / 256) * ((cols + bn - 1) / bn);
           double us = 1e30;
-          const int s = tiles <= pairs ? tile_gemm_splits(d, tiles, num_kb, bn, true, elt, lines ? 1.0 : 1.2, &us) : 0;
+          const int s = tiles <= pairs ? tile_gemm_splits(d, tiles, num_kb, bn, true, elt, block_us(bn, 1, cr, cc), &us) : 0;
           if (s > 0 && us < best) {
             best = us;
             pl.kind = PLAIN_TILE; pl.swap = swap != 0; pl.pair = true; pl.bn = bn; pl.splits = s;
@@ -117,7 +118,7 @@ static PlainPlan plain_plan(const DeviceState* d, int M, int N, int K, int elt, 
         for (int rb = 1; rb <= 2; ++rb) {
           if (rb == 2 && rows <= 256) continue;
           // a transposed store writes shorter runs: row-major unless the other way saves something
-          const double us = flow_us(rows, cols, num_kb, bn, rb, pairs, lines) * (swap ? 1.02 : 1.0);
+          const double us = flow_us(rows, cols, num_kb, bn, rb, pairs, cr, cc) * (swap ? 1.02 : 1.0);
           if (us < best) {
             best = us;
             pl.kind = PLAIN_FLOW; pl.swap = swap != 0; pl.pair = true; pl.bn = bn; pl.rb = rb; pl.splits = 0; pl.workers = pairs;
@@ -137,7 +138,7 @@ static PlainPlan plain_plan(const DeviceState* d, int M, int N, int K, int elt, 
   if (elt == 4 && pl.bn == 128) pl.bn = 256;
   const int tiles = ((rows + kBM - 1) / kBM) * ((cols + pl.bn - 1) / pl.bn);
   if (swap_ab < 0 && bn_override <= 0 && whole_chip && tiles <= d->num_sms) {
-    pl.splits = tile_gemm_splits(d, tiles, num_kb, pl.bn, false, elt, 1.0, nullptr);
+    pl.splits = tile_gemm_splits(d, tiles, num_kb, pl.bn, false, elt, 0.25, nullptr);
     if (pl.splits > 0) {
       pl.kind = PLAIN_TILE;
       return pl;
@@ -151,19 +152,20 @@ static PlainPlan plain_plan(const DeviceState* d, int M, int N, int K, int elt, 
 // The plan of a problem, remembered per thread for the shapes a program repeats (a decode step calls the
 // same few again and again; working a plan out takes microseconds).
 static PlainPlan known_plan(const DeviceState* d, int M, int N, int K, int elt, int swap_ab, int bn_override, int use_pair,
-                            int max_ctas) {
+                            int max_ctas, long long lda, long long ldb) {
+  const int class_a = row_class(lda, elt), class_b = row_class(ldb, elt);
   struct Entry {
-    int key[10];
+    int key[11];
     PlainPlan plan;
   };
   static thread_local Entry table[64];
-  if (emu_recorder().active) return plain_plan(d, M, N, K, elt, swap_ab, bn_override, use_pair, max_ctas);
-  const int key[10] = {1, d->device, M, N, K, elt, swap_ab, bn_override, use_pair, max_ctas};
+  if (emu_recorder().active) return plain_plan(d, M, N, K, elt, swap_ab, bn_override, use_pair, max_ctas, class_a, class_b);
+  const int key[11] = {1, d->device, M, N, K, elt, swap_ab, bn_override, use_pair, max_ctas, class_a * 3 + class_b};
   unsigned h = 2166136261u;
   for (int k : key) h = (h ^ (unsigned)k) * 16777619u;
   Entry& e = table[(h ^ (h >> 15)) % 64];
   if (memcmp(e.key, key, sizeof(key)) != 0) {
-    e.plan = plain_plan(d, M, N, K, elt, swap_ab, bn_override, use_pair, max_ctas);
+    e.plan = plain_plan(d, M, N, K, elt, swap_ab, bn_override, use_pair, max_ctas, class_a, class_b);
     memcpy(e.key, key, sizeof(key));
   }
   return e.plan;
@@ -182,12 +184,12 @@ static int launch_plain(const GemmParams& p, unsigned ctas, unsigned threads, cu
 using namespace kraken;
 
 // Counter words a call with these arguments needs (0: none).
-KR_API int kr_gemm_scratch(int M, int N, int K, int in_fp32, int swap_ab, int bn_override, int use_pair, int max_ctas,
+KR_API int kr_gemm_scratch(int M, int N, int K, long long lda, long long ldb, int in_fp32, int swap_ab, int bn_override, int use_pair, int max_ctas,
                            unsigned long long* counter_words) {
   DeviceState* d = device_state();
   if (!d) return KR_FAIL_CUDA;
   KR_REQUIRE(M >= 1 && N >= 1 && K >= 1, "GEMM needs positive sizes");
-  *counter_words = known_plan(d, M, N, K, in_fp32 ? 4 : 2, swap_ab, bn_override, use_pair, max_ctas).kind == PLAIN_FLOW ? 2 : 0;
+  *counter_words = known_plan(d, M, N, K, in_fp32 ? 4 : 2, swap_ab, bn_override, use_pair, max_ctas, lda, ldb).kind == PLAIN_FLOW ? 2 : 0;
   return KR_SUCCESS;
 }
 
@@ -207,7 +209,7 @@ KR_API int kr_gemm(const void* a, long long lda, const void* bt, long long ldb, 
   if (!d) return KR_FAIL_CUDA;
   KR_REQUIRE(M >= 1 && N >= 1, "GEMM needs positive sizes");
   const int elt = in_fp32 ? 4 : 2;
-  const PlainPlan pl = known_plan(d, M, N, K, elt, swap_ab, bn_override, use_pair, max_ctas);
+  const PlainPlan pl = known_plan(d, M, N, K, elt, swap_ab, bn_override, use_pair, max_ctas, lda, ldb);
   const bool pair = pl.kind == PLAIN_FLOW || pl.pair;
   GemmParams p;
   memset(&p, 0, sizeof(p));

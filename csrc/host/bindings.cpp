@@ -26,7 +26,7 @@ struct Api {
   int (*rms_norm)(const void*, const void*, void*, int, int, float, void*);
   int (*local_bias_rms_norm)(const void*, int, const void*, u64, const void*, void*, int, int, float, int, void*);
   int (*local_all_reduce)(const void*, void*, const void*, u64, u64, void*);
-  int (*gemm_scratch)(int, int, int, int, int, int, int, int, u64*);
+  int (*gemm_scratch)(int, int, int, long long, long long, int, int, int, int, int, u64*);
   int (*gemm)(const void*, long long, const void*, long long, void*, long long, int, int, int, int, int, int, int, int, int, int,
               uint32_t*, void*, void*);
 };
@@ -99,24 +99,27 @@ bool gemm_operands(const at::Tensor& a, const at::Tensor& bt, int64_t N, int64_t
          ldb % unit == 0 && lda >= K && ldb >= K && aligned(a) && aligned(bt);
 }
 int run_gemm(const at::Tensor& a, const at::Tensor& bt, int64_t N, int64_t ldb, bool out_fp32, int act, int swap, int bn, int max_ctas, int pair,
-             void* copy_dst, c10::cuda::CUDAStream stream, at::Tensor& out) {
+             void* copy_dst, c10::cuda::CUDAStream stream, bool pad_rows, at::Tensor& out) {
   const int64_t M = a.size(0), K = a.size(1);
   const bool fp32 = a.scalar_type() == at::kFloat;
-  out = at::detail::empty_cuda({M, N}, out_fp32 ? at::kFloat : at::kBFloat16, a.device(), std::nullopt);
+  // pad_rows: rows of whole 128-byte lines, for a result that the next GEMM reads
+  const int64_t line = out_fp32 ? 32 : 64, ldo = pad_rows ? (N + line - 1) / line * line : N;
+  out = at::detail::empty_cuda({M, ldo}, out_fp32 ? at::kFloat : at::kBFloat16, a.device(), std::nullopt);
+  if (ldo != N) out = out.narrow(1, 0, N);
   u64 words = 0;
-  int rc = api.gemm_scratch((int)M, (int)N, (int)K, fp32, swap, bn, pair, max_ctas, &words);
+  int rc = api.gemm_scratch((int)M, (int)N, (int)K, a.stride(0), ldb, fp32, swap, bn, pair, max_ctas, &words);
   if (rc) return rc;
   at::Tensor counters;
   if (words) counters = counters_for(a.device().index(), stream, (int64_t)words);
-  return api.gemm(a.data_ptr(), a.stride(0), bt.data_ptr(), ldb, out.data_ptr(), N, (int)M, (int)N, (int)K, out_fp32, act, swap, bn, max_ctas,
+  return api.gemm(a.data_ptr(), a.stride(0), bt.data_ptr(), ldb, out.data_ptr(), ldo, (int)M, (int)N, (int)K, out_fp32, act, swap, bn, max_ctas,
                   pair, fp32, words ? (uint32_t*)counters.data_ptr() : nullptr, copy_dst, (void*)stream.stream());
 }
 
-// gemm(a, b, out_fp32, act, tf32, swap_ab, bn, max_ctas, pair, copy_dst): act(a @ b). a [M, K] with K contiguous, b
+// gemm(a, b, out_fp32, act, tf32, swap_ab, bn, max_ctas, pair, copy_dst, pad_rows): act(a @ b). a [M, K] with K contiguous, b
 // [K, N] stored transposed (N rows of contiguous K), both bf16 or, with tf32, both fp32.
 PyObject* py_gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
-  if (n != 10) {
-    PyErr_SetString(PyExc_TypeError, "gemm takes 10 arguments");
+  if (n != 11) {
+    PyErr_SetString(PyExc_TypeError, "gemm takes 11 arguments");
     return nullptr;
   }
   const c10::DeviceIndex dev = c10::cuda::current_device();
@@ -133,7 +136,7 @@ PyObject* py_gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
   }
   at::Tensor out;
   const int rc = run_gemm(*a, *b, b->size(1), b->stride(1), args[2] == Py_True, act, swap, bn, max_ctas, pair, copy_dst,
-                          c10::cuda::getCurrentCUDAStream(dev), out);
+                          c10::cuda::getCurrentCUDAStream(dev), args[10] == Py_True, out);
   if (rc) return failed(rc);
   return THPVariable_Wrap(std::move(out));
 }
@@ -155,7 +158,7 @@ PyObject* py_decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (PyErr_Occurred()) return nullptr;
   auto stream = c10::cuda::getCurrentCUDAStream(dev);
   at::Tensor p;
-  int rc = run_gemm(*h, *wt, N, wt->stride(0), false, 0, -1, 0, 0, 1, nullptr, stream, p);
+  int rc = run_gemm(*h, *wt, N, wt->stride(0), false, 0, -1, 0, 0, 1, nullptr, stream, false, p);
   if (rc) return failed(rc);
   at::Tensor y = at::detail::empty_cuda(p.sizes(), at::kBFloat16, p.device(), std::nullopt);
   rc = api.local_bias_rms_norm(p.data_ptr(), 0, bias->data_ptr(), (u64)N, w->data_ptr(), y.data_ptr(), (int)p.size(0), (int)N, (float)eps, 1,

@@ -26,8 +26,8 @@ int launch_gemm_ar(int bn, const GemmParams& p, unsigned nb, cudaStream_t stream
 // Routes a parameter block to the kernel family of its mode and operand type (gemm.cu).
 int launch_gemm(int bn, const GemmParams& p, unsigned nb, cudaStream_t stream);
 // One-wave GEMM (gemm_tile.cu): the most K splits with which `tiles` tiles of this kernel run at once,
-// 0 when it does not apply, and its estimated time (off_line: factor for rows off 128-byte lines); and its launch.
-int tile_gemm_splits(const DeviceState* d, int tiles, int num_kb, int bn, bool pair, int elt, double off_line, double* us);
+// 0 when it does not apply, and its estimated time (block_us: one K block of a tile); and its launch.
+int tile_gemm_splits(const DeviceState* d, int tiles, int num_kb, int bn, bool pair, int elt, double block_us, double* us);
 // Persistent pairs that draw their tiles in order (gemm_flow.cu); sched: two zero words, zero again afterwards.
 int launch_flow_gemm(const GemmParams& g, int bn, int rb, int pairs, uint32_t* sched, cudaStream_t stream);
 int launch_tile_gemm(const GemmParams& g, int bn, bool pair, int splits, cudaStream_t stream);

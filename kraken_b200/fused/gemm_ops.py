@@ -43,7 +43,7 @@ _ACT = {None: 0, "gelu_tanh": 1}
 def _gemm(a: torch.Tensor, b: torch.Tensor, out_fp32: bool, tf32: bool, swap_ab: int = -1, bn: int = 0, max_ctas: int = 0,
           pair: int = 1, act: str | None = None, copy_dst: torch.Tensor | None = None) -> torch.Tensor:
     """act(a @ b) on this GPU alone; `copy_dst` additionally receives a copy of `a`."""
-    out = _host.gemm(a, b, out_fp32, _ACT[act], tf32, swap_ab, bn, max_ctas, pair, copy_dst)
+    out = _host.gemm(a, b, out_fp32, _ACT[act], tf32, swap_ab, bn, max_ctas, pair, copy_dst, False)
     if out is not None:
         return out
     # operands of another type or layout: cast and laid out K-major first
@@ -54,7 +54,7 @@ def _gemm(a: torch.Tensor, b: torch.Tensor, out_fp32: bool, tf32: bool, swap_ab:
     N = bt.shape[0]
     if bt.shape[1] != K:
         raise ValueError("inner dimensions differ")
-    out = _host.gemm(a2, bt.t(), out_fp32, _ACT[act], tf32, swap_ab, bn, max_ctas, pair, copy_dst)
+    out = _host.gemm(a2, bt.t(), out_fp32, _ACT[act], tf32, swap_ab, bn, max_ctas, pair, copy_dst, False)
     if out is not None:
         return out
     out = torch.empty((M, N), dtype=torch.float32 if out_fp32 else torch.bfloat16, device=a.device)
@@ -121,11 +121,12 @@ _AG_FLAG_BANK = 2048      # chunk flags per bank in the signal pad (two banks fr
 
 def all_gather_matmul_act(a_shared: torch.Tensor, b: torch.Tensor, act: str, group=None) -> torch.Tensor:
     """act(gathered A @ b), without the gathered A: the activation is applied to the fp32 sums in the
-    GEMM's epilogue. act="gelu_tanh"."""
+    GEMM's epilogue. act="gelu_tanh". The result's rows may be padded to whole 128-byte lines (a view with a
+    larger row stride), which is how the next GEMM fetches them fastest."""
     if a_shared.is_cuda and symm_mem.solo(group):
         alloc = symm_mem.native_allocation(a_shared)
         if alloc is not None and alloc.local_ptr == a_shared.data_ptr():
-            c = _host.gemm(a_shared, b, False, _ACT[act], False, -1, 0, 0, 1, None)
+            c = _host.gemm(a_shared, b, False, _ACT[act], False, -1, 0, 0, 1, None, True)
             if c is not None:
                 return c
     if a_shared.device.type != "cuda":
@@ -161,7 +162,7 @@ def all_gather_matmul(a_shared: torch.Tensor, b: torch.Tensor, a_out: torch.Tens
         alloc = symm_mem.native_allocation(a_shared)
         if alloc is not None and alloc.local_ptr == a_shared.data_ptr() and a_shared.is_contiguous() and not _log.dump_enabled():
             gathered = torch.empty_like(a_shared) if a_out is None else a_out
-            c = _host.gemm(a_shared, b, False, 0, False, -1, 0, 0, 1, gathered)
+            c = _host.gemm(a_shared, b, False, 0, False, -1, 0, 0, 1, gathered, False)
             if c is not None:
                 if progress is not None:
                     progress.fill_(1)
@@ -298,7 +299,7 @@ def gemm_one_shot_all_reduce(a: torch.Tensor, b: torch.Tensor, **kwargs) -> torc
     if a.device.type != "cuda":
         return ref.gemm_all_reduce(a, b, group)
     if symm_mem.solo(group):
-        out = _host.gemm(a, b, True, 0, True, -1, 0, 0, 1, None)
+        out = _host.gemm(a, b, True, 0, True, -1, 0, 0, 1, None, False)
         if out is not None:
             return out
     tf32 = use_tf32(a, b)
@@ -365,7 +366,7 @@ def gemm_reduce_scatter(a: torch.Tensor, b: torch.Tensor, **kwargs) -> torch.Ten
     if a.device.type != "cuda":
         return ref.gemm_reduce_scatter(a, b, group)
     if not kwargs.keys() - {"group"} and symm_mem.solo(group) and not _log.dump_enabled():
-        out = _host.gemm(a, b, False, 0, False, -1, 0, 0, 1, None)
+        out = _host.gemm(a, b, False, 0, False, -1, 0, 0, 1, None, False)
         if out is not None:
             return out
     a2, lda = as_k_major_a(a)

@@ -442,7 +442,7 @@ def test_one_rank_all_gather_matmul_and_activation(M, N, K):
     _close(h, torch.nn.functional.gelu(ref, approximate="tanh"), K)
 
 
-@pytest.mark.parametrize("bn", [1128, 1160, 1192, 1224, 1256, 2128, 2160, 2192, 2224, 2256])
+@pytest.mark.parametrize("bn", [1064, 1096, 2064, 2096, 1128, 1160, 1192, 1224, 1256, 2128, 2160, 2192, 2224, 2256])
 @pytest.mark.parametrize("swap", [0, 1])
 def test_gemm_persistent_pairs_every_tile_shape(bn, swap):
     # row blocks x columns as 1000 * b + n; the last wave of two-block tiles is dealt as single blocks
