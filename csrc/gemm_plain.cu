@@ -47,26 +47,24 @@ struct PlainPlan {
 // (a row length of an odd number of 16-byte units): each 128 bytes then cost a fifth sector.
 static int row_class(long long ld, int elt) { return ld * elt % 128 == 0 ? 0 : ld * elt % 32 == 0 ? 1 : 2; }
 
-// Time model of the pair kernels, in microseconds, fitted to long runs on a B200 with every SM busy, i.e. at
-// the power limit: per K block (64 bf16 or 32 fp32 columns of K) 0.299 for the MMAs of 256 x 256 and 0.0054 per
-// KB of operands a CTA fetches, by the class of their rows (4096 x 4096 x 9512 against x 9472: 256 x 256 tiles
-// 308 / 256 us, 512 x 256 266 / 249, 256 x 128 388 / 292).
+// Time model of the pair kernels, in microseconds, fitted to runs of every tile shape and split on 35 ragged and 4
+// aligned problems on a B200 (it picks within 5 % of the best on average): per K block (64 bf16 or 32 fp32
+// columns of K) 0.284 for the MMAs of 256 x 256 and a price per KB of operands that a CTA fetches, by the class
+// of their rows (4096 x 4096 x 9512 against x 9472: 256 x 256 tiles 308 / 256 us, 512 x 256 266 / 249).
 static double block_us(int bn, int rb, int class_r, int class_c) {
-  static const double kByClass[3] = {1.0, 1.07, 1.5};
-  return (0.299 * rb * bn / 256 + 0.0054 * (16 * rb * kByClass[class_r] + bn / 16.0 * kByClass[class_c])) * (rb == 2 ? 1.03 : 1.0);
+  static const double kPerKb[3] = {0.0035, 0.0051, 0.0105};
+  return 0.284 * rb * bn / 256 + kPerKb[class_r] * 16 * rb + kPerKb[class_c] * bn / 16.0;
 }
-// With fewer SMs busy the rest run faster, up to full clock.
-static double clock_factor(double busy) { return std::max(0.64, std::sqrt(busy)); }
 
-static double flow_us(int rows, int cols, int num_kb, int bn, int rb, int pairs, int class_r, int class_c) {
+static double flow_us(int rows, int cols, int num_kb, int bn, int rb, int pairs, int class_r, int class_c, double hbm_us) {
   const int T = ((rows + 256 * rb - 1) / (256 * rb)) * ((cols + bn - 1) / bn);
   const int whole = T / pairs, rest = T % pairs;
   const double full = num_kb * block_us(bn, rb, class_r, class_c);
-  double last = rest ? full * clock_factor((double)rest / pairs) : 0.0;
-  if (rb == 2 && rest && 2 * rest <= pairs) last = num_kb * block_us(bn, 1, class_r, class_c) * clock_factor(2.0 * rest / pairs);
+  double last = rest ? full * busy_factor((double)rest / pairs) : 0.0;
+  if (rb == 2 && rest && 2 * rest <= pairs) last = num_kb * block_us(bn, 1, class_r, class_c) * busy_factor(2.0 * rest / pairs);
   // what is not hidden: start and last epilogue, and with one accumulator set the epilogue of every tile
-  const double bubble = 2 * rb * bn <= 512 ? 0.0 : 3.5;
-  return whole * (full + bubble) + last + 8.0;
+  const double bubble = 2 * rb * bn <= 512 ? 0.0 : 3.8;
+  return std::max(whole * (full + bubble) + last, hbm_us) + 6.3;
 }
 
 static PlainPlan plain_plan(const DeviceState* d, int M, int N, int K, int elt, int swap_ab, int bn_override, int use_pair,
@@ -79,6 +77,7 @@ static PlainPlan plain_plan(const DeviceState* d, int M, int N, int K, int elt, 
   if (max_ctas > 0 && max_ctas < cap) cap = max_ctas;
   const bool pair_ok = use_pair != 0 && pair_enabled() && !emu && cap >= 2;
   const int num_kb = (K + 128 / elt - 1) / (128 / elt), pairs = cap / 2;
+  const double hbm_us = ((double)M + N) * K * elt / 5e6;         // with the rate that short kernels reach
   const bool whole_chip = max_ctas <= 0 && !emu;
   pl.swap = swap_ab < 0 ? (M <= 64 && N >= 128) : swap_ab != 0;
   if (bn_override >= 1000 && pair_ok) {
@@ -97,8 +96,9 @@ static PlainPlan plain_plan(const DeviceState* d, int M, int N, int K, int elt, 
       if (whole_chip && cols <= 128) {
         // single CTAs of 128 x 128: up to eight K splits (100 x 4000 x 9000 21 us, with pairs 27)
         const int tiles = (rows + kBM - 1) / kBM;
+        const double single_us = 1.06 * (0.142 + 2 * (block_us(128, 1, cr, cc) - 0.142) / 1.5);      // 32 KB a stage, not 24
         double us = 1e30;
-        const int s = tiles <= d->num_sms ? tile_gemm_splits(d, tiles, num_kb, 128, false, elt, 0.36 / 0.324 * (block_us(128, 1, cr, cc) + 0.0054 * 8), &us) : 0;
+        const int s = tiles <= d->num_sms ? tile_gemm_splits(d, tiles, num_kb, 128, false, elt, single_us, hbm_us, &us) : 0;
         if (s > 0 && us < best) {
           best = us;
           pl.kind = PLAIN_TILE; pl.swap = swap != 0; pl.pair = false; pl.bn = 128; pl.splits = s; pl.rb = 1;
@@ -109,7 +109,7 @@ static PlainPlan plain_plan(const DeviceState* d, int M, int N, int K, int elt, 
         if (whole_chip && bn >= 128) {
           const int tiles = ((rows + 255) / 256) * ((cols + bn - 1) / bn);
           double us = 1e30;
-          const int s = tiles <= pairs ? tile_gemm_splits(d, tiles, num_kb, bn, true, elt, block_us(bn, 1, cr, cc), &us) : 0;
+          const int s = tiles <= pairs ? tile_gemm_splits(d, tiles, num_kb, bn, true, elt, block_us(bn, 1, cr, cc), hbm_us, &us) : 0;
           if (s > 0 && us < best) {
             best = us;
             pl.kind = PLAIN_TILE; pl.swap = swap != 0; pl.pair = true; pl.bn = bn; pl.splits = s;
@@ -118,7 +118,7 @@ static PlainPlan plain_plan(const DeviceState* d, int M, int N, int K, int elt, 
         for (int rb = 1; rb <= 2; ++rb) {
           if (rb == 2 && rows <= 256) continue;
           // a transposed store writes shorter runs: row-major unless the other way saves something
-          const double us = flow_us(rows, cols, num_kb, bn, rb, pairs, cr, cc) * (swap ? 1.02 : 1.0);
+          const double us = flow_us(rows, cols, num_kb, bn, rb, pairs, cr, cc, hbm_us) * (swap ? 1.056 : 1.0);
           if (us < best) {
             best = us;
             pl.kind = PLAIN_FLOW; pl.swap = swap != 0; pl.pair = true; pl.bn = bn; pl.rb = rb; pl.splits = 0; pl.workers = pairs;
@@ -138,7 +138,7 @@ static PlainPlan plain_plan(const DeviceState* d, int M, int N, int K, int elt, 
   if (elt == 4 && pl.bn == 128) pl.bn = 256;
   const int tiles = ((rows + kBM - 1) / kBM) * ((cols + pl.bn - 1) / pl.bn);
   if (swap_ab < 0 && bn_override <= 0 && whole_chip && tiles <= d->num_sms) {
-    pl.splits = tile_gemm_splits(d, tiles, num_kb, pl.bn, false, elt, 0.25, nullptr);
+    pl.splits = tile_gemm_splits(d, tiles, num_kb, pl.bn, false, elt, 0.25, hbm_us, nullptr);
     if (pl.splits > 0) {
       pl.kind = PLAIN_TILE;
       return pl;

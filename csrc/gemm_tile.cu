@@ -379,23 +379,24 @@ static int max_clusters(int device, const TileVariant& v, unsigned cluster) {
 }
 
 // The split count of a one-wave problem, 0 when its tiles do not fit the chip at once, and its time (us).
-// block_us: one K block with every SM busy (less when fewer are; single CTAs of narrow tiles are bound by
-// their loads, not by the clock), but never below the operands' time out of HBM, plus what summing S splits
-// adds: little for the narrow tiles of single CTAs, a lot once a cluster of pairs spans more than four CTAs
-// (M = 256, N = 4096, K = 2048: 1 / 2 / 3 splits 17.5 / 14.2 / 20.5 us).
-int tile_gemm_splits(const DeviceState* d, int tiles, int num_kb, int bn, bool pair, int elt, double block_us, double* us_out) {
+// block_us: one K block with every SM busy (less when fewer are; single CTAs of up to 64 columns are bound by
+// their loads, not by the clock), but never below the operands' time out of HBM (hbm_us), plus what summing S
+// splits adds: little for single CTAs, a lot once a cluster of pairs spans more than four CTAs (M = 256,
+// N = 4096, K = 2048: 1 / 2 / 3 splits 17.5 / 14.2 / 20.5 us). A pair without splits is left to the persistent
+// kernel, which stores faster (373 x 8000 x 7768: 57 us against 71).
+int tile_gemm_splits(const DeviceState* d, int tiles, int num_kb, int bn, bool pair, int elt, double block_us, double hbm_us,
+                     double* us_out) {
   const TileVariant v = elt == 4 ? tile_variant<4>(bn, pair) : tile_variant<2>(bn, pair);
   if (v.fn == nullptr) return 0;
   const int ctas = pair ? 2 : 1, most = 8 / ctas;
-  const double hbm_us = (double)tiles * ctas * num_kb * kBM * 128 / 6.5e6;
-  auto sum_us = [&](int s) { return !pair ? 0.25 * s : (s <= 2 ? 1.5 * s : 4.0 * s - 2.0) * bn / 256; };
+  auto sum_us = [&](int s) { return !pair ? 0.25 * s : (s <= 2 ? 0.6 * s : 3.3 * s - 2.0) * bn / 256; };
   int best = 0;
   double best_us = 1e30;
-  for (int s = 1; s <= most && (s == 1 || num_kb >= 4 * s); ++s) {
+  for (int s = pair ? 2 : 1; s <= most && (s == 1 || num_kb >= 4 * s); ++s) {
     if (tiles * s * ctas > d->num_sms || tiles > max_clusters(d->device, v, (unsigned)(s * ctas))) continue;
     const double busy = (double)tiles * s * ctas / d->num_sms;
-    const double kb_us = pair ? block_us * std::max(0.64, std::sqrt(busy)) : block_us;
-    const double us = std::max((num_kb + s - 1) / s * kb_us, hbm_us) + sum_us(s) + 8.0;
+    const double kb_us = pair || bn == 128 ? block_us * busy_factor(busy) : block_us;
+    const double us = std::max((num_kb + s - 1) / s * kb_us, hbm_us) + sum_us(s) + 6.9;
     if (us < best_us) {
       best_us = us;
       best = s;

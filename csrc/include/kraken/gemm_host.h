@@ -1,6 +1,8 @@
 // Host-side helpers shared by the GEMM translation units: the tensor-map cache, tiling defaults
 // and the operand set-up of C[M,N] = A[M,K] * Bt[N,K]^T. Defined in gemm.cu.
 #pragma once
+#include <algorithm>
+#include <cmath>
 #include "kraken/driver_api.h"
 #include "kraken/gemm_core.cuh"
 
@@ -25,9 +27,11 @@ int launch_gemm_tf32(int bn, const GemmParams& p, unsigned nb, cudaStream_t stre
 int launch_gemm_ar(int bn, const GemmParams& p, unsigned nb, cudaStream_t stream);
 // Routes a parameter block to the kernel family of its mode and operand type (gemm.cu).
 int launch_gemm(int bn, const GemmParams& p, unsigned nb, cudaStream_t stream);
+// Fewer SMs busy run faster (power), up to full clock.
+inline double busy_factor(double busy) { return std::max(0.75, std::pow(busy, 0.28)); }
 // One-wave GEMM (gemm_tile.cu): the most K splits with which `tiles` tiles of this kernel run at once,
-// 0 when it does not apply, and its estimated time (block_us: one K block of a tile); and its launch.
-int tile_gemm_splits(const DeviceState* d, int tiles, int num_kb, int bn, bool pair, int elt, double block_us, double* us);
+// 0 when it does not apply, and its estimated time (block_us: one K block of a tile, hbm_us: the operands' time out of HBM); and its launch.
+int tile_gemm_splits(const DeviceState* d, int tiles, int num_kb, int bn, bool pair, int elt, double block_us, double hbm_us, double* us);
 // Persistent pairs that draw their tiles in order (gemm_flow.cu); sched: two zero words, zero again afterwards.
 int launch_flow_gemm(const GemmParams& g, int bn, int rb, int pairs, uint32_t* sched, cudaStream_t stream);
 int launch_tile_gemm(const GemmParams& g, int bn, bool pair, int splits, cudaStream_t stream);

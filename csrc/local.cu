@@ -170,6 +170,8 @@ __global__ void __launch_bounds__(T) norm_stream_kernel(const LocalNormParams p,
 // Rows longer than the register budget: two passes over global memory.
 __global__ void __launch_bounds__(kNormMaxThreads) rms_norm_long_kernel(const LocalNormParams p) {
   __shared__ float smem[32];
+  pdl_launch();
+  pdl_wait();
   const int nvec = p.D / 8;
   const char* xrow = (const char*)p.x + (size_t)blockIdx.x * p.D * 2;
   char* yrow = (char*)p.y + (size_t)blockIdx.x * p.D * 2;
