@@ -437,7 +437,7 @@ constexpr size_t kTmapCacheEntries = 4096;
 static unsigned long long g_tmap_hits = 0, g_tmap_misses = 0;
 
 // Tensor map of a row-major matrix [rows, cols] of bf16 (elt 2) or fp32 (elt 4) elements (cols
-// contiguous, `ld` elements per row), box = box_bytes (128 or 64) of columns x box_rows rows, swizzled by as much,
+// contiguous, `ld` elements per row), box = box_bytes (128, 64 or, unswizzled, 32) of columns x box_rows rows, swizzled by as much,
 // out-of-range elements read as zero.
 int get_tmap(const void* ptr, unsigned long long rows, unsigned long long cols, unsigned long long ld,
                     unsigned box_rows, CUtensorMap* out, int elt, unsigned box_bytes, bool promote_256) {
@@ -462,7 +462,7 @@ int get_tmap(const void* ptr, unsigned long long rows, unsigned long long cols, 
   CUtensorMap m;
   KR_CU(cuTensorMapEncodeTiled, &m, elt == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
         const_cast<void*>(ptr), gdim, gstride, box,
-        estr, CU_TENSOR_MAP_INTERLEAVE_NONE, box_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, promote_256 ? CU_TENSOR_MAP_L2_PROMOTION_L2_256B : CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+        estr, CU_TENSOR_MAP_INTERLEAVE_NONE, box_bytes == 32 ? CU_TENSOR_MAP_SWIZZLE_NONE : box_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, promote_256 ? CU_TENSOR_MAP_L2_PROMOTION_L2_256B : CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   {
     std::lock_guard<std::mutex> lk(g_tmap_mu);

@@ -9,7 +9,7 @@
 //  * RB = 2 row blocks: a pair computes 512 x 256, each operand stage feeds twice the MMAs (48 KB instead of 64
 //    per CTA and 256 x 256 x 64 block pair). The accumulators then fill TMEM, so a tile's first MMAs wait for the
 //    epilogue of the one before, row block by row block. RB = 1 keeps two accumulators in turn.
-// Narrower column tiles (BN) fit ragged sizes and waves better; the launcher picks (flow_plan).
+// Column tiles (BN) of 64 ... 256, in steps of 16 from 128 on for bf16, fit ragged sizes and waves; the launcher picks.
 //
 // Warps: 0 TMA producer (the leader's also draws the tiles), 1 MMA issuer (leader), 2-5 epilogue (one per TMEM
 // lane quarter), 6-7 optional copy of the row operand. The common epilogues (MODE) are kernels of their own: with
@@ -26,7 +26,7 @@ constexpr int kFlowCopyThreads = 64;
 constexpr int kFlowSlots = 16;                            // more than the slowest role can be behind the producer, see next_item
 
 struct alignas(64) FlowParams {
-  CUtensorMap tmap_r, tmap_c, tmap_out;
+  CUtensorMap tmap_r, tmap_c, tmap_out, tmap_tail;      // tmap_tail: the last 16 columns of tiles with BN % 32 == 16
   int tiles_r, tiles_c, num_kb, group_r;                  // tiles of RB * 256 rows
   int items, split_from;                                  // tiles from split_from on are drawn as single row blocks
   int transposed, out_fp32, act;
@@ -48,11 +48,12 @@ struct FlowCfg {
   static constexpr int EPI = kFlowEpiWarps * 8192;       // two panel slots per warp
   static constexpr int RAW_STAGES = (kSmemLimit - 1024 - EPI - 512) / STAGE;
   static constexpr int STAGES = RAW_STAGES > 8 ? 8 : RAW_STAGES;
-  static constexpr int BUFS = 2 * RB * BN <= 512 ? 2 : 1;
-  static constexpr int UNITS = BUFS * RB;                 // accumulators of BN columns
-  static constexpr int TMEM_COLS = UNITS * BN <= 256 ? 256 : 512;
+  static constexpr int UNIT = (BN + 31) / 32 * 32;        // TMEM columns of an accumulator: read in chunks of 32
+  static constexpr int BUFS = 2 * RB * UNIT <= 512 ? 2 : 1;
+  static constexpr int UNITS = BUFS * RB;                 // accumulators
+  static constexpr int TMEM_COLS = UNITS * UNIT <= 256 ? 256 : 512;
   static constexpr int SMEM = 1024 + STAGES * STAGE + EPI + 512;
-  static_assert(BN % 32 == 0 && BN >= 64 && BN <= 256 && UNITS <= 4 && STAGES >= 3, "tile shape");
+  static_assert(BN % 16 == 0 && BN >= 64 && BN <= 256 && UNITS <= 4 && STAGES >= 3, "tile shape");
   static_assert(16 * STAGES + 16 * UNITS + 12 * kFlowSlots + 8 <= 512, "barrier area");
   static_assert(STAGES + BUFS + 2 < kFlowSlots, "a role could be lapped");
 };
@@ -139,12 +140,12 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
   pdl_launch();
   pdl_wait();
 
-  // A staged panel of 32 rows x `cols` columns to an output that TMA cannot describe (rows not whole 16-byte
+  // A staged panel of `rows` x `cols` to an output that TMA cannot describe (rows not whole 16-byte
   // units), element by element.
-  auto store_plain = [&](uint32_t panel, int gx, int gy, int cols, bool fp32, int ln) {
-    const int elt = fp32 ? 4 : 2, pitch = cols * elt, mask = pitch == 128 ? 7 : 3;
-    for (int r = 0; r < 32 && gy + r < p.out_rows; ++r) {
-      const int perm = pitch == 128 ? (r & mask) : ((r >> 1) & mask);
+  auto store_plain = [&](uint32_t panel, int gx, int gy, int cols, int rows, bool fp32, int ln) {
+    const int elt = fp32 ? 4 : 2, pitch = cols * elt;
+    for (int r = 0; r < rows && gy + r < p.out_rows; ++r) {
+      const int perm = pitch == 128 ? (r & 7) : pitch == 64 ? ((r >> 1) & 3) : 0;
       for (int c = ln; c < cols && gx + c < p.out_cols; c += 32) {
         const uint32_t a = panel + (uint32_t)(r * pitch + ((((c * elt) >> 4) ^ perm) << 4) + ((c * elt) & 15));
         const long long o = (long long)(gy + r) * p.ldo + gx + c;
@@ -244,7 +245,7 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
               tc_fence_after();
             }
             const uint64_t adesc = make_smem_desc_sw128(sa + rb * Cfg::A_BYTES);
-            const uint32_t d_tmem = tmem_base + (uint32_t)(u * BN);
+            const uint32_t d_tmem = tmem_base + (uint32_t)(u * Cfg::UNIT);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               const uint32_t accumulate = (kb > 0 || i != 0) ? 1u : 0u;
@@ -270,7 +271,8 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
     const int q = warp & 3;                                // TMEM lane quarter
     const uint32_t slots = epi0 + (uint32_t)(warp - 2) * 8192u;
     constexpr int PW = BN % 64 == 0 ? 64 : 32;             // columns per panel of a bf16 row-major tile
-    constexpr int CHUNKS = BN / 32;
+    constexpr int CHUNKS = Cfg::UNIT / 32;
+    constexpr bool TAIL = BN % 32 != 0;                    // the last chunk is 16 columns wide
     const bool fp32 = MODE == FLOW_ANY && p.out_fp32 != 0, transposed = MODE == FLOW_ANY && p.transposed != 0;
     const bool act = MODE == FLOW_ROWS_ACT || (MODE == FLOW_ANY && p.act != 0);
     uint32_t uph = 0, sent = 0;
@@ -287,7 +289,7 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
         if (!ok) break;
         uph ^= 1u << u;
         tc_fence_after();
-        const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(u * BN);
+        const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(u * Cfg::UNIT);
         const int drow = it.tr * (RB * 256) + rb * 256 + (int)cta * kBM + q * 32;      // first row of D of this warp
         auto release = [&] {      // this warp has read its part of the accumulator
           tc_fence_before();
@@ -301,19 +303,20 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
           return slots + (sent++ & 1u) * 4096u;
         };
         // A panel in a slot goes out: rows gy ..., columns gx ... of the output
-        auto send = [&](uint32_t slot, int gx, int gy, int cols) {
+        auto send = [&](uint32_t slot, int gx, int gy, int cols, int rows, bool tail) {
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
-            if ((MODE != FLOW_ANY || p.out == nullptr) && gx < p.out_cols && gy < p.out_rows) tma_store_2d(&p.tmap_out, slot, gx, gy);
+            if ((MODE != FLOW_ANY || p.out == nullptr) && gx < p.out_cols && gy < p.out_rows) tma_store_2d(tail ? &p.tmap_tail : &p.tmap_out, slot, gx, gy);
             bulk_commit_group();
           }
-          if (MODE == FLOW_ANY && p.out != nullptr) store_plain(slot, gx, gy, cols, fp32, lane);
+          if (MODE == FLOW_ANY && p.out != nullptr) store_plain(slot, gx, gy, cols, rows, fp32, lane);
         };
         if (MODE == FLOW_ANY && (fp32 || transposed)) {
 #pragma unroll 1
           for (int i = 0; i < CHUNKS; ++i) {
             const int col = i * 32;
+            const bool tail = TAIL && i + 1 == CHUNKS;
             uint32_t r[32];
             tmem_ld32(t_addr + (uint32_t)col, r);
             tmem_ld_wait();
@@ -337,12 +340,15 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
                                "h"(*reinterpret_cast<const unsigned short*>(&v)) : "memory");
                 }
               }
-              send(slot, drow, it.tc * BN + col, 32);
+              send(slot, drow, it.tc * BN + col, 32, tail ? 16 : 32, tail);
             } else {
 #pragma unroll
-              for (int v = 0; v < 8; ++v)
-                st_shared_u4(slot + lane * 128u + (uint32_t)((v ^ (lane & 7)) << 4), r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3]);
-              send(slot, it.tc * BN + col, drow, 32);
+              for (int v = 0; v < 8; ++v) {
+                if (tail && v >= 4) continue;
+                const uint32_t a = tail ? slot + lane * 64u + (uint32_t)((v ^ ((lane >> 1) & 3)) << 4) : slot + lane * 128u + (uint32_t)((v ^ (lane & 7)) << 4);
+                st_shared_u4(a, r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3]);
+              }
+              send(slot, it.tc * BN + col, drow, tail ? 16 : 32, 32, tail);
             }
           }
         } else {
@@ -374,12 +380,15 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
             if (PW == 32 || (i & 1) == 0) slot = next_slot();
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
-              const uint32_t a = PW == 64 ? slot + lane * 128u + (uint32_t)((((i & 1) * 4 + v) ^ (lane & 7)) << 4)
+              const bool tail = TAIL && i + 1 == CHUNKS;
+              if (tail && v >= 2) continue;
+              const uint32_t a = tail ? slot + lane * 32u + v * 16u : PW == 64 ? slot + lane * 128u + (uint32_t)((((i & 1) * 4 + v) ^ (lane & 7)) << 4)
                                           : slot + lane * 64u + (uint32_t)((v ^ ((lane >> 1) & 3)) << 4);
               st_shared_u4(a, packed[i][4 * v], packed[i][4 * v + 1], packed[i][4 * v + 2], packed[i][4 * v + 3]);
             }
-            if (PW == 32) send(slot, it.tc * BN + i * 32, drow, 32);
-            else if ((i & 1) == 1) send(slot, it.tc * BN + i * 32 - 32, drow, 64);
+            if (TAIL && i + 1 == CHUNKS) send(slot, it.tc * BN + i * 32, drow, 16, 32, true);
+            else if (PW == 32) send(slot, it.tc * BN + i * 32, drow, 32, 32, false);
+            else if ((i & 1) == 1) send(slot, it.tc * BN + i * 32 - 32, drow, 64, 32, false);
           }
         }
       }
@@ -434,6 +443,16 @@ static FlowVariant flow_variant(int bn, int rb) {
   KR_FLOW(128, 1)
   KR_FLOW(96, 1)
   KR_FLOW(64, 1)
+  if constexpr (ELT == 2) {
+    KR_FLOW(240, 2)
+    KR_FLOW(208, 2)
+    KR_FLOW(176, 2)
+    KR_FLOW(144, 2)
+    KR_FLOW(240, 1)
+    KR_FLOW(208, 1)
+    KR_FLOW(176, 1)
+    KR_FLOW(144, 1)
+  }
 #undef KR_FLOW
   return {nullptr, 0};
 }
@@ -452,6 +471,9 @@ int launch_flow_gemm(const GemmParams& g, int bn, int rb, int pairs, uint32_t* s
   const unsigned box_bytes = (out_elt == 4 || (!g.transposed && bn % 64 == 0)) ? 128u : 64u;
   if (tma_out) {
     int rc = get_tmap(g.out, g.out_rows, g.out_cols, g.ldo, 32, &p.tmap_out, out_elt, box_bytes);
+    if (!rc && bn % 32 != 0)
+      rc = g.transposed ? get_tmap(g.out, g.out_rows, g.out_cols, g.ldo, 16, &p.tmap_tail, out_elt, box_bytes)
+                        : get_tmap(g.out, g.out_rows, g.out_cols, g.ldo, 32, &p.tmap_tail, out_elt, 16u * out_elt);
     if (rc) return rc;
   } else {
     p.tmap_out = g.tmap_r;          // prefetched, not used

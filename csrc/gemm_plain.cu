@@ -53,7 +53,10 @@ static int row_class(long long ld, int elt) { return ld * elt % 128 == 0 ? 0 : l
 // of their rows (4096 x 4096 x 9512 against x 9472: 256 x 256 tiles 308 / 256 us, 512 x 256 266 / 249).
 static double block_us(int bn, int rb, int class_r, int class_c) {
   static const double kPerKb[3] = {0.0035, 0.0051, 0.0105};
-  return 0.284 * rb * bn / 256 + kPerKb[class_r] * 16 * rb + kPerKb[class_c] * bn / 16.0;
+  // Two row blocks: fewer and larger stages in flight, which shows while the fetches are not what bounds the block
+  // (2048 x 3584 x 8192: 512 x 224 tiles in one wave 90-100 us, 256 x 208 in two 86-92).
+  const double two = rb == 2 && class_r < 2 && class_c < 2 ? 1.045 : 1.0;
+  return (0.284 * rb * bn / 256 + kPerKb[class_r] * 16 * rb + kPerKb[class_c] * bn / 16.0) * two;
 }
 
 static double flow_us(int rows, int cols, int num_kb, int bn, int rb, int pairs, int class_r, int class_c, double hbm_us) {
@@ -63,7 +66,7 @@ static double flow_us(int rows, int cols, int num_kb, int bn, int rb, int pairs,
   double last = rest ? full * busy_factor((double)rest / pairs) : 0.0;
   if (rb == 2 && rest && 2 * rest <= pairs) last = num_kb * block_us(bn, 1, class_r, class_c) * busy_factor(2.0 * rest / pairs);
   // what is not hidden: start and last epilogue, and with one accumulator set the epilogue of every tile
-  const double bubble = 2 * rb * bn <= 512 ? 0.0 : 3.8;
+  const double bubble = 2 * rb * bn <= 512 ? 0.0 : 3.2;
   return std::max(whole * (full + bubble) + last, hbm_us) + 6.3;
 }
 
@@ -104,9 +107,10 @@ static PlainPlan plain_plan(const DeviceState* d, int M, int N, int K, int elt, 
           pl.kind = PLAIN_TILE; pl.swap = swap != 0; pl.pair = false; pl.bn = 128; pl.splits = s; pl.rb = 1;
         }
       }
-      for (int bn = 64; bn <= 256; bn += 32) {
-        if (bn > 64 && bn - 32 >= cols) continue;                    // wider than needed
-        if (whole_chip && bn >= 128) {
+      for (int bn = 64, step; bn <= 256; bn += step) {
+        step = bn >= 128 && elt == 2 ? 16 : 32;
+        if (bn > 64 && bn - step >= cols) continue;                  // wider than needed
+        if (whole_chip && bn >= 128 && bn % 32 == 0) {
           const int tiles = ((rows + 255) / 256) * ((cols + bn - 1) / bn);
           double us = 1e30;
           const int s = tiles <= pairs ? tile_gemm_splits(d, tiles, num_kb, bn, true, elt, block_us(bn, 1, cr, cc), hbm_us, &us) : 0;
