@@ -33,7 +33,7 @@ HOST_PATH = OUT_DIR / (HOST_NAME + ".so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
-    "-std=c++17", "-O3", "-lineinfo",
+    "-std=c++17", "-O3", "-lineinfo", "--split-compile=0",
     "-Xcompiler", "-fPIC",
     "-Xcompiler", "-fvisibility=hidden",
 ]
