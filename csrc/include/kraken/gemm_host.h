@@ -30,11 +30,12 @@ int launch_gemm(int bn, const GemmParams& p, unsigned nb, cudaStream_t stream);
 // Fewer SMs busy run faster (power), up to full clock.
 inline double busy_factor(double busy) { return std::max(0.75, std::pow(busy, 0.28)); }
 // One-wave GEMM (gemm_tile.cu): the most K splits with which `tiles` tiles of this kernel run at once,
-// 0 when it does not apply, and its estimated time (block_us: one K block of a tile, hbm_us: the operands' time out of HBM); and its launch.
+// 0 when it does not apply, and its estimated time (block_us: one K block of a tile, hbm_us:
+// the operands' time out of HBM); and its launch.
 int tile_gemm_splits(const DeviceState* d, int tiles, int num_kb, int bn, bool pair, int elt, double block_us, double hbm_us, double* us);
+int launch_tile_gemm(const GemmParams& g, int bn, bool pair, int splits, cudaStream_t stream);
 // Persistent pairs that draw their tiles in order (gemm_flow.cu); sched: two zero words, zero again afterwards.
 int launch_flow_gemm(const GemmParams& g, int bn, int rb, int pairs, uint32_t* sched, cudaStream_t stream);
-int launch_tile_gemm(const GemmParams& g, int bn, bool pair, int splits, cudaStream_t stream);
 int pick_bn(int rows_c);      // column-tile width for `rows_c` rows of the column operand
 int tf32_bn(int rows_c);      // the same among the widths the tf32 kernels exist for
 
