@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
     constexpr int CHUNKS = Cfg::UNIT / 32;
     constexpr bool TAIL = BN % 32 != 0;                    // the last chunk is 16 columns wide
     const bool fp32 = MODE == FLOW_ANY && p.out_fp32 != 0, transposed = MODE == FLOW_ANY && p.transposed != 0;
-    const bool act = MODE == FLOW_ROWS_ACT || (MODE == FLOW_ANY && p.act != 0);
+    const bool act = MODE == FLOW_ANY && p.act != 0;
     uint32_t uph = 0, sent = 0;
     bool ok = true;
     int t = pair;
@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
           }
           if (MODE == FLOW_ANY && p.out != nullptr) store_plain(slot, gx, gy, cols, rows, fp32, lane);
         };
-        if (MODE == FLOW_ANY && (fp32 || transposed)) {
+        if (MODE == FLOW_ANY && (fp32 || transposed || act)) {
 #pragma unroll 1
           for (int i = 0; i < CHUNKS; ++i) {
             const int col = i * 32;
@@ -341,6 +341,17 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
                 }
               }
               send(slot, drow, it.tc * BN + col, 32, tail ? 16 : 32, tail);
+            } else if (!fp32) {
+#pragma unroll
+              for (int v = 0; v < 4; ++v) {
+                if (tail && v >= 2) continue;
+                uint32_t w[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) w[j] = pack_bf16x2(__uint_as_float(r[8 * v + 2 * j]), __uint_as_float(r[8 * v + 2 * j + 1]));
+                const uint32_t a = tail ? slot + lane * 32u + v * 16u : slot + lane * 64u + (uint32_t)((v ^ ((lane >> 1) & 3)) << 4);
+                st_shared_u4(a, w[0], w[1], w[2], w[3]);
+              }
+              send(slot, it.tc * BN + col, drow, tail ? 16 : 32, 32, tail);
             } else {
 #pragma unroll
               for (int v = 0; v < 8; ++v) {
@@ -352,31 +363,38 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
             }
           }
         } else {
-          // bf16 rows: everything is read and rounded before anything is stored, so that the next tile's MMAs
-          // wait for nothing but TMEM reads; the activation follows on the rounded values, as it would on a
-          // bf16 tensor.
+          // bf16 rows: everything is read, activated (on the fp32 sums) and rounded before anything is stored, so
+          // that the next tile's MMAs do not wait for stores. With an activation 16 columns at a time: more raw
+          // sums next to the rounded ones would spill.
           uint32_t packed[CHUNKS][16];
+          if (MODE == FLOW_ROWS_ACT) {
 #pragma unroll
-          for (int i = 0; i < CHUNKS; i += 2) {
-            uint32_t r0[32], r1[32];
-            tmem_ld32(t_addr + (uint32_t)(i * 32), r0);
-            if (i + 1 < CHUNKS) tmem_ld32(t_addr + (uint32_t)(i * 32 + 32), r1);
-            tmem_ld_wait();
+            for (int i = 0; i < BN / 16; ++i) {
+              uint32_t raw[32];
+              tmem_ld16(t_addr + (uint32_t)(i * 16), raw);
+              tmem_ld_wait();
 #pragma unroll
-            for (int v = 0; v < 16; ++v) {
-              packed[i][v] = pack_bf16x2(__uint_as_float(r0[2 * v]), __uint_as_float(r0[2 * v + 1]));
-              if (i + 1 < CHUNKS) packed[i + 1 < CHUNKS ? i + 1 : i][v] = pack_bf16x2(__uint_as_float(r1[2 * v]), __uint_as_float(r1[2 * v + 1]));
+              for (int v = 0; v < 8; ++v)
+                packed[i / 2][i % 2 * 8 + v] = pack_bf16x2(gelu_tanh(__uint_as_float(raw[2 * v])), gelu_tanh(__uint_as_float(raw[2 * v + 1])));
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < CHUNKS; i += 2) {
+              uint32_t r0[32], r1[32];
+              tmem_ld32(t_addr + (uint32_t)(i * 32), r0);
+              if (i + 1 < CHUNKS) tmem_ld32(t_addr + (uint32_t)(i * 32 + 32), r1);
+              tmem_ld_wait();
+#pragma unroll
+              for (int v = 0; v < 16; ++v) {
+                packed[i][v] = pack_bf16x2(__uint_as_float(r0[2 * v]), __uint_as_float(r0[2 * v + 1]));
+                if (i + 1 < CHUNKS) packed[i + 1 < CHUNKS ? i + 1 : i][v] = pack_bf16x2(__uint_as_float(r1[2 * v]), __uint_as_float(r1[2 * v + 1]));
+              }
             }
           }
           release();
           uint32_t slot = 0;
 #pragma unroll
           for (int i = 0; i < CHUNKS; ++i) {
-            if (act) {
-#pragma unroll
-              for (int v = 0; v < 16; ++v)
-                packed[i][v] = pack_bf16x2(gelu_tanh(bf16lo(packed[i][v])), gelu_tanh(bf16hi(packed[i][v])));
-            }
             if (PW == 32 || (i & 1) == 0) slot = next_slot();
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
@@ -468,7 +486,8 @@ int launch_flow_gemm(const GemmParams& g, int bn, int rb, int pairs, uint32_t* s
   p.tmap_r = g.tmap_r;
   p.tmap_c = g.tmap_c;
   const int out_elt = g.out_fp32 ? 4 : 2;
-  const unsigned box_bytes = (out_elt == 4 || (!g.transposed && bn % 64 == 0)) ? 128u : 64u;
+  // panels of 64 columns from the kernels that hold a tile's rounded rows, of 32 from those that go chunk by chunk
+  const unsigned box_bytes = (out_elt == 4 || (!g.transposed && bn % 64 == 0 && (rows || !g.act))) ? 128u : 64u;
   if (tma_out) {
     int rc = get_tmap(g.out, g.out_rows, g.out_cols, g.ldo, 32, &p.tmap_out, out_elt, box_bytes);
     if (!rc && bn % 32 != 0)

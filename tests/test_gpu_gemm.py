@@ -3,6 +3,8 @@
 matmuls of the same bf16 inputs. Shapes include the reference's test shapes scaled to fit one GPU
 (test/test_gemm_allreduce.py:57-117: 512x256x128, 256^3, rank-valued 32^3 with 1e-5 tolerance;
 test/test_gemm_reduce_scatter.py:44-115; test/test_allgather_matmul.py:47-81)."""
+import math
+
 import pytest
 import torch
 
@@ -459,3 +461,22 @@ def test_gemm_persistent_pairs_every_tile_shape(bn, swap):
                 assert ((c.float() - ref).norm() / ref.norm()).item() < 3e-3
     c = fused.matmul(a, bt.t(), bn=bn, swap_ab=swap, max_ctas=6)        # many tiles per pair
     assert ((c.float() - ref).norm() / ref.norm()).item() < 3e-3
+
+
+@pytest.mark.parametrize("M,N,bn,swap", [(520, 1024, 1256, 0), (1500, 2080, 2256, 0), (520, 1024, 2144, 0), (777, 1160, 1096, 0), (520, 1024, 1192, 1),
+                                         (520, 1001, 1144, 0), (520, 1001, 2128, 1), (16, 1024, 0, -1), (200, 520, 0, -1), (64, 136, 64, 0), (77, 520, 256, 0)])
+@pytest.mark.parametrize("out_fp32", [False, True])
+def test_activation_is_applied_to_the_fp32_sums_in_every_kernel(M, N, bn, swap, out_fp32):
+    # Operands are multiples of 1/32, so the sums are exact in fp32 and mostly not in bf16. What remains is one
+    # rounding of the result (8 significant bits: 2**-8 of the value) and the error of the device's exp and divide (below 1e-4).
+    from kraken_b200.fused.gemm_ops import _gemm
+
+    K = 72
+    g = torch.Generator().manual_seed(61)
+    a = (torch.randint(-32, 33, (M, K), generator=g) / 32).to(torch.bfloat16).cuda()
+    bt = (torch.randint(-32, 33, (N, K), generator=g) / 32).to(torch.bfloat16).cuda()
+    s = a.double() @ bt.double().t()
+    ref = s * torch.sigmoid(2 * (2 / math.pi) ** 0.5 * (s + 0.044715 * s ** 3))      # the tanh form, without its cancellation
+    h = _gemm(a, bt.t(), out_fp32, False, swap, bn, act="gelu_tanh").double()
+    worst = float(((h - ref).abs() / (ref.abs() + 1e-30)).max())
+    assert worst <= (0 if out_fp32 else 2.0 ** -8) + 1e-4, worst
