@@ -160,7 +160,9 @@ def all_gather_matmul(a_shared: torch.Tensor, b: torch.Tensor, a_out: torch.Tens
     if a_shared.is_cuda and a_shared.dim() == 2 and kwargs.get("backend") in (None, "auto", "push", "ce", "sm") and symm_mem.solo(group):
         # nothing to gather: one launch multiplies the shard in place and copies it to a_out on the side
         alloc = symm_mem.native_allocation(a_shared)
-        if alloc is not None and alloc.local_ptr == a_shared.data_ptr() and a_shared.is_contiguous() and not _log.dump_enabled():
+        # any other a_out that a copy accepts (or refuses) is the general path's to fill (or to refuse)
+        plain_out = a_out is None or (a_out.shape == a_shared.shape and not a_out.requires_grad)
+        if plain_out and alloc is not None and alloc.local_ptr == a_shared.data_ptr() and a_shared.is_contiguous() and not _log.dump_enabled():
             gathered = torch.empty_like(a_shared) if a_out is None else a_out
             c = _host.gemm(a_shared, b, False, 0, False, -1, 0, 0, 1, gathered, False)
             if c is not None:

@@ -480,3 +480,23 @@ def test_activation_is_applied_to_the_fp32_sums_in_every_kernel(M, N, bn, swap, 
     h = _gemm(a, bt.t(), out_fp32, False, swap, bn, act="gelu_tanh").double()
     worst = float(((h - ref).abs() / (ref.abs() + 1e-30)).max())
     assert worst <= (0 if out_fp32 else 2.0 ** -8) + 1e-4, worst
+
+
+def test_one_rank_all_gather_matmul_fills_a_out_like_a_copy():
+    # what a_out.copy_(a_shared) accepts is filled, what it refuses is refused
+    from kraken_b200.parallel import symm_mem
+
+    M, N, K = 96, 136, 64
+    a, bt = _ab(M, N, K, seed=42)
+    x = symm_mem.empty(M, K, dtype=torch.bfloat16, device="cuda")
+    x.copy_(a)
+    ref = fused.matmul(a, bt.t())
+    for out in (torch.zeros_like(a), torch.zeros(1, M, K, dtype=torch.bfloat16, device="cuda"), torch.zeros(M, K, device="cuda"),
+                torch.zeros(M, 2 * K, dtype=torch.bfloat16, device="cuda")[:, :K]):
+        gathered, c = fused.all_gather_matmul(x, bt.t(), a_out=out)
+        assert gathered is out and torch.equal(out.reshape(M, K).to(torch.bfloat16), a)
+        _close(c, ref.float(), K)
+    for out in (torch.zeros(K, M, dtype=torch.bfloat16, device="cuda"), torch.zeros(M * K, dtype=torch.bfloat16, device="cuda"),
+                torch.zeros(M, K, dtype=torch.bfloat16, device="cuda", requires_grad=True)):
+        with pytest.raises(RuntimeError):
+            fused.all_gather_matmul(x, bt.t(), a_out=out)
