@@ -491,7 +491,7 @@ int default_group_r() {
   return v;
 }
 
-static bool tma_store_enabled() {
+bool tma_store_enabled() {
   static int v = -1;
   if (v < 0) {
     const char* e = getenv("KRAKEN_TMA_STORE");

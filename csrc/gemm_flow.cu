@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
   pdl_wait();
 
   // A staged panel of `rows` x `cols` to an output that TMA cannot describe (rows not whole 16-byte
-  // units), element by element.
+  // units) or may not store to (KRAKEN_TMA_STORE=0), element by element.
   auto store_plain = [&](uint32_t panel, int gx, int gy, int cols, int rows, bool fp32, int ln) {
     const int elt = fp32 ? 4 : 2, pitch = cols * elt;
     for (int r = 0; r < rows && gy + r < p.out_rows; ++r) {
@@ -476,7 +476,7 @@ static FlowVariant flow_variant(int bn, int rb) {
 }
 
 int launch_flow_gemm(const GemmParams& g, int bn, int rb, int pairs, uint32_t* sched, cudaStream_t stream) {
-  const bool tma_out = (g.ldo * (g.out_fp32 ? 4 : 2)) % 16 == 0 && ((uintptr_t)g.out & 15) == 0;
+  const bool tma_out = tma_store_enabled() && (g.ldo * (g.out_fp32 ? 4 : 2)) % 16 == 0 && ((uintptr_t)g.out & 15) == 0;
   const bool rows = tma_out && !g.out_fp32 && !g.transposed && !g.in_fp32;
   const FlowVariant v = g.in_fp32 ? flow_variant<4, FLOW_ANY>(bn, rb) : !rows ? flow_variant<2, FLOW_ANY>(bn, rb)
                         : g.act ? flow_variant<2, FLOW_ROWS_ACT>(bn, rb) : flow_variant<2, FLOW_ROWS>(bn, rb);

@@ -16,6 +16,7 @@ int get_tmap(const void* ptr, unsigned long long rows, unsigned long long cols, 
 // Tensor map for TMA stores of bf16 tiles (box of 32 rows); false when the matrix cannot be
 // described to TMA or TMA stores are switched off.
 bool store_tmap(const void* ptr, long long rows, long long cols, long long ld, CUtensorMap* m);
+bool tma_store_enabled();       // KRAKEN_TMA_STORE
 int default_group_r();
 bool pair_enabled();
 unsigned grid_cap(const DeviceState* d);

@@ -10,7 +10,7 @@ kraken/comm/two_shot_all_reduce.py:153).
 ``KRAKEN_NUM_COMM_SMS``     comm CTAs of the in-kernel all-gather engine (default: from the problem shape)
 ``KRAKEN_GEMM_PAIR``        ``0`` forces the single-CTA GEMM kernel (default: CTA pairs when eligible)
 ``KRAKEN_GEMM_GROUP``       row tiles per column sweep of the GEMM tile order (default 16)
-``KRAKEN_TMA_STORE``        ``0`` makes the epilogue of the fused GEMMs use vector stores instead of TMA stores
+``KRAKEN_TMA_STORE``        ``0`` makes the GEMM epilogues use vector or element stores instead of TMA stores
 ``KRAKEN_AG_MODE``          engine of the fused all-gather GEMM: ``auto`` (default: ``push``; ``ce`` above 2 ranks when
                             the workspace has no multicast mapping),
                             ``push`` (comm CTAs write the own shard into the peers' gathered buffers), ``ce`` (copy

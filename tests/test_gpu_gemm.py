@@ -500,3 +500,38 @@ def test_one_rank_all_gather_matmul_fills_a_out_like_a_copy():
                 torch.zeros(M, K, dtype=torch.bfloat16, device="cuda", requires_grad=True)):
         with pytest.raises(RuntimeError):
             fused.all_gather_matmul(x, bt.t(), a_out=out)
+
+
+_TMA_STORE_PROBE = """
+import ctypes, torch
+from kraken_b200 import fused
+from kraken_b200.ops import lib as klib
+g = torch.Generator().manual_seed(71)
+a = torch.randn(520, 264, generator=g).to(torch.bfloat16).cuda()
+bt = (0.05 * torch.randn(1032, 264, generator=g)).to(torch.bfloat16).cuda()
+ref = a.float() @ bt.float().t()
+hits, before, after = ctypes.c_ulonglong(0), ctypes.c_ulonglong(0), ctypes.c_ulonglong(0)
+keep = []
+for bn in ({bn}):
+    for out_dtype in (torch.bfloat16, torch.float32):
+        klib.check(klib.lib().kr_tmap_cache_stats(ctypes.byref(hits), ctypes.byref(before)))
+        c = fused.matmul(a, bt.t(), out_dtype=out_dtype, bn=bn, swap_ab=0)
+        assert ((c.float() - ref).norm() / ref.norm()).item() < 3e-3
+        klib.check(klib.lib().kr_tmap_cache_stats(ctypes.byref(hits), ctypes.byref(after)))
+        print("maps", after.value - before.value)
+        keep.append((a, bt, c))          # fresh addresses for the next call
+        a, bt = a.clone(), bt.clone()
+"""
+
+
+@pytest.mark.parametrize("setting,maps", [("1", 3), ("0", 2)])
+def test_tma_store_setting_reaches_the_persistent_pairs(setting, maps):
+    # read once per process; without TMA stores a call describes its two operands and no output
+    import os
+    import subprocess
+    import sys
+
+    r = subprocess.run([sys.executable, "-c", _TMA_STORE_PROBE.format(bn="1256, 2192")], env={**os.environ, "KRAKEN_TMA_STORE": setting},
+                       cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stderr[-2000:]
+    assert [int(line.split()[1]) for line in r.stdout.splitlines() if line.startswith("maps")] == [maps] * 4, r.stdout
