@@ -547,6 +547,8 @@ __device__ __forceinline__ void gemm_mainloop(const GemmParams& p, unsigned bid,
         if (ok) umma_commit(tfull_bar(acc));   // accumulator complete
         trace_put(p, 0, it, 2);
       }
+      // an epilogue that gave up on a peer no longer waits for these MMAs: TMEM is not freed under them
+      if (ok && it > 0) mbar_wait(tfull_bar((it - 1) & 1), (uint32_t)((it - 1) >> 1) & 1u, p.sync, 48);
     }
   } else if (warp >= 6) {
     hooks.side_role(p, bid, nb, -1, (int)threadIdx.x - kGemmThreads);
@@ -761,6 +763,7 @@ __device__ __forceinline__ void gemm_mainloop_pair(const GemmParams& p, unsigned
         }
         trace_put(p, 0, it, 2);
       }
+      if (ok && it > 0) mbar_wait(tfull_bar((it - 1) & 1), (uint32_t)((it - 1) >> 1) & 1u, p.sync, 48);   // as in gemm_mainloop
     }
   } else if (warp >= 6) {
     hooks.side_role(p, pair_id, num_pairs, (int)cta, (int)threadIdx.x - kGemmThreads);

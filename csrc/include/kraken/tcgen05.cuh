@@ -36,7 +36,12 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
       : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
   return ok != 0;
 }
-// Bounded wait for the phase with the given parity. On expiry: status word set, returns false.
+// Bounded wait for the phase with the given parity. On expiry: status word set, returns false. An error that is
+// already recorded (another role of this kernel, or an earlier kernel whose status the host has not read yet)
+// shortens the wait to kMbarGraceNs, not to nothing: a bulk copy or MMA that is in flight completes in
+// far less, so nobody leaves while its own copies still write shared memory, and a kernel that needs no other
+// rank still computes its whole result.
+constexpr uint64_t kMbarGraceNs = 20000000;
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const SyncCtx& c, uint32_t site) {
   if (mbar_try_wait(bar, parity)) return true;
   const uint64_t t0 = globaltimer_ns();
@@ -44,11 +49,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const S
   while (true) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((++n & 255u) == 0u) {
-      if (!status_ok(c)) return false;
-      if (globaltimer_ns() - t0 > c.timeout_ns) {
+      const uint64_t waited = globaltimer_ns() - t0;
+      if (waited > c.timeout_ns) {
         set_status(c, make_status(KR_ERR_TIMEOUT_MBAR, site, 0, blockIdx.x));
         return false;
       }
+      if (waited > kMbarGraceNs && !status_ok(c)) return false;
     }
   }
 }

@@ -87,3 +87,45 @@ def test_symm_mem_sync_single_pattern(ws, prev, subseq):
         with world.rank(r):
             hdl = symm_mem.rendezvous(ts[r])
         assert int(hdl.get_signal_pad(r).to(torch.int64).abs().sum()) == 0      # every token consumed
+
+
+@pytest.mark.expects_timeout
+def test_kernels_after_an_unread_error_still_compute_their_whole_result():
+    # A wait of an earlier kernel ran out and the host has not looked yet. Kernels that need no other rank must
+    # not cut their own pipelines short over it: every tile is there, with nothing of theirs left in flight.
+    from kraken_b200 import fused
+
+    L = klib.lib()
+    g = torch.Generator().manual_seed(81)
+    a = torch.randn(2048, 264, generator=g).to(torch.bfloat16).cuda()
+    bt = (0.05 * torch.randn(2056, 264, generator=g)).to(torch.bfloat16).cuda()
+    h = torch.randn(16, 4096, generator=g).to(torch.bfloat16).cuda()
+    wt = (0.02 * torch.randn(1024, 4096, generator=g)).to(torch.bfloat16).cuda()
+    rows = torch.randn(3552, 1024, generator=g).to(torch.bfloat16).cuda()
+    w = torch.ones(1024, dtype=torch.bfloat16, device="cuda")
+
+    def run():
+        # persistent pairs that draw their tiles, with many and with few tiles per pair; single CTAs; one wave
+        # with K splits; rows through shared memory
+        return [fused.matmul(a, bt.t(), max_ctas=6, bn=2256, swap_ab=0), fused.matmul(a, bt.t()), fused.matmul(a, bt.t(), pair=0, max_ctas=7),
+                fused.matmul(h, wt.t()), fused.rms_norm(rows, w)]
+
+    want = run()
+    torch.cuda.synchronize()
+    kraken_b200.check_status()
+    old = L.kr_get_timeout_ms()
+    klib.check(L.kr_set_timeout_ms(5.0))
+    try:
+        ptx.wait_timeout_test(num_blocks=4)
+        klib.check(L.kr_set_timeout_ms(old))
+        got = run()
+        torch.cuda.synchronize()
+        again = run()                # the tile counters are back at zero although nobody has read the status
+        with pytest.raises(kraken_b200.KrakenSyncTimeout):
+            kraken_b200.check_status()
+    finally:
+        klib.check(L.kr_set_timeout_ms(old))
+    for outs in (got, again, run()):
+        for x, y in zip(outs, want):
+            assert torch.equal(x, y)
+    kraken_b200.check_status()
