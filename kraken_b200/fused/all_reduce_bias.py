@@ -130,8 +130,10 @@ def one_shot_all_reduce_bias_rms_norm(symm_mem_input: torch.Tensor, x: torch.Ten
 
 def two_shot_all_reduce_bias_rms_norm(symm_mem_input: torch.Tensor, x: torch.Tensor, bias: torch.Tensor | None,
                                       w: torch.Tensor, y: torch.Tensor, eps: float = 1e-5, group=None) -> None:
-    """Same result with the two-shot exchange: rank k reduces columns [k*D/ws, (k+1)*D/ws) of each
-    row and publishes them, then every rank normalises. Needs D % (8 * world_size) == 0."""
+    """The same with the two-shot exchange: rank k reduces columns [k*D/ws, (k+1)*D/ws) of each row (+ bias) and
+    publishes them as bf16, then every rank normalises those bf16 sums. One rank publishes nothing and
+    normalises its fp32 sums, as the one-shot form does at any world size; so does a D that is not a multiple of
+    8 * world_size, which takes the one-shot form."""
     if _alone(symm_mem_input, group) and _host.bias_rms_norm(symm_mem_input, x, bias, w, y, eps):
         return
     D = x.shape[-1]

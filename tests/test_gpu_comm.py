@@ -269,3 +269,35 @@ def test_rms_norm_of_thousands_of_rows(rows, D):
     x = torch.randn(rows, D, device="cuda").to(torch.bfloat16)
     w = (1 + 0.1 * torch.randn(D, device="cuda")).to(torch.bfloat16)
     torch.testing.assert_close(fused.rms_norm(x, w).float(), _rms_ref(x, w, 1e-5), atol=4e-2, rtol=2e-2)
+
+
+@pytest.mark.parametrize("ws", [1, 2, 4])
+@pytest.mark.parametrize("form", ["one_shot", "two_shot"])
+@pytest.mark.parametrize("rows,D", [(3, 1024), (300, 5120)])
+def test_where_bias_rms_norm_rounds_its_sums(ws, form, rows, D):
+    # Inputs are multiples of 1/64 below 4, so the sums are exact in fp32. What is normalised: the bf16 sums where they are
+    # published (two-shot, several ranks), else the fp32 sums. Left over: one bf16 rounding of the result (2**-8) and
+    # a few fp32 roundings (below 1e-5); the other choice of sums is off by about 2**-8 more for many elements.
+    g = torch.Generator().manual_seed(91)
+    grid = lambda *shape: (torch.randint(-255, 256, shape, generator=g) / 64).to(torch.bfloat16).cuda()
+    xs, bias = [grid(rows, D) for _ in range(ws)], grid(D)
+    w = (1 + 0.1 * torch.randn(D, generator=g)).to(torch.bfloat16).cuda()
+    op = fused.one_shot_all_reduce_bias_rms_norm if form == "one_shot" else fused.two_shot_all_reduce_bias_rms_norm
+    ys = [torch.empty_like(x) for x in xs]
+    if ws == 1:
+        scratch = symm_mem.empty(rows, D, dtype=torch.bfloat16, device="cuda")
+        op(scratch, xs[0], bias, w, ys[0])
+    else:
+        world = EmuWorld(ws)
+        scratch = world.symmetric((rows, D), torch.bfloat16)
+        world.run(lambda r: op(scratch[r], xs[r], bias, w, ys[r]))
+    s = sum(x.double() for x in xs) + bias.double()
+    published = form == "two_shot" and ws > 1
+
+    def worst(sums):
+        ref = sums * torch.rsqrt(sums.pow(2).mean(-1, keepdim=True) + 1e-5) * w.double()
+        return max(float(((y.double() - ref).abs() / (ref.abs() + 1e-30)).max()) for y in ys)
+
+    rounded = s.to(torch.bfloat16).double()
+    assert worst(rounded if published else s) <= 2.0 ** -8 + 1e-5
+    assert worst(s if published else rounded) > 2.0 ** -8 + 1e-5
