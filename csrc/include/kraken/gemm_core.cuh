@@ -180,8 +180,8 @@ __device__ __forceinline__ void trace_put(const GemmParams& p, int role, int slo
     p.trace[(((size_t)blockIdx.x * kTraceRoles + role) * kTraceTiles + slot) * kTraceFields + field] = globaltimer_ns();
 }
 
-// The work of one CTA (or CTA pair): tiles worker, worker + workers, ... With k_splits > 1 items are
-// (split, tile), split-major, so that one wave of CTAs covers every tile once.
+// The work of one CTA: tiles worker, worker + workers, ... With k_splits > 1 items are (split, tile),
+// split-major, so that one wave of CTAs covers every tile once.
 struct WorkIter {
   int t, stride, total, tiles_rc, ksp, num_kb;
   __device__ __forceinline__ WorkIter(const GemmParams& p, int worker, int workers, int num_kb_) {
@@ -222,7 +222,7 @@ __device__ __forceinline__ void epi_bar_sync() { asm volatile("bar.sync 1, 128;"
 //   side_role (work of the warps beyond the six pipeline warps, if the launch has any),
 //   helper_role (what the six pipeline warps do after their last tile, before the teardown).
 struct HookDefaults {
-  static constexpr bool kOverlap = false;   // whether the kernel is launched with launch_overlapped()
+  static constexpr bool kOverlap = false;   // whether the (single-CTA) kernel is launched with launch_overlapped()
   static constexpr bool kAct = false;       // whether its epilogue can apply an activation (GemmParams::act)
   int k_split = 0;           // which K split the tile in hand belongs to (set by the main loop)
   __device__ __forceinline__ bool may_wait(const GemmParams&, int) const { return false; }
@@ -684,14 +684,9 @@ __device__ __forceinline__ void gemm_mainloop_pair(const GemmParams& p, unsigned
   cluster_sync_all();            // both CTAs' barriers exist before anyone signals across the pair
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  if (Hooks::kOverlap) {
-    pdl_launch();
-    pdl_wait();
-  }
 
   const int num_kb = (p.K + kBK - 1) / kBK;
-  WorkIter work(p, (int)pair_id, (int)num_pairs, num_kb);   // tiles_r counts 256-row pair tiles here
-  int tile, split, kb_lo, kb_hi;
+  const int tiles = p.tiles_r * p.tiles_c;                  // tiles_r counts 256-row pair tiles here
 
   if (warp == 0) {
     // ================= TMA producer (both CTAs) =================
@@ -701,14 +696,14 @@ __device__ __forceinline__ void gemm_mainloop_pair(const GemmParams& p, unsigned
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
-      while (ok && work.next(tile, split, kb_lo, kb_hi)) {
+      for (int tile = (int)pair_id; ok && tile < tiles; tile += (int)num_pairs) {
         int tr2, tc;
         tile_coords(p, tile, tr2, tc);
         const int tr = 2 * tr2 + (int)cta;
         const CUtensorMap* rmap = &p.tmap_r;
         int row0 = tr * kBM;
         ok = hooks.before_load(p, tr, rmap, row0);
-        for (int kb = kb_lo; kb < kb_hi && ok; ++kb) {
+        for (int kb = 0; kb < num_kb && ok; ++kb) {
           ok = mbar_wait(empty_bar(s), ph ^ 1u, p.sync, 44);
           if (!ok) break;
           const uint32_t lead_full = mapa_shared(full_bar(s), 0);
@@ -734,7 +729,7 @@ __device__ __forceinline__ void gemm_mainloop_pair(const GemmParams& p, unsigned
       uint32_t ph = 0;
       int it = 0;
       bool ok = true;
-      for (; ok && work.next(tile, split, kb_lo, kb_hi); ++it) {
+      for (int tile = (int)pair_id; ok && tile < tiles; tile += (int)num_pairs, ++it) {
         const int acc = it & 1;
         const uint32_t acc_ph = (uint32_t)(it >> 1) & 1u;
         ok = mbar_wait(tempty_bar(acc), acc_ph ^ 1u, p.sync, 45);
@@ -742,17 +737,17 @@ __device__ __forceinline__ void gemm_mainloop_pair(const GemmParams& p, unsigned
         tc_fence_after();
         trace_put(p, 0, it, 0);
         const uint32_t d_tmem = tmem_base + (uint32_t)(acc * Cfg::BN);
-        for (int kb = kb_lo; kb < kb_hi; ++kb) {
+        for (int kb = 0; kb < num_kb; ++kb) {
           ok = mbar_wait(full_bar(s), ph, p.sync, 46);
           if (!ok) break;
           tc_fence_after();
-          if (kb == kb_lo) trace_put(p, 0, it, 1);
+          if (kb == 0) trace_put(p, 0, it, 1);
           const uint32_t sa = stage0 + s * Cfg::STAGE;
           const uint64_t adesc = make_smem_desc_sw128(sa);
           const uint64_t bdesc = make_smem_desc_sw128(sa + Cfg::A_BYTES);
 #pragma unroll
           for (int k = 0; k < kBK / 16; ++k)
-            umma_bf16_pair(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, (kb > kb_lo || k != 0) ? 1u : 0u);
+            umma_bf16_pair(d_tmem, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, (kb > 0 || k != 0) ? 1u : 0u);
           umma_commit_pair(empty_bar(s));      // own stage free
           umma_commit_pair(peer_empty[s]);     // peer's stage free
           if (++s == Cfg::STAGES) { s = 0; ph ^= 1u; }
@@ -776,7 +771,7 @@ __device__ __forceinline__ void gemm_mainloop_pair(const GemmParams& p, unsigned
     int prev_tr = -1, prev_tc = -1;
     int it = 0;
     bool ok = true;
-    for (; ok && work.next(tile, split, kb_lo, kb_hi); ++it) {
+    for (int tile = (int)pair_id; ok && tile < tiles; tile += (int)num_pairs, ++it) {
       int tr2, tc;
       tile_coords(p, tile, tr2, tc);
       const int tr = 2 * tr2 + (int)cta;

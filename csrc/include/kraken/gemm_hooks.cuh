@@ -10,9 +10,8 @@ struct PlainHooks : HookDefaults {
   static constexpr bool kAct = true;
   int bn;
   // The copy warps: this CTA's contiguous share of the row operand, eight 16-byte loads in flight per thread.
-  __device__ __forceinline__ void side_role(const GemmParams& p, unsigned worker, unsigned workers, int half, int tid) {
-    const size_t ctas = half < 0 ? workers : 2 * workers, id = half < 0 ? worker : 2 * worker + half;
-    const size_t nvec = p.cp_bytes / 16, lo = nvec * id / ctas, hi = nvec * (id + 1) / ctas;
+  __device__ __forceinline__ void side_role(const GemmParams& p, unsigned cta, unsigned ctas, int, int tid) {
+    const size_t nvec = p.cp_bytes / 16, lo = nvec * cta / ctas, hi = nvec * (cta + 1) / ctas;
     const char* src = (const char*)p.cp_src;
     char* dst = (char*)p.cp_dst;
     size_t v = lo + tid;
