@@ -301,3 +301,37 @@ def test_where_bias_rms_norm_rounds_its_sums(ws, form, rows, D):
     rounded = s.to(torch.bfloat16).double()
     assert worst(rounded if published else s) <= 2.0 ** -8 + 1e-5
     assert worst(s if published else rounded) > 2.0 ** -8 + 1e-5
+
+
+@pytest.mark.parametrize("rows,D,K", [(128, 40960, 2048), (3600, 4096, 1024), (16, 8192, 4096), (600, 5120, 2048), (40, 16392, 2048)])
+def test_chain_of_overlapped_launches(rows, D, K):
+    # Each kernel starts while the one before it still runs and must wait for it before it reads; the norms here are
+    # the long-row, the streaming and the row-per-block kernels. Same bits as with a synchronisation after every step.
+    g = torch.Generator().manual_seed(95)
+    bt = (0.05 * torch.randn(D, K, generator=g)).to(torch.bfloat16).cuda()
+    w = (1 + 0.1 * torch.randn(D, generator=g)).to(torch.bfloat16).cuda()
+    scratch = symm_mem.empty(rows, D, dtype=torch.bfloat16, device="cuda")
+    bias = torch.randn(D, generator=g).to(torch.bfloat16).cuda()
+    bufs = [torch.empty(rows, D, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+
+    def chain(a, after):
+        x = fused.matmul(a, bt.t())
+        after()
+        x = fused.rms_norm(x, w)
+        after()
+        fused.one_shot_all_reduce_bias(scratch, x, bias, bufs[0])
+        after()
+        x = fused.rms_norm(bufs[0], w)
+        after()
+        fused.two_shot_all_reduce_bias(scratch, x, bias, bufs[1])
+        after()
+        return fused.rms_norm(bufs[1], w)
+
+    for _ in range(4):
+        a = torch.randn(rows, K, generator=g).to(torch.bfloat16).cuda()
+        want = chain(a, torch.cuda.synchronize)
+        torch.cuda.synchronize()
+        for b in bufs:
+            _poison(b)
+        torch.cuda.synchronize()
+        assert torch.equal(chain(a, lambda: None), want)

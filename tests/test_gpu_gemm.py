@@ -535,3 +535,60 @@ def test_tma_store_setting_reaches_the_persistent_pairs(setting, maps):
                        cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))), capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stderr[-2000:]
     assert [int(line.split()[1]) for line in r.stdout.splitlines() if line.startswith("maps")] == [maps] * 4, r.stdout
+
+
+@pytest.mark.parametrize("M,hidden,ffn", [(65, 264, 1096), (300, 512, 1032), (777, 520, 2024), (2100, 1160, 4104), (300, 512, 1088)])
+def test_prefill_at_one_rank_with_ragged_ffn(M, hidden, ffn):
+    # the up projection's rows are padded to whole 128-byte lines when ffn is not a multiple of 64; what the padding
+    # holds (NaN here) must not reach the down projection
+    from kraken_b200.fused.gemm_ops import all_gather_matmul_act
+    from kraken_b200.models import TPMLP
+
+    mlp = TPMLP(hidden, ffn, device="cuda", seed=5)
+    x = (0.5 * torch.randn(M, hidden, generator=torch.Generator().manual_seed(92))).to(torch.bfloat16).cuda()
+    xs = mlp.stage_input(x)
+    padded = -(-ffn // 64) * 64
+    h = all_gather_matmul_act(xs, mlp.w_up_t.t(), "gelu_tanh")
+    assert h.shape == (M, ffn) and h.stride(0) == padded
+    if padded != ffn:
+        torch.as_strided(h, (M, padded - ffn), (padded, 1), ffn).fill_(float("nan"))
+    s = x.double() @ mlp.w_up_t.double().t()
+    gelu = s * torch.sigmoid(2 * (2 / math.pi) ** 0.5 * (s + 0.044715 * s ** 3))
+    # one bf16 rounding per element: at most 2**-8, half of that root mean square or less
+    assert ((h.double() - gelu).norm() / gelu.norm()).item() < 2.0 ** -9 + 1e-4
+    ref = gelu.to(torch.bfloat16).double() @ mlp.w_down_t.double().t()
+    y = fused.gemm_reduce_scatter(h, mlp.w_down_t.t())
+    assert y.shape == (M, hidden) and ((y.double() - ref).norm() / ref.norm()).item() < 3e-3
+    assert torch.equal(mlp.prefill(xs), y)
+
+
+def test_tile_counters_of_many_streams_and_threads():
+    # Every stream has counter words of its own, more streams than the pool keeps among them, used by two threads
+    # at a time. Whole tiles would be missing or stale if two launches drew from the same words.
+    import threading
+
+    a, bt = _ab(2048, 2600, 264, seed=93)
+    want = fused.matmul(a, bt.t())
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(priority=p) for p in (0, -1) for _ in range(24)]
+    outs, errors = {}, []
+
+    def work(mine):
+        try:
+            for i in mine:
+                with torch.cuda.stream(streams[i]):
+                    outs[i] = [fused.matmul(a, bt.t()) for _ in range(4)]
+        except Exception as e:
+            errors.append(e)
+
+    for _ in range(2):
+        threads = [threading.Thread(target=work, args=(range(k, len(streams), 2),)) for k in range(2)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        torch.cuda.synchronize()
+        assert not errors, errors
+        for i in range(len(streams)):
+            assert all(torch.equal(c, want) for c in outs[i]), i
+        outs.clear()

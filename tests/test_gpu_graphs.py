@@ -73,3 +73,26 @@ def test_capability_queries_are_safe_inside_stream_capture():
     g.replay()
     torch.cuda.synchronize()
     torch.testing.assert_close(y, x * 2)
+
+
+def test_gemms_that_draw_their_tiles_replay_under_cuda_graph():
+    # more tiles than CTA pairs: the tile counter is allocated and zeroed inside the graph, and is zero again for the replay
+    g = torch.Generator().manual_seed(94)
+    a = torch.randn(4096, 264, generator=g).to(torch.bfloat16).cuda()
+    b1 = (0.05 * torch.randn(4104, 264, generator=g)).to(torch.bfloat16).cuda()
+    b2 = (0.02 * torch.randn(4096, 4104, generator=g)).to(torch.bfloat16).cuda()
+
+    def chain():
+        return fused.matmul(fused.matmul(a, b1.t()), b2.t())
+
+    chain()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = chain()
+    for _ in range(4):
+        a.copy_(torch.randn(4096, 264, generator=g).to(torch.bfloat16))
+        out.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, chain())
