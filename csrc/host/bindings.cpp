@@ -10,6 +10,7 @@
 #include <Python.h>
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAException.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -67,16 +68,22 @@ constexpr int64_t kCounterWords = 32;
 std::mutex g_pool_mu;
 std::map<std::pair<int, void*>, at::Tensor> g_pool;
 
+// Not through the dispatcher: nobody's dispatch mode may see, replace or delay these words (the lock is held).
+at::Tensor zero_words(c10::DeviceIndex dev, c10::cuda::CUDAStream stream, int64_t words) {
+  at::Tensor t = at::detail::empty_cuda({words}, at::kInt, at::Device(at::kCUDA, dev), std::nullopt);
+  C10_CUDA_CHECK(cudaMemsetAsync(t.data_ptr(), 0, (size_t)words * sizeof(int32_t), stream.stream()));
+  return t;
+}
+
 at::Tensor counters_for(c10::DeviceIndex dev, c10::cuda::CUDAStream stream, int64_t words) {
-  const auto opt = at::TensorOptions().dtype(at::kInt).device(at::kCUDA, dev);
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(stream.stream(), &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) return at::zeros({words}, opt);
+  if (cudaStreamIsCapturing(stream.stream(), &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) return zero_words(dev, stream, words);
   std::lock_guard<std::mutex> lk(g_pool_mu);
   auto key = std::make_pair((int)dev, (void*)stream.stream());
   auto it = g_pool.find(key);
   if (it != g_pool.end() && it->second.numel() >= words) return it->second;
   if (g_pool.size() >= kMaxStreams) g_pool.clear();
-  at::Tensor t = at::zeros({std::max(words, kCounterWords)}, opt);
+  at::Tensor t = zero_words(dev, stream, std::max(words, kCounterWords));
   g_pool[key] = t;
   return t;
 }

@@ -592,3 +592,30 @@ def test_tile_counters_of_many_streams_and_threads():
         for i in range(len(streams)):
             assert all(torch.equal(c, want) for c in outs[i]), i
         outs.clear()
+
+
+def test_tile_counters_stay_out_of_dispatch_modes():
+    # the counter words of a new stream are made under a lock: a mode that sees their allocation could replace them
+    # or wait in Python while it is held
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Recorder(TorchDispatchMode):
+        def __init__(self):
+            super().__init__()
+            self.seen = []
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    a, bt = _ab(2048, 2600, 264, seed=96)
+    b = bt.t()
+    want = fused.matmul(a, b)
+    for _ in range(2):                      # the first call on a stream, and on one whose words are there
+        for stream in [torch.cuda.Stream() for _ in range(40)]:
+            with torch.cuda.stream(stream), Recorder() as mode:
+                stream.wait_stream(torch.cuda.default_stream())
+                c = fused.matmul(a, b)
+            assert mode.seen == []
+            stream.synchronize()
+            assert torch.equal(c, want)
