@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
           }
           if (MODE == FLOW_ANY && p.out != nullptr) store_plain(slot, gx, gy, cols, rows, fp32, lane);
         };
-        if (MODE == FLOW_ANY && (fp32 || transposed)) {
+        if (MODE == FLOW_ANY && (fp32 || transposed || act)) {
 #pragma unroll 1
           for (int i = 0; i < CHUNKS; ++i) {
             const int col = i * 32;
@@ -341,6 +341,17 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
                 }
               }
               send(slot, drow, it.tc * BN + col, 32, tail ? 16 : 32, tail);
+            } else if (!fp32) {
+#pragma unroll
+              for (int v = 0; v < 4; ++v) {
+                if (tail && v >= 2) continue;
+                uint32_t w[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) w[j] = pack_bf16x2(__uint_as_float(r[8 * v + 2 * j]), __uint_as_float(r[8 * v + 2 * j + 1]));
+                const uint32_t a = tail ? slot + lane * 32u + v * 16u : slot + lane * 64u + (uint32_t)((v ^ ((lane >> 1) & 3)) << 4);
+                st_shared_u4(a, w[0], w[1], w[2], w[3]);
+              }
+              send(slot, it.tc * BN + col, drow, tail ? 16 : 32, 32, tail);
             } else {
 #pragma unroll
               for (int v = 0; v < 8; ++v) {
@@ -350,27 +361,6 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
               }
               send(slot, it.tc * BN + col, drow, tail ? 16 : 32, 32, tail);
             }
-          }
-        } else if (MODE == FLOW_ANY && act) {
-#pragma unroll 1
-          for (int i = 0; i < CHUNKS; ++i) {
-            const bool tail = TAIL && i + 1 == CHUNKS;
-            uint32_t r[32];
-            tmem_ld32(t_addr + (uint32_t)(i * 32), r);
-            tmem_ld_wait();
-            if (i + 1 == CHUNKS) release();
-            const uint32_t slot = next_slot();
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-              if (tail && v >= 2) continue;
-              uint32_t w[4];
-#pragma unroll
-              for (int j = 0; j < 4; ++j)
-                w[j] = pack_bf16x2(gelu_tanh(__uint_as_float(r[8 * v + 2 * j])), gelu_tanh(__uint_as_float(r[8 * v + 2 * j + 1])));
-              const uint32_t a = tail ? slot + lane * 32u + v * 16u : slot + lane * 64u + (uint32_t)((v ^ ((lane >> 1) & 3)) << 4);
-              st_shared_u4(a, w[0], w[1], w[2], w[3]);
-            }
-            send(slot, it.tc * BN + i * 32, drow, tail ? 16 : 32, 32, tail);
           }
         } else {
           // bf16 rows: everything is read, activated (on the fp32 sums) and rounded before anything is stored, so
