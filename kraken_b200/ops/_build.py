@@ -31,9 +31,11 @@ HOST_NAME = "kraken_b200_host"
 HOST_SRC = CSRC / "host" / "bindings.cpp"
 HOST_PATH = OUT_DIR / (HOST_NAME + ".so")
 
+# Without --split-compile: where it cuts a file depends on the run, and with it registers and spills (three builds of
+# gemm_rs.cu: 116, 144 and 116 bytes spilled by the pair kernel) and times (256 x 8192 x 8192 34.7 or 37.4 us).
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
-    "-std=c++17", "-O3", "-lineinfo", "--split-compile=0",
+    "-std=c++17", "-O3", "-lineinfo",
     "-Xcompiler", "-fPIC",
     "-Xcompiler", "-fvisibility=hidden",
 ]

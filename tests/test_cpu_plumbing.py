@@ -159,3 +159,9 @@ def test_config_sizing_overrides(monkeypatch):
     assert config.comm_cta_bytes_per_s("push") == 33e9
     # push-style one-shot: the limit shrinks with the world size and stops where pulling was measured faster
     assert push_limit_bytes(2) == 2 << 20 and push_limit_bytes(8) == 1 << 20 and push_limit_bytes(4) == 1 << 20
+
+
+def test_build_flags_give_the_same_program_every_time():
+    from kraken_b200.ops import _build
+
+    assert not any("split-compile" in f for f in _build.NVCC_FLAGS)
