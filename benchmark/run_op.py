@@ -4,7 +4,8 @@ Ops: gemm, gemm_swap (decode shape, operands swapped), gemm_tf32, rms_norm, ag_m
 rs_pull / rs_scatter / rs_push (the fused reduce-scatter GEMM kernels at world size 1: CTA pairs,
 reducer warps, counters), the memory-bound collectives at world size 1 (one_shot_ar, one_shot_ar_pull,
 two_shot_ar, reduce_scatter, all_gather: M x K bf16 elements; ar_bias_norm_one_shot / _pull /
-_two_shot: M rows of K), cublas (torch.matmul, for comparison). Prints the CUDA-event time of each
+_two_shot: M rows of K; on one rank these and ag_matmul run the one-rank kernels, not the exchanges that
+several ranks run), cublas (torch.matmul, for comparison). Prints the CUDA-event time of each
 iteration; with --flush-l2 a 256 MB buffer is overwritten before each timed call."""
 from __future__ import annotations
 

@@ -88,7 +88,8 @@ at::Tensor counters_for(c10::DeviceIndex dev, c10::cuda::CUDAStream stream, int6
   return t;
 }
 
-// reset(): drops the counters (after a reported timeout a kernel may have left without resetting them)
+// reset(): drops the counters. Every path of the kernels, a wait that ran out included, puts them back to zero; a
+// recovery should not have to rely on that.
 PyObject* py_reset(PyObject*, PyObject*) {
   std::lock_guard<std::mutex> lk(g_pool_mu);
   g_pool.clear();

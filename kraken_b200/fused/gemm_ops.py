@@ -5,8 +5,9 @@ kraken/fused/gemm_one_shot_all_reduce_fused.py:106-178,
 kraken/fused/gemm_reduce_scatter_fused.py:152-235,
 kraken/fused/gemm_reduce_scatter_ce_persistent.py:326-375. The Triton tiling kwargs
 (``block_size_*``, ``BLOCK_SIZE_*``, ``group_size_m``, ``num_stages``, ``num_warps``) are accepted and
-ignored: tile shapes are chosen by the library (128 x 256 x 64, or 128 x {16..128} with the
-operands swapped for decode-sized M).
+ignored: tile shapes are chosen by the library. Several ranks: 256 x 256 on CTA pairs or 128 x {16..256} on
+single CTAs; one rank: 256 or 512 rows x {64..256} columns on persistent pairs, or one wave of 128 x {16..128} or
+256 x {128..256} tiles with K splits. Decode-sized M swaps the operands.
 """
 from __future__ import annotations
 

@@ -185,5 +185,5 @@ def check_status(stream: int | None = None, clear: bool = True) -> None:
             check(lib().kr_clear_status(s))
         from . import host
 
-        host.reset_if_loaded()      # a kernel that gave up may have left its scratch counters set
+        host.reset_if_loaded()      # start over with fresh tile counters
         raise KrakenSyncTimeout(decode_status(word.value))
