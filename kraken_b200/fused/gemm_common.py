@@ -46,6 +46,9 @@ def as_k_major_bt(b: torch.Tensor, keep_fp32: bool = False) -> tuple[torch.Tenso
     if b.dtype == want and b.stride(0) == 1 and b.stride(1) % unit == 0 and b.stride(1) >= b.shape[0] \
             and b.data_ptr() % 16 == 0:
         return b.t(), b.stride(1)
+    if b.is_inference():              # a changed inference tensor looks like the old one: no cache
+        bt = b.t().to(want).contiguous()
+        return bt, bt.stride(0)
     key = (b.data_ptr(), tuple(b.shape), tuple(b.stride()), b.dtype, b._version, want)
     hit = _bt_cache.get(key)
     if hit is not None:

@@ -165,3 +165,20 @@ def test_build_flags_give_the_same_program_every_time():
     from kraken_b200.ops import _build
 
     assert not any("split-compile" in f for f in _build.NVCC_FLAGS)
+
+
+def test_transposed_weight_follows_a_changed_inference_tensor():
+    import torch
+
+    from kraken_b200.fused.gemm_common import as_k_major_bt
+
+    with torch.inference_mode():
+        b = torch.randn(16, 24).to(torch.bfloat16)
+        for _ in range(3):
+            assert torch.equal(as_k_major_bt(b)[0], b.t())
+            b.mul_(2)
+    c = torch.randn(16, 24).to(torch.bfloat16)
+    first = as_k_major_bt(c)[0]
+    assert as_k_major_bt(c)[0] is first          # an ordinary tensor that has not changed is laid out once
+    c.mul_(2)
+    assert torch.equal(as_k_major_bt(c)[0], c.t())
