@@ -5,7 +5,8 @@ transpose ``bt`` [N, K] with K contiguous (the layout of an ``nn.Linear`` weight
 reference's all-gather matmul insists on: kraken/fused/all_gather_matmul.py:158-160). A ``b`` that is
 row-major [K, N] is transposed once and cached per (storage, version) — weights are static in
 inference, whereas the reference's copy-engine variant re-transposes on every call
-(kraken/fused/gemm_reduce_scatter_ce_persistent.py:192). bf16 operands run on the bf16 tensor-core
+(kraken/fused/gemm_reduce_scatter_ce_persistent.py:192). Changes that torch does not count (through raw pointers, by
+a replayed graph) are not seen: a weight that changes that way has to be K-major. bf16 operands run on the bf16 tensor-core
 path; when BOTH operands are fp32 the plain GEMM and the GEMM all-reduce multiply them as tf32
 (``keep_fp32=True`` below), as ``tl.dot`` does for the reference's fp32 tests; every other
 combination is cast to bf16. Accumulation is always fp32.
@@ -15,6 +16,10 @@ from __future__ import annotations
 import torch
 
 _bt_cache: dict[tuple, tuple] = {}
+
+
+def _capturing(t: torch.Tensor) -> bool:
+    return t.is_cuda and torch.cuda.is_current_stream_capturing()
 
 
 def use_tf32(a: torch.Tensor, b: torch.Tensor) -> bool:
@@ -46,7 +51,9 @@ def as_k_major_bt(b: torch.Tensor, keep_fp32: bool = False) -> tuple[torch.Tenso
     if b.dtype == want and b.stride(0) == 1 and b.stride(1) % unit == 0 and b.stride(1) >= b.shape[0] \
             and b.data_ptr() % 16 == 0:
         return b.t(), b.stride(1)
-    if b.is_inference():              # a changed inference tensor looks like the old one: no cache
+    # A changed inference tensor looks like the old one, and what a capture lays out is only there when the graph runs
+    # (and may be dropped here while the graph still reads it): no cache for either.
+    if b.is_inference() or _capturing(b):
         bt = b.t().to(want).contiguous()
         return bt, bt.stride(0)
     key = (b.data_ptr(), tuple(b.shape), tuple(b.stride()), b.dtype, b._version, want)

@@ -96,3 +96,22 @@ def test_gemms_that_draw_their_tiles_replay_under_cuda_graph():
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(out, chain())
+
+
+def test_row_major_weight_first_used_inside_a_capture():
+    g = torch.Generator().manual_seed(97)
+    a = torch.randn(256, 264, generator=g).to(torch.bfloat16).cuda()
+    b = (0.05 * torch.randn(264, 520, generator=g)).to(torch.bfloat16).cuda()        # row-major: laid out K-major by the op
+    fused.matmul(a, (0.05 * torch.randn(264, 520, generator=g)).to(torch.bfloat16).cuda())
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = fused.matmul(a, b)
+    ref = a.float() @ b.float()
+    c = fused.matmul(a, b)                       # before the graph has run
+    torch.testing.assert_close(c.float(), ref, atol=2e-2, rtol=2e-2)
+    for _ in range(2):
+        graph.replay()
+        torch.cuda.synchronize()
+        torch.testing.assert_close(out.float(), a.float() @ b.float(), atol=2e-2, rtol=2e-2)
+        b.mul_(-1)                               # the graph lays out what the weight holds when it runs
