@@ -57,11 +57,17 @@ def as_k_major_bt(b: torch.Tensor, keep_fp32: bool = False) -> tuple[torch.Tenso
         bt = b.t().to(want).contiguous()
         return bt, bt.stride(0)
     key = (b.data_ptr(), tuple(b.shape), tuple(b.stride()), b.dtype, b._version, want)
+    stream = torch.cuda.current_stream(b.device) if b.is_cuda else None
     hit = _bt_cache.get(key)
     if hit is not None:
-        return hit[0], hit[0].stride(0)
+        bt, _, made_on, ready = hit
+        if made_on is not None and made_on != stream:
+            stream.wait_event(ready)
+            bt.record_stream(stream)     # dropped from the cache, it may still be read here
+        return bt, bt.stride(0)
     bt = b.t().to(want).contiguous()
     if len(_bt_cache) > 64:
         _bt_cache.clear()
-    _bt_cache[key] = (bt, b)     # keep `b` alive so the key's data_ptr cannot be recycled
+    # keep `b` alive so the key's data_ptr cannot be recycled
+    _bt_cache[key] = (bt, b, stream, stream.record_event() if stream is not None else None)
     return bt, bt.stride(0)

@@ -115,3 +115,22 @@ def test_row_major_weight_first_used_inside_a_capture():
         torch.cuda.synchronize()
         torch.testing.assert_close(out.float(), a.float() @ b.float(), atol=2e-2, rtol=2e-2)
         b.mul_(-1)                               # the graph lays out what the weight holds when it runs
+
+
+def test_row_major_weight_laid_out_on_another_stream():
+    g = torch.Generator().manual_seed(98)
+    a = torch.randn(256, 4096, generator=g).to(torch.bfloat16).cuda()
+    busy = torch.randn(8192, 8192, generator=g).cuda()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    for i in range(3):
+        b = (0.02 * torch.randn(4096, 4096, generator=g)).to(torch.bfloat16).cuda()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(streams[0]):
+            for _ in range(4):
+                busy @ busy                      # the layout waits behind these
+            first = fused.matmul(a, b)
+        with torch.cuda.stream(streams[1]):
+            second = fused.matmul(a, b)          # must wait for it
+        torch.cuda.synchronize()
+        assert torch.equal(first, second)
+        torch.testing.assert_close(second.float(), a.float() @ b.float(), atol=2e-2, rtol=2e-2)
