@@ -83,7 +83,14 @@ static PlainPlan plain_plan(const DeviceState* d, int M, int N, int K, int elt, 
   const double hbm_us = ((double)M + N) * K * elt / 5e6;         // with the rate that short kernels reach
   const bool whole_chip = max_ctas <= 0 && !emu;
   pl.swap = swap_ab < 0 ? (M <= 64 && N >= 128) : swap_ab != 0;
-  if (bn_override >= 1000 && pair_ok) {
+  if (bn_override >= 10000 && !emu) {
+    pl.kind = PLAIN_TILE;
+    pl.splits = bn_override / 10000;
+    pl.pair = bn_override / 1000 % 10 != 0;
+    pl.bn = bn_override % 1000;
+    return pl;
+  }
+  if (bn_override >= 1000 && bn_override < 10000 && pair_ok) {
     pl.kind = PLAIN_FLOW;
     pl.bn = bn_override % 1000;
     pl.rb = bn_override / 1000;
@@ -200,7 +207,8 @@ KR_API int kr_gemm_scratch(int M, int N, int K, long long lda, long long ldb, in
 // out[M,N] (bf16 or fp32, row stride ldo) = act(a[M,K] (row stride lda) * bt[N,K]^T (row stride ldb)).
 // act: 0 none, 1 GELU (tanh form), on the fp32 sums.
 // swap_ab: -1 auto, 0/1 forced (1: the weights are the row operand).
-// bn_override: 0 auto, 16 ... 256 a column tile, 1000 * b + n persistent pairs with b row blocks x n columns.
+// bn_override: 0 auto, 16 ... 256 a column tile, 1000 * b + n persistent pairs with b row blocks x n columns, 10000 * s +
+// 1000 * p + n the one-wave kernel with s K ranges, single CTAs (p 0) or pairs (p 1) and n columns.
 // use_pair: 0 forces the single-CTA kernels, anything else lets eligible shapes use CTA pairs.
 // in_fp32: a and bt hold fp32 and are multiplied as tf32 (strides in elements).
 // counters: as many zero words as kr_gemm_scratch says for the same arguments (zero again after the call;

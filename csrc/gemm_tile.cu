@@ -8,12 +8,15 @@
 //
 // Why clusters and not partial sums in global memory: a 256 x 256 tile split in two costs 15-18 us there
 // (slots out to L2, an atomic, slots back in: measured with %globaltimer stamps) and about 4 us here.
-// The accumulators go TMEM -> own shared memory (the operand stages are free by then); after one
-// cluster barrier every CTA of the cluster sums and stores an equal share of the tile, reading the
-// others' shared memory, with all ten warps, so that the store is shared out as well. A warp reads 512
-// consecutive bytes of a peer at a time (scattered 16-byte units measured a third of the rate), hence two
-// staging layouts: [unit of four columns][row] for a transposed store, [row][unit] with the units of a row
-// permuted by the row number (no bank conflicts for the row-per-lane writes) for a row-major one.
+//
+// The sums are SENT: every CTA owns an equal share of the tile's rows, and the others store their partial sums of it
+// straight from registers into its shared memory (st.async, counted on an mbarrier of the owner; the operand stages are
+// free by then). The owner adds them in split order and stores its rows. One cluster barrier, whose latency the first
+// read of the accumulator hides, says that the stages are free; nothing follows the stores. Against the other order
+// (accumulator into own shared memory, cluster barrier, owners fetch, cluster barrier before anybody may leave), us a call
+// in a stream of them: 8 x 4096 x 4096 9.9 to 9.5, 35 x 4064 x 5416 14.4 to 12.9, 102 x 1240 x 2816 9.9 to 8.1,
+// 100 x 4000 x 9000 21.6 to 19.8. What bounds this part now is the way between SMs: 64 KB leave an SM in 2700 clocks
+// (24 bytes each; bulk copies 3400, plain remote stores and a barrier 4200, fetches 3900), whatever the cluster size.
 #include <algorithm>
 #include <cmath>
 #include <map>
@@ -47,45 +50,42 @@ struct TileCfg {
   static constexpr int STAGES = RAW_STAGES > 12 ? 12 : RAW_STAGES;
   static constexpr int TMEM_COLS = BN <= 32 ? 32 : BN <= 64 ? 64 : BN <= 128 ? 128 : 256;
   static constexpr int SMEM = 1024 + STAGES * STAGE + 512;
-  static_assert(BN * kBM * 4 <= STAGES * STAGE, "the accumulator has to fit the stages");
+  // what arrives for the largest share: 48 rows of three pairs, 32 rows of seven CTAs, or 128 of one
+  static_assert(BN / 4 * (PAIR ? 3 * 49 : 7 * 33) * 16 <= STAGES * STAGE && BN / 4 * 129 * 16 <= STAGES * STAGE, "the sums have to fit the stages");
 };
 
-__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
+__device__ __forceinline__ float4 ld_shared_f4(uint32_t addr) {
   float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
   return v;
 }
+// 16 bytes into the shared memory of a CTA of the cluster, counted on an mbarrier there.
+__device__ __forceinline__ void push_cluster_u4(uint32_t addr, uint32_t bar, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1,%2,%3,%4}, [%5];"
+               ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ uint32_t cluster_size() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
   return r;
 }
 
-// acc[k] = sum over the splits, in order, of the four columns at staging offset off[k]. Loops, not
-// straight-line code: the epilogue runs once per launch out of a cold instruction cache, and code that
-// was unrolled over splits and units spent more time on fetching itself than on the sums.
-template <int UN>
-__device__ __forceinline__ void sum_splits(uint32_t slot0, uint32_t ctas, uint32_t half, int splits, const uint32_t (&off)[UN], float4 (&acc)[UN]) {
-#pragma unroll
-  for (int k = 0; k < UN; ++k) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 1
-  for (int i = 0; i < splits; i += 2) {
-    const uint32_t a = mapa_shared(slot0, (uint32_t)i * ctas + half), b = mapa_shared(slot0, (uint32_t)min(i + 1, splits - 1) * ctas + half);
-    float4 x[UN], y[UN];
-#pragma unroll
-    for (int k = 0; k < UN; ++k) x[k] = ld_cluster_f4(a + off[k]);
-#pragma unroll
-    for (int k = 0; k < UN; ++k) y[k] = ld_cluster_f4(b + off[k]);
-    const float s = i + 1 < splits ? 1.f : 0.f;
-#pragma unroll
-    for (int k = 0; k < UN; ++k) {
-      acc[k].x = (acc[k].x + x[k].x) + s * y[k].x;
-      acc[k].y = (acc[k].y + x[k].y) + s * y[k].y;
-      acc[k].z = (acc[k].z + x[k].z) + s * y[k].z;
-      acc[k].w = (acc[k].w + x[k].w) + s * y[k].w;
+// Until all partial sums of this CTA's share are here. Longer than any other wait of the cluster can take, recorded
+// error or not: who leaves early is written to after it has left.
+__device__ __forceinline__ void wait_sums(uint32_t bar, const SyncCtx& c) {
+  const uint64_t t0 = globaltimer_ns();
+  while (!mbar_try_wait(bar, 0))
+    if (globaltimer_ns() - t0 > 4 * c.timeout_ns + 50 * kMbarGraceNs) {
+      set_status(c, make_status(KR_ERR_TIMEOUT_MBAR, 83, 0, blockIdx.x));
+      return;
     }
-  }
 }
+
+// The rows of a CTA's 128 x BN part of the tile that split k sums and stores: groups of 16 rows (whole 32-byte
+// sectors of a transposed bf16 store), as even as eight groups go.
+__device__ __forceinline__ int share_begin(int k, int splits) { return (8 * k + splits - 1) / splits * 16; }
 
 template <int BN, int ELT, bool PAIR>
 __global__ void __launch_bounds__(kTileThreads, 1) gemm_tile_kernel(const __grid_constant__ TileParams p) {
@@ -108,12 +108,17 @@ __global__ void __launch_bounds__(kTileThreads, 1) gemm_tile_kernel(const __grid
   const uint32_t bars = stage0 + Cfg::STAGES * Cfg::STAGE;
   auto full_bar = [&](int s) { return bars + 8u * s; };
   auto empty_bar = [&](int s) { return bars + 8u * (Cfg::STAGES + s); };
-  auto row_unit_off = [](int row, int unit) {
-    constexpr int PERM = BN / 4 < 8 ? BN / 4 - 1 : 7;
-    return (uint32_t)(row * (BN / 4) + (unit ^ (row & PERM))) * 16u;
-  };
   const uint32_t done_bar = bars + 8u * (2 * Cfg::STAGES);
-  const uint32_t tmem_slot = done_bar + 8;
+  const uint32_t sum_bar = done_bar + 8, tmem_slot = done_bar + 16;
+
+  // Shares of this CTA's part of the tile. A split's partial sums arrive at the owner of a row as 16-byte units of
+  // four columns, [split][unit][row]: what a warp sends is contiguous. Units past the output are not sent.
+  const int valid_cols = (p.transposed ? p.out_rows : p.out_cols) - tc * BN;
+  const int units = min(BN, valid_cols + 3) / 4;
+  const int row_lo = share_begin(split, splits), rows = share_begin(split + 1, splits) - row_lo;
+  const uint32_t unit_bytes = (uint32_t)rows * 16u + 16u;      // a row of padding against bank conflicts
+  const int valid_rows = (p.transposed ? p.out_cols : p.out_rows) - tr * kBM;
+  const int rows_left = min(max(valid_rows - row_lo, 0), rows);   // of the share; rows past the output are not sent either
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < Cfg::STAGES; ++s) {
@@ -121,7 +126,9 @@ __global__ void __launch_bounds__(kTileThreads, 1) gemm_tile_kernel(const __grid
       mbar_init(empty_bar(s), 1);
     }
     mbar_init(done_bar, 1);
+    mbar_init(sum_bar, 1 + kTileThreads / 32 - 2);
     mbar_fence_init();
+    mbar_expect_tx(sum_bar, (uint32_t)((splits - 1) * units * rows_left) * 16u);
     tma_prefetch_desc(&p.tmap_r);
     tma_prefetch_desc(&p.tmap_c);
   }
@@ -215,106 +222,119 @@ __global__ void __launch_bounds__(kTileThreads, 1) gemm_tile_kernel(const __grid
       }
       for (; v < hi; v += T) st16((char*)p.cp_dst + v * 16, ld16((const char*)p.cp_src + v * 16));
     }
-    // ---- accumulator -> own shared memory, as 16-byte units of four columns
-    bool ok = mbar_wait(done_bar, 0, p.sync, 82);
-    ok = __all_sync(0xffffffffu, ok);
-    tc_fence_after();
-    constexpr int CH = BN < 32 ? BN : 32;                  // two warps per TMEM lane quarter take turns
-    const int q = warp & 3, h = (warp - 2) >> 2;
-    if (ok) {
-      const int row = q * 32 + lane;
-#pragma unroll 1
-      for (int c0 = h * CH; c0 < BN; c0 += 2 * CH) {
-        uint32_t r[32];
-        const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c0;
-        if (CH == 32) tmem_ld32(t_addr, r);
-        else tmem_ld16(t_addr, r);
-        tmem_ld_wait();
-#pragma unroll
-        for (int u = 0; u < CH / 4; ++u)
-          st_shared_u4(stage0 + (p.transposed ? (uint32_t)((c0 / 4 + u) * kBM + row) * 16u : row_unit_off(row, c0 / 4 + u)), r[4 * u], r[4 * u + 1], r[4 * u + 2], r[4 * u + 3]);
-      }
-    }
+    mbar_wait(done_bar, 0, p.sync, 82);      // what a wait that ran out leaves is sent all the same: the others count on it
   }
   __syncwarp();
-  tc_fence_before();
-  if (csize > 1) cluster_sync_all();
-  else __syncthreads();
   tc_fence_after();
+  // From here on this CTA's stages are free for what the others send. Nobody waits for more than that: the sums are
+  // sent, not fetched, and whoever has them all stores and leaves.
+  if (csize > 1) cluster_arrive();
+  if (warp >= 2) {
+    constexpr int CH = BN < 32 ? BN : 32;                  // two warps per TMEM lane quarter take turns
+    const int q = warp & 3, h = (warp - 2) >> 2, row = q * 32 + lane;
+    const int to = (row / 16) * splits / 8, to_lo = share_begin(to, splits);
+    const uint32_t to_bytes = (uint32_t)(share_begin(to + 1, splits) - to_lo) * 16u + 16u;
+    const uint32_t to_rank = (uint32_t)to * CTAS + half;
+    const uint32_t slot = (uint32_t)(split * units) * to_bytes + (uint32_t)(row - to_lo) * 16u;
+    const uint32_t dst = to == split ? stage0 + slot : mapa_shared(stage0, to_rank) + slot, dst_bar = mapa_shared(sum_bar, to_rank);
+    bool waited = csize == 1;
+#pragma unroll 1
+    for (int c0 = h * CH; c0 < units * 4; c0 += 2 * CH) {
+      uint32_t r[32];
+      const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c0;
+      if (CH == 32) tmem_ld32(t_addr, r);
+      else tmem_ld16(t_addr, r);
+      tmem_ld_wait();
+      if (!waited) cluster_wait();
+      waited = true;
+#pragma unroll
+      for (int u = 0; u < CH / 4; ++u) {
+        if (c0 / 4 + u >= units || row >= valid_rows) continue;
+        const uint32_t a = dst + (uint32_t)(c0 / 4 + u) * to_bytes;
+        if (to == split) st_shared_u4(a, r[4 * u], r[4 * u + 1], r[4 * u + 2], r[4 * u + 3]);
+        else push_cluster_u4(a, dst_bar, r[4 * u], r[4 * u + 1], r[4 * u + 2], r[4 * u + 3]);
+      }
+    }
+    if (!waited) cluster_wait();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(sum_bar);
+  } else if (csize > 1) {
+    cluster_wait();
+  }
+  __syncwarp();
+  wait_sums(sum_bar, p.sync);
 
-  // ---- sum over the splits and store: share `split` of this CTA's 128 x BN part of the tile
-  constexpr int UN = 2;                                    // 16-byte units per thread and split in flight
-  constexpr int UNITS = BN / 4 * kBM;
-  const int lo = UNITS / 64 * split / splits * 64, hi = UNITS / 64 * (split + 1) / splits * 64;
-  const uint32_t slot0 = stage0;
+  // ---- sum over the splits, in order, and store
   const bool fp32 = p.out_fp32 != 0, act = p.act != 0;
+  const uint32_t split_bytes = (uint32_t)units * unit_bytes;
+  auto unit_addr = [&](int unit, int row) { return stage0 + (uint32_t)unit * unit_bytes + (uint32_t)row * 16u; };
+  // two units at a time: the loads of a split are in flight together
+  auto sum_units = [&](uint32_t a, uint32_t b, float (&v)[8]) {
+    float4 x = ld_shared_f4(a), y = ld_shared_f4(b);
+#pragma unroll 1
+    for (int k = 1; k < splits; ++k) {
+      const float4 s = ld_shared_f4(a += split_bytes), t = ld_shared_f4(b += split_bytes);
+      x = make_float4(x.x + s.x, x.y + s.y, x.z + s.z, x.w + s.w);
+      y = make_float4(y.x + t.x, y.y + t.y, y.z + t.z, y.w + t.w);
+    }
+    v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+    v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
+  };
   if (p.transposed) {
     // D(i, j) -> out[tc*BN + j][tr*128 + i]; lanes = consecutive i
-    const int cols_left = p.out_rows - tc * BN, rows_left = p.out_cols - tr * kBM;
-    char* const out = (char*)p.out + ((long long)tc * BN * p.ldo + tr * kBM) * (fp32 ? 4 : 2);
+    char* const out = (char*)p.out + ((long long)tc * BN * p.ldo + tr * kBM + row_lo) * (fp32 ? 4 : 2);
 #pragma unroll 1
-    for (int e0 = lo + (int)threadIdx.x; e0 < hi; e0 += UN * kTileThreads) {
-      float4 acc[UN];
-      uint32_t off[UN];
+    for (int e = (int)threadIdx.x; e < (units + 1) / 2 * rows; e += kTileThreads) {
+      const int u = e / rows * 2, i = e - u / 2 * rows;
+      if (i >= rows_left) continue;
+      float v[8];
+      sum_units(unit_addr(u, i), unit_addr(min(u + 1, units - 1), i), v);
 #pragma unroll
-      for (int k = 0; k < UN; ++k) off[k] = (uint32_t)min(e0 + k * kTileThreads, hi - 1) * 16u;
-      sum_splits<UN>(slot0, CTAS, half, splits, off, acc);
-#pragma unroll
-      for (int k = 0; k < UN; ++k) {
-        const int e = e0 + k * kTileThreads, i = e % kBM;
-        if (e < hi && i < rows_left) {
-          const float v[4] = {acc[k].x, acc[k].y, acc[k].z, acc[k].w};
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const int j = e / kBM * 4 + c;
-            if (j < cols_left) {
-              const float y = act ? gelu_tanh(v[c]) : v[c];
-              if (fp32) ((float*)out)[(long long)j * p.ldo + i] = y;
-              else ((__nv_bfloat16*)out)[(long long)j * p.ldo + i] = __float2bfloat16(y);
-            }
-          }
+      for (int c = 0; c < 8; ++c) {
+        const int j = u * 4 + c;
+        if (j < valid_cols) {
+          const float y = act ? gelu_tanh(v[c]) : v[c];
+          if (fp32) ((float*)out)[(long long)j * p.ldo + i] = y;
+          else ((__nv_bfloat16*)out)[(long long)j * p.ldo + i] = __float2bfloat16(y);
         }
       }
     }
   } else {
     // D(i, j) -> out[tr*128 + i][tc*BN + j]; lanes = consecutive groups of eight columns
-    constexpr int GROUPS = BN / 8;                         // per row
+    const int groups = (units + 1) / 2;
     const bool vec_ok = (p.ldo * (fp32 ? 4 : 2)) % 16 == 0 && ((uintptr_t)p.out & 15) == 0;
 #pragma unroll 1
-    for (int e = lo / 2 + (int)threadIdx.x; e < hi / 2; e += kTileThreads) {
-      const int i = e / GROUPS, u = e % GROUPS * 2;
-      const int row = tr * kBM + i, col = tc * BN + u * 4;
-      float4 acc[2];
-      const uint32_t off[2] = {row_unit_off(i, u), row_unit_off(i, u + 1)};
-      sum_splits<2>(slot0, CTAS, half, splits, off, acc);
-      if (row < p.out_rows && col < p.out_cols) {
-        float v[8] = {acc[0].x, acc[0].y, acc[0].z, acc[0].w, acc[1].x, acc[1].y, acc[1].z, acc[1].w};
-        if (act) {
+    for (int e = (int)threadIdx.x; e < rows_left * groups; e += kTileThreads) {
+      const int i = e / groups, u = (e - i * groups) * 2;
+      const int row = tr * kBM + row_lo + i, col = tc * BN + u * 4;
+      float v[8];
+      sum_units(unit_addr(u, i), unit_addr(min(u + 1, units - 1), i), v);
+      if (act) {
 #pragma unroll
-          for (int c = 0; c < 8; ++c) v[c] = gelu_tanh(v[c]);
-        }
-        char* o = (char*)p.out + ((long long)row * p.ldo + col) * (fp32 ? 4 : 2);
-        if (vec_ok && col + 8 <= p.out_cols) {
-          if (fp32) {
-            st16(o, U4{__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3])});
-            st16(o + 16, U4{__float_as_uint(v[4]), __float_as_uint(v[5]), __float_as_uint(v[6]), __float_as_uint(v[7])});
-          } else {
-            st16(o, pack8(v));
-          }
+        for (int c = 0; c < 8; ++c) v[c] = gelu_tanh(v[c]);
+      }
+      char* o = (char*)p.out + ((long long)row * p.ldo + col) * (fp32 ? 4 : 2);
+      if (vec_ok && col + 8 <= p.out_cols) {
+        if (fp32) {
+          st16(o, U4{__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3])});
+          st16(o + 16, U4{__float_as_uint(v[4]), __float_as_uint(v[5]), __float_as_uint(v[6]), __float_as_uint(v[7])});
         } else {
-#pragma unroll
-          for (int c = 0; c < 8; ++c)
-            if (col + c < p.out_cols) {
-              if (fp32) ((float*)o)[c] = v[c];
-              else ((__nv_bfloat16*)o)[c] = __float2bfloat16(v[c]);
-            }
+          st16(o, pack8(v));
         }
+      } else {
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+          if (col + c < p.out_cols) {
+            if (fp32) ((float*)o)[c] = v[c];
+            else ((__nv_bfloat16*)o)[c] = __float2bfloat16(v[c]);
+          }
       }
     }
   }
-  // nobody leaves while the cluster may still read its shared memory (or the pair its barriers)
+  // Everything sent to this CTA has arrived, and who it sent to is still waiting for that: a single CTA may leave. The
+  // CTAs of a pair give back their tensor memory together.
   tc_fence_before();
-  if (csize > 1) cluster_sync_all();
+  if (PAIR) cluster_sync_all();
   else __syncthreads();
   if (warp == 1) {
     tc_fence_after();
@@ -336,7 +356,8 @@ static TileVariant tile_variant(int bn, bool pair) {
       case 160: return {(const void*)gemm_tile_kernel<160, ELT, true>, TileCfg<160, true>::SMEM};
       case 192: return {(const void*)gemm_tile_kernel<192, ELT, true>, TileCfg<192, true>::SMEM};
       case 224: return {(const void*)gemm_tile_kernel<224, ELT, true>, TileCfg<224, true>::SMEM};
-      default: return {(const void*)gemm_tile_kernel<256, ELT, true>, TileCfg<256, true>::SMEM};
+      case 256: return {(const void*)gemm_tile_kernel<256, ELT, true>, TileCfg<256, true>::SMEM};
+      default: return {nullptr, 0};
     }
   }
   switch (bn) {
@@ -408,13 +429,15 @@ int tile_gemm_splits(const DeviceState* d, int tiles, int num_kb, int bn, bool p
 
 int launch_tile_gemm(const GemmParams& g, int bn, bool pair, int splits, cudaStream_t stream) {
   const TileVariant v = g.in_fp32 ? tile_variant<4>(bn, pair) : tile_variant<2>(bn, pair);
-  if (v.fn == nullptr) return fail(KR_FAIL_ARG, "no one-wave kernel of this tile width");
+  const int num_kb = (g.K + (g.in_fp32 ? 32 : 64) - 1) / (g.in_fp32 ? 32 : 64);
+  if (v.fn == nullptr || (pair && bn % 32 != 0)) return fail(KR_FAIL_ARG, "no one-wave kernel of this tile width");
+  if (splits < 1 || splits * (pair ? 2 : 1) > 8 || splits > num_kb) return fail(KR_FAIL_ARG, "no such number of K ranges");
   TileParams p;
   p.tmap_r = g.tmap_r;
   p.tmap_c = g.tmap_c;
   p.tiles_r = g.tiles_r;
   p.tiles_c = g.tiles_c;
-  p.num_kb = (g.K + (g.in_fp32 ? 32 : 64) - 1) / (g.in_fp32 ? 32 : 64);
+  p.num_kb = num_kb;
   p.transposed = g.transposed;
   p.out_fp32 = g.out_fp32;
   p.act = g.act;

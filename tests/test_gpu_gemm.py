@@ -463,6 +463,26 @@ def test_gemm_persistent_pairs_every_tile_shape(bn, swap):
     assert ((c.float() - ref).norm() / ref.norm()).item() < 3e-3
 
 
+@pytest.mark.parametrize("splits", [1, 2, 3, 4, 5, 6, 7, 8])
+@pytest.mark.parametrize("swap", [0, 1])
+def test_gemm_one_wave_every_split_and_tile(splits, swap):
+    # 10000 * splits + 1000 * pairs + columns: each split owns 16 ... 128 rows of a tile; rows and columns past the
+    # output are neither sent nor waited for (last row block of 1 and of 0 rows in a pair, 1 ... 4 columns of a unit)
+    for bn, dtype in [(16, 0), (32, 0), (64, 0), (128, 0), (16, 1), (128, 1), (1128, 0), (1160, 0), (1224, 1), (1256, 0)]:
+        if bn >= 1000 and splits > 4:
+            continue
+        dtype = torch.float32 if dtype else torch.bfloat16
+        for M, N, K in [(129, 264, 584), (1, 136, 1096), (300, 1032, 512)]:
+            g = torch.Generator().manual_seed(71)
+            a = torch.randn(M, K, generator=g).to(dtype).cuda()
+            bt = (0.05 * torch.randn(N, K, generator=g)).to(dtype).cuda()
+            ref = (a.double() @ bt.double().t()).float()
+            for out_dtype, limit in ((torch.float32, 1e-5 if dtype == torch.bfloat16 else 1e-3), (torch.bfloat16, 3e-3)):
+                c = fused.matmul(a, bt.t(), out_dtype=out_dtype, bn=10000 * splits + bn, swap_ab=swap)
+                assert ((c.float() - ref).norm() / ref.norm()).item() < limit
+                assert torch.equal(c, fused.matmul(a, bt.t(), out_dtype=out_dtype, bn=10000 * splits + bn, swap_ab=swap))
+
+
 @pytest.mark.parametrize("M,N,bn,swap", [(520, 1024, 1256, 0), (1500, 2080, 2256, 0), (520, 1024, 2144, 0), (777, 1160, 1096, 0), (520, 1024, 1192, 1),
                                          (520, 1001, 1144, 0), (520, 1001, 2128, 1), (16, 1024, 0, -1), (200, 520, 0, -1), (64, 136, 64, 0), (77, 520, 256, 0)])
 @pytest.mark.parametrize("out_fp32", [False, True])
