@@ -64,7 +64,7 @@ __device__ __forceinline__ void push_cluster_u4(uint32_t addr, uint32_t bar, uin
   asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1,%2,%3,%4}, [%5];"
                ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d), "r"(bar) : "memory");
 }
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ uint32_t cluster_size() {
   uint32_t r;
@@ -144,6 +144,20 @@ __global__ void __launch_bounds__(kTileThreads, 1) gemm_tile_kernel(const __grid
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
   pdl_launch();
   pdl_wait();
+
+  // Worked out now, while nothing waits for it (the divisions took 300 clocks of the tail): where this thread's row of the
+  // accumulator goes, and which of the sums it stores first.
+  constexpr int CH = BN < 32 ? BN : 32;                    // two warps per TMEM lane quarter take turns
+  const int q = warp & 3, h = (warp - 2) >> 2, acc_row = q * 32 + lane;
+  const int to = acc_row / 16 * splits / 8, to_lo = share_begin(to, splits);
+  uint32_t to_bytes = (uint32_t)(share_begin(to + 1, splits) - to_lo) * 16u + 16u;
+  const uint32_t to_rank = (uint32_t)to * CTAS + half;
+  const uint32_t slot = (uint32_t)(split * units) * to_bytes + (uint32_t)(acc_row - to_lo) * 16u;
+  uint32_t dst = to == split ? stage0 + slot : mapa_shared(stage0, to_rank) + slot, dst_bar = mapa_shared(sum_bar, to_rank);
+  const int groups = (units + 1) / 2;                      // of eight columns
+  const int items = p.transposed ? groups * rows : rows_left * groups, per = p.transposed ? rows : groups;
+  int hi = (int)threadIdx.x / per, lo = (int)threadIdx.x - hi * per;
+  asm volatile("" : "+r"(to_bytes), "+r"(dst), "+r"(dst_bar), "+r"(hi), "+r"(lo));
 
   if (warp == 0) {
     if (elect_one()) {
@@ -230,13 +244,6 @@ __global__ void __launch_bounds__(kTileThreads, 1) gemm_tile_kernel(const __grid
   // sent, not fetched, and whoever has them all stores and leaves.
   if (csize > 1) cluster_arrive();
   if (warp >= 2) {
-    constexpr int CH = BN < 32 ? BN : 32;                  // two warps per TMEM lane quarter take turns
-    const int q = warp & 3, h = (warp - 2) >> 2, row = q * 32 + lane;
-    const int to = (row / 16) * splits / 8, to_lo = share_begin(to, splits);
-    const uint32_t to_bytes = (uint32_t)(share_begin(to + 1, splits) - to_lo) * 16u + 16u;
-    const uint32_t to_rank = (uint32_t)to * CTAS + half;
-    const uint32_t slot = (uint32_t)(split * units) * to_bytes + (uint32_t)(row - to_lo) * 16u;
-    const uint32_t dst = to == split ? stage0 + slot : mapa_shared(stage0, to_rank) + slot, dst_bar = mapa_shared(sum_bar, to_rank);
     bool waited = csize == 1;
 #pragma unroll 1
     for (int c0 = h * CH; c0 < units * 4; c0 += 2 * CH) {
@@ -249,7 +256,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) gemm_tile_kernel(const __grid
       waited = true;
 #pragma unroll
       for (int u = 0; u < CH / 4; ++u) {
-        if (c0 / 4 + u >= units || row >= valid_rows) continue;
+        if (c0 / 4 + u >= units || acc_row >= valid_rows) continue;
         const uint32_t a = dst + (uint32_t)(c0 / 4 + u) * to_bytes;
         if (to == split) st_shared_u4(a, r[4 * u], r[4 * u + 1], r[4 * u + 2], r[4 * u + 3]);
         else push_cluster_u4(a, dst_bar, r[4 * u], r[4 * u + 1], r[4 * u + 2], r[4 * u + 3]);
@@ -265,7 +272,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) gemm_tile_kernel(const __grid
   wait_sums(sum_bar, p.sync);
 
   // ---- sum over the splits, in order, and store
-  const bool fp32 = p.out_fp32 != 0, act = p.act != 0;
+  const bool fp32 = p.out_fp32 != 0, act = p.act != 0, vec_ok = (p.ldo * (fp32 ? 4 : 2)) % 16 == 0 && ((uintptr_t)p.out & 15) == 0;
   const uint32_t split_bytes = (uint32_t)units * unit_bytes;
   auto unit_addr = [&](int unit, int row) { return stage0 + (uint32_t)unit * unit_bytes + (uint32_t)row * 16u; };
   // two units at a time: the loads of a split are in flight together
@@ -280,55 +287,55 @@ __global__ void __launch_bounds__(kTileThreads, 1) gemm_tile_kernel(const __grid
     v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
     v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
   };
-  if (p.transposed) {
-    // D(i, j) -> out[tc*BN + j][tr*128 + i]; lanes = consecutive i
-    char* const out = (char*)p.out + ((long long)tc * BN * p.ldo + tr * kBM + row_lo) * (fp32 ? 4 : 2);
 #pragma unroll 1
-    for (int e = (int)threadIdx.x; e < (units + 1) / 2 * rows; e += kTileThreads) {
-      const int u = e / rows * 2, i = e - u / 2 * rows;
-      if (i >= rows_left) continue;
-      float v[8];
-      sum_units(unit_addr(u, i), unit_addr(min(u + 1, units - 1), i), v);
+  for (int e = (int)threadIdx.x; e < items;) {
+    const int u = (p.transposed ? hi : lo) * 2, i = p.transposed ? lo : hi;
+    float v[8];
+    sum_units(unit_addr(u, i), unit_addr(min(u + 1, units - 1), i), v);
+    if (act) {
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const int j = u * 4 + c;
-        if (j < valid_cols) {
-          const float y = act ? gelu_tanh(v[c]) : v[c];
-          if (fp32) ((float*)out)[(long long)j * p.ldo + i] = y;
-          else ((__nv_bfloat16*)out)[(long long)j * p.ldo + i] = __float2bfloat16(y);
+      for (int c = 0; c < 8; ++c) v[c] = gelu_tanh(v[c]);
+    }
+    const int left = valid_cols - u * 4;                   // of the eight columns, those inside the output
+    if (p.transposed) {
+      // D(i, j) -> out[tc*BN + j][tr*128 + i]; lanes = consecutive i
+      const long long o = (long long)(tc * BN + u * 4) * p.ldo + tr * kBM + row_lo + i;
+      if (i < rows_left) {
+        if (fp32) {
+          float* out = (float*)p.out + o;
+#pragma unroll
+          for (int c = 0; c < 8; ++c, out += p.ldo)
+            if (c < left) *out = v[c];
+        } else {
+          __nv_bfloat16* out = (__nv_bfloat16*)p.out + o;
+#pragma unroll
+          for (int c = 0; c < 8; ++c, out += p.ldo)
+            if (c < left) *out = __float2bfloat16(v[c]);
         }
       }
-    }
-  } else {
-    // D(i, j) -> out[tr*128 + i][tc*BN + j]; lanes = consecutive groups of eight columns
-    const int groups = (units + 1) / 2;
-    const bool vec_ok = (p.ldo * (fp32 ? 4 : 2)) % 16 == 0 && ((uintptr_t)p.out & 15) == 0;
-#pragma unroll 1
-    for (int e = (int)threadIdx.x; e < rows_left * groups; e += kTileThreads) {
-      const int i = e / groups, u = (e - i * groups) * 2;
-      const int row = tr * kBM + row_lo + i, col = tc * BN + u * 4;
-      float v[8];
-      sum_units(unit_addr(u, i), unit_addr(min(u + 1, units - 1), i), v);
-      if (act) {
-#pragma unroll
-        for (int c = 0; c < 8; ++c) v[c] = gelu_tanh(v[c]);
-      }
-      char* o = (char*)p.out + ((long long)row * p.ldo + col) * (fp32 ? 4 : 2);
-      if (vec_ok && col + 8 <= p.out_cols) {
+    } else {
+      // D(i, j) -> out[tr*128 + i][tc*BN + j]; lanes = consecutive groups of eight columns
+      const long long o = (long long)(tr * kBM + row_lo + i) * p.ldo + tc * BN + u * 4;
+      if (vec_ok && left >= 8) {
         if (fp32) {
-          st16(o, U4{__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3])});
-          st16(o + 16, U4{__float_as_uint(v[4]), __float_as_uint(v[5]), __float_as_uint(v[6]), __float_as_uint(v[7])});
+          float* out = (float*)p.out + o;
+          st16(out, U4{__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3])});
+          st16(out + 4, U4{__float_as_uint(v[4]), __float_as_uint(v[5]), __float_as_uint(v[6]), __float_as_uint(v[7])});
         } else {
-          st16(o, pack8(v));
+          st16((__nv_bfloat16*)p.out + o, pack8(v));
         }
       } else {
 #pragma unroll
         for (int c = 0; c < 8; ++c)
-          if (col + c < p.out_cols) {
-            if (fp32) ((float*)o)[c] = v[c];
-            else ((__nv_bfloat16*)o)[c] = __float2bfloat16(v[c]);
+          if (c < left) {
+            if (fp32) ((float*)p.out)[o + c] = v[c];
+            else ((__nv_bfloat16*)p.out)[o + c] = __float2bfloat16(v[c]);
           }
       }
+    }
+    if ((e += kTileThreads) < items) {
+      hi = e / per;
+      lo = e - hi * per;
     }
   }
   // Everything sent to this CTA has arrived, and who it sent to is still waiting for that: a single CTA may leave. The
