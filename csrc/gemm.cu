@@ -418,20 +418,25 @@ struct TmapKey {
   int elt;
   unsigned box_bytes;
   int promote;
+  unsigned narrow_rows;
   bool operator==(const TmapKey& o) const {
-    return ptr == o.ptr && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows && elt == o.elt && box_bytes == o.box_bytes && promote == o.promote;
+    return ptr == o.ptr && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows && elt == o.elt && box_bytes == o.box_bytes && promote == o.promote &&
+           narrow_rows == o.narrow_rows;
   }
 };
 struct TmapHash {
   size_t operator()(const TmapKey& k) const {
     unsigned long long h = (unsigned long long)(uintptr_t)k.ptr >> 4;
-    for (unsigned long long v : {k.rows, k.cols, k.ld, (unsigned long long)k.box_rows * 4096 + (unsigned long long)k.promote * 8 + k.box_bytes * 16 + (unsigned long long)k.elt})
+    for (unsigned long long v : {k.rows, k.cols, k.ld, (unsigned long long)k.narrow_rows << 32 | (unsigned long long)k.box_rows * 4096 + (unsigned long long)k.promote * 8 + k.box_bytes * 16 + (unsigned long long)k.elt})
       h = (h ^ v) * 0x9e3779b97f4a7c15ull;
     return (size_t)(h ^ (h >> 32));
   }
 };
 static std::mutex g_tmap_mu;
-static std::unordered_map<TmapKey, CUtensorMap, TmapHash> g_tmap_cache;
+struct TmapEntry {
+  CUtensorMap map, narrow;        // narrow: the same matrix with boxes of narrow_rows rows
+};
+static std::unordered_map<TmapKey, TmapEntry, TmapHash> g_tmap_cache;
 static std::deque<TmapKey> g_tmap_order;             // insertion order, for eviction
 constexpr size_t kTmapCacheEntries = 4096;
 static unsigned long long g_tmap_hits = 0, g_tmap_misses = 0;
@@ -439,14 +444,15 @@ static unsigned long long g_tmap_hits = 0, g_tmap_misses = 0;
 // Tensor map of a row-major matrix [rows, cols] of bf16 (elt 2) or fp32 (elt 4) elements (cols
 // contiguous, `ld` elements per row), box = box_bytes (128, 64 or, unswizzled, 32) of columns x box_rows rows, swizzled by as much,
 // out-of-range elements read as zero.
-int get_tmap(const void* ptr, unsigned long long rows, unsigned long long cols, unsigned long long ld,
-                    unsigned box_rows, CUtensorMap* out, int elt, unsigned box_bytes, bool promote_256) {
-  TmapKey key{ptr, rows, cols, ld, box_rows, elt, box_bytes, promote_256 ? 1 : 0};
+int get_tmap(const void* ptr, unsigned long long rows, unsigned long long cols, unsigned long long ld, unsigned box_rows, CUtensorMap* out,
+             int elt, unsigned box_bytes, bool promote_256, unsigned narrow_rows, CUtensorMap* narrow) {
+  TmapKey key{ptr, rows, cols, ld, box_rows, elt, box_bytes, promote_256 ? 1 : 0, narrow_rows};
   {
     std::lock_guard<std::mutex> lk(g_tmap_mu);
     auto it = g_tmap_cache.find(key);
     if (it != g_tmap_cache.end()) {
-      *out = it->second;
+      *out = it->second.map;
+      if (narrow_rows) *narrow = it->second.narrow;
       ++g_tmap_hits;
       return KR_SUCCESS;
     }
@@ -454,16 +460,19 @@ int get_tmap(const void* ptr, unsigned long long rows, unsigned long long cols, 
   KR_REQUIRE(((uintptr_t)ptr & 15) == 0, "GEMM operand must be 16-byte aligned");
   KR_REQUIRE(elt == 2 || elt == 4, "GEMM operands are bf16 or fp32");
   KR_REQUIRE((ld * elt) % 16 == 0, "GEMM operand row stride must be a multiple of 16 bytes");
-  KR_REQUIRE(box_rows >= 1 && box_rows <= 256, "bad TMA box");
+  KR_REQUIRE(box_rows >= 1 && box_rows <= 256 && narrow_rows <= 256, "bad TMA box");
   cuuint64_t gdim[2] = {cols, rows};
   cuuint64_t gstride[1] = {ld * (unsigned long long)elt};
-  cuuint32_t box[2] = {(cuuint32_t)(box_bytes / elt), box_rows};
   cuuint32_t estr[2] = {1, 1};
-  CUtensorMap m;
-  KR_CU(cuTensorMapEncodeTiled, &m, elt == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
-        const_cast<void*>(ptr), gdim, gstride, box,
-        estr, CU_TENSOR_MAP_INTERLEAVE_NONE, box_bytes == 32 ? CU_TENSOR_MAP_SWIZZLE_NONE : box_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, promote_256 ? CU_TENSOR_MAP_L2_PROMOTION_L2_256B : CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  TmapEntry e;
+  memset(&e, 0, sizeof(e));
+  for (int k = 0; k < (narrow_rows ? 2 : 1); ++k) {
+    cuuint32_t box[2] = {(cuuint32_t)(box_bytes / elt), k ? narrow_rows : box_rows};
+    KR_CU(cuTensorMapEncodeTiled, k ? &e.narrow : &e.map, elt == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
+          const_cast<void*>(ptr), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+          box_bytes == 32 ? CU_TENSOR_MAP_SWIZZLE_NONE : box_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
+          promote_256 ? CU_TENSOR_MAP_L2_PROMOTION_L2_256B : CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  }
   {
     std::lock_guard<std::mutex> lk(g_tmap_mu);
     // bounded: the oldest descriptors go first, so a loop over a few operands keeps hitting
@@ -471,10 +480,11 @@ int get_tmap(const void* ptr, unsigned long long rows, unsigned long long cols, 
       g_tmap_cache.erase(g_tmap_order.front());
       g_tmap_order.pop_front();
     }
-    if (g_tmap_cache.emplace(key, m).second) g_tmap_order.push_back(key);
+    if (g_tmap_cache.emplace(key, e).second) g_tmap_order.push_back(key);
     ++g_tmap_misses;
   }
-  *out = m;
+  *out = e.map;
+  if (narrow_rows) *narrow = e.narrow;
   return KR_SUCCESS;
 }
 
@@ -598,7 +608,8 @@ unsigned grid_cap(const DeviceState* d) {
 // Fills the operand/tiling part of the parameter block for C[M,N] = A[M,K] * Bt[N,K]^T.
 // swap: the weights (Bt) become the 128-row operand and the tile is stored transposed.
 int setup_problem(GemmParams& p, const void* a, long long lda, const void* bt, long long ldb, int M, int N,
-                         int K, bool swap, int bn_override, int* bn_out, int elt, int c_box_rows, bool promote_256) {
+                         int K, bool swap, int bn_override, int* bn_out, int elt, int c_box_rows, bool promote_256, int narrow_rows,
+                         CUtensorMap* narrow) {
   KR_REQUIRE(M >= 1 && N >= 1 && K >= 8 && (K * elt) % 16 == 0, "GEMM needs K rows of whole 16-byte units and positive sizes");
   p.in_fp32 = elt == 4 ? 1 : 0;
   const void* r = swap ? bt : a;
@@ -616,7 +627,7 @@ int setup_problem(GemmParams& p, const void* a, long long lda, const void* bt, l
   p.transposed = swap ? 1 : 0;
   int rc = get_tmap(r, p.rows_r, K, ldr, kBM, &p.tmap_r, elt, 128, promote_256);
   if (rc) return rc;
-  rc = get_tmap(c, p.rows_c, K, ldc, c_box_rows > 0 ? c_box_rows : bn, &p.tmap_c, elt, 128, promote_256);
+  rc = get_tmap(c, p.rows_c, K, ldc, c_box_rows > 0 ? c_box_rows : bn, &p.tmap_c, elt, 128, promote_256, (unsigned)narrow_rows, narrow);
   if (rc) return rc;
   p.host_c_ptr = c;
   p.host_ldc = ldc;

@@ -10,6 +10,9 @@
 //    per CTA and 256 x 256 x 64 block pair). The accumulators then fill TMEM, so a tile's first MMAs wait for the
 //    epilogue of the one before, row block by row block. RB = 1 keeps two accumulators in turn.
 // Column tiles (BN) of 64 ... 256, in steps of 16 from 128 on for bf16, fit ragged sizes and waves; the launcher picks.
+// The last column tile is as narrow as the output leaves it (16s), and a pair draws its next tile shortly before the end of
+// the one in hand: drawn at its start, the last tiles of 777 x 5120 x 13704 (256 columns, three wide and one narrow tile per
+// row of tiles) went to the pairs with the wide ones (172 us, now 141), those of 522 x 6156 x 4440 (tf32) as well (88, 73).
 // For fp32 operands the steps of 16 are neither built nor measured; nothing in the kernel forbids them.
 //
 // Warps: 0 TMA producer (the leader's also draws the tiles), 1 MMA issuer (leader), 2-5 epilogue (one per TMEM
@@ -27,7 +30,8 @@ constexpr int kFlowCopyThreads = 64;
 constexpr int kFlowSlots = 16;                            // more than the slowest role can be behind the producer, see next_item
 
 struct alignas(64) FlowParams {
-  CUtensorMap tmap_r, tmap_c, tmap_out, tmap_tail;      // tmap_tail: the last 16 columns of tiles with BN % 32 == 16
+  CUtensorMap tmap_r, tmap_c, tmap_last, tmap_out, tmap_tail;      // tmap_tail: the last 16 columns of tiles with BN % 32 == 16
+  int last_cols;                                          // columns of the last column tile, in 16s (tmap_last: boxes of half as many rows)
   int tiles_r, tiles_c, num_kb, group_r;                  // tiles of RB * 256 rows
   int items, split_from;                                  // tiles from split_from on are drawn as single row blocks
   int transposed, out_fp32, act;
@@ -127,6 +131,7 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
     mbar_fence_init();
     tma_prefetch_desc(&p.tmap_r);
     tma_prefetch_desc(&p.tmap_c);
+    tma_prefetch_desc(&p.tmap_last);
     tma_prefetch_desc(&p.tmap_out);
   }
   if (warp == 1) {
@@ -182,13 +187,17 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
       int t = pair;
       for (int k = 0; ok && t < p.items; ++k) {
         int drawn = 0;
-        // Drawn now and published a few K blocks on, when the atomic has long returned: the peer's producer goes
-        // on to the next tile without a gap. Without a counter every pair takes its fixed share.
-        if (leader) drawn = p.sched != nullptr ? (int)atomicAdd(p.sched, 1u) + pairs : t + pairs;
+        // Drawn shortly before the end of this tile, so that the pair that is done first takes it, and published a few
+        // K blocks on, when the atomic has returned: the peer's producer goes on to the next tile without a gap.
+        // Without a counter every pair takes its fixed share.
+        const int draw_kb = max(0, p.num_kb - 10), publish_kb = max(min(3, p.num_kb - 1), p.num_kb - 4);
         const FlowItem it = flow_item<RB>(p, t);
-        const uint32_t bytes = 2u * (uint32_t)((it.rb_hi - it.rb_lo) * Cfg::A_BYTES + Cfg::B_BYTES);
-        const int row0 = it.tr * (RB * 256) + (int)cta * kBM, col0 = it.tc * BN + (int)cta * (BN / 2);
+        const int cols = it.tc + 1 == p.tiles_c ? p.last_cols : BN;
+        const CUtensorMap* const map_c = it.tc + 1 == p.tiles_c ? &p.tmap_last : &p.tmap_c;
+        const uint32_t bytes = 2u * (uint32_t)((it.rb_hi - it.rb_lo) * Cfg::A_BYTES + cols * 64);
+        const int row0 = it.tr * (RB * 256) + (int)cta * kBM, col0 = it.tc * BN + (int)cta * (cols / 2);
         for (int kb = 0; kb < p.num_kb; ++kb) {
+          if (leader && kb == draw_kb) drawn = p.sched != nullptr ? (int)atomicAdd(p.sched, 1u) + pairs : t + pairs;
           ok = mbar_wait(empty_bar(s), ph ^ 1u, p.sync, 92);
           if (!ok) break;
           const uint32_t lead_full = mapa_shared(full_bar(s), 0);
@@ -198,9 +207,9 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
           for (int rb = 0; rb < RB; ++rb)
             if (rb >= it.rb_lo && rb < it.rb_hi)
               tma_load_2d_pair(sa + rb * Cfg::A_BYTES, &p.tmap_r, lead_full, kb * kStageK, row0 + rb * 256);
-          tma_load_2d_pair(sa + RB * Cfg::A_BYTES, &p.tmap_c, lead_full, kb * kStageK, col0);
+          tma_load_2d_pair(sa + RB * Cfg::A_BYTES, map_c, lead_full, kb * kStageK, col0);
           if (++s == Cfg::STAGES) { s = 0; ph ^= 1u; }
-          if (leader && kb == min(3, p.num_kb - 1)) {
+          if (leader && kb == publish_kb) {
             // to both CTAs, even past the end (that is how the other roles learn of it)
             const uint32_t slot = (uint32_t)(k % kFlowSlots);
 #pragma unroll
@@ -223,13 +232,14 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
   } else if (warp == 1) {
     // ================= MMA issuer (leader CTA only) =================
     if (leader && elect_one()) {
-      constexpr uint32_t idesc = ELT == 2 ? make_idesc_bf16(256, BN) : make_idesc_tf32(256, BN);
       int s = 0;
       uint32_t ph = 0, uph = 0;                            // uph: one phase bit per accumulator
       bool ok = true;
       int t = pair;
       for (int k = 0; ok && t < p.items; ++k) {
         const FlowItem it = flow_item<RB>(p, t);
+        const int cols = it.tc + 1 == p.tiles_c ? p.last_cols : BN;
+        const uint32_t idesc = ELT == 2 ? make_idesc_bf16(256, cols) : make_idesc_tf32(256, cols);
         const int u0 = Cfg::BUFS == 2 ? (k & 1) * RB : 0;
         for (int kb = 0; kb < p.num_kb; ++kb) {
           ok = mbar_wait(full_bar(s), ph, p.sync, 94);
@@ -477,7 +487,8 @@ static FlowVariant flow_variant(int bn, int rb) {
   return {nullptr, 0};
 }
 
-int launch_flow_gemm(const GemmParams& g, int bn, int rb, int pairs, uint32_t* sched, cudaStream_t stream) {
+int launch_flow_gemm(const GemmParams& g, int bn, int rb, int pairs, int last_cols, const CUtensorMap& tmap_last, uint32_t* sched,
+                     cudaStream_t stream) {
   const bool tma_out = tma_store_enabled() && (g.ldo * (g.out_fp32 ? 4 : 2)) % 16 == 0 && ((uintptr_t)g.out & 15) == 0;
   const bool rows = tma_out && !g.out_fp32 && !g.transposed && !g.in_fp32;
   const FlowVariant v = g.in_fp32 ? flow_variant<4, FLOW_ANY>(bn, rb) : !rows ? flow_variant<2, FLOW_ANY>(bn, rb)
@@ -504,6 +515,8 @@ int launch_flow_gemm(const GemmParams& g, int bn, int rb, int pairs, uint32_t* s
   p.tiles_r = (g.rows_r + 256 * rb - 1) / (256 * rb);
   p.tiles_c = (g.rows_c + bn - 1) / bn;
   p.num_kb = (g.K + (g.in_fp32 ? 32 : 64) - 1) / (g.in_fp32 ? 32 : 64);
+  p.last_cols = last_cols;
+  p.tmap_last = last_cols < bn ? tmap_last : p.tmap_c;
   p.group_r = std::max(1, g.group_r / (2 * rb));
   const int tiles = p.tiles_r * p.tiles_c;
   // A last wave that is at most half full is dealt as single row blocks

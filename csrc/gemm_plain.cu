@@ -226,10 +226,13 @@ KR_API int kr_gemm(const void* a, long long lda, const void* bt, long long ldb, 
   GemmParams p;
   memset(&p, 0, sizeof(p));
   int bn = 0;
+  CUtensorMap tmap_last;
+  const int cols = pl.swap ? M : N, last_cols = pl.bn > 0 ? ((cols - 1) % pl.bn + 16) / 16 * 16 : 0;
+  const int narrow = pl.kind == PLAIN_FLOW && last_cols < pl.bn ? last_cols / 2 : 0;
   int rc = setup_problem(p, a, lda, bt, ldb, M, N, K, pl.swap, pl.bn, &bn, elt, pair ? pl.bn / 2 : pl.bn,
                          // Persistent pairs on rows off the 128-byte lines: fetching past the line into L2 only gets in the
                          // way there (777 x 5120 x 13704 153 to 140 us); elsewhere it helps (16 x 8192 x 28672 78.6 to 76.0).
-                         pl.kind != PLAIN_FLOW || (lda * elt % 128 == 0 && ldb * elt % 128 == 0));
+                         pl.kind != PLAIN_FLOW || (lda * elt % 128 == 0 && ldb * elt % 128 == 0), narrow, &tmap_last);
   if (rc) return rc;
   p.mode = GEMM_PLAIN;
   p.out = out;
@@ -246,7 +249,7 @@ KR_API int kr_gemm(const void* a, long long lda, const void* bt, long long ldb, 
     p.cp_dst = copy_dst;
     p.cp_bytes = (unsigned long long)M * K * elt;
   }
-  if (pl.kind == PLAIN_FLOW) return launch_flow_gemm(p, bn, pl.rb, pl.workers, counters, stream);
+  if (pl.kind == PLAIN_FLOW) return launch_flow_gemm(p, bn, pl.rb, pl.workers, last_cols, tmap_last, counters, stream);
   if (pl.kind == PLAIN_TILE) {
     if (pl.pair) p.tiles_r = (p.rows_r + 255) / 256;
     return launch_tile_gemm(p, bn, pl.pair, pl.splits, stream);

@@ -10,9 +10,10 @@ namespace kraken {
 
 // Tensor map of a row-major bf16 (elt 2) or fp32 (elt 4) matrix [rows, cols] (cols contiguous, `ld`
 // elements per row), box = box_bytes (128 or 64) of columns x box_rows rows, swizzled by as much, out-of-range
-// elements read as zero. Cached.
+// elements read as zero. narrow_rows > 0: *narrow is the same with boxes of so many rows. Cached.
 int get_tmap(const void* ptr, unsigned long long rows, unsigned long long cols, unsigned long long ld,
-             unsigned box_rows, CUtensorMap* out, int elt = 2, unsigned box_bytes = 128, bool promote_256 = true);
+             unsigned box_rows, CUtensorMap* out, int elt = 2, unsigned box_bytes = 128, bool promote_256 = true,
+             unsigned narrow_rows = 0, CUtensorMap* narrow = nullptr);
 // Tensor map for TMA stores of bf16 tiles (box of 32 rows); false when the matrix cannot be
 // described to TMA or TMA stores are switched off.
 bool store_tmap(const void* ptr, long long rows, long long cols, long long ld, CUtensorMap* m);
@@ -21,7 +22,8 @@ int default_group_r();
 bool pair_enabled();
 unsigned grid_cap(const DeviceState* d);
 int setup_problem(GemmParams& p, const void* a, long long lda, const void* bt, long long ldb, int M, int N, int K,
-                  bool swap, int bn_override, int* bn_out, int elt = 2, int c_box_rows = 0, bool promote_256 = true);
+                  bool swap, int bn_override, int* bn_out, int elt = 2, int c_box_rows = 0, bool promote_256 = true, int narrow_rows = 0,
+                  CUtensorMap* narrow = nullptr);
 // Single-CTA kernels for fp32 operands multiplied as tf32 (GEMM -> all-reduce; column tiles of 16, 64 or 256). Defined in gemm_tf32.cu.
 int launch_gemm_tf32(int bn, const GemmParams& p, unsigned nb, cudaStream_t stream);
 // Single-CTA kernels of the decode GEMM -> all-reduce. Defined in gemm_ar.cu.
@@ -36,7 +38,9 @@ inline double busy_factor(double busy) { return std::max(0.75, std::pow(busy, 0.
 int tile_gemm_splits(const DeviceState* d, int tiles, int num_kb, int bn, bool pair, int elt, double block_us, double hbm_us, double* us);
 int launch_tile_gemm(const GemmParams& g, int bn, bool pair, int splits, cudaStream_t stream);
 // Persistent pairs that draw their tiles in order (gemm_flow.cu); sched: two zero words, zero again afterwards.
-int launch_flow_gemm(const GemmParams& g, int bn, int rb, int pairs, uint32_t* sched, cudaStream_t stream);
+// last_cols: columns of the last column tile, in 16s; below bn with a tensor map of half as many rows of the column operand.
+int launch_flow_gemm(const GemmParams& g, int bn, int rb, int pairs, int last_cols, const CUtensorMap& tmap_last, uint32_t* sched,
+                     cudaStream_t stream);
 int pick_bn(int rows_c);      // column-tile width for `rows_c` rows of the column operand
 int tf32_bn(int rows_c);      // the same among the widths the tf32 kernels exist for
 
