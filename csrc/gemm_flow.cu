@@ -34,7 +34,7 @@ struct alignas(64) FlowParams {
   int last_cols;                                          // columns of the last column tile, in 16s (tmap_last: boxes of half as many rows)
   int tiles_r, tiles_c, num_kb, group_r;                  // tiles of RB * 256 rows
   int items, split_from;                                  // tiles from split_from on are drawn as single row blocks
-  int transposed, out_fp32, act;
+  int transposed, out_fp32, act, rest_follows;
   int out_rows, out_cols;
   uint32_t* sched;                                        // [0] items drawn beyond the first of each pair, [1] pairs done; or nullptr
   void* out;                                              // output without a tensor map (else nullptr) and its row stride
@@ -143,8 +143,11 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
   cluster_sync_all();            // both CTAs' barriers exist before anyone signals across the pair
   tc_fence_after();
   const uint32_t tmem_base = ld_shared_u32(tmem_slot);
-  pdl_launch();
+  // With a second launch for the rest of the problem, that one relies on the operands as this one does: it may only
+  // start once they are there.
+  if (p.rest_follows == 0) pdl_launch();
   pdl_wait();
+  if (p.rest_follows != 0) pdl_launch();
 
   // A staged panel of `rows` x `cols` to an output that TMA cannot describe (rows not whole 16-byte
   // units) or may not store to (KRAKEN_TMA_STORE=0), element by element.
@@ -526,6 +529,7 @@ int launch_flow_gemm(const GemmParams& g, int bn, int rb, int pairs, int last_co
   p.transposed = g.transposed;
   p.out_fp32 = g.out_fp32;
   p.act = g.act;
+  p.rest_follows = g.rest_follows;
   p.out_rows = g.out_rows;
   p.out_cols = g.out_cols;
   p.sched = sched;

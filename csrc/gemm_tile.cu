@@ -12,15 +12,14 @@
 // The sums are SENT: every CTA owns an equal share of the tile's rows, and the others store their partial sums of it
 // straight from registers into its shared memory (st.async, counted on an mbarrier of the owner; the operand stages are
 // free by then). The owner adds them in split order and stores its rows. One cluster barrier, whose latency the first
-// read of the accumulator hides, says that the stages are free; nothing follows the stores. Against the other order
-// (accumulator into own shared memory, cluster barrier, owners fetch, cluster barrier before anybody may leave), us a call
-// in a stream of them: 8 x 4096 x 4096 9.9 to 9.5, 35 x 4064 x 5416 14.4 to 12.9, 102 x 1240 x 2816 9.9 to 8.1,
-// 100 x 4000 x 9000 21.6 to 19.8. What bounds this part now is the way between SMs: 64 KB leave an SM in 2700 clocks
+// read of the accumulator hides, says that the stages are free; nothing follows the stores. With
+// the other order (own shared memory, cluster barrier, owners fetch, cluster barrier before anybody may leave) and the
+// places of a thread's rows worked out here instead of before, us a call in a stream of them: 8 x 4096 x 4096 9.8, now 8.8;
+// 35 x 4064 x 5416 14.4, 12.5; 102 x 1240 x 2816 9.8, 7.3; 100 x 4000 x 9000 20.8, 19.5. What bounds this part now is the way between SMs: 64 KB leave an SM in 2700 clocks
 // (24 bytes each; bulk copies 3400, plain remote stores and a barrier 4200, fetches 3900), whatever the cluster size.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
-#include <map>
-#include <mutex>
 #include "kraken/gemm_host.h"
 
 namespace kraken {
@@ -30,7 +29,7 @@ constexpr int kTileThreads = 320;      // TMA warp, MMA warp, eight warps that e
 struct alignas(64) TileParams {
   CUtensorMap tmap_r, tmap_c;
   int tiles_r, tiles_c, num_kb;
-  int transposed, out_fp32, act;
+  int transposed, out_fp32, act, is_rest;
   int out_rows, out_cols;
   void* out;
   long long ldo;
@@ -64,6 +63,8 @@ __device__ __forceinline__ void push_cluster_u4(uint32_t addr, uint32_t bar, uin
   asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1,%2,%3,%4}, [%5];"
                ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d), "r"(bar) : "memory");
 }
+// Relaxed: what it announces are this CTA's copies and MMAs, which mbarriers have shown to be over, and no store of the
+// thread (with release semantics the arrival took 500 clocks).
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ uint32_t cluster_size() {
@@ -143,7 +144,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) gemm_tile_kernel(const __grid
   uint32_t tmem_base;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
   pdl_launch();
-  pdl_wait();
+  if (p.is_rest == 0) pdl_wait();
 
   // Worked out now, while nothing waits for it (the divisions took 300 clocks of the tail): where this thread's row of the
   // accumulator goes, and which of the sums it stores first.
@@ -348,6 +349,9 @@ __global__ void __launch_bounds__(kTileThreads, 1) gemm_tile_kernel(const __grid
     if (PAIR) tmem_dealloc_pair(tmem_base, Cfg::TMEM_COLS);
     else tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
   }
+  // The rest of a problem starts when all blocks of the launch before it run and have seen their own predecessor
+  // complete, reads what they read, writes other rows or columns, and is complete no sooner than they are.
+  if (p.is_rest != 0) pdl_wait();
 }
 
 // ---- host ---------------------------------------------------------------------------------------
@@ -377,13 +381,12 @@ static TileVariant tile_variant(int bn, bool pair) {
 }
 
 // How many clusters of `cluster` CTAs of this kernel the device holds at once (asked once; 0: none).
-static int max_clusters(int device, const TileVariant& v, unsigned cluster) {
-  static std::mutex mu;
-  static std::map<std::tuple<int, const void*, unsigned>, int> known;
-  std::lock_guard<std::mutex> lk(mu);
-  auto key = std::make_tuple(device, v.fn, cluster);
-  auto it = known.find(key);
-  if (it != known.end()) return it->second;
+static int max_clusters(int device, const TileVariant& v, int elt, int bn, bool pair, unsigned cluster) {
+  constexpr int kDevices = 16;
+  static std::atomic<int> known[kDevices][2][2][17][9];        // answer + 1
+  std::atomic<int>* slot = device < kDevices ? &known[device][elt == 4][pair][bn / 16][cluster] : nullptr;
+  if (slot != nullptr)
+    if (const int n = slot->load(std::memory_order_relaxed)) return n - 1;
   int n = 0;
   if (ensure_dynamic_smem(v.fn, v.smem) == KR_SUCCESS) {
     cudaLaunchAttribute attr[1];
@@ -402,29 +405,28 @@ static int max_clusters(int device, const TileVariant& v, unsigned cluster) {
       n = 0;
     }
   }
-  known[key] = n;
+  if (slot != nullptr) slot->store(n + 1, std::memory_order_relaxed);
   return n;
 }
 
-// The split count of a one-wave problem, 0 when its tiles do not fit the chip at once, and its time (us).
-// block_us: one K block with every SM busy (less when fewer are; single CTAs of up to 64 columns are bound by
-// their loads, not by the clock), but never below the operands' time out of HBM (hbm_us), plus what summing S
-// splits adds: little for single CTAs, a lot once a cluster of pairs spans more than four CTAs (M = 256,
-// N = 4096, K = 2048: 1 / 2 / 3 splits 17.5 / 14.2 / 20.5 us). A pair without splits is left to the persistent
-// kernel, which stores faster (373 x 8000 x 7768: 57 us against 71).
-int tile_gemm_splits(const DeviceState* d, int tiles, int num_kb, int bn, bool pair, int elt, double block_us, double hbm_us,
+// The split count of a one-wave problem, 0 when its tiles do not fit the chip at once, and its time (us). kb_us: one K
+// block with every SM busy (less when fewer are, the clock being what power leaves; not so for single CTAs of up to 64
+// columns). Near the operands' time out of HBM (hbm_us) the two slow each other down (norm of order 4). Then the partial
+// sums' way between SMs (44 KB a us and SM); clusters of six CTAs and more start later.
+int tile_gemm_splits(const DeviceState* d, int tiles, int num_kb, int bn, bool pair, int elt, double kb_us, double hbm_us,
                      double* us_out) {
   const TileVariant v = elt == 4 ? tile_variant<4>(bn, pair) : tile_variant<2>(bn, pair);
   if (v.fn == nullptr) return 0;
   const int ctas = pair ? 2 : 1, most = 8 / ctas;
-  auto sum_us = [&](int s) { return !pair ? 0.25 * s : (s <= 2 ? 0.6 * s : 3.3 * s - 2.0) * bn / 256; };
   int best = 0;
   double best_us = 1e30;
-  for (int s = pair ? 2 : 1; s <= most && (s == 1 || num_kb >= 4 * s); ++s) {
-    if (tiles * s * ctas > d->num_sms || tiles > max_clusters(d->device, v, (unsigned)(s * ctas))) continue;
-    const double busy = (double)tiles * s * ctas / d->num_sms;
-    const double kb_us = pair || bn == 128 ? block_us * busy_factor(busy) : block_us;
-    const double us = std::max((num_kb + s - 1) / s * kb_us, hbm_us) + sum_us(s) + 6.9;
+  for (int s = 1; s <= most && (s == 1 || num_kb >= 4 * s); ++s) {
+    if (tiles * s * ctas > d->num_sms || tiles > max_clusters(d->device, v, elt, bn, pair, (unsigned)(s * ctas))) continue;
+    const double busy = (double)tiles * s * ctas / d->num_sms, sent = (double)(s - 1) / s * kBM * bn * 4;
+    const double blocks = (num_kb + s - 1) / s * kb_us * (pair || bn > 64 ? busy_factor(busy) : 1.0), b2 = blocks * blocks, h2 = hbm_us * hbm_us;
+    // (unsplit pairs: the persistent kernel stores faster)
+    const double us = std::sqrt(std::sqrt(b2 * b2 + h2 * h2)) * (pair && s == 1 ? 1.05 : 1.0) + sent / 44500 + (pair ? kTilePairUs : kTileSingleUs) +
+                      (pair && s >= 3 ? 0.5 : 0.0);
     if (us < best_us) {
       best_us = us;
       best = s;
@@ -448,6 +450,7 @@ int launch_tile_gemm(const GemmParams& g, int bn, bool pair, int splits, cudaStr
   p.transposed = g.transposed;
   p.out_fp32 = g.out_fp32;
   p.act = g.act;
+  p.is_rest = g.is_rest;
   p.out_rows = g.out_rows;
   p.out_cols = g.out_cols;
   p.out = g.out;

@@ -131,6 +131,7 @@ struct alignas(64) GemmParams {
   // launcher can re-encode its tensor map with another box height
   const void* host_c_ptr;
   long long host_ldc;
+  int rest_follows, is_rest;        // first and second launch of one plain GEMM
 };
 
 // Linear persistent tile index -> (row tile, column tile): row tiles advance in groups of

@@ -3,12 +3,14 @@
 matmuls of the same bf16 inputs. Shapes include the reference's test shapes scaled to fit one GPU
 (test/test_gemm_allreduce.py:57-117: 512x256x128, 256^3, rank-valued 32^3 with 1e-5 tolerance;
 test/test_gemm_reduce_scatter.py:44-115; test/test_allgather_matmul.py:47-81)."""
+import ctypes
 import math
 
 import pytest
 import torch
 
 from kraken_b200 import fused
+from kraken_b200.ops import lib as klib
 from kraken_b200.parallel import EmuWorld
 
 pytestmark = pytest.mark.gpu
@@ -481,6 +483,79 @@ def test_gemm_one_wave_every_split_and_tile(splits, swap):
                 c = fused.matmul(a, bt.t(), out_dtype=out_dtype, bn=10000 * splits + bn, swap_ab=swap)
                 assert ((c.float() - ref).norm() / ref.norm()).item() < limit
                 assert torch.equal(c, fused.matmul(a, bt.t(), out_dtype=out_dtype, bn=10000 * splits + bn, swap_ab=swap))
+
+
+def _plan(M, N, K, fp32):
+    plan = (ctypes.c_int * 11)()
+    klib.check(klib.lib().kr_gemm_plan(M, N, K, K, K, int(fp32), plan))
+    return list(plan)
+
+
+# whole waves on persistent pairs, the rest of the rows or columns by the one-wave kernel in a launch that overlaps it
+@pytest.mark.parametrize("M,N,K,fp32", [(1823, 4616, 2024, 0), (1885, 5040, 2616, 0), (1572, 3032, 3048, 0), (2481, 3720, 2264, 0),
+                                        (2534, 3712, 2536, 0), (2307, 1984, 2448, 1), (1588, 2792, 2840, 1)])
+def test_gemm_in_two_launches(M, N, K, fp32):
+    from kraken_b200.fused.gemm_ops import _gemm
+    from kraken_b200.parallel import symm_mem
+
+    assert _plan(M, N, K, fp32)[5] == 1
+    dtype = torch.float32 if fp32 else torch.bfloat16
+    g = torch.Generator(device="cuda").manual_seed(91)
+    a = torch.randn(M, K, generator=g, device="cuda").to(dtype)
+    bt = (0.05 * torch.randn(N, K, generator=g, device="cuda")).to(dtype)
+    ref = (a.double() @ bt.double().t()).float()
+    for out_dtype, limit in ((torch.float32, 1e-3 if fp32 else 1e-5), (torch.bfloat16, 3e-3)):
+        c = fused.matmul(a, bt.t(), out_dtype=out_dtype)
+        assert ((c.float() - ref).norm() / ref.norm()).item() < limit
+        assert ((c.float() - ref).abs().amax(0) < 0.05 * ref.abs().amax()).all()              # no column or row left out
+    h = _gemm(a, bt.t(), True, True, act="gelu_tanh")
+    href = torch.nn.functional.gelu(ref, approximate="tanh")
+    assert ((h - href).norm() / href.norm()).item() < 1e-3
+    if not fp32:
+        x = symm_mem.empty(M, K, dtype=dtype, device="cuda")
+        x.copy_(a)
+        gathered, c = fused.all_gather_matmul(x, bt.t())
+        assert torch.equal(gathered, a) and ((c.float() - ref).norm() / ref.norm()).item() < 3e-3
+
+
+def test_gemms_in_two_launches_chained_and_captured():
+    # The second launch does not wait for the first one, but nothing after them may start before both are complete, and it
+    # must not start before what the first one waits for: every call reads the result of the one before, whose memory the
+    # one after next writes.
+    M, N, K = 1885, 5040, 2616
+    assert _plan(M, N, K, 0)[5] == 1 and _plan(M, K, N, 0)[5] in (0, 1)
+    g = torch.Generator(device="cuda").manual_seed(92)
+    x = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    w1 = (torch.randn(N, K, generator=g, device="cuda") / K ** 0.5).to(torch.bfloat16)
+    w2 = (torch.randn(K, N, generator=g, device="cuda") / N ** 0.5).to(torch.bfloat16)
+
+    def chain(n, sync):
+        y = x
+        for _ in range(n):
+            y = fused.matmul(y, w1.t())
+            if sync:
+                torch.cuda.synchronize()
+            y = fused.matmul(y, w2.t())
+            if sync:
+                torch.cuda.synchronize()
+        return y
+
+    want = chain(6, True)
+    for _ in range(5):
+        assert torch.equal(chain(6, False), want)
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        chain(1, False)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=s):
+            y = chain(6, False)
+    torch.cuda.current_stream().wait_stream(s)
+    for _ in range(3):
+        y.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, want)
 
 
 @pytest.mark.parametrize("M,N,bn,swap", [(520, 1024, 1256, 0), (1500, 2080, 2256, 0), (520, 1024, 2144, 0), (777, 1160, 1096, 0), (520, 1024, 1192, 1),
