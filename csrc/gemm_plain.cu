@@ -173,7 +173,7 @@ static PlainPlan plain_plan(const DeviceState* d, int M, int N, int K, int elt, 
       const int rows = swap ? N : M, cols = swap ? M : N, cr = swap ? class_b : class_a, cc = swap ? class_a : class_b;
       if (rows <= 128) continue;
       for (int bn = 64, step; bn <= 256; bn += step) {
-        step = bn >= 128 && elt == 2 ? 16 : 32;
+        step = bn >= 128 ? 16 : 32;
         if (bn > 64 && bn - step >= cols) continue;                  // wider than needed
         for (int rb = 1; rb <= 2; ++rb) {
           if (rb == 2 && rows <= 256) continue;

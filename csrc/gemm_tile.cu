@@ -424,8 +424,9 @@ int tile_gemm_splits(const DeviceState* d, int tiles, int num_kb, int bn, bool p
     if (tiles * s * ctas > d->num_sms || tiles > max_clusters(d->device, v, elt, bn, pair, (unsigned)(s * ctas))) continue;
     const double busy = (double)tiles * s * ctas / d->num_sms, sent = (double)(s - 1) / s * kBM * bn * 4;
     const double blocks = (num_kb + s - 1) / s * kb_us * (pair || bn > 64 ? busy_factor(busy) : 1.0), b2 = blocks * blocks, h2 = hbm_us * hbm_us;
-    // (unsplit pairs: the persistent kernel stores faster)
-    const double us = std::sqrt(std::sqrt(b2 * b2 + h2 * h2)) * (pair && s == 1 ? 1.05 : 1.0) + sent / 44500 + (pair ? kTilePairUs : kTileSingleUs) +
+    // (unsplit pairs: the persistent kernel stores bf16 rows faster, 636 x 4080 x 3152 29 us against 33; fp32 does not, 500 x
+    // 4000 x 4000 34.6 against 29.4)
+    const double us = std::sqrt(std::sqrt(b2 * b2 + h2 * h2)) * (pair && s == 1 && elt == 2 ? 1.05 : 1.0) + sent / 44500 + (pair ? kTilePairUs : kTileSingleUs) +
                       (pair && s >= 3 ? 0.5 : 0.0);
     if (us < best_us) {
       best_us = us;
