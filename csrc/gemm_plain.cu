@@ -177,8 +177,10 @@ static PlainPlan plain_plan(const DeviceState* d, int M, int N, int K, int elt, 
         if (bn > 64 && bn - step >= cols) continue;                  // wider than needed
         for (int rb = 1; rb <= 2; ++rb) {
           if (rb == 2 && rows <= 256) continue;
-          // a transposed store writes shorter runs: row-major unless the other way saves something
-          const double factor = swap ? 1.08 : 1.0, us = flow_us(rows, cols, num_kb, bn, rb, pairs, cr, cc, hbm_us) * factor;
+          // A transposed store writes shorter runs: row-major unless the other way saves something. fp32 operands: both store
+          // chunk by chunk, and take longer to the end (334 x 4444 x 1312 14.8 us, the one-wave kernel 13.6).
+          const double factor = !swap ? 1.0 : elt == 4 ? 1.03 : 1.08, fp32_us = elt == 4 ? 1.0 : 0.0;
+          const double us = flow_us(rows, cols, num_kb, bn, rb, pairs, cr, cc, hbm_us) * factor + fp32_us;
           if (us < best) {
             best = us;
             pl.kind = PLAIN_FLOW; pl.swap = swap != 0; pl.pair = true; pl.bn = bn; pl.rb = rb; pl.splits = 0; pl.workers = pairs;
