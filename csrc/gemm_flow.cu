@@ -184,6 +184,8 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
   if (warp == 0) {
     // ================= TMA producer (both CTAs) =================
     if (elect_one()) {
+      // One thread has 130 ns a K block of 256 x 128 x 64: what does not change is kept out of the loop.
+      const uint32_t lead_full0 = mapa_shared(full_bar(0), 0);
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
@@ -199,20 +201,25 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
         const CUtensorMap* const map_c = it.tc + 1 == p.tiles_c ? &p.tmap_last : &p.tmap_c;
         const uint32_t bytes = 2u * (uint32_t)((it.rb_hi - it.rb_lo) * Cfg::A_BYTES + cols * 64);
         const int row0 = it.tr * (RB * 256) + (int)cta * kBM, col0 = it.tc * BN + (int)cta * (cols / 2);
-        for (int kb = 0; kb < p.num_kb; ++kb) {
-          if (leader && kb == draw_kb) drawn = p.sched != nullptr ? (int)atomicAdd(p.sched, 1u) + pairs : t + pairs;
-          ok = mbar_wait(empty_bar(s), ph ^ 1u, p.sync, 92);
-          if (!ok) break;
-          const uint32_t lead_full = mapa_shared(full_bar(s), 0);
-          if (leader) mbar_expect_tx(full_bar(s), bytes);             // both CTAs' bytes complete on the leader's barrier
-          const uint32_t sa = stage0 + s * Cfg::STAGE;
+        auto load_blocks = [&](int kb, int end) {
+          for (; kb < end; ++kb) {
+            ok = mbar_wait(empty_bar(s), ph ^ 1u, p.sync, 92);
+            if (!ok) return;
+            const uint32_t lead_full = lead_full0 + 8u * s, sa = stage0 + s * Cfg::STAGE;
+            if (leader) mbar_expect_tx(full_bar(s), bytes);           // both CTAs' bytes complete on the leader's barrier
 #pragma unroll
-          for (int rb = 0; rb < RB; ++rb)
-            if (rb >= it.rb_lo && rb < it.rb_hi)
-              tma_load_2d_pair(sa + rb * Cfg::A_BYTES, &p.tmap_r, lead_full, kb * kStageK, row0 + rb * 256);
-          tma_load_2d_pair(sa + RB * Cfg::A_BYTES, map_c, lead_full, kb * kStageK, col0);
-          if (++s == Cfg::STAGES) { s = 0; ph ^= 1u; }
-          if (leader && kb == publish_kb) {
+            for (int rb = 0; rb < RB; ++rb)
+              if (RB == 1 || (rb >= it.rb_lo && rb < it.rb_hi))
+                tma_load_2d_pair(sa + rb * Cfg::A_BYTES, &p.tmap_r, lead_full, kb * kStageK, row0 + rb * 256);
+            tma_load_2d_pair(sa + RB * Cfg::A_BYTES, map_c, lead_full, kb * kStageK, col0);
+            if (++s == Cfg::STAGES) { s = 0; ph ^= 1u; }
+          }
+        };
+#pragma unroll 1
+        for (int part = 0; ok && part < 3; ++part) {
+          load_blocks(part == 0 ? 0 : part == 1 ? draw_kb : publish_kb + 1, part == 0 ? draw_kb : part == 1 ? publish_kb + 1 : p.num_kb);
+          if (leader && part == 0) drawn = p.sched != nullptr ? (int)atomicAdd(p.sched, 1u) + pairs : t + pairs;
+          if (leader && ok && part == 1) {
             // to both CTAs, even past the end (that is how the other roles learn of it)
             const uint32_t slot = (uint32_t)(k % kFlowSlots);
 #pragma unroll
@@ -235,6 +242,8 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
   } else if (warp == 1) {
     // ================= MMA issuer (leader CTA only) =================
     if (leader && elect_one()) {
+      const uint32_t peer_empty0 = mapa_shared(empty_bar(0), 1);
+      const uint64_t desc0 = make_smem_desc_sw128(stage0);
       int s = 0;
       uint32_t ph = 0, uph = 0;                            // uph: one phase bit per accumulator
       bool ok = true;
@@ -248,17 +257,16 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
           ok = mbar_wait(full_bar(s), ph, p.sync, 94);
           if (!ok) break;
           tc_fence_after();
-          const uint32_t sa = stage0 + s * Cfg::STAGE;
-          const uint64_t bdesc = make_smem_desc_sw128(sa + RB * Cfg::A_BYTES);
+          const uint64_t sdesc = desc0 + (uint64_t)(s * (Cfg::STAGE >> 4)), bdesc = sdesc + (uint64_t)(RB * Cfg::A_BYTES >> 4);
 #pragma unroll
           for (int rb = 0; rb < RB; ++rb) {
-            if (rb < it.rb_lo || rb >= it.rb_hi) continue;
+            if (RB > 1 && (rb < it.rb_lo || rb >= it.rb_hi)) continue;
             const int u = u0 + rb;
             if (kb == 0) {
               ok = mbar_wait(tempty_bar(u), ((uph >> u) & 1u) ^ 1u, p.sync, 95) && ok;
               tc_fence_after();
             }
-            const uint64_t adesc = make_smem_desc_sw128(sa + rb * Cfg::A_BYTES);
+            const uint64_t adesc = sdesc + (uint64_t)(rb * Cfg::A_BYTES >> 4);
             const uint32_t d_tmem = tmem_base + (uint32_t)(u * Cfg::UNIT);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -273,7 +281,7 @@ __global__ void __launch_bounds__(kFlowThreads + kFlowCopyThreads, 1) gemm_flow_
           }
           if (!ok) break;
           umma_commit_pair(empty_bar(s));
-          umma_commit_pair(mapa_shared(empty_bar(s), 1));
+          umma_commit_pair(peer_empty0 + 8u * s);
           if (++s == Cfg::STAGES) { s = 0; ph ^= 1u; }
         }
         for (int rb = it.rb_lo; rb < it.rb_hi; ++rb) uph ^= 1u << (u0 + rb);
