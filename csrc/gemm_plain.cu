@@ -82,6 +82,7 @@ constexpr double kHbmBytesPerUs = 6.45e6;
 
 static double flow_us(int rows, int cols, int num_kb, int bn, int rb, int pairs, int class_r, int class_c, double hbm_us) {
   const int tiles_r = (rows + 256 * rb - 1) / (256 * rb), tiles_c = (cols + bn - 1) / bn, last_cols = (cols - (tiles_c - 1) * bn + 15) / 16 * 16;
+  if (tiles_c == 1) bn = last_cols;                        // every tile is that narrow
   // what is not hidden: start and last epilogue, and with one accumulator set the epilogue of every tile
   const double bubble = 2 * rb * bn <= 512 ? 0.0 : kEpilogueUs;
   const int narrow = last_cols < bn ? tiles_r : 0, T = tiles_r * tiles_c - narrow, whole = T / pairs, rest = T % pairs;
@@ -96,7 +97,9 @@ static double flow_us(int rows, int cols, int num_kb, int bn, int rb, int pairs,
     const double thin = std::min(full, num_kb * std::max(0.26 * rb, 1.35 * block_us(last_cols, rb, class_r, class_c, last_cols)));
     const int fit = rest ? (pairs - rest) * (int)(full / thin) : 0, left = std::max(0, narrow - fit);
     if (rest) last = full * busy_factor(std::min(1.0, (rest + narrow * thin / full) / pairs));
-    last += (left + pairs - 1) / pairs * thin * busy_factor(std::min(1.0, (double)left / pairs));
+    const double then = (left + pairs - 1) / pairs * thin * busy_factor(std::min(1.0, (double)left / pairs));
+    // all of them on the pairs that the last wave leaves free, or what is left of them after it
+    last = rest ? std::min(last + then, std::max(last, (narrow + pairs - rest - 1) / (pairs - rest) * thin)) : then;
   } else if (rb == 2 && rest && 2 * rest <= pairs) {
     last = num_kb * block_us(bn, 1, class_r, class_c, bn) * busy_factor(2.0 * rest / pairs);
   }
@@ -179,7 +182,7 @@ static PlainPlan plain_plan(const DeviceState* d, int M, int N, int K, int elt, 
           if (rb == 2 && rows <= 256) continue;
           // A transposed store writes shorter runs: row-major unless the other way saves something. fp32 operands: both store
           // chunk by chunk, and take longer to the end (334 x 4444 x 1312 14.8 us, the one-wave kernel 13.6).
-          const double factor = !swap ? 1.0 : elt == 4 ? 1.03 : 1.08, fp32_us = elt == 4 ? 1.0 : 0.0;
+          const double factor = !swap ? 1.0 : elt == 4 ? 1.03 : ((rows + 256 * rb - 1) / (256 * rb)) * ((cols + bn - 1) / bn) >= 2 * pairs ? 1.05 : 1.08, fp32_us = elt == 4 ? 1.0 : 0.0;
           const double us = flow_us(rows, cols, num_kb, bn, rb, pairs, cr, cc, hbm_us) * factor + fp32_us;
           if (us < best) {
             best = us;
