@@ -118,7 +118,6 @@ static TileChoice best_tile(const DeviceState* d, int M, int N, int num_kb, int 
   TileChoice best = {1e30, false, false, 0, 0};
   for (int swap = 0; swap < 2; ++swap) {
     const int rows = swap ? N : M, cols = swap ? M : N, cr = swap ? class_b : class_a, cc = swap ? class_a : class_b;
-    if (rows <= 128) continue;
     auto offer = [&](bool pair, int bn, double kb_us) {
       const int tiles = ((rows + (pair ? 255 : 127)) / (pair ? 256 : 128)) * ((cols + bn - 1) / bn);
       double us = 1e30;
@@ -129,7 +128,9 @@ static TileChoice best_tile(const DeviceState* d, int M, int N, int num_kb, int 
       const int bn = pick_bn(cols);
       offer(false, bn, single_us(bn, cr, cc, cols));
     }
-    for (int bn = 128; bn <= 256; bn += 32)
+    // Pairs only where the second CTA has rows. Single CTAs always: one tile of both dimensions up to 128 is eight K ranges in
+    // a cluster instead of one CTA that walks all of K (64 x 128 x 8192 6.6 us against 26.1, 1 x 128 x 7168 5.0 against 19.5).
+    for (int bn = 128; rows > 128 && bn <= 256; bn += 32)
       if (pair_enabled() && (bn == 128 || bn - 32 < cols)) offer(true, bn, block_us(bn, 1, cr, cc, cols));
   }
   return best;
@@ -388,6 +389,15 @@ KR_API int kr_gemm(const void* a, long long lda, const void* bt, long long ldb, 
   KR_REQUIRE(M >= 1 && N >= 1, "GEMM needs positive sizes");
   const int elt = in_fp32 ? 4 : 2;
   PlainPlan pl = known_plan(d, M, N, K, elt, swap_ab, bn_override, use_pair, max_ctas, lda, ldb);
+  // One tile whose K is too short to cut: bf16 rows that TMA stores leave the persistent kernel sooner (128 x 128 x 256 3.9 us,
+  // the one-wave kernel 4.7); element stores take longer there (100 x 100 x 256 11.5 and 6.4), tiles of 64 columns as long.
+  if (pl.kind == PLAIN_TILE && pl.splits == 1 && swap_ab < 0 && bn_override <= 0 && std::min(M, N) > 64 && std::max(M, N) <= 128 && elt == 2 &&
+      !out_fp32 && ldo % 8 == 0 && ((uintptr_t)out & 15) == 0 && tma_store_enabled()) {
+    pl.kind = PLAIN_SINGLE;
+    pl.swap = pl.pair = false;
+    pl.bn = 128;
+    pl.workers = 1;
+  }
   PlainCall c = {a, lda, bt, ldb, out, ldo, M, N, K, out_fp32, act, in_fp32, counters, copy_dst, stream};
   if (pl.cut == 0) return run_plain(d, pl, c, false, false);
   PlainCall rest = c;

@@ -505,6 +505,35 @@ def _plan(M, N, K, fp32):
     return list(plan)
 
 
+# Both dimensions up to 128: one tile, whose K is what can be shared out (router and gate projections of a decode step).
+@pytest.mark.parametrize("M,N,K,fp32", [(64, 128, 8192, 0), (128, 128, 16384, 0), (1, 128, 7168, 0), (16, 64, 4096, 0), (128, 1, 520, 0),
+                                        (33, 17, 5000, 0), (128, 128, 4096, 1), (8, 127, 260, 1)])
+def test_one_tile_problems_are_cut_along_k(M, N, K, fp32):
+    plan = _plan(M, N, K, fp32)
+    assert plan[0] == 1 and plan[4] > 1, plan
+    dtype = torch.float32 if fp32 else torch.bfloat16
+    g = torch.Generator().manual_seed(97)
+    a = torch.randn(M, K, generator=g).to(dtype).cuda()
+    bt = (0.05 * torch.randn(N, K, generator=g)).to(dtype).cuda()
+    ref = (a.double() @ bt.double().t()).float()
+    # fp32 sums: one cut of the running sum (2**-23 of it) per MMA of 16 columns; tf32 operands: 10 bits; bf16 results: 2**-9
+    for out_dtype, limit in ((torch.float32, 1e-3 if fp32 else 1e-6 + K / 16 * 2.0 ** -23), (torch.bfloat16, 3e-3)):
+        c = fused.matmul(a, bt.t(), out_dtype=out_dtype)
+        assert ((c.float() - ref).norm() / ref.norm()).item() < limit
+        assert torch.equal(c, fused.matmul(a, bt.t(), out_dtype=out_dtype))
+
+
+@pytest.mark.parametrize("M,N,K", [(128, 128, 256), (65, 72, 8), (72, 66, 448), (128, 128, 440)])
+def test_one_tile_problems_too_short_to_cut(M, N, K):
+    # the kernel depends on how the result can be stored: bf16 rows of whole 16 bytes, others, fp32
+    assert _plan(M, N, K, 0)[4] == 1
+    a, bt = _ab(M, N, K, seed=98)
+    ref = (a.double() @ bt.double().t()).float()
+    for out_dtype, limit in ((torch.float32, 1e-6 + K / 16 * 2.0 ** -23), (torch.bfloat16, 3e-3)):
+        c = fused.matmul(a, bt.t(), out_dtype=out_dtype)
+        assert ((c.float() - ref).norm() / ref.norm()).item() < limit
+
+
 def _two_launch_problem(index, fp32, same=lambda M, N, K: True):
     """The index-th of a fixed series of ragged problems that the launcher gives to two launches."""
     import random
