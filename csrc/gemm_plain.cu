@@ -114,7 +114,7 @@ struct TileChoice {
   bool swap, pair;
   int bn, splits;
 };
-static TileChoice best_tile(const DeviceState* d, int M, int N, int num_kb, int elt, int class_a, int class_b, double hbm_us) {
+static TileChoice best_tile(const DeviceState* d, int M, int N, int num_kb, int elt, int class_a, int class_b, double hbm_us, bool pairs_ok) {
   TileChoice best = {1e30, false, false, 0, 0};
   for (int swap = 0; swap < 2; ++swap) {
     const int rows = swap ? N : M, cols = swap ? M : N, cr = swap ? class_b : class_a, cc = swap ? class_a : class_b;
@@ -130,8 +130,8 @@ static TileChoice best_tile(const DeviceState* d, int M, int N, int num_kb, int 
     }
     // Pairs only where the second CTA has rows. Single CTAs always: one tile of both dimensions up to 128 is eight K ranges in
     // a cluster instead of one CTA that walks all of K (64 x 128 x 8192 6.6 us against 26.1, 1 x 128 x 7168 5.0 against 19.5).
-    for (int bn = 128; rows > 128 && bn <= 256; bn += 32)
-      if (pair_enabled() && (bn == 128 || bn - 32 < cols)) offer(true, bn, block_us(bn, 1, cr, cc, cols));
+    for (int bn = 128; pairs_ok && rows > 128 && bn <= 256; bn += 32)
+      if (bn == 128 || bn - 32 < cols) offer(true, bn, block_us(bn, 1, cr, cc, cols));
   }
   return best;
 }
@@ -167,7 +167,7 @@ static PlainPlan plain_plan(const DeviceState* d, int M, int N, int K, int elt, 
     // the whole choice is open: both orientations, every tile width, one wave with K splits or many
     double best = 1e30;
     if (whole_chip) {
-      const TileChoice c = best_tile(d, M, N, num_kb, elt, class_a, class_b, hbm_us);
+      const TileChoice c = best_tile(d, M, N, num_kb, elt, class_a, class_b, hbm_us, true);
       if (c.splits > 0) {
         best = c.us;
         pl.kind = PLAIN_TILE; pl.swap = c.swap; pl.pair = c.pair; pl.bn = c.bn; pl.splits = c.splits;
@@ -204,7 +204,7 @@ static PlainPlan plain_plan(const DeviceState* d, int M, int N, int K, int elt, 
             const int at = strips * (by_col ? bn : 256 * rb);
             const bool cut_n = (by_col != 0) != (swap != 0);
             const int m = cut_n ? M : M - at, n = cut_n ? N - at : N;
-            const TileChoice c = best_tile(d, m, n, num_kb, elt, class_a, class_b, ((double)m + n) * K * elt / kHbmBytesPerUs);
+            const TileChoice c = best_tile(d, m, n, num_kb, elt, class_a, class_b, ((double)m + n) * K * elt / kHbmBytesPerUs, true);
             const double both = std::max(main_us + c.us - (c.pair ? kTilePairUs : kTileSingleUs) + kRestUs, hbm_us + kFlowUs);
             if (c.splits == 0 || both * 1.02 >= best) continue;      // not for what the model cannot tell
             best = both;
@@ -227,8 +227,8 @@ static PlainPlan plain_plan(const DeviceState* d, int M, int N, int K, int elt, 
   const int tiles = ((rows + kBM - 1) / kBM) * ((cols + pl.bn - 1) / pl.bn);
   if (swap_ab < 0 && bn_override <= 0 && whole_chip && tiles <= d->num_sms) {
     // up to 64 rows of either operand: one wave with K splits
-    const TileChoice c = best_tile(d, M, N, num_kb, elt, class_a, class_b, hbm_us);
-    if (c.splits > 0 && (use_pair != 0 || !c.pair)) {
+    const TileChoice c = best_tile(d, M, N, num_kb, elt, class_a, class_b, hbm_us, pair_ok);
+    if (c.splits > 0) {
       pl.kind = PLAIN_TILE; pl.swap = c.swap; pl.pair = c.pair; pl.bn = c.bn; pl.splits = c.splits;
       return pl;
     }
@@ -274,13 +274,14 @@ using namespace kraken;
 
 // What a call with these arguments would run. plan[0..5]: kernel (0 single CTAs, 1 one wave, 2 persistent pairs), weights as
 // row operand, column tile, row blocks, K ranges, 1 when in two launches; plan[6..10] of the second launch: first row (column
-// when plan[7] is 1) of the output, by column, weights as row operand, column tile, K ranges.
-KR_API int kr_gemm_plan(int M, int N, int K, long long lda, long long ldb, int in_fp32, int* plan) {
+// when plan[7] is 1) of the output, by column, weights as row operand, column tile, K ranges; plan[11]: 1 when the one-wave
+// kernel runs in CTA pairs.
+KR_API int kr_gemm_plan(int M, int N, int K, long long lda, long long ldb, int in_fp32, int use_pair, int* plan) {
   DeviceState* d = device_state();
   if (!d) return KR_FAIL_CUDA;
   KR_REQUIRE(M >= 1 && N >= 1 && K >= 1, "GEMM needs positive sizes");
-  const PlainPlan pl = known_plan(d, M, N, K, in_fp32 ? 4 : 2, -1, 0, 1, 0, lda, ldb);
-  const int v[11] = {pl.kind, pl.swap, pl.bn, pl.rb, pl.splits, pl.cut > 0, pl.cut, pl.cut_n, pl.rest_swap, pl.rest_bn, pl.rest_splits};
+  const PlainPlan pl = known_plan(d, M, N, K, in_fp32 ? 4 : 2, -1, 0, use_pair, 0, lda, ldb);
+  const int v[12] = {pl.kind, pl.swap, pl.bn, pl.rb, pl.splits, pl.cut > 0, pl.cut, pl.cut_n, pl.rest_swap, pl.rest_bn, pl.rest_splits, pl.pair};
   memcpy(plan, v, sizeof(v));
   return KR_SUCCESS;
 }

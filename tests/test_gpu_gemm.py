@@ -499,9 +499,9 @@ def test_gemm_persistent_pairs_fp32_steps_of_16(bn, swap):
             assert ((c.float() - ref).norm() / ref.norm()).item() < (1e-3 if out_dtype == torch.float32 else 3e-3)
 
 
-def _plan(M, N, K, fp32):
-    plan = (ctypes.c_int * 11)()
-    klib.check(klib.lib().kr_gemm_plan(M, N, K, K, K, int(fp32), plan))
+def _plan(M, N, K, fp32, pair=1):
+    plan = (ctypes.c_int * 12)()
+    klib.check(klib.lib().kr_gemm_plan(M, N, K, K, K, int(fp32), pair, plan))
     return list(plan)
 
 
@@ -532,6 +532,22 @@ def test_one_tile_problems_too_short_to_cut(M, N, K):
     for out_dtype, limit in ((torch.float32, 1e-6 + K / 16 * 2.0 ** -23), (torch.bfloat16, 3e-3)):
         c = fused.matmul(a, bt.t(), out_dtype=out_dtype)
         assert ((c.float() - ref).norm() / ref.norm()).item() < limit
+
+
+# Without pairs the one-wave kernel runs on single CTAs, also where pairs would be the faster choice.
+@pytest.mark.parametrize("M,N,K,fp32,with_pairs", [(6120, 106, 8272, 0, 1), (100, 6152, 6200, 0, 1), (2, 9622, 8216, 0, 1), (4280, 122, 6472, 1, 1),
+                                                   (16, 4096, 4096, 0, 0)])
+def test_one_wave_without_pairs(M, N, K, fp32, with_pairs):
+    assert _plan(M, N, K, fp32)[11] == with_pairs
+    plan = _plan(M, N, K, fp32, pair=0)
+    assert plan[0] == 1 and plan[11] == 0, plan
+    dtype = torch.float32 if fp32 else torch.bfloat16
+    g = torch.Generator(device="cuda").manual_seed(99)
+    a = torch.randn(M, K, generator=g, device="cuda").to(dtype)
+    bt = (0.05 * torch.randn(N, K, generator=g, device="cuda")).to(dtype)
+    ref = a.double() @ bt.double().t()
+    c = fused.matmul(a, bt.t(), out_dtype=torch.float32, pair=0)
+    assert ((c - ref).norm() / ref.norm()).item() < (1e-3 if fp32 else 1e-6 + K / 16 * 2.0 ** -23)
 
 
 def _two_launch_problem(index, fp32, same=lambda M, N, K: True):
