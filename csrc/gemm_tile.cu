@@ -409,31 +409,37 @@ static int max_clusters(int device, const TileVariant& v, int elt, int bn, bool 
   return n;
 }
 
-// The split count of a one-wave problem, 0 when its tiles do not fit the chip at once, and its time (us). kb_us: one K
-// block with every SM busy (less when fewer are, the clock being what power leaves; not so for single CTAs of up to 64
-// columns). Near the operands' time out of HBM (hbm_us) the two slow each other down (norm of order 4). Then the partial
+// The split count with which a one-wave problem takes less than *us, and its time there; 0 when there is none or its tiles do
+// not fit the chip at once. kb_us: one K block with every SM busy (less when fewer are, the clock being what power leaves; not
+// so for single CTAs of up to 64 columns). Near the operands' time out of HBM (hbm_us) the two slow each other down (norm of order 4). Then the partial
 // sums' way between SMs (44 KB a us and SM); clusters of six CTAs and more start later.
 int tile_gemm_splits(const DeviceState* d, int tiles, int num_kb, int bn, bool pair, int elt, double kb_us, double hbm_us,
-                     double* us_out) {
+                     double* us, PlanStats* stats) {
   const TileVariant v = elt == 4 ? tile_variant<4>(bn, pair) : tile_variant<2>(bn, pair);
   if (v.fn == nullptr) return 0;
   const int ctas = pair ? 2 : 1, most = 8 / ctas;
+  const bool powered = pair || bn > 64;
+  const double start_us = pair ? kTilePairUs : kTileSingleUs;
+  // Most problems are asked for in vain, so whatever costs (roots and powers, 20 ns each) comes after a bound that does not.
+  const int room = std::min(most, d->num_sms / (tiles * ctas));
+  if (room < 1 || std::max((powered ? kBusyFloor : 1.0) * kb_us * num_kb / room, hbm_us) + start_us >= *us) return 0;
   int best = 0;
-  double best_us = 1e30;
-  for (int s = 1; s <= most && (s == 1 || num_kb >= 4 * s); ++s) {
-    if (tiles * s * ctas > d->num_sms || tiles > max_clusters(d->device, v, elt, bn, pair, (unsigned)(s * ctas))) continue;
-    const double busy = (double)tiles * s * ctas / d->num_sms, sent = (double)(s - 1) / s * kBM * bn * 4;
-    const double blocks = (num_kb + s - 1) / s * kb_us * (pair || bn > 64 ? busy_factor(busy) : 1.0), b2 = blocks * blocks, h2 = hbm_us * hbm_us;
+  for (int s = 1; s <= room && (s == 1 || num_kb >= 4 * s); ++s) {
+    if (tiles > max_clusters(d->device, v, elt, bn, pair, (unsigned)(s * ctas))) continue;
+    const double all_busy = (num_kb + s - 1) / s * kb_us, sent = (double)(s - 1) / s * kBM * bn * 4;
+    const double ends = sent / 44500 + start_us + (pair && s >= 3 ? 0.5 : 0.0);
+    if (std::max(powered ? kBusyFloor * all_busy : all_busy, hbm_us) + ends >= *us) continue;
+    ++stats->timed;
+    const double busy = (double)tiles * s * ctas / d->num_sms;
+    const double blocks = all_busy * (powered ? busy_factor(busy) : 1.0), b2 = blocks * blocks, h2 = hbm_us * hbm_us;
     // (unsplit pairs: the persistent kernel stores bf16 rows faster, 636 x 4080 x 3152 29 us against 33; fp32 does not, 500 x
     // 4000 x 4000 34.6 against 29.4)
-    const double us = std::sqrt(std::sqrt(b2 * b2 + h2 * h2)) * (pair && s == 1 && elt == 2 ? 1.05 : 1.0) + sent / 44500 + (pair ? kTilePairUs : kTileSingleUs) +
-                      (pair && s >= 3 ? 0.5 : 0.0);
-    if (us < best_us) {
-      best_us = us;
+    const double t = std::sqrt(std::sqrt(b2 * b2 + h2 * h2)) * (pair && s == 1 && elt == 2 ? 1.05 : 1.0) + ends;
+    if (t < *us) {
+      *us = t;
       best = s;
     }
   }
-  if (us_out) *us_out = best_us;
   return best;
 }
 

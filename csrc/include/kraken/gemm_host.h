@@ -31,12 +31,16 @@ int launch_gemm_ar(int bn, const GemmParams& p, unsigned nb, cudaStream_t stream
 // Routes a parameter block to the kernel family of its mode and operand type (gemm.cu).
 int launch_gemm(int bn, const GemmParams& p, unsigned nb, cudaStream_t stream);
 // Fewer SMs busy run faster (power), up to full clock.
-inline double busy_factor(double busy) { return std::max(0.79, std::pow(busy, 0.24)); }
-// One-wave GEMM (gemm_tile.cu): the most K splits with which `tiles` tiles of this kernel run at once,
-// 0 when it does not apply, and its estimated time (kb_us: one K block of a tile, hbm_us:
-// the operands' time out of HBM); and its launch.
+constexpr double kBusyFloor = 0.79;
+inline double busy_factor(double busy) { return std::max(kBusyFloor, std::pow(busy, 0.24)); }
+// What planning cost this thread: plans worked out, kernels whose time was worked out for them.
+struct PlanStats {
+  unsigned long long plans, timed;
+};
+// One-wave GEMM (gemm_tile.cu): the K splits with which `tiles` tiles of this kernel run at once in less than *us, and that
+// time in *us; 0 when there are none (kb_us: one K block of a tile, hbm_us: the operands' time out of HBM); and its launch.
 constexpr double kTilePairUs = 5.5, kTileSingleUs = 4.6;       // its start and end
-int tile_gemm_splits(const DeviceState* d, int tiles, int num_kb, int bn, bool pair, int elt, double kb_us, double hbm_us, double* us);
+int tile_gemm_splits(const DeviceState* d, int tiles, int num_kb, int bn, bool pair, int elt, double kb_us, double hbm_us, double* us, PlanStats* stats);
 int launch_tile_gemm(const GemmParams& g, int bn, bool pair, int splits, cudaStream_t stream);
 // Persistent pairs that draw their tiles in order (gemm_flow.cu); sched: two zero words, zero again afterwards.
 // last_cols: columns of the last column tile, in 16s; below bn with a tensor map of half as many rows of the column operand.

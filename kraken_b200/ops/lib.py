@@ -101,6 +101,7 @@ _PROTOS = {
     "kr_gemm": (c_int, [_P, c_longlong, _P, c_longlong, _P, c_longlong, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                         c_int, c_int, _P, _P, _P]),
     "kr_gemm_plan": (c_int, [c_int, c_int, c_int, c_longlong, c_longlong, c_int, c_int, POINTER(c_int)]),
+    "kr_gemm_plan_stats": (c_int, [POINTER(c_ulonglong), POINTER(c_ulonglong)]),
     "kr_gemm_scratch": (c_int, [c_int, c_int, c_int, c_longlong, c_longlong, c_int, c_int, c_int, c_int, c_int, POINTER(c_ulonglong)]),
     "kr_ag_gemm_bf16": (c_int, [_P, _P, _P, c_int, c_int, _P, _P, c_longlong, _P, c_longlong, c_int, c_int, c_int,
                                 c_int, _P, _P, c_int, c_uint32, c_int, c_ulonglong, c_uint32, c_ulonglong, c_int, _P, _P, c_int, _P]),
