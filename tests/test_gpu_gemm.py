@@ -573,6 +573,16 @@ def test_a_plan_is_worked_out_in_microseconds():
     assert sum(timed) / len(timed) < 70 and max(timed) < 200, (sum(timed) / len(timed), max(timed))
 
 
+def test_plans_of_a_programs_shapes_are_all_remembered():
+    # a block's four projections at 8 row counts, and at 32; a second pass over them works nothing out
+    for row_counts in ([1, 7, 16, 64, 200, 777, 2048, 8192], list(range(100, 1700, 50))):
+        shapes = [(m, n, k) for m in row_counts for n, k in ((10240, 8192), (8192, 8192), (28672, 8192), (8192, 28672))]
+        want = [_plan(*s, 0) for s in shapes]
+        before = _plan_stats()[0]
+        assert [_plan(*s, 0) for s in shapes] == want
+        assert _plan_stats()[0] == before, _plan_stats()[0] - before
+
+
 def _two_launch_problem(index, fp32, same=lambda M, N, K: True):
     """The index-th of a fixed series of ragged problems that the launcher gives to two launches."""
     import random
