@@ -318,14 +318,15 @@ using namespace kraken;
 
 // What a call with these arguments would run. plan[0..5]: kernel (0 single CTAs, 1 one wave, 2 persistent pairs), weights as
 // row operand, column tile, row blocks, K ranges, 1 when in two launches; plan[6..10] of the second launch: first row (column
-// when plan[7] is 1) of the output, by column, weights as row operand, column tile, K ranges; plan[11]: 1 when the one-wave
-// kernel runs in CTA pairs.
+// when plan[7] is 1) of the output, by column, weights as row operand, column tile, K ranges; plan[11], plan[12]: 1 when the
+// one-wave kernel, as all of it or as the second launch, runs in CTA pairs.
 KR_API int kr_gemm_plan(int M, int N, int K, long long lda, long long ldb, int in_fp32, int use_pair, int* plan) {
   DeviceState* d = device_state();
   if (!d) return KR_FAIL_CUDA;
   KR_REQUIRE(M >= 1 && N >= 1 && K >= 1, "GEMM needs positive sizes");
   const PlainPlan pl = known_plan(d, M, N, K, in_fp32 ? 4 : 2, -1, 0, use_pair, 0, lda, ldb);
-  const int v[12] = {pl.kind, pl.swap, pl.bn, pl.rb, pl.splits, pl.cut > 0, pl.cut, pl.cut_n, pl.rest_swap, pl.rest_bn, pl.rest_splits, pl.pair};
+  const int v[13] = {pl.kind, pl.swap, pl.bn, pl.rb, pl.splits, pl.cut > 0, pl.cut, pl.cut_n, pl.rest_swap, pl.rest_bn, pl.rest_splits,
+                     pl.kind == PLAIN_TILE && pl.pair, pl.rest_pair};
   memcpy(plan, v, sizeof(v));
   return KR_SUCCESS;
 }

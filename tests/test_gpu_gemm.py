@@ -499,9 +499,9 @@ def test_gemm_persistent_pairs_fp32_steps_of_16(bn, swap):
             assert ((c.float() - ref).norm() / ref.norm()).item() < (1e-3 if out_dtype == torch.float32 else 3e-3)
 
 
-def _plan(M, N, K, fp32, pair=1):
-    plan = (ctypes.c_int * 12)()
-    klib.check(klib.lib().kr_gemm_plan(M, N, K, K, K, int(fp32), pair, plan))
+def _plan(M, N, K, fp32, pair=1, lda=None):
+    plan = (ctypes.c_int * 13)()
+    klib.check(klib.lib().kr_gemm_plan(M, N, K, lda or K, K, int(fp32), pair, plan))
     return list(plan)
 
 
@@ -583,14 +583,14 @@ def test_plans_of_a_programs_shapes_are_all_remembered():
         assert _plan_stats()[0] == before, _plan_stats()[0] - before
 
 
-def _two_launch_problem(index, fp32, same=lambda M, N, K: True):
+def _two_launch_problem(index, fp32, same=lambda M, N, K: True, more_n=0, more_lda=0):
     """The index-th of a fixed series of ragged problems that the launcher gives to two launches."""
     import random
 
     r = random.Random(3)
     for _ in range(20000):
-        M, N, K = r.randint(300, 3000), r.randint(60, 700) * 8, r.randint(64, 400) * 8
-        if _plan(M, N, K, fp32)[5] == 1 and same(M, N, K):
+        M, N, K = r.randint(300, 3000), r.randint(60, 700) * 8 + more_n, r.randint(64, 400) * 8
+        if _plan(M, N, K, fp32, lda=K + more_lda)[5] == 1 and same(M, N, K):
             if index == 0:
                 return M, N, K
             index -= 1
@@ -621,6 +621,67 @@ def test_gemm_in_two_launches(index, fp32):
         x.copy_(a)
         gathered, c = fused.all_gather_matmul(x, bt.t())
         assert torch.equal(gathered, a) and ((c.float() - ref).norm() / ref.norm()).item() < 3e-3
+
+
+# The forms of the first launch and what it shares with the second one: stores of whole rows, transposed, element by element
+# (an output that TMA cannot describe), and a left operand with padded rows; cut by rows and by columns.
+@pytest.mark.parametrize("by_col", [0, 1])
+@pytest.mark.parametrize("swap,more_n,more_lda", [(0, 0, 0), (1, 0, 0), (0, 1, 0), (1, 1, 0), (0, 0, 72)])
+@pytest.mark.parametrize("act", [None, "gelu_tanh"])
+def test_forms_of_the_first_of_two_launches(by_col, swap, more_n, more_lda, act):
+    from kraken_b200.fused.gemm_ops import _gemm
+
+    def same(M, N, K):
+        plan = _plan(M, N, K, 0, lda=K + more_lda)
+        return plan[1] == swap and plan[7] == by_col
+
+    M, N, K = _two_launch_problem(0, 0, same, more_n, more_lda)
+    g = torch.Generator(device="cuda").manual_seed(93)
+    a = torch.full((M, K + more_lda), float("nan"), device="cuda", dtype=torch.bfloat16)[:, :K]
+    a.copy_(torch.randn(M, K, generator=g, device="cuda"))
+    bt = (torch.randn(N, K, generator=g, device="cuda") / K ** 0.5).to(torch.bfloat16)
+    ref = a.double() @ bt.double().t()
+    if act is not None:
+        ref = ref * torch.sigmoid(2 * (2 / math.pi) ** 0.5 * (ref + 0.044715 * ref ** 3))
+    for out_fp32 in (False, True):
+        c = _gemm(a, bt.t(), out_fp32, False, act=act)
+        # One rounding of a bf16 result, 2**-8 of the value. The sums (rms 1, below 6) are cut once per MMA of 16 columns, at most
+        # 200 * 2**-23 * 6; the device's exp and divide: 1e-4 of the value.
+        assert (((c.double() - ref).abs() - (0 if out_fp32 else 2.0 ** -8) * ref.abs()).max()).item() < 1e-3
+        assert torch.equal(c, _gemm(a, bt.t(), out_fp32, False, act=act))
+
+
+def test_plans_can_be_launched():
+    # every plan fits the chip and the kernels that exist, and the two launches of a problem share it out without a gap
+    import random
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    r = random.Random(12)
+
+    def one_wave(M, N, kb, swap, pair, bn, splits):
+        rows, cols = (N, M) if swap else (M, N)
+        tiles = -(-rows // (256 if pair else 128)) * -(-cols // bn)
+        assert bn in ((128, 160, 192, 224, 256) if pair else (16, 32, 64, 128))
+        assert 1 <= splits <= kb and splits * (1 + pair) <= 8 and tiles * splits * (1 + pair) <= sms
+
+    kinds = set()
+    for _ in range(4000):
+        M, N = (int(2 ** r.uniform(0, 13)) for _ in range(2))
+        fp32, pair = r.randint(0, 1), int(r.random() < 0.8)
+        K = int(2 ** r.uniform(0, 12)) * (4 if fp32 else 8)
+        kb = -(-K // (32 if fp32 else 64))
+        kind, swap, bn, rb, splits, two, cut, cut_n, rest_swap, rest_bn, rest_splits, pairs, rest_pairs = _plan(M, N, K, fp32, pair)
+        kinds.add((kind, two))
+        assert pair or (kind != 2 and not pairs)
+        if kind == 1:
+            one_wave(M, N, kb, swap, pairs, bn, splits)
+        elif kind == 2:
+            assert bn in (64, 96, 128, 144, 160, 176, 192, 208, 224, 240, 256) and rb in (1, 2)
+            if two:
+                assert 0 < cut < (N if cut_n else M) and cut % (bn if cut_n != swap else 256 * rb) == 0
+                one_wave(*((M, N - cut) if cut_n else (M - cut, N)), kb, rest_swap, rest_pairs, rest_bn, rest_splits)
+        assert two in (0, int(kind == 2))
+    assert kinds == {(0, 0), (1, 0), (2, 0), (2, 1)}
 
 
 def test_gemms_in_two_launches_chained_and_captured():
