@@ -57,8 +57,9 @@ static int row_class(long long ld, int elt) { return ld * elt % 128 == 0 ? 0 : l
 // picks is 1.5 % slower on average than the best plan measured for a problem.
 //
 // A K block (64 bf16 or 32 fp32 columns of K) takes the longer of its MMAs and of bringing its operand rows into shared
-// memory, plus a sixth of the other. The second is no matter of L2 or HBM but of what an SM takes in: per 128-byte row 1.1
-// clocks where rows start on lines, 1.6 on sectors, 2.5 in the middle of sectors (a loop of loads alone: 235, 139 and 94 GB/s).
+// memory, plus a sixth of the other. The second is no matter of L2 or HBM but of what an SM takes in: per 128-byte row 1.19
+// clocks where rows start on lines, 1.62 on sectors, 2.52 in the middle of sectors (fitted; a loop of loads alone at full clock:
+// 235, 139 and 94 GB/s, which are 1.07, 1.81 and 2.68).
 constexpr double kClocksPerUs = 1465;
 static double stage_us(double mma_clocks, double fill_clocks) {
   return (std::max({mma_clocks, fill_clocks, 255.0}) + 0.156 * std::min(mma_clocks, fill_clocks)) / kClocksPerUs;

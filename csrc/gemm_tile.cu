@@ -7,16 +7,17 @@
 //   (split by split), bf16 or fp32 result.
 //
 // Why clusters and not partial sums in global memory: a 256 x 256 tile split in two costs 15-18 us there
-// (slots out to L2, an atomic, slots back in: measured with %globaltimer stamps) and about 4 us here.
+// (slots out to L2, an atomic, slots back in: measured with %globaltimer stamps) and about 1.5 us here.
 //
 // The sums are SENT: every CTA owns an equal share of the tile's rows, and the others store their partial sums of it
 // straight from registers into its shared memory (st.async, counted on an mbarrier of the owner; the operand stages are
 // free by then). The owner adds them in split order and stores its rows. One cluster barrier, whose latency the first
-// read of the accumulator hides, says that the stages are free; nothing follows the stores. With
-// the other order (own shared memory, cluster barrier, owners fetch, cluster barrier before anybody may leave) and the
-// places of a thread's rows worked out here instead of before, us a call in a stream of them: 8 x 4096 x 4096 9.8, now 8.8;
-// 35 x 4064 x 5416 14.4, 12.5; 102 x 1240 x 2816 9.8, 7.3; 100 x 4000 x 9000 20.8, 19.5. What bounds this part now is the way between SMs: 64 KB leave an SM in 2700 clocks
-// (24 bytes each; bulk copies 3400, plain remote stores and a barrier 4200, fetches 3900), whatever the cluster size.
+// read of the accumulator hides, says that the stages are free; nothing follows the stores. The other order was: own
+// shared memory, cluster barrier, owners fetch, cluster barrier before anybody may leave, and the places of a thread's rows
+// worked out here. With the plans of either, us a call in a graph of them, then and now: 8 x 4096 x 4096 9.3, 8.7;
+// 35 x 4064 x 5416 13.7, 11.5; 102 x 1240 x 2816 8.5, 5.9; 100 x 4000 x 9000 21.4, 20.0. What bounds this part now is the
+// way between SMs: 64 KB leave an SM in 2700 clocks (24 bytes each; bulk copies 3400, plain remote stores and a barrier
+// 4200, fetches 3900), whatever the cluster size.
 #include <algorithm>
 #include <atomic>
 #include <cmath>
