@@ -395,7 +395,7 @@ static int run_plain(const DeviceState* d, const PlainPlan& pl, const PlainCall&
   p.sync = sync_ctx(d);
   if (copy_dst != nullptr) {
     const int copy_rows = c.copy_rows > 0 ? c.copy_rows : M;
-    KR_REQUIRE(lda == K && ((uintptr_t)copy_dst & 15) == 0 && ((unsigned long long)copy_rows * K * elt) % 16 == 0, "the copied operand must be contiguous and 16-byte aligned");
+    KR_REQUIRE((lda == K || copy_rows == 1) && ((uintptr_t)copy_dst & 15) == 0 && ((unsigned long long)copy_rows * K * elt) % 16 == 0, "the copied operand must be contiguous and 16-byte aligned");
     p.cp_src = a;
     p.cp_dst = copy_dst;
     p.cp_bytes = (unsigned long long)copy_rows * K * elt;

@@ -762,6 +762,19 @@ def test_one_rank_all_gather_matmul_fills_a_out_like_a_copy():
             fused.all_gather_matmul(x, bt.t(), a_out=out)
 
 
+def test_one_rank_all_gather_matmul_of_one_row_of_a_wider_buffer():
+    # one row is contiguous whatever its stride
+    from kraken_b200.parallel import symm_mem
+
+    wide = symm_mem.empty(1, 520, dtype=torch.bfloat16, device="cuda")
+    a, bt = _ab(1, 136, 264, seed=43)
+    x = wide[:, :264]
+    x.copy_(a)
+    gathered, c = fused.all_gather_matmul(x, bt.t())
+    assert torch.equal(gathered, a)
+    _close(c, a.float() @ bt.float().t(), 264)
+
+
 _TMA_STORE_PROBE = """
 import ctypes, torch
 from kraken_b200 import fused
