@@ -534,6 +534,33 @@ def test_one_tile_problems_too_short_to_cut(M, N, K):
         assert ((c.float() - ref).norm() / ref.norm()).item() < limit
 
 
+# The same in every form that these calls take, against the persistent kernel on one CTA (bn=64, weights as columns): padded rows on
+# the left, weights as columns of a wider matrix, activation, a copy of the operand, results that TMA cannot store.
+@pytest.mark.parametrize("M,N,K", [(128, 128, 256), (128, 72, 440), (65, 127, 1032), (1, 128, 2056), (128, 1, 2048), (17, 24, 8)])
+@pytest.mark.parametrize("fp32", [0, 1])
+@pytest.mark.parametrize("act", [None, "gelu_tanh"])
+def test_forms_of_one_tile_problems(M, N, K, fp32, act):
+    from kraken_b200.fused.gemm_ops import _gemm
+
+    dtype = torch.float32 if fp32 else torch.bfloat16
+    g = torch.Generator(device="cuda").manual_seed(100)
+    a = torch.full((M, K + 24), float("nan"), device="cuda", dtype=dtype)[:, :K]
+    a.copy_(torch.randn(M, K, generator=g, device="cuda"))
+    bt = torch.full((N, K + 8), float("nan"), device="cuda", dtype=dtype)[:, :K]
+    bt.copy_(torch.randn(N, K, generator=g, device="cuda") / K ** 0.5)
+    # sums below 6, cut once per MMA of 32 bytes of K; the device's exp and divide: 1e-4; bf16 results: 2**-8 of the value, on
+    # either side of what the sums differ by
+    slack = 2 * 6 * (K * a.element_size() / 32) * 2.0 ** -23 + (6e-4 if act else 0)
+    for out_fp32 in (True, False):
+        want = _gemm(a, bt.t(), out_fp32, bool(fp32), 0, 64, act=act).double()
+        c = _gemm(a, bt.t(), out_fp32, bool(fp32), act=act).double()
+        assert (((c - want).abs() - (0 if out_fp32 else 2.0 ** -7) * want.abs()).max()).item() < slack
+        whole = a.contiguous()
+        copied = torch.zeros_like(whole)
+        c = _gemm(whole, bt.t(), out_fp32, bool(fp32), act=act, copy_dst=copied).double()
+        assert torch.equal(copied, whole) and (((c - want).abs() - (0 if out_fp32 else 2.0 ** -7) * want.abs()).max()).item() < slack
+
+
 # Without pairs the one-wave kernel runs on single CTAs, also where pairs would be the faster choice.
 @pytest.mark.parametrize("M,N,K,fp32,with_pairs", [(6120, 106, 8272, 0, 1), (100, 6152, 6200, 0, 1), (2, 9622, 8216, 0, 1), (4280, 122, 6472, 1, 1),
                                                    (16, 4096, 4096, 0, 0)])
